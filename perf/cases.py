@@ -89,8 +89,9 @@ def _expert(gen, D, F):
     return 1.0 + 0.01 * normal(D), normal(F, D).div_(math.sqrt(D)), normal(F, D).div_(math.sqrt(D)), normal(D, F).div_(math.sqrt(F))
 
 
-def prepare(case, seed):
-    E, D, F, T = case["experts"], case["d_model"], case["d_ff"], case["tokens"]
+def _inputs(case, seed):
+    """Routing parameters, tokens and the generator that the experts' weights come from, all made from the seed."""
+    E, D, T = case["experts"], case["d_model"], case["tokens"]
     rng = np.random.default_rng(seed)
     gen = torch.Generator(device="cuda")
     gen.manual_seed(seed)
@@ -104,6 +105,12 @@ def prepare(case, seed):
         scale = math.sqrt(6.0) / math.pi * 0.02 * math.sqrt(max(1, D - 1))
         x[:, 0] = 1.0
         centroids[:, 0] = scale * np.log(share / share.sum())
+    return centroids, gating_ln, x, gen
+
+
+def prepare(case, seed):
+    E, D, F = case["experts"], case["d_model"], case["d_ff"]
+    centroids, gating_ln, x, gen = _inputs(case, seed)
     layer = MoELayer.create(E, D, F, 2, centroids, None, "T5_FF", case["variant"], gating_ln)
     host = case["kind"] in ("streamed", "cached")
     for e in range(E):
@@ -141,3 +148,32 @@ def tolerance(case):
     # FP32 in and out.  The layer output x + FFN(x) of the split-operand tensor-core products is 1e-6 to 3e-6
     # (2-norm) from an evaluation in 64 bits; a stack adds its layers' errors.
     return {"rel": 1e-5 * case["layers"], "max": 2e-4 * case["layers"]}
+
+
+def exact(case, seed):
+    """The layer's definition in 64 bits."""
+    centroids, gating_ln, x, gen = _inputs(case, seed)
+    D, F = case["d_model"], case["d_ff"]
+    experts = [_expert(gen, D, F) for _ in range(case["experts"])]
+    centroids = torch.from_numpy(centroids).cuda().double()
+
+    def layer_norm(v, gamma):
+        centred = v - v.mean(1, keepdim=True)
+        return gamma.double() * centred / torch.sqrt(centred.square().mean(1, keepdim=True) + 1e-6)
+
+    x = x.double()
+    for _ in range(case["layers"]):
+        scored = x if gating_ln is None else layer_norm(x, torch.from_numpy(gating_ln).cuda())
+        score, gate = (scored @ centroids.T).max(1)
+        out = x.clone()
+        for e, (ln, wi0, wi1, wo) in enumerate(experts):
+            rows = (gate == e).nonzero()[:, 0]
+            if rows.numel():
+                h = layer_norm(x[rows], ln)
+                g = torch.nn.functional.gelu(h @ wi0.double().T, approximate="tanh") * (h @ wi1.double().T)
+                out[rows] += g @ wo.double().T
+        if case["variant"] == "base_layer":
+            alpha = torch.sigmoid(score)[:, None]
+            out = alpha * out + (1.0 - alpha) * x
+        x = out
+    return x.cpu() if case["kind"] == "host" else x
