@@ -1,6 +1,7 @@
 // Shared host/device helpers of the B200 MoE-layer kernels.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -53,6 +54,11 @@ inline void note_launch(int n = 1) { g_kernel_launches += n; }
 // with explicit round-to-nearest adds / fused multiply-adds, and the 32 lane
 // partials are combined by a butterfly (xor 16, 8, 4, 2, 1).
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+}
 __device__ __forceinline__ float warp_xor_sum(float v) {
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, off));
@@ -128,7 +134,7 @@ __device__ __forceinline__ float ln_apply(float x, float mean, float rstd, float
     return __fmul_rn(gamma, __fmul_rn(__fsub_rn(x, mean), rstd));
 }
 
-// Splits an FP32 value into a TF32-representable head and an FP32 remainder:
+// Splits an FP32 value into a TF32-representable head and an FP32 remainder (CUDA-core path):
 // hi = x rounded to 10 mantissa bits (round to nearest, ties away), lo = x - hi (exact).
 __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
     uint32_t h;
@@ -137,22 +143,60 @@ __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
     lo = __fsub_rn(x, hi);
 }
 
-// Two FP32 values rounded to BF16 (round to nearest even) in one 32-bit word: `even` in the lower half.
-__device__ __forceinline__ uint32_t pack_bf16x2(float even, float odd) {
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(odd), "f"(even));
-    return r;
+// Operand of the tensor-core GEMM: an FP32 value, scaled by a power of two of its row, as a pair of FP16 values,
+// hi = x rounded to 11 significant bits, lo = x - hi rounded to 11 (in the lower / upper half of the word).  |lo| is at
+// most half a unit of hi, so together they hold x to within 2^-23 relative (the last bit of an FP32 value) down to
+// |x| = 2^-3, and to within 2^-25 absolute below that.
+__device__ __forceinline__ uint32_t split_f16(float x) {
+    const __half hi = __float2half_rn(x);
+    const __half lo = __float2half_rn(__fsub_rn(x, __half2float(hi)));
+    return (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
 }
-
-// Token operand of the tensor-core GEMM, per value x: hi = x rounded to TF32 (FP32 plane `hi`), and the BF16
-// roundings of hi and of lo = x - hi in a packed plane.  The packed plane has one 128-byte group per 32 values
-// of a row: 32 x bf16(hi) followed by 32 x bf16(lo); rows are padded with zeros to a multiple of 32 values.
-__host__ __device__ __forceinline__ size_t pack_pitch(int K) { return (size_t)((K + 31) / 32) * 64; }   // in BF16 elements
-// Stores the packed entries of four consecutive values k0..k0+3 (k0 a multiple of 4) of one row.
-__device__ __forceinline__ void store_pack4(uint16_t* __restrict__ pack_row, int k0, const float hi[4], const float lo[4]) {
+// Rows of pairs are stored in 128-byte groups of 32 values: 32 x hi followed by 32 x lo; rows are padded with zeros to
+// a multiple of 32 values.
+__host__ __device__ __forceinline__ size_t pack_pitch(int K) { return (size_t)((K + 31) / 32) * 64; }   // in 16-bit elements
+// Stores four consecutive values k0..k0+3 (k0 a multiple of 4) of one row.
+__device__ __forceinline__ void store_pack4(uint16_t* __restrict__ pack_row, int k0, const float v[4]) {
     uint16_t* g = pack_row + (size_t)(k0 >> 5) * 64 + (k0 & 31);
-    *reinterpret_cast<uint2*>(g) = make_uint2(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]));
-    *reinterpret_cast<uint2*>(g + 32) = make_uint2(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]));
+    const uint32_t a = split_f16(v[0]), b = split_f16(v[1]), c = split_f16(v[2]), d = split_f16(v[3]);
+    *reinterpret_cast<uint2*>(g) = make_uint2(__byte_perm(a, b, 0x5410), __byte_perm(c, d, 0x5410));
+    *reinterpret_cast<uint2*>(g + 32) = make_uint2(__byte_perm(a, b, 0x7632), __byte_perm(c, d, 0x7632));
+}
+// 2^e as a float, e in [-126, 127].
+__device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
+// Exponent s that brings the largest magnitude of a row into [2^14, 2^15) (FP16 ends at 65504); 0 for a row of zeros
+// or with an infinity.  At most 126, so that 2^s and 2^-s are both normal floats.
+__device__ __forceinline__ int row_exponent(float max_abs) {
+    if (!(max_abs > 0.f) || !(max_abs <= FLT_MAX)) return 0;
+    return min(126, 14 - ((__float_as_int(max_abs) >> 23) - 127));
+}
+// Exponent of the gate activations g of one token.  |g_f| = |gelu(a_f) b_f| <= |a_f| |b_f| <= |h|^2 |wi_0[f]| |wi_1[f]|
+// (2-norms), so with h2 = log2 |h|^2 and w = max_f log2(|wi_0[f]| |wi_1[f]|) no g 2^s exceeds 2^15.  The bound is about
+// 2^13 above a typical g at d_model 4096, which leaves typical values near 2^2 and their lo parts well inside the
+// normal range of FP16.  Both GEMMs compute it from the same two numbers.
+__device__ __forceinline__ int g_exponent(float h2, float w) {
+    float b = h2 + w + 0.01f;
+    if (!(b > -111.f)) b = -111.f;
+    if (!(b < 141.f)) b = 141.f;
+    return 15 - (int)ceilf(b);
+}
+// Order-preserving map of floats onto unsigned integers above 0, for atomicMax.
+__device__ __forceinline__ uint32_t encode_bound(float x) {
+    const uint32_t u = __float_as_uint(x);
+    return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float decode_bound(float stored) {
+    const uint32_t u = __float_as_uint(stored);
+    return __uint_as_float((u & 0x80000000u) ? u & 0x7fffffffu : ~u);
+}
+// sum 2^-s of the weight row 2^-s of the token row; the smaller factor first, so that nothing overflows on the way.
+__device__ __forceinline__ float unscale(float sum, float w_inv, float x_inv) {
+    return __fmul_rn(__fmul_rn(sum, fminf(w_inv, x_inv)), fmaxf(w_inv, x_inv));
+}
+// Row statistics the tensor-core path keeps of a token row: 2^-s and log2 of the squared norm, from the exponent and
+// the sum of squares of the row times 2^s.
+__device__ __forceinline__ float2 token_row_info(int s, float scaled_square_sum) {
+    return make_float2(exp2_int(-s), scaled_square_sum > 0.f ? log2f(scaled_square_sum) - 2.f * (float)s : -300.f);
 }
 
 // base_layer output mix (plugin/cuda/moe.cu:115-127, sigmoid plugin/cuda/common.cuh:24-27):

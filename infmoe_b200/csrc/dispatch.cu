@@ -55,7 +55,7 @@ constexpr int DISPATCH_TABLES = 5 + DISPATCH_WARPS;
 __global__ void __launch_bounds__(DISPATCH_THREADS)
 dispatch_kernel(const int* __restrict__ gate, long long T, int E, const int* __restrict__ region_count,
                 int region_size, int* __restrict__ pos, int* __restrict__ count, int* __restrict__ offset,
-                int* __restrict__ status) {
+                int* __restrict__ status, int* __restrict__ zero, int zero_count) {
     cg::cluster_group cluster = cg::this_cluster();
     const int C = (int)cluster.num_blocks(), r = (int)cluster.block_rank();
     extern __shared__ int smem[];
@@ -84,6 +84,8 @@ dispatch_kernel(const int* __restrict__ gate, long long T, int E, const int* __r
     };
 
     for (int e = tid; e < B; e += DISPATCH_THREADS) s_count[e] = 0;
+    if (r == 0)
+        for (int i = tid; i < zero_count; i += DISPATCH_THREADS) zero[i] = 0;
     __syncthreads();
     bool bad = false;
     const long long super = (long long)C * DISPATCH_THREADS;
@@ -172,7 +174,7 @@ dispatch_kernel(const int* __restrict__ gate, long long T, int E, const int* __r
 size_t dispatch_smem_bytes(int E) { return sizeof(int) * (size_t)DISPATCH_TABLES * (size_t)(E + 1); }
 
 int launch_dispatch(const int* gate, long long T, int E, int* pos, int* count, int* offset, int* status,
-                    cudaStream_t stream, const int* region_count, int region_size) {
+                    cudaStream_t stream, const int* region_count, int region_size, int* zero, int zero_count) {
     if (T < 0 || T > 0x7fffffffLL || E <= 0 || (T > 0 && (!gate || !pos)) || !count || !offset ||
         (region_count && region_size <= 0)) {
         set_error("expert_count: bad argument (T=%lld E=%d)", T, E);
@@ -207,7 +209,7 @@ int launch_dispatch(const int* gate, long long T, int E, int* pos, int* count, i
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     INFMOE_CUDA_TRY(cudaLaunchKernelEx(&cfg, dispatch_kernel, gate, T, E, region_count, region_size, pos, count, offset,
-                                       status));
+                                       status, zero, zero ? zero_count : 0));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

@@ -15,15 +15,22 @@ int launch_select_top1(long long T, int E, const float* aff, int* gate, float* w
                        cudaStream_t stream);
 // region_count != NULL: the T slots are regions of region_size slots, of which only the first region_count[s]
 // hold rows (receive buffer of the expert-parallel path); the other slots are skipped silently.
+// zero[0 .. zero_count) (may be NULL) is cleared on the way: the counters of the GEMMs' cut tiles.
 int launch_dispatch(const int* gate, long long T, int E, int* pos, int* count, int* offset, int* status,
-                    cudaStream_t stream, const int* region_count = nullptr, int region_size = 0);
+                    cudaStream_t stream, const int* region_count = nullptr, int region_size = 0, int* zero = nullptr,
+                    int zero_count = 0);
 int launch_scatter(long long T, int D, const float* X, const float* coeff, const int* pos, float* routed,
                    float* rcoeff, cudaStream_t stream);
 // valid_rows (device, may be NULL): rows at or past *valid_rows are skipped (tokens without an expert sit at
-// the tail of pos[]; the dispatch kernel stores their start in offset[E]).  routed may be NULL.
+// the tail of pos[]; the dispatch kernel stores their start in offset[E]).
+// CUDA-core GEMM: routed rows and FP32 head / tail planes of the LayerNorm output.
 int launch_scatter_ln_split(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
                             const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h_hi,
-                            float* h_lo, bool pack, cudaStream_t stream);
+                            float* h_lo, cudaStream_t stream);
+// Tensor-core GEMM: packed FP16-pair plane `h` (pack_bytes) and two floats per row in row_info (token_row_info).
+int launch_scatter_ln_pack(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
+                           const float* gamma_all, const int* valid_rows, float* rscore, void* h, float* row_info,
+                           cudaStream_t stream);
 int launch_gather(long long T, int D, const float* in, const int* pos, float* out, cudaStream_t stream,
                   const int* valid_rows = nullptr);
 int launch_mix_gather(long long T, int D, const int* pos, const float* routed, const float* post,
@@ -32,19 +39,26 @@ int launch_layernorm(float* out, const float* in, long long n, int D, const floa
 int launch_gelu_dot(const float* a, float* b, size_t len, cudaStream_t stream);
 int launch_split(const float* src, float* hi, float* lo, size_t len, cudaStream_t stream);
 int launch_fill_int(int* dst, int value, cudaStream_t stream);   // *dst = value, stream ordered
-// Tile-contiguous weight layout (see rows.cu); src1 != NULL interleaves the rows of two matrices.
+// Tile-contiguous weight layouts (see rows.cu); src1 != NULL interleaves the rows of two matrices.
+//   launch_retile       raw FP32 tiles, for the CUDA-core GEMM (tiled_elems floats)
+//   launch_split_tiles  FP16-pair tiles, the rows' 2^-s and, of two matrices, the gate bound, for the tensor-core GEMM
+//                       (split_plane_elems floats: tiles, one float per padded row, 32 floats for the bound)
 int launch_retile(const float* src0, const float* src1, int M, int K, float* dst, cudaStream_t stream);
+int launch_split_tiles(const float* src0, const float* src1, int M, int K, float* dst, cudaStream_t stream);
 inline size_t tiled_elems(int M, int K) { return (size_t)((M + 127) / 128) * 128 * (size_t)((K + 31) / 32) * 32; }
-int launch_ln_split(long long n, int D, const float* in, const float* gamma, float* h_hi, float* h_lo, bool pack,
+inline size_t split_bound_at(int M, int K) { return tiled_elems(M, K) + (size_t)((M + 127) / 128) * 128; }
+inline size_t split_plane_elems(int M, int K) { return split_bound_at(M, K) + 32; }
+// h = LN(x; gamma) for rows already in place, as launch_scatter_ln_split / _pack write it.
+int launch_ln_split(long long n, int D, const float* in, const float* gamma, float* h_hi, float* h_lo,
                     cudaStream_t stream);
-// Bytes of the second activation plane of a [rows][K] operand: FP32 tail plane (CUDA-core GEMM) or packed BF16
-// plane with rows padded to whole groups of 32 values (tensor-core GEMM); the larger of the two.
-inline size_t second_plane_bytes(long long rows, int K) { return (size_t)rows * (size_t)((K + 31) / 32) * 128; }
+int launch_ln_pack(long long n, int D, const float* in, const float* gamma, void* h, float* row_info,
+                   cudaStream_t stream);
+// Bytes of a packed FP16-pair plane [rows][K] (rows padded to whole groups of 32 values).
+inline size_t pack_bytes(long long rows, int K) { return (size_t)rows * (size_t)((K + 31) / 32) * 128; }
 
-// Expert weights live in two raw FP32 planes in tile-contiguous layout (128 x 32 tiles, see launch_retile):
-// w01 [slots] x tiled(2F x D) (row 2f = wi_0[f], row 2f+1 = wi_1[f]) and wo [slots] x tiled(D x F).  
-// Activations travel as two planes: hi = value rounded to TF32 (FP32 [rows][K]) and either lo = value - hi
-// (FP32 [rows][K], CUDA-core GEMM) or the packed BF16 plane of common.cuh (tensor-core GEMM).
+// CUDA-core GEMM.  Expert weights live in two raw FP32 planes in tile-contiguous layout (128 x 32 tiles):
+// w01 [slots] x tiled(2F x D) (row 2f = wi_0[f], row 2f+1 = wi_1[f]) and wo [slots] x tiled(D x F).
+// Activations travel as two FP32 planes: hi = value rounded to TF32, lo = value - hi.
 int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int* offset, const int* slot_of_expert,
                     const float* h_hi, const float* h_lo, const float* w01, const float* wo, const float* routed,
                     float* g_hi, float* g_lo, float* post, cudaStream_t stream);
@@ -53,14 +67,32 @@ int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int
 int launch_wait_probe(unsigned long long limit_ns, int* status, unsigned long long* waited_ns, cudaStream_t stream);
 
 bool ffn_umma_supported(int D, int F, int E);
-// out_pos != NULL: `post` is the layer output in token order, row j of the experts' result goes to row out_pos[j]
-// (and mix_score != NULL applies the base_layer output mix on the way): the combine step fused into the epilogue.
-// out_row_ptr != NULL: row out_pos[j] is written to the address out_row_ptr[out_pos[j]] instead.
-int launch_ffn_umma(long long T, int D, int F, int E, int e_begin, int e_end, const int* offset,
-                    const int* slot_of_expert, int slots, const float* h_hi, const float* h_lo, const float* w01,
-                    const float* wo, const float* routed, float* g_hi, float* g_lo, float* post, int* status,
-                    int num_sms, cudaStream_t stream, cudaEvent_t mid_event = nullptr, const int* out_pos = nullptr,
-                    const float* mix_score = nullptr, const unsigned long long* out_row_ptr = nullptr);
+// Buffers of one tensor-core FFN call (all on the device).
+struct FfnUmma {
+    const int* offset;              // [E+1] first row of each expert
+    const int* slot_of_expert;      // expert -> weight slot (NULL: identity)
+    int slots;                      // weight slots in the planes
+    const float *w01, *wo;          // split planes (launch_split_tiles), [slots] x split_plane_elems
+    const void* h;                  // packed LayerNorm output [T][D]
+    const float* row_info;          // [T][2]
+    void* g;                        // packed gate activations [T][F] (scratch)
+    const float* resid;             // rows the experts were applied to
+    // Output rows: row j of the experts' result goes to row out_pos[j] of `out` (out_pos NULL: row j), or to the
+    // address out_row_ptr[out_pos[j]]; mix_score != NULL applies the base_layer output mix on the way.
+    float* out;
+    const int* out_pos;
+    const float* mix_score;
+    const unsigned long long* out_row_ptr;
+    void* part;                     // scratch for cut tiles (ffn_umma_part_bytes; NULL: no tile is cut) and its
+    size_t part_bytes;              // counters (FFN_COUNTERS, zero before the first launch of a call; every
+    int* part_count;                // launch leaves them zero)
+    int* status;
+};
+int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_begin, int e_end, int num_sms,
+                    cudaStream_t stream, cudaEvent_t mid_event = nullptr);
+constexpr int FFN_CTAS = 148;                   // most CTAs of a launch (SMs of a B200); the workspace is sized for them
+constexpr int FFN_COUNTERS = FFN_CTAS * 8;      // ints in part_count: one per cut tile and accumulate warp
+size_t ffn_umma_part_bytes(long long T, int D, int F);
 // Rows of `in` [n][D] copied to the addresses dst[i] (one per row; they may point into a peer GPU's memory).
 int launch_rows_to_ptrs(long long n, int D, const float* in, const unsigned long long* dst, cudaStream_t stream);
 

@@ -72,9 +72,11 @@ struct ExpertStore {
     // device: LayerNorm weights of all experts [E][D] (always resident, 4*E*D bytes)
     float* d_ln = nullptr;
     std::vector<char> ln_on_device;
-    // device-resident raw FP32 weights in the GEMM's tile-contiguous layout (launch_retile):
-    //   [0] w01 [E] x tiled(2F x D)  (row 2f = wi_0[f], row 2f+1 = wi_1[f])
-    //   [1] wo  [E] x tiled(D x F)
+    // device-resident weights in the GEMM's tile-contiguous layout: FP16 pairs with their row scales for the
+    // tensor-core GEMM (launch_split_tiles), raw FP32 for the CUDA-core one (launch_retile)
+    //   [0] w01 [E] x plane(2F x D)  (row 2f = wi_0[f], row 2f+1 = wi_1[f])
+    //   [1] wo  [E] x plane(D x F)
+    bool split = false;
     float* d_plane[2] = {nullptr, nullptr};
     float* d_staging = nullptr;   // 3*D*F floats: landing area of host weights before they are retiled
     std::vector<char> on_device;
@@ -87,7 +89,10 @@ struct ExpertStore {
     bool upload_recorded = false;
 
     size_t matrix_elems() const { return (size_t)D * (size_t)F; }
-    size_t plane_elems(int p) const { return p == 0 ? tiled_elems(2 * F, D) : tiled_elems(D, F); }   // per expert
+    size_t plane_elems(int p) const {   // floats per expert
+        const int M = p == 0 ? 2 * F : D, K = p == 0 ? D : F;
+        return split ? split_plane_elems(M, K) : tiled_elems(M, K);
+    }
     size_t resident_bytes() const { return (plane_elems(0) + plane_elems(1)) * (size_t)E * sizeof(float); }
 
     ~ExpertStore() {
@@ -107,8 +112,9 @@ struct ExpertStore {
 };
 
 struct WsLayout {
-    size_t gate, pos, count, offset, slot_map, score, rscore, routed, post, h_hi, h_lo, g_hi, g_lo, slots, custom_slots,
-        custom_ws, total;
+    size_t gate, pos, count, offset, slot_map, score, rscore, routed, post, h_hi, h_lo, g_hi, g_lo, row_info, part, part_count, slots,
+        custom_slots, custom_ws, total;
+    size_t part_bytes;
 };
 
 // Sublayer types registered through infmoe_register_sublayer (the reference's extension point is deriving from
@@ -241,12 +247,18 @@ WsLayout ws_layout(const infmoe_layer* L, long long T, bool streamed) {
     const bool row_planes = L->identity || L->custom || !uses_umma(L);
     w.routed = take(row_planes ? 4 * t * D : 0);
     w.post = take(row_planes ? 4 * t * D : 0);
-    w.h_hi = take(4 * t * D);
-    w.h_lo = take(second_plane_bytes((long long)t, L->D));
-    w.g_hi = take(4 * t * F);
-    w.g_lo = take(second_plane_bytes((long long)t, L->F));
+    // activations: one packed plane each on the tensor-core path (h_lo / g_lo stay empty), FP32 head and tail planes
+    // on the CUDA-core path
+    w.h_hi = take(row_planes ? 4 * t * D : pack_bytes((long long)t, L->D));
+    w.h_lo = take(row_planes ? 4 * t * D : 0);
+    w.g_hi = take(row_planes ? 4 * t * F : pack_bytes((long long)t, L->F));
+    w.g_lo = take(row_planes ? 4 * t * F : 0);
+    w.row_info = take(row_planes ? 0 : 8 * t);
+    w.part_bytes = row_planes ? 0 : ffn_umma_part_bytes((long long)t, L->D, L->F);
+    w.part = take(w.part_bytes);
+    w.part_count = take(row_planes ? 0 : FFN_COUNTERS * sizeof(int));
     w.slots = take(streamed && !L->identity && !L->custom
-                       ? 4 * (size_t)L->mc * (tiled_elems(2 * L->F, L->D) + tiled_elems(L->D, L->F) + 3 * D * F)
+                       ? 4 * (size_t)L->mc * (L->store->plane_elems(0) + L->store->plane_elems(1) + 3 * D * F)
                        : 0);
     // registered sublayer: max_concurrency weight slots (MoESubLayer::weightSize each) and its own scratch
     const size_t sub_weight = L->custom && L->sub.weight_size ? align_up(L->sub.weight_size(L->sub.user)) : 0;
@@ -279,10 +291,9 @@ int ensure_resident_planes(ExpertStore* s) {
     return INFMOE_OK;
 }
 
-// Puts one expert's matrices into its two planes (tile-contiguous, wi_0 / wi_1 rows interleaved).  Host
-// sources first land in `staging` (device, 3*D*F floats); the weights stay raw FP32 (the GEMM kernel splits
-// them into TF32 head and tail on the fly).
-int load_expert_planes(int D, int F, const float* wi0, const float* wi1, const float* wo, float* w01, float* wo_dst,
+// Puts one expert's matrices into its two planes (tile-contiguous, wi_0 / wi_1 rows interleaved; FP16 pairs with
+// `split`, else raw FP32).  Host sources first land in `staging` (device, 3*D*F floats).
+int load_expert_planes(bool split, int D, int F, const float* wi0, const float* wi1, const float* wo, float* w01, float* wo_dst,
                        bool src_on_host, float* staging, cudaStream_t stream) {
     const size_t n = (size_t)D * F;
     if (src_on_host) {
@@ -297,8 +308,9 @@ int load_expert_planes(int D, int F, const float* wi0, const float* wi1, const f
         wi1 = staging + n;
         wo = staging + 2 * n;
     }
-    INFMOE_TRY(launch_retile(wi0, wi1, 2 * F, D, w01, stream));
-    INFMOE_TRY(launch_retile(wo, nullptr, D, F, wo_dst, stream));
+    const auto layout = split ? launch_split_tiles : launch_retile;
+    INFMOE_TRY(layout(wi0, wi1, 2 * F, D, w01, stream));
+    INFMOE_TRY(layout(wo, nullptr, D, F, wo_dst, stream));
     return INFMOE_OK;
 }
 
@@ -313,7 +325,7 @@ int upload_resident(ExpertStore* s, cudaStream_t stream) {
     for (int e = 0; e < s->E; ++e) {
         if (s->on_device[e] || !s->on_host[e]) continue;
         if (!s->d_staging) INFMOE_CUDA_TRY(cudaMalloc(&s->d_staging, sizeof(float) * 3 * s->matrix_elems()));
-        INFMOE_TRY(load_expert_planes(s->D, s->F, s->h_wi0[e], s->h_wi1[e], s->h_wo[e],
+        INFMOE_TRY(load_expert_planes(s->split, s->D, s->F, s->h_wi0[e], s->h_wi1[e], s->h_wo[e],
                                       s->d_plane[0] + s->plane_elems(0) * e, s->d_plane[1] + s->plane_elems(1) * e,
                                       true, s->d_staging, stream));
         s->on_device[e] = 1;
@@ -418,16 +430,41 @@ struct FfnOutput {
     const unsigned long long* row_ptr = nullptr;   // address of output row i instead of out + i * D
 };
 
+// Workspace pieces the experts work in.
+struct FfnBuffers {
+    float *h_hi, *h_lo, *g_hi, *g_lo;   // tensor-core path: packed planes in h_hi / g_hi
+    float* row_info;
+    void* part;
+    size_t part_bytes;
+    int* part_count;
+};
+
 int run_ffn(infmoe_layer* L, long long T, int e_begin, int e_end, const int* d_offset, const int* d_slot_map,
-            int slots, float* const planes[2], const float* h_hi, const float* h_lo, const float* routed, float* g_hi,
-            float* g_lo, const FfnOutput& o, cudaStream_t stream, cudaEvent_t mid = nullptr) {
-    if (uses_umma(L))
-        return launch_ffn_umma(T, L->D, L->F, L->E, e_begin, e_end, d_offset, d_slot_map, slots, h_hi, h_lo, planes[0],
-                               planes[1], routed, g_hi, g_lo, o.out ? o.out : o.post, L->d_status, L->num_sms, stream,
-                               mid, o.out ? o.pos : nullptr, o.out ? o.mix_score : nullptr, o.out ? o.row_ptr : nullptr);
-    float* post = o.post;
-    return launch_ffn_simt(T, L->D, L->F, e_begin, e_end, d_offset, d_slot_map, h_hi, h_lo, planes[0], planes[1],
-                           routed, g_hi, g_lo, post, stream);
+            int slots, float* const planes[2], const FfnBuffers& w, const float* routed, const FfnOutput& o,
+            cudaStream_t stream, cudaEvent_t mid = nullptr) {
+    if (uses_umma(L)) {
+        FfnUmma f{};
+        f.offset = d_offset;
+        f.slot_of_expert = d_slot_map;
+        f.slots = slots;
+        f.w01 = planes[0];
+        f.wo = planes[1];
+        f.h = w.h_hi;
+        f.row_info = w.row_info;
+        f.g = w.g_hi;
+        f.resid = routed;
+        f.out = o.out ? o.out : o.post;
+        f.out_pos = o.out ? o.pos : nullptr;
+        f.mix_score = o.out ? o.mix_score : nullptr;
+        f.out_row_ptr = o.out ? o.row_ptr : nullptr;
+        f.part = w.part;
+        f.part_bytes = w.part_bytes;
+        f.part_count = w.part_count;
+        f.status = L->d_status;
+        return launch_ffn_umma(f, T, L->D, L->F, L->E, e_begin, e_end, L->num_sms, stream, mid);
+    }
+    return launch_ffn_simt(T, L->D, L->F, e_begin, e_end, d_offset, d_slot_map, w.h_hi, w.h_lo, planes[0], planes[1],
+                           routed, w.g_hi, w.g_lo, o.post, stream);
 }
 
 void free_device_state(infmoe_layer* L) {
@@ -578,6 +615,7 @@ int infmoe_layer_create(const infmoe_layer_config* cfg, infmoe_layer** out) {
     // decided here, not at the first enqueue: the workspace size depends on it
     const char* path = getenv("INFMOE_FFN");
     if (path && strcmp(path, "simt") == 0) L->ffn_path = 1;
+    L->store->split = uses_umma(L);
     *out = L;
     return INFMOE_OK;
 }
@@ -732,7 +770,7 @@ int infmoe_layer_set_expert(infmoe_layer* L, int32_t e, const float* ln_w, const
         INFMOE_TRY(ensure_resident_planes(s));
         INFMOE_CUDA_TRY(cudaMemcpy(s->d_ln + (size_t)e * s->D, ln_w, sizeof(float) * s->D, cudaMemcpyDeviceToDevice));
         s->ln_on_device[e] = 1;
-        INFMOE_TRY(load_expert_planes(s->D, s->F, wi0, wi1, wo, s->d_plane[0] + s->plane_elems(0) * e,
+        INFMOE_TRY(load_expert_planes(s->split, s->D, s->F, wi0, wi1, wo, s->d_plane[0] + s->plane_elems(0) * e,
                                       s->d_plane[1] + s->plane_elems(1) * e, false, nullptr, 0));
         INFMOE_CUDA_TRY(cudaStreamSynchronize(0));
         s->on_device[e] = 1;
@@ -1012,10 +1050,15 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     float* rscore = (float*)(base + w.rscore);
     float* routed = (float*)(base + w.routed);
     float* post = (float*)(base + w.post);
-    float* h_hi = (float*)(base + w.h_hi);
-    float* h_lo = (float*)(base + w.h_lo);
-    float* g_hi = (float*)(base + w.g_hi);
-    float* g_lo = (float*)(base + w.g_lo);
+    FfnBuffers buf;
+    buf.h_hi = (float*)(base + w.h_hi);
+    buf.h_lo = (float*)(base + w.h_lo);
+    buf.g_hi = (float*)(base + w.g_hi);
+    buf.g_lo = (float*)(base + w.g_lo);
+    buf.row_info = (float*)(base + w.row_info);
+    buf.part = w.part_bytes ? base + w.part : nullptr;
+    buf.part_bytes = w.part_bytes;
+    buf.part_count = (int*)(base + w.part_count);
     const int* gate_in = given_gate ? given_gate : gate;
     if (given_gate) score = const_cast<float*>(row_score);   // scores of the caller's rows, or none
     L->last_gate = gate_in;
@@ -1031,7 +1074,8 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                                 L->D, L->E, gate, score, L->d_status, stream));
     INFMOE_TRY(prof_mark(L, 1, stream));
     // 2. dispatch metadata (:350-352)
-    INFMOE_TRY(launch_dispatch(gate_in, T, L->E, pos, count, offset, L->d_status, stream, region_count, region_size));
+    INFMOE_TRY(launch_dispatch(gate_in, T, L->E, pos, count, offset, L->d_status, stream, region_count, region_size,
+                               w.part_bytes ? buf.part_count : nullptr, FFN_COUNTERS));
     const int* valid_rows = offset + L->E;   // rows past it have no expert (or are empty slots): nobody touches them
     INFMOE_TRY(prof_mark(L, 2, stream));
     // whole layer: the variant decides; experts alone: the caller asks for the mix by passing the scores
@@ -1096,23 +1140,26 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
             ++j;
         }
     } else {
-        // 3. scatter fused with the experts' LayerNorm and the TF32 split (:354-355, T5FFLayer.cc:99-103)
+        // 3. scatter fused with the experts' LayerNorm and the operand split (:354-355, T5FFLayer.cc:99-103)
         const bool pack = uses_umma(L);   // the GEMM run_ffn picks
         // tensor-core path: no routed copy, the second GEMM's epilogue reads its residual from d_in through pos[]
-        if (pack) routed = nullptr;
-        INFMOE_TRY(launch_scatter_ln_split(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, routed, rscore,
-                                           h_hi, h_lo, pack, stream));
-        if (pack) routed = const_cast<float*>(d_in);   // run_ffn's residual operand
+        if (pack) {
+            INFMOE_TRY(launch_scatter_ln_pack(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, rscore, buf.h_hi,
+                                              buf.row_info, stream));
+            routed = const_cast<float*>(d_in);   // run_ffn's residual operand
+        } else {
+            INFMOE_TRY(launch_scatter_ln_split(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, routed, rscore,
+                                               buf.h_hi, buf.h_lo, stream));
+        }
         INFMOE_TRY(prof_mark(L, 3, stream));
         // 4. experts (:360-402)
         if (!streamed) {
             cudaEvent_t mid = nullptr;
             if (L->profiling) mid = L->prof_events[(size_t)(L->prof_calls % PROF_CALLS) * PROF_MARKS + 4];
-            INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, nullptr, L->E, s->d_plane, h_hi, h_lo, routed, g_hi, g_lo,
-                               ffn_out, stream, mid));
+            INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, nullptr, L->E, s->d_plane, buf, routed, ffn_out, stream, mid));
         } else {
             const size_t n = s->matrix_elems();
-            // slot planes: w01 [mc] x tiled(2F x D), wo [mc] x tiled(D x F), then one raw landing area per slot
+            // slot planes: w01 [mc], wo [mc], then one raw landing area per slot
             const size_t n0 = s->plane_elems(0), n1 = s->plane_elems(1);
             float* planes[2];
             planes[0] = (float*)(base + w.slots);
@@ -1158,8 +1205,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
             if (all_cached) {
                 // nothing to copy: one grouped launch over all experts, as in resident mode
                 for (const CachePlan& pl : plan) INFMOE_CUDA_TRY(cudaStreamWaitEvent(stream, L->ev_ready[pl.slot], 0));
-                INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, slot_map, nslots, planes, h_hi, h_lo, routed, g_hi, g_lo,
-                                   ffn_out, stream));
+                INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, slot_map, nslots, planes, buf, routed, ffn_out, stream));
                 for (const CachePlan& pl : plan) INFMOE_CUDA_TRY(cudaEventRecord(L->ev_freed[pl.slot], stream));
             }
             for (size_t j = 0; j < active.size() && !all_cached; ++j) {
@@ -1174,7 +1220,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                     // rotation for the cache, each reusable once its retile kernels are done
                     const int area = cached ? (int)(loads % (size_t)L->mc) : slot;
                     if (cached) INFMOE_CUDA_TRY(cudaStreamWaitEvent(cs, L->ev_stage[area], 0));
-                    INFMOE_TRY(load_expert_planes(L->D, L->F, s->h_wi0[e], s->h_wi1[e], s->h_wo[e],
+                    INFMOE_TRY(load_expert_planes(s->split, L->D, L->F, s->h_wi0[e], s->h_wi1[e], s->h_wo[e],
                                                   planes[0] + n0 * slot, planes[1] + n1 * slot, true,
                                                   staging + 3 * n * area, cs));
                     if (cached) INFMOE_CUDA_TRY(cudaEventRecord(L->ev_stage[area], cs));
@@ -1183,8 +1229,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                     ++loads;
                 }
                 INFMOE_CUDA_TRY(cudaStreamWaitEvent(stream, L->ev_ready[slot], 0));
-                INFMOE_TRY(run_ffn(L, T, e, e + 1, offset, slot_map, nslots, planes, h_hi, h_lo, routed, g_hi, g_lo,
-                                   ffn_out, stream));
+                INFMOE_TRY(run_ffn(L, T, e, e + 1, offset, slot_map, nslots, planes, buf, routed, ffn_out, stream));
                 INFMOE_CUDA_TRY(cudaEventRecord(L->ev_freed[slot], stream));
             }
             INFMOE_TRY(prof_mark(L, 4, stream));   // streamed: copies and both GEMMs are timed together
@@ -1196,7 +1241,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     } else {
         // with per-row addresses the rows are first combined in the caller's row order (g_hi is free by now:
         // T x d_ff floats), then copied out
-        float* ordered = row_dst ? g_hi : d_out;
+        float* ordered = row_dst ? buf.g_hi : d_out;
         if (mix)
             INFMOE_TRY(launch_mix_gather(T, L->D, pos, routed, post, rscore, ordered, stream, valid_rows));
         else
@@ -1762,38 +1807,62 @@ int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_
         p += align_up(bytes);
         return at;
     };
-    float* h_hi = (float*)take(4 * r * d);
-    float* h_lo = (float*)take(second_plane_bytes(rows, D));
-    float* g_hi = (float*)take(4 * r * f);
-    float* g_lo = (float*)take(second_plane_bytes(rows, F));
+    const char* path = getenv("INFMOE_FFN");
+    const bool simt = (path && strcmp(path, "simt") == 0) || !ffn_umma_supported(D, F, 1);
+    float* h_hi = (float*)take(simt ? 4 * r * d : pack_bytes(rows, D));
+    float* h_lo = (float*)take(simt ? 4 * r * d : 0);
+    float* g_hi = (float*)take(simt ? 4 * r * f : pack_bytes(rows, F));
+    float* g_lo = (float*)take(simt ? 4 * r * f : 0);
+    float* row_info = (float*)take(simt ? 0 : 8 * r);
     float* planes[2];
-    planes[0] = (float*)take(4 * tiled_elems(2 * F, D));
-    planes[1] = (float*)take(4 * tiled_elems(D, F));
+    planes[0] = (float*)take(4 * (simt ? tiled_elems(2 * F, D) : split_plane_elems(2 * F, D)));
+    planes[1] = (float*)take(4 * (simt ? tiled_elems(D, F) : split_plane_elems(D, F)));
     int* offset = (int*)take(8);
     int* status = (int*)take(4);
     // offset[] = {0, rows}: the row count travels as a kernel parameter, so no host buffer has to outlive the call
     INFMOE_CUDA_TRY(cudaMemsetAsync(offset, 0, 4, stream));
     INFMOE_TRY(launch_fill_int(offset + 1, (int)rows, stream));
     INFMOE_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), stream));
-    const char* path = getenv("INFMOE_FFN");
-    const bool simt = (path && strcmp(path, "simt") == 0) || !ffn_umma_supported(D, F, 1);
-    INFMOE_TRY(launch_ln_split(rows, D, x, ln_w, h_hi, h_lo, !simt, stream));
-    INFMOE_TRY(load_expert_planes(D, F, wi0, wi1, wo, planes[0], planes[1], false, nullptr, stream));
+    if (simt) INFMOE_TRY(launch_ln_split(rows, D, x, ln_w, h_hi, h_lo, stream));
+    else INFMOE_TRY(launch_ln_pack(rows, D, x, ln_w, h_hi, row_info, stream));
+    INFMOE_TRY(load_expert_planes(!simt, D, F, wi0, wi1, wo, planes[0], planes[1], false, nullptr, stream));
     int dev = 0, sms = 0;
     INFMOE_CUDA_TRY(cudaGetDevice(&dev));
     INFMOE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (simt)
+    if (simt) {
         INFMOE_TRY(launch_ffn_simt(rows, D, F, 0, 1, offset, nullptr, h_hi, h_lo, planes[0], planes[1], x, g_hi, g_lo,
                                    y, stream));
-    else
-        INFMOE_TRY(launch_ffn_umma(rows, D, F, 1, 0, 1, offset, nullptr, 1, h_hi, h_lo, planes[0], planes[1], x, g_hi,
-                                   g_lo, y, status, sms, stream));
+    } else {
+        FfnUmma u{};
+        u.offset = offset;
+        u.slots = 1;
+        u.w01 = planes[0];
+        u.wo = planes[1];
+        u.h = h_hi;
+        u.row_info = row_info;
+        u.g = g_hi;
+        u.resid = x;
+        u.out = y;
+        u.status = status;
+        INFMOE_TRY(launch_ffn_umma(u, rows, D, F, 1, 0, 1, sms, stream));
+    }
     int h_status = 0;
     INFMOE_CUDA_TRY(cudaMemcpyAsync(&h_status, status, sizeof(int), cudaMemcpyDeviceToHost, stream));
     INFMOE_CUDA_TRY(cudaStreamSynchronize(stream));
     return status_to_rc(h_status);
 }
 
+}  // namespace
+
+namespace {
+// Scratch of the CUDA-core form, the larger one but for the row scales and row_info of the tensor-core form (which
+// are at most 2 MB beside a scratch of 32 MB: 512 bytes per 128-row weight block, which has at least one 16 KB tile).
+// It is also the measure of what infmoe_t5ff_run_static takes.
+size_t t5ff_scratch_bytes(int64_t rows, int32_t D, int32_t F) {
+    const size_t r = (size_t)rows, d = (size_t)D, f = (size_t)F;
+    return align_up(4 * r * d) + align_up(pack_bytes(rows, D)) + align_up(4 * r * f) + align_up(pack_bytes(rows, F)) +
+           align_up(4 * tiled_elems(2 * F, D)) + align_up(4 * tiled_elems(D, F)) + 2 * ALIGN + ALIGN;
+}
 }  // namespace
 
 extern "C" {
@@ -1803,10 +1872,9 @@ int infmoe_t5ff_workspace_bytes(int64_t rows, int32_t D, int32_t F, size_t* byte
         set_error("t5ff_workspace_bytes: bad argument");
         return INFMOE_ERR_INVALID_ARGUMENT;
     }
-    const size_t r = (size_t)rows, d = (size_t)D, f = (size_t)F;
-    *bytes = align_up(4 * r * d) + align_up(second_plane_bytes(rows, D)) + align_up(4 * r * f) +
-             align_up(second_plane_bytes(rows, F)) + align_up(4 * tiled_elems(2 * F, D)) +
-             align_up(4 * tiled_elems(D, F)) + 2 * ALIGN + ALIGN;
+    const size_t scales = 4 * (split_plane_elems(2 * F, D) - tiled_elems(2 * F, D)) +
+                          4 * (split_plane_elems(D, F) - tiled_elems(D, F)) + 8 * (size_t)rows;
+    *bytes = t5ff_scratch_bytes(rows, D, F) + align_up(scales) + 3 * ALIGN;
     return INFMOE_OK;
 }
 
@@ -1843,7 +1911,8 @@ int infmoe_t5ff_run(int64_t rows, int32_t D, int32_t F, const float* ln_w, const
 // larger problems are rejected and belong to infmoe_t5ff_run.  Like infmoe_t5ff_run the call
 // blocks the host until the result is there.
 #define INFMOE_STATIC_SCRATCH_BYTES (32u << 20)
-static __device__ __align__(256) unsigned char g_static_scratch[INFMOE_STATIC_SCRATCH_BYTES];
+#define INFMOE_STATIC_SCALE_BYTES (2u << 20)   // row scales beside the scratch, see t5ff_scratch_bytes
+static __device__ __align__(256) unsigned char g_static_scratch[INFMOE_STATIC_SCRATCH_BYTES + INFMOE_STATIC_SCALE_BYTES];
 
 namespace {
 
@@ -1879,9 +1948,11 @@ int static_scratch_address(unsigned char** out) {
 extern "C" {
 
 int infmoe_t5ff_static_limit(int64_t rows, int32_t D, int32_t F, size_t* needed, size_t* available) {
-    size_t need = 0;
-    INFMOE_TRY(infmoe_t5ff_workspace_bytes(rows, D, F, &need));
-    if (needed) *needed = need;
+    if (rows < 0 || D <= 0 || F <= 0) {
+        set_error("t5ff_workspace_bytes: bad argument");
+        return INFMOE_ERR_INVALID_ARGUMENT;
+    }
+    if (needed) *needed = t5ff_scratch_bytes(rows, D, F);
     if (available) *available = (size_t)INFMOE_STATIC_SCRATCH_BYTES;
     return INFMOE_OK;
 }
@@ -1893,8 +1964,7 @@ int infmoe_t5ff_run_static(int64_t rows, int32_t D, int32_t F, const float* ln_w
         return INFMOE_ERR_INVALID_ARGUMENT;
     }
     if (rows == 0) return INFMOE_OK;
-    size_t need = 0;
-    INFMOE_TRY(infmoe_t5ff_workspace_bytes(rows, D, F, &need));
+    const size_t need = t5ff_scratch_bytes(rows, D, F);
     if (need > (size_t)INFMOE_STATIC_SCRATCH_BYTES) {
         set_error("t5ff_run_static: rows=%lld d_model=%d d_ff=%d needs %zu bytes of scratch but the built-in array "
                   "holds %u; use infmoe_t5ff_run with a workspace of your own", (long long)rows, D, F, need,

@@ -1,6 +1,6 @@
 // Row-wise kernels of the MoE layer: scatter into expert-contiguous order,
-// gather / mix back to token order, LayerNorm, gelu-dot and the TF32 head/tail
-// split that feeds the tensor-core GEMMs.  All of them are pure HBM streaming:
+// gather / mix back to token order, LayerNorm, gelu-dot and the splits that feed
+// the GEMMs.  All of them are pure HBM streaming:
 // one warp per row, 128-bit loads and stores, rows of one warp contiguous.
 //
 // Reference counterparts (all scalar 4-byte copies, one CTA of 256 threads per row):
@@ -10,6 +10,7 @@
 //   cuApplyLayerNorm                         plugin/cuda/ops/layernorm.cu:136-174
 //   gelu_dot functor via thrust::transform   plugin/cuda/ops/gelu.cu:6-25
 #include "common.cuh"
+#include "kernels.h"
 
 namespace infmoe {
 
@@ -40,16 +41,11 @@ scatter_kernel(long long T, int D, int vec, const float* __restrict__ X, const f
     if (lane == 0 && coeff && rcoeff) rcoeff[j] = coeff[p];
 }
 
-// The layer's fused scatter: one read of X[pos[j],:] produces its per-expert
-// LayerNorm h = LN(x; gamma_e) (T5FFLayer.cc:99-103) already split for the
-// grouped GEMM, the routed score and, when `routed` is given, the routed row
-// itself (the tensor-core GEMM reads its residual from X through pos[] and needs
-// no such copy).  gamma is [E][D]; the expert of row j is gate[pos[j]].  Rows at or
-// past *valid_rows (tokens without an expert, empty receive slots) are skipped.
-// PACK = false: TF32 head and FP32 tail planes h_hi / h_lo [T][D] (exact split,
-// CUDA-core GEMM); PACK = true: head plane h_hi and the packed BF16 plane (see
-// store_pack4) in h_lo (tensor-core GEMM).
-template <bool PACK>
+// The layer's fused scatter: X[pos[j],:] -> its per-expert LayerNorm h = LN(x; gamma_e) (T5FFLayer.cc:99-103), ready
+// for the grouped GEMM.  gamma is [E][D]; the expert of row j is gate[pos[j]].  Rows at or past *valid_rows (tokens
+// without an expert, empty receive slots) are skipped.
+//
+// For the CUDA-core GEMM: the routed row, the routed score, and TF32 head and FP32 tail planes h_hi / h_lo [T][D].
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 scatter_ln_split_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ score,
                         const int* __restrict__ pos, const int* __restrict__ gate,
@@ -65,48 +61,94 @@ scatter_ln_split_kernel(long long T, int D, int vec, const float* __restrict__ X
     const float* gamma = gamma_all + (long long)e * D;
     float mean, rstd;
     warp_row_stats(src, D, vec != 0, mean, rstd);
-    uint16_t* pack_row = PACK ? reinterpret_cast<uint16_t*>(h_lo) + j * (long long)pack_pitch(D) : nullptr;
-    const int k_end = PACK ? ((D + 31) & ~31) : D;   // the packed plane is zero padded to whole groups
-    for (int base = 4 * lane; base < k_end; base += 128) {
+    for (int base = 4 * lane; base < D; base += 128) {
         float hh[4] = {0.f, 0.f, 0.f, 0.f}, ll[4] = {0.f, 0.f, 0.f, 0.f};
-        if (base < D) {
-            const float4 v = load_row4(src, base, D, vec != 0);
-            const float4 g = load_row4(gamma, base, D, vec != 0);
-            const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
+        const float4 v = load_row4(src, base, D, vec != 0);
+        const float4 g = load_row4(gamma, base, D, vec != 0);
+        const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (base + k < D) split_tf32(ln_apply(vv[k], mean, rstd, gg[k]), hh[k], ll[k]);
-            const long long o = j * D + base;
-            if (vec) {
-                if (routed) *reinterpret_cast<float4*>(routed + o) = v;
-                *reinterpret_cast<float4*>(h_hi + o) = make_float4(hh[0], hh[1], hh[2], hh[3]);
-                if (!PACK) *reinterpret_cast<float4*>(h_lo + o) = make_float4(ll[0], ll[1], ll[2], ll[3]);
-            } else {
-                for (int k = 0; k < 4 && base + k < D; ++k) {
-                    if (routed) routed[o + k] = vv[k];
-                    h_hi[o + k] = hh[k];
-                    if (!PACK) h_lo[o + k] = ll[k];
-                }
+        for (int k = 0; k < 4; ++k)
+            if (base + k < D) split_tf32(ln_apply(vv[k], mean, rstd, gg[k]), hh[k], ll[k]);
+        const long long o = j * D + base;
+        if (vec) {
+            *reinterpret_cast<float4*>(routed + o) = v;
+            *reinterpret_cast<float4*>(h_hi + o) = make_float4(hh[0], hh[1], hh[2], hh[3]);
+            *reinterpret_cast<float4*>(h_lo + o) = make_float4(ll[0], ll[1], ll[2], ll[3]);
+        } else {
+            for (int k = 0; k < 4 && base + k < D; ++k) {
+                routed[o + k] = vv[k];
+                h_hi[o + k] = hh[k];
+                h_lo[o + k] = ll[k];
             }
         }
-        if (PACK) store_pack4(pack_row, base, hh, ll);
     }
+    if (lane == 0 && rscore && score) rscore[j] = score[p];
+}
+
+// One warp: h = LN(src; gamma) as FP16 pairs scaled by a power of two of the row, and the row's two numbers.
+__device__ __forceinline__ void warp_ln_pack(const float* __restrict__ src, const float* __restrict__ gamma, int D,
+                                             bool vec, uint16_t* __restrict__ pack_row, float2* __restrict__ info) {
+    const int lane = threadIdx.x & 31;
+    float mean, rstd;
+    warp_row_stats(src, D, vec, mean, rstd);
+    auto load_h = [&](int base, float (&h)[4]) {
+        const float4 v = load_row4(src, base, D, vec), g = load_row4(gamma, base, D, vec);
+        const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) h[k] = base + k < D ? ln_apply(vv[k], mean, rstd, gg[k]) : 0.f;
+    };
+    float top = 0.f;
+    for (int base = 4 * lane; base < D; base += 128) {
+        float h[4];
+        load_h(base, h);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) top = fmaxf(top, fabsf(h[k]));
+    }
+    const int s = row_exponent(warp_max(top));
+    const float scale = exp2_int(s);
+    float squares = 0.f;
+    for (int base = 4 * lane; base < ((D + 31) & ~31); base += 128) {
+        float h[4] = {0.f, 0.f, 0.f, 0.f};
+        if (base < D) load_h(base, h);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            h[k] = __fmul_rn(h[k], scale);
+            squares = fmaf(h[k], h[k], squares);
+        }
+        store_pack4(pack_row, base, h);
+    }
+    squares = warp_xor_sum(squares);
+    if (lane == 0) *info = token_row_info(s, squares);
+}
+
+// The scatter for the tensor-core GEMM (which reads its residual from X through pos[], so no routed row is written).
+__global__ void __launch_bounds__(ROW_WARPS * 32)
+scatter_ln_pack_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ score,
+                       const int* __restrict__ pos, const int* __restrict__ gate, const float* __restrict__ gamma_all,
+                       const int* __restrict__ valid_rows, float* __restrict__ rscore, uint16_t* __restrict__ h,
+                       float2* __restrict__ row_info) {
+    const int lane = threadIdx.x & 31;
+    const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
+    if (j >= T || (valid_rows && j >= *valid_rows)) return;
+    const int p = pos[j];
+    warp_ln_pack(X + (long long)p * D, gamma_all + (long long)gate[p] * D, D, vec != 0,
+                 h + j * (long long)pack_pitch(D), row_info + j);
     if (lane == 0 && rscore && score) rscore[j] = score[p];
 }
 
 // The same for aligned rows of up to 128 * NV floats, with more bytes in flight per warp: the whole row is
 // fetched into registers by back-to-back 128-bit loads (NV per lane) before any of it is used, so it crosses HBM
-// once in one burst and both statistics passes and the split run from registers.  The additions happen in the
-// order of warp_row_stats, so the results are the same bits.  Few rows per SM (4096 rows on 148 SMs) would
+// once in one burst and the statistics passes and the split run from registers.  The additions of the LayerNorm happen
+// in the order of warp_row_stats, so h has the same bits.  Few rows per SM (4096 rows on 148 SMs) would
 // otherwise leave the memory system half idle.  The expert's LayerNorm weights are fetched into shared memory by
 // cp.async while the row is on its way, so the output loop never waits for L2.
-template <bool PACK, int NV>
+// Bound by HBM: reads 4 D and writes 4 D bytes per row (a third less than the two planes it wrote before).
+template <int NV>
 __global__ void __launch_bounds__(128)
-scatter_ln_split_reg_kernel(long long T, int D, const float* __restrict__ X, const float* __restrict__ score,
-                            const int* __restrict__ pos, const int* __restrict__ gate,
-                            const float* __restrict__ gamma_all, const int* __restrict__ valid_rows,
-                            float* __restrict__ routed, float* __restrict__ rscore, float* __restrict__ h_hi,
-                            float* __restrict__ h_lo) {
+scatter_ln_pack_reg_kernel(long long T, int D, const float* __restrict__ X, const float* __restrict__ score,
+                           const int* __restrict__ pos, const int* __restrict__ gate,
+                           const float* __restrict__ gamma_all, const int* __restrict__ valid_rows,
+                           float* __restrict__ rscore, uint16_t* __restrict__ h, float2* __restrict__ row_info) {
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;
@@ -151,28 +193,39 @@ scatter_ln_split_reg_kernel(long long T, int D, const float* __restrict__ X, con
         }
     const float var = __fdiv_rn(warp_xor_sum(q), (float)D);
     const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, 1e-6f)));
-    uint16_t* pack_row = PACK ? reinterpret_cast<uint16_t*>(h_lo) + j * (long long)pack_pitch(D) : nullptr;
-    const int k_end = PACK ? ((D + 31) & ~31) : D;
+    uint16_t* pack_row = h + j * (long long)pack_pitch(D);
     asm volatile("cp.async.wait_group 0;" ::: "memory");   // every lane reads back only what it fetched itself
+    float top = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int base = 4 * lane + 128 * i;
+        if (base >= D) continue;
+        const float4 g = s_gamma[base >> 2];
+        v[i].x = ln_apply(v[i].x, mean, rstd, g.x);
+        v[i].y = ln_apply(v[i].y, mean, rstd, g.y);
+        v[i].z = ln_apply(v[i].z, mean, rstd, g.z);
+        v[i].w = ln_apply(v[i].w, mean, rstd, g.w);
+        top = fmaxf(fmaxf(fmaxf(top, fabsf(v[i].x)), fmaxf(fabsf(v[i].y), fabsf(v[i].z))), fabsf(v[i].w));
+    }
+    const int exponent = row_exponent(warp_max(top));
+    const float scale = exp2_int(exponent);
+    const int k_end = (D + 31) & ~31;
+    float squares = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int base = 4 * lane + 128 * i;
         if (base >= k_end) continue;
-        float hh[4] = {0.f, 0.f, 0.f, 0.f}, ll[4] = {0.f, 0.f, 0.f, 0.f};
-        if (base < D) {
-            const float4 g = s_gamma[base >> 2];
-            split_tf32(ln_apply(v[i].x, mean, rstd, g.x), hh[0], ll[0]);
-            split_tf32(ln_apply(v[i].y, mean, rstd, g.y), hh[1], ll[1]);
-            split_tf32(ln_apply(v[i].z, mean, rstd, g.z), hh[2], ll[2]);
-            split_tf32(ln_apply(v[i].w, mean, rstd, g.w), hh[3], ll[3]);
-            const long long o = j * D + base;
-            if (routed) *reinterpret_cast<float4*>(routed + o) = v[i];
-            *reinterpret_cast<float4*>(h_hi + o) = make_float4(hh[0], hh[1], hh[2], hh[3]);
-            if (!PACK) *reinterpret_cast<float4*>(h_lo + o) = make_float4(ll[0], ll[1], ll[2], ll[3]);
-        }
-        if (PACK) store_pack4(pack_row, base, hh, ll);
+        const float x[4] = {__fmul_rn(v[i].x, scale), __fmul_rn(v[i].y, scale), __fmul_rn(v[i].z, scale),
+                            __fmul_rn(v[i].w, scale)};     // zeros past the row
+#pragma unroll
+        for (int k = 0; k < 4; ++k) squares = fmaf(x[k], x[k], squares);
+        store_pack4(pack_row, base, x);
     }
-    if (lane == 0 && rscore && score) rscore[j] = score[p];
+    squares = warp_xor_sum(squares);
+    if (lane == 0) {
+        row_info[j] = token_row_info(exponent, squares);
+        if (rscore && score) rscore[j] = score[p];
+    }
 }
 
 // out[pos[j],:] = in[j,:] for the rows below *valid_rows (all rows when valid_rows is NULL)
@@ -237,8 +290,7 @@ layernorm_kernel(long long n, int D, int vec, const float* __restrict__ in, cons
     }
 }
 
-// h = LN(x; gamma) split for the grouped GEMM (rows already in place); planes as in scatter_ln_split_kernel.
-template <bool PACK>
+// h = LN(x; gamma) for rows already in place, as the scatter kernels write it.
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 ln_split_kernel(long long n, int D, int vec, const float* __restrict__ in, const float* __restrict__ gamma,
                 float* __restrict__ h_hi, float* __restrict__ h_lo) {
@@ -248,22 +300,20 @@ ln_split_kernel(long long n, int D, int vec, const float* __restrict__ in, const
     const float* src = in + j * D;
     float mean, rstd;
     warp_row_stats(src, D, vec != 0, mean, rstd);
-    uint16_t* pack_row = PACK ? reinterpret_cast<uint16_t*>(h_lo) + j * (long long)pack_pitch(D) : nullptr;
-    const int k_end = PACK ? ((D + 31) & ~31) : D;
-    for (int base = 4 * lane; base < k_end; base += 128) {
-        float hh[4] = {0.f, 0.f, 0.f, 0.f}, ll[4] = {0.f, 0.f, 0.f, 0.f};
-        if (base < D) {
-            const float4 v = load_row4(src, base, D, vec != 0);
-            const float4 g = load_row4(gamma, base, D, vec != 0);
-            const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
-            for (int k = 0; k < 4 && base + k < D; ++k) {
-                split_tf32(ln_apply(vv[k], mean, rstd, gg[k]), hh[k], ll[k]);
-                h_hi[j * D + base + k] = hh[k];
-                if (!PACK) h_lo[j * D + base + k] = ll[k];
-            }
-        }
-        if (PACK) store_pack4(pack_row, base, hh, ll);
+    for (int base = 4 * lane; base < D; base += 128) {
+        const float4 v = load_row4(src, base, D, vec != 0);
+        const float4 g = load_row4(gamma, base, D, vec != 0);
+        const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
+        for (int k = 0; k < 4 && base + k < D; ++k)
+            split_tf32(ln_apply(vv[k], mean, rstd, gg[k]), h_hi[j * D + base + k], h_lo[j * D + base + k]);
     }
+}
+__global__ void __launch_bounds__(ROW_WARPS * 32)
+ln_pack_kernel(long long n, int D, int vec, const float* __restrict__ in, const float* __restrict__ gamma,
+               uint16_t* __restrict__ h, float2* __restrict__ row_info) {
+    const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
+    if (j >= n) return;
+    warp_ln_pack(in + j * D, gamma, D, vec != 0, h + j * (long long)pack_pitch(D), row_info + j);
 }
 
 __global__ void gelu_dot_kernel(const float* __restrict__ a, float* __restrict__ b, size_t len) {
@@ -289,10 +339,12 @@ __global__ void split_kernel(const float* __restrict__ src, float* __restrict__ 
         split_tf32(src[i], hi[i], lo[i]);
 }
 
-// Weight matrix -> tile-contiguous layout for the tensor-core GEMM: tiles of 128 rows x 32 floats (16 KB),
+// Weight matrix -> tile-contiguous layout: tiles of 128 rows x 32 values (16 KB),
 // tile (mb, kb) at ((mb * KB + kb) * 128 rows; rows and columns past the matrix are zero.  With two sources
 // the rows are interleaved: row 2f = src0[f], row 2f+1 = src1[f] (wi_0 / wi_1).  One warp moves one 128-byte
 // row segment, so both the read and the write are coalesced.
+//
+// retile_kernel: raw FP32 tiles for the CUDA-core GEMM.
 __global__ void __launch_bounds__(256)
 retile_kernel(const float* __restrict__ src0, const float* __restrict__ src1, int M, int K, int MB, int KB,
               float* __restrict__ dst) {
@@ -310,6 +362,62 @@ retile_kernel(const float* __restrict__ src0, const float* __restrict__ src1, in
         else v = src0[(size_t)m * K + k];
     }
     dst[seg * 32 + lane] = v;
+}
+
+// Tensor-core GEMM, first pass: 2^-s of every (padded) row from its largest magnitude, and the gate bound, the largest
+// log2(|wi_0[f]| |wi_1[f]|) of the expert (g_exponent).  One warp per row of the sources, all rows read once; squares
+// are summed in 64 bits because the magnitudes may be anywhere in the FP32 range.
+__global__ void __launch_bounds__(256)
+row_scale_kernel(const float* __restrict__ src0, const float* __restrict__ src1, int M, int K, int padded,
+                 float* __restrict__ inv, uint32_t* __restrict__ bound) {
+    const int lane = threadIdx.x & 31;
+    const int step = src1 ? 2 : 1;
+    const int m0 = ((int)blockIdx.x * 8 + (int)(threadIdx.x >> 5)) * step;   // rows m0 (and m0 + 1)
+    if (m0 >= padded) return;
+    double norm[2] = {0.0, 0.0};
+    for (int i = 0; i < step; ++i) {
+        const int m = m0 + i;
+        float top = 0.f;
+        double sum = 0.0;
+        if (m < M) {
+            const float* row = src1 ? (i ? src1 : src0) + (size_t)(m >> 1) * K : src0 + (size_t)m * K;
+#pragma unroll 8
+            for (int k = lane; k < K; k += 32) {
+                const float v = row[k];
+                top = fmaxf(top, fabsf(v));
+                sum += (double)v * (double)v;
+            }
+        }
+        top = warp_max(top);
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        norm[i] = sum;
+        if (lane == 0) inv[m] = exp2_int(-row_exponent(top));
+    }
+    if (src1 && lane == 0 && m0 < M)
+        atomicMax(bound, encode_bound(0.5f * ((float)log2(norm[0]) + (float)log2(norm[1]))));
+}
+
+// Second pass: the tiles as FP16 pairs, a row of a tile being 32 x hi, 32 x lo of the values times 2^s.
+__global__ void __launch_bounds__(256)
+split_tiles_kernel(const float* __restrict__ src0, const float* __restrict__ src1, int M, int K, int MB, int KB,
+                   const float* __restrict__ inv, uint16_t* __restrict__ dst) {
+    const int lane = threadIdx.x & 31;
+    const long long seg = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);   // (mb, kb, r) flattened
+    if (seg >= (long long)MB * KB * 128) return;
+    const int r = (int)(seg % 128);
+    const long long tile = seg / 128;
+    const int kb = (int)(tile % KB), mb = (int)(tile / KB);
+    const int m = mb * 128 + r, k = kb * 32 + lane;
+    float v = 0.f;
+    if (m < M && k < K) {
+        if (src1) v = (m & 1) ? src1[(size_t)(m >> 1) * K + k] : src0[(size_t)(m >> 1) * K + k];
+        else v = src0[(size_t)m * K + k];
+    }
+    // 2^s = 1 / 2^-s exactly (both are normal)
+    const uint32_t p = split_f16(__fmul_rn(v, __fdiv_rn(1.0f, inv[m])));
+    dst[seg * 64 + lane] = (uint16_t)p;
+    dst[seg * 64 + 32 + lane] = (uint16_t)(p >> 16);
 }
 
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
@@ -333,37 +441,42 @@ int launch_scatter(long long T, int D, const float* X, const float* coeff, const
 
 int launch_scatter_ln_split(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
                             const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h_hi,
-                            float* h_lo, bool pack, cudaStream_t stream) {
+                            float* h_lo, cudaStream_t stream) {
     if (T == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && aligned16(X) && aligned16(routed) && aligned16(h_hi) && aligned16(h_lo) &&
                     aligned16(gamma_all);
+    scatter_ln_split_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, X, score, pos, gate, gamma_all,
+                                                                        valid_rows, routed, rscore, h_hi, h_lo);
+    note_launch();
+    INFMOE_CUDA_TRY(cudaGetLastError());
+    return INFMOE_OK;
+}
+
+int launch_scatter_ln_pack(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
+                           const float* gamma_all, const int* valid_rows, float* rscore, void* h, float* row_info,
+                           cudaStream_t stream) {
+    if (T == 0) return INFMOE_OK;
+    const int vec = (D % 4 == 0) && aligned16(X) && aligned16(gamma_all);
+    uint16_t* pack = (uint16_t*)h;
+    float2* info = (float2*)row_info;
     if (vec && D <= 4096) {
         const unsigned grid = (unsigned)((T + 3) / 4);
-#define INFMOE_SCATTER_REG(PACK, NV)                                                                               \
+#define INFMOE_SCATTER_REG(NV)                                                                                     \
     do {                                                                                                           \
-        auto kern = scatter_ln_split_reg_kernel<PACK, NV>;                                                         \
+        auto kern = scatter_ln_pack_reg_kernel<NV>;                                                                \
         constexpr int smem = 4 * NV * 32 * 16;                                                                     \
         if (smem > 48 * 1024)                                                                                      \
             INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));        \
-        kern<<<grid, 128, smem, stream>>>(T, D, X, score, pos, gate, gamma_all, valid_rows, routed, rscore, h_hi,  \
-                                          h_lo);                                                                   \
+        kern<<<grid, 128, smem, stream>>>(T, D, X, score, pos, gate, gamma_all, valid_rows, rscore, pack, info);   \
     } while (0)
-        if (pack) {
-            if (D <= 1024) INFMOE_SCATTER_REG(true, 8);
-            else if (D <= 2048) INFMOE_SCATTER_REG(true, 16);
-            else INFMOE_SCATTER_REG(true, 32);
-        } else {
-            if (D <= 1024) INFMOE_SCATTER_REG(false, 8);
-            else if (D <= 2048) INFMOE_SCATTER_REG(false, 16);
-            else INFMOE_SCATTER_REG(false, 32);
-        }
+        if (D <= 1024) INFMOE_SCATTER_REG(8);
+        else if (D <= 2048) INFMOE_SCATTER_REG(16);
+        else INFMOE_SCATTER_REG(32);
 #undef INFMOE_SCATTER_REG
-    } else if (pack)
-        scatter_ln_split_kernel<true><<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(
-            T, D, vec, X, score, pos, gate, gamma_all, valid_rows, routed, rscore, h_hi, h_lo);
-    else
-        scatter_ln_split_kernel<false><<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(
-            T, D, vec, X, score, pos, gate, gamma_all, valid_rows, routed, rscore, h_hi, h_lo);
+    } else {
+        scatter_ln_pack_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, X, score, pos, gate, gamma_all,
+                                                                           valid_rows, rscore, pack, info);
+    }
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
@@ -441,15 +554,36 @@ int launch_layernorm(float* out, const float* in, long long n, int D, const floa
     return INFMOE_OK;
 }
 
-int launch_ln_split(long long n, int D, const float* in, const float* gamma, float* h_hi, float* h_lo, bool pack,
+int launch_ln_split(long long n, int D, const float* in, const float* gamma, float* h_hi, float* h_lo,
                     cudaStream_t stream) {
     if (n == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && aligned16(in) && aligned16(gamma);
-    if (pack)
-        ln_split_kernel<true><<<row_grid(n), ROW_WARPS * 32, 0, stream>>>(n, D, vec, in, gamma, h_hi, h_lo);
-    else
-        ln_split_kernel<false><<<row_grid(n), ROW_WARPS * 32, 0, stream>>>(n, D, vec, in, gamma, h_hi, h_lo);
+    ln_split_kernel<<<row_grid(n), ROW_WARPS * 32, 0, stream>>>(n, D, vec, in, gamma, h_hi, h_lo);
     note_launch();
+    INFMOE_CUDA_TRY(cudaGetLastError());
+    return INFMOE_OK;
+}
+
+int launch_ln_pack(long long n, int D, const float* in, const float* gamma, void* h, float* row_info,
+                   cudaStream_t stream) {
+    if (n == 0) return INFMOE_OK;
+    const int vec = (D % 4 == 0) && aligned16(in) && aligned16(gamma);
+    ln_pack_kernel<<<row_grid(n), ROW_WARPS * 32, 0, stream>>>(n, D, vec, in, gamma, (uint16_t*)h, (float2*)row_info);
+    note_launch();
+    INFMOE_CUDA_TRY(cudaGetLastError());
+    return INFMOE_OK;
+}
+
+int launch_split_tiles(const float* src0, const float* src1, int M, int K, float* dst, cudaStream_t stream) {
+    const int MB = (M + 127) / 128, KB = (K + 31) / 32, padded = MB * 128;
+    float* inv = dst + tiled_elems(M, K);
+    uint32_t* bound = (uint32_t*)(dst + split_bound_at(M, K));
+    INFMOE_CUDA_TRY(cudaMemsetAsync(bound, 0, 32 * sizeof(float), stream));
+    const int warps = src1 ? padded / 2 : padded;
+    row_scale_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(src0, src1, M, K, padded, inv, bound);
+    const long long segs = (long long)MB * KB * 128;
+    split_tiles_kernel<<<(unsigned)((segs + 7) / 8), 256, 0, stream>>>(src0, src1, M, K, MB, KB, inv, (uint16_t*)dst);
+    note_launch(2);
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
 }
