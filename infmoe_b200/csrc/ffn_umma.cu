@@ -146,6 +146,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
         : "memory");
 }
+// True for one thread of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -451,29 +457,25 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
     } else if (warp == MMA_WARP) {
         // ================= MMA issuer =================
-        // The whole warp runs the loop so that addresses and descriptors stay warp-uniform; one lane issues the
-        // tcgen05 instructions.
-        uint32_t it = 0, cc = 0;
-        bool ok = true;
-        while (ok && sched.next(item) && !*abort_flag) {
-            const TileInfo t = decode_tile<NMAX>(item.tile, s_prefix, s_order, args);
-            const uint32_t idesc = make_idesc(t.n_pad);
-            for (int c = item.c0; ok && c < item.c1; ++c, ++cc) {
-                const uint32_t acc = cc % C::NACC;
-                const uint32_t d = tmem_base + acc * NMAX;
-                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_acc_empty[acc]), ((cc / C::NACC) & 1) ^ 1, abort_flag))) {
-                    ok = false;
-                    break;
-                }
-                const int kb0 = c * CHUNK_BLOCKS, kb_end = min(KB, kb0 + CHUNK_BLOCKS);
-                for (int kb = kb0; kb < kb_end; ++kb, ++it) {
-                    const uint32_t s = it % STAGES;
-                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[s]), (it / STAGES) & 1, abort_flag))) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    if (lane == 0) {
+        // One elected thread runs the whole loop (elect.sync tells the compiler so).  With the warp running it and lane 0
+        // issuing, the operands of every MMA had to be moved to uniform registers behind a divergent branch: ~148
+        // cycles per MMA whatever its N, which held a decode step of 27 experts at 1694 us of first GEMM where the
+        // same bytes stream in 1269.  Elected: 1259 us (7.2 TB/s); 4096 tokens 2780 -> 2383.
+        if (elect_one()) {
+            uint32_t it = 0, cc = 0;
+            bool ok = true;
+            while (ok && sched.next(item) && !*abort_flag) {
+                const TileInfo t = decode_tile<NMAX>(item.tile, s_prefix, s_order, args);
+                const uint32_t idesc = make_idesc(t.n_pad);
+                for (int c = item.c0; ok && c < item.c1; ++c, ++cc) {
+                    const uint32_t acc = cc % C::NACC;
+                    const uint32_t d = tmem_base + acc * NMAX;
+                    if (!mbar_wait(smem_u32(&s_acc_empty[acc]), ((cc / C::NACC) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                    const int kb0 = c * CHUNK_BLOCKS, kb_end = min(KB, kb0 + CHUNK_BLOCKS);
+                    for (int kb = kb0; kb < kb_end; ++kb, ++it) {
+                        const uint32_t s = it % STAGES;
+                        if (!mbar_wait(smem_u32(&s_full[s]), (it / STAGES) & 1, abort_flag)) { ok = false; break; }
+                        tc_fence_after();
                         const uint64_t dw = make_smem_desc(ring + s * C::STAGE), dx = make_smem_desc(ring + s * C::STAGE + W_TILE);
                         // In a row hi is bytes 0..63, lo bytes 64..127; 32 bytes along K = 2 units of the descriptor
                         // address.  Corrections first (small terms).
@@ -490,6 +492,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 }
             }
         }
+        __syncwarp();
     } else if (warp >= EPI_WARP0) {
         // ================= accumulate + epilogue =================
         // Each chunk is accumulated in TMEM (its first MMA overwrites the accumulator) and added here, with

@@ -479,3 +479,28 @@ def test_enqueue_argument_checks(torch_cuda):
     with pytest.raises(capi.InfMoEError) as e:
         empty.forward_host(np.zeros((2, 8), np.float32))
     assert e.value.status == 8
+
+
+# (tokens, d_model, d_ff) of one expert.  infmoe_t5ff_run never cuts a tile; the layer does when the last round of tiles
+# leaves enough SMs idle: few long tiles (several CTAs to a tile), a K that ends inside a chunk of 256 and inside a block
+# of 32, token tiles of 16, 64 and two of 112 columns, and a tail behind whole rounds.
+@pytest.mark.parametrize("T,D,F", [(1, 4096, 512), (16, 2048, 4096), (5, 600, 2724), (64, 1032, 3000), (210, 1000, 2724),
+                                   (300, 1024, 9600)])
+def test_tiles_cut_along_k_have_the_bits_of_uncut_ones(oracle, T, D, F):
+    import torch
+    from infmoe_b200 import MoELayer
+    from tests import gpu_util as g
+    rng = np.random.default_rng(T + D + F)
+    x = rng.standard_normal((T, D)).astype(np.float32)
+    ln = (1 + 0.01 * rng.standard_normal(D)).astype(np.float32)
+    wi0, wi1 = ((rng.standard_normal((F, D)) / np.sqrt(D)).astype(np.float32) for _ in range(2))
+    wo = (rng.standard_normal((D, F)) / np.sqrt(F)).astype(np.float32)
+    layer = MoELayer.create(1, D, F, 2, np.ones((1, D), np.float32), None, "T5_FF", "default", None)
+    layer.set_expert(0, *(torch.from_numpy(a).cuda() for a in (ln, wi0, wi1, wo)))
+    got = [layer.forward(torch.from_numpy(x).cuda()).cpu().numpy() for _ in range(3)]
+    layer.sync_status()
+    layer.terminate()
+    want = g.t5ff_run(x, ln, wi0, wi1, wo)
+    for out in got:                                # also again: the counters of the cut tiles are back at zero
+        np.testing.assert_array_equal(out, want)
+    assert oracle.rel_l2(want[:4], oracle.expert_ffn_f64(x[:4], ln, wi0, wi1, wo)) <= TOL
