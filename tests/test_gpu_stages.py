@@ -50,6 +50,17 @@ def test_route_bit_exact(g, oracle, T, D, E, ln):
     assert status == 0
 
 
+# The few-token kernel: tokens per cluster (4), experts per CTA and warp (8), a centroid row of one, just under and just
+# over 128 floats, its longest row (12800 floats) and one past it; and the tiled kernels, which now start at
+# T * max(E, 8) = 24576, aligned and unaligned.
+@pytest.mark.parametrize("T,D,E,ln", [(1, 4, 1, False), (3, 127, 7, True), (4, 128, 8, True), (5, 132, 9, False),
+                                      (9, 510, 65, True), (2, 64, 300, True), (6, 12800, 3, True), (6, 12804, 3, True),
+                                      (3071, 36, 8, True), (3072, 36, 8, True), (3100, 510, 5, True),
+                                      (800, 516, 33, False)])
+def test_route_few_and_many_tokens(g, oracle, T, D, E, ln):
+    test_route_bit_exact(g, oracle, T, D, E, ln)
+
+
 def test_route_ties_and_nan(g, oracle):
     x = np.ones((5, 16), np.float32)
     c = np.ones((6, 16), np.float32)
