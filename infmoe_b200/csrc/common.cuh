@@ -134,15 +134,6 @@ __device__ __forceinline__ float ln_apply(float x, float mean, float rstd, float
     return __fmul_rn(gamma, __fmul_rn(__fsub_rn(x, mean), rstd));
 }
 
-// Splits an FP32 value into a TF32-representable head and an FP32 remainder (CUDA-core path):
-// hi = x rounded to 10 mantissa bits (round to nearest, ties away), lo = x - hi (exact).
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-    uint32_t h;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-    hi = __uint_as_float(h);
-    lo = __fsub_rn(x, hi);
-}
-
 // Operand of the tensor-core GEMM: an FP32 value, scaled by a power of two of its row, as a pair of FP16 values,
 // hi = x rounded to 11 significant bits, lo = x - hi rounded to 11 (in the lower / upper half of the word).  |lo| is at
 // most half a unit of hi, so together they hold x to within 2^-23 relative (the last bit of an FP32 value) down to
@@ -155,6 +146,8 @@ __device__ __forceinline__ uint32_t split_f16(float x) {
 // Rows of pairs are stored in 128-byte groups of 32 values: 32 x hi followed by 32 x lo; rows are padded with zeros to
 // a multiple of 32 values.
 __host__ __device__ __forceinline__ size_t pack_pitch(int K) { return (size_t)((K + 31) / 32) * 64; }   // in 16-bit elements
+// Floats of a padded FP32 row (CUDA-core GEMM).
+__host__ __device__ __forceinline__ size_t padded_row(int K) { return (size_t)((K + 31) / 32) * 32; }
 // Stores four consecutive values k0..k0+3 (k0 a multiple of 4) of one row.
 __device__ __forceinline__ void store_pack4(uint16_t* __restrict__ pack_row, int k0, const float v[4]) {
     uint16_t* g = pack_row + (size_t)(k0 >> 5) * 64 + (k0 & 31);

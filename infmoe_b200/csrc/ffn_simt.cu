@@ -1,37 +1,47 @@
 // Exact-FP32 grouped expert FFN on CUDA cores.  This is the path for shapes the
-// tensor-core kernels cannot take (row strides that are not multiples of 16
-// bytes, i.e. d_model or d_ff not divisible by 4) and the cross-check used while
-// validating the tcgen05 kernels on the device.  It is not a fallback for a
-// missing GPU: it runs on the same device from the same buffers.
+// tensor-core kernels cannot take (d_model or d_ff not divisible by 4) and the
+// cross-check used while validating the tcgen05 kernels on the device.  It is not a
+// fallback for a missing GPU: it runs on the same device from the same buffers.
 //
 // Math (T5FFLayer::run, plugin/sublayers/T5FFLayer.cc:112-138), per expert e on
 // its rows [offset[e], offset[e+1]):
-//   g = gelu(h wi_0^T) * (h wi_1^T)        h = h_hi + h_lo (exact recombination)
+//   g = gelu(h wi_0^T) * (h wi_1^T)
 //   y = x + g wo^T
-// Activations are stored as TF32 head/tail planes; head + tail is the original
-// FP32 value exactly, so these kernels compute with full FP32 inputs.  Weights are
-// raw FP32 in the tile-contiguous layout of the tensor-core path; wi_0 and wi_1 share
-// one matrix with interleaved rows (row 2f = wi_0[f], row 2f+1 = wi_1[f]).
+// Activations are FP32 rows padded with zeros to a multiple of 32 values; weights are raw FP32 in tiles of 128 rows x
+// 32 values (launch_retile), wi_0 and wi_1 sharing one matrix with interleaved rows (row 2f = wi_0[f], row
+// 2f+1 = wi_1[f]).  So whatever the widths are, every row of a k block is 128 aligned bytes.
+//
+// Bound by FP32 FMA issue for many rows per expert, by the number of CTAs for few.  A CTA computes 16 RI token rows x 32
+// outputs; a thread RI x 4 (x 2 when both matrices are multiplied) of them.  K blocks of 32 are fetched by 16-byte
+// cp.async into two buffers.  Both operands stay row-major in shared memory at a pitch of 36 floats, and a thread reads
+// four k of a row at a time: 4 + 8 128-bit loads for 128 multiply-adds, without bank conflicts (the eight weight rows a
+// warp reads at once start 4 banks apart; token rows are broadcasts).  Every output is one chain of FMAs in ascending k.
+// Layer of 300 tokens, 6 experts, 510 x 1022: 423 -> 103 us (it was 64 x 64 tiles of scalar loads, one buffer, TF32 head
+// and tail planes added on the fly).
 #include "common.cuh"
+#include "kernels.h"
 
 namespace infmoe {
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
+constexpr int SIMT_THREADS = 128;
+constexpr int TN = 32;       // outputs per CTA
+constexpr int TK = 32;       // one k block of the weight tiles
+constexpr int PITCH = TK + 4;
 
-// Finds the (expert, first row, valid rows) of row-tile `tile` when every expert's
-// rows are tiled separately by TM.  Returns false when `tile` is past the end.
-__device__ bool locate_tile(const int* __restrict__ offset, int e_begin, int e_end, int tile, int& expert,
+// Finds the (expert, first row, valid rows) of row tile `tile` when every expert's rows are tiled separately by `tm`.
+// Returns false when `tile` is past the end.
+__device__ bool locate_tile(const int* __restrict__ offset, int e_begin, int e_end, int tm, int tile, int& expert,
                             int& row0, int& rows) {
     int seen = 0;
     for (int e = e_begin; e < e_end; ++e) {
         const int beg = offset[e], cnt = offset[e + 1] - beg;
-        const int nt = (cnt + TM - 1) / TM;
+        const int nt = (cnt + tm - 1) / tm;
         if (tile < seen + nt) {
             expert = e;
-            row0 = beg + (tile - seen) * TM;
-            rows = min(TM, beg + cnt - row0);
+            row0 = beg + (tile - seen) * tm;
+            rows = min(tm, beg + cnt - row0);
             return true;
         }
         seen += nt;
@@ -39,21 +49,27 @@ __device__ bool locate_tile(const int* __restrict__ offset, int e_begin, int e_e
     return false;
 }
 
-// DUAL = true : out_hi/out_lo[j][n] = split(gelu(A W0^T) * (A W1^T))   (N = d_ff, K = d_model)
-// DUAL = false: out_hi[j][n] = resid[j][n] + A W0^T                      (N = d_model, K = d_ff)
-template <bool DUAL>
-__global__ void __launch_bounds__(256)
-ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, int K,
-                const float* __restrict__ a_hi, const float* __restrict__ a_lo,
+// 16 bytes to shared memory, or zeros
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int bytes = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
+// DUAL = true : out[j][n] = gelu(A W0^T) * (A W1^T), padded rows of N outputs   (N = d_ff, K = d_model)
+// DUAL = false: out[j][n] = resid[j][n] + A W0^T, dense rows                    (N = d_model, K = d_ff)
+template <bool DUAL, int RI>
+__global__ void __launch_bounds__(SIMT_THREADS)
+ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, int K, const float* __restrict__ act,
                 const float* __restrict__ w, const int* __restrict__ slot_of_expert, const float* __restrict__ resid,
-                float* __restrict__ out_hi, float* __restrict__ out_lo) {
-    __shared__ float As[TK][TM + 1];
-    __shared__ float B0s[TK][TN + 1];
-    __shared__ float B1s[DUAL ? TK : 1][TN + 1];
+                float* __restrict__ out) {
+    constexpr int TM = 16 * RI, WROWS = DUAL ? 2 * TN : TN, NB = DUAL ? 2 : 1;
+    __shared__ __align__(16) float As[2][TM][PITCH];
+    __shared__ __align__(16) float Ws[2][WROWS][PITCH];
     __shared__ int s_info[4];
     if (threadIdx.x == 0) {
         int e = 0, r0 = 0, rows = 0;
-        const bool ok = locate_tile(offset, e_begin, e_end, blockIdx.y, e, r0, rows);
+        const bool ok = locate_tile(offset, e_begin, e_end, TM, blockIdx.y, e, r0, rows);
         s_info[0] = ok ? 1 : 0;
         s_info[1] = e;
         s_info[2] = r0;
@@ -63,82 +79,72 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
     if (!s_info[0]) return;
     const int expert = s_info[1], row0 = s_info[2], rows = s_info[3];
     const int slot = slot_of_expert ? slot_of_expert[expert] : expert;
-    const int n0 = blockIdx.x * TN;
-    // tile-contiguous weight plane: 128 x 32 tiles, tile (mb, kb) at (mb * KB + kb) * 4096 floats
-    const int Mw = DUAL ? 2 * N : N, MBw = (Mw + 127) / 128, KBw = (K + 31) / 32;
-    const size_t wbase = (size_t)slot * (size_t)MBw * (size_t)KBw * 4096;
-    auto w_at = [&](int m, int k) -> float {
-        return w[wbase + ((size_t)(m >> 7) * KBw + (k >> 5)) * 4096 + (size_t)(m & 127) * 32 + (k & 31)];
+    const int n0 = blockIdx.x * TN, m0 = NB * n0;    // first output, first weight row (inside one 128-row block)
+    const int KB = (K + TK - 1) / TK, MB = (NB * N + 127) / 128;
+    const float* wt = w + (size_t)slot * (size_t)MB * KB * 4096 + ((size_t)(m0 >> 7) * KB) * 4096 + (size_t)(m0 & 127) * TK;
+    const float* at = act + (size_t)row0 * KB * TK;
+
+    auto fetch = [&](int kb, int buf) {
+        for (int i = threadIdx.x; i < TM * 8; i += SIMT_THREADS) {
+            const int r = i >> 3, c = (i & 7) * 4;
+            const bool valid = r < rows;
+            copy16(&As[buf][r][c], at + (size_t)(valid ? r : 0) * KB * TK + kb * TK + c, valid);
+        }
+        for (int i = threadIdx.x; i < WROWS * 8; i += SIMT_THREADS) {
+            const int r = i >> 3, c = (i & 7) * 4;
+            // wi_0 and wi_1 rows apart, so that neighbouring outputs are neighbouring rows
+            copy16(&Ws[buf][DUAL ? (r & 1) * TN + (r >> 1) : r][c], wt + (size_t)kb * 4096 + r * TK + c, true);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    float acc0[4][4], acc1[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc0[i][j] = acc1[i][j] = 0.f;
-
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        for (int i = threadIdx.x; i < TM * TK; i += 256) {
-            const int r = i / TK, k = i % TK;
-            float v = 0.f;
-            if (r < rows && k0 + k < K) {
-                const size_t o = (size_t)(row0 + r) * K + k0 + k;
-                v = a_hi[o] + a_lo[o];
-            }
-            As[k][r] = v;
-        }
-        for (int i = threadIdx.x; i < TN * TK; i += 256) {
-            const int n = i / TK, k = i % TK;
-            float v0 = 0.f, v1 = 0.f;
-            if (n0 + n < N && k0 + k < K) {
-                if (DUAL) {
-                    v0 = w_at(2 * (n0 + n), k0 + k);
-                    v1 = w_at(2 * (n0 + n) + 1, k0 + k);
-                } else {
-                    v0 = w_at(n0 + n, k0 + k);
-                }
-            }
-            B0s[k][n] = v0;
-            if (DUAL) B1s[k][n] = v1;
+    // token rows ty + 16 i, outputs tx + 8 j
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    float acc[NB][RI][4] = {};
+    fetch(0, 0);
+    for (int kb = 0; kb < KB; ++kb) {
+        const int buf = kb & 1;
+        if (kb + 1 < KB) {
+            fetch(kb + 1, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < TK; ++k) {
-            float a[4], b0[4], b1[4];
+        for (int k = 0; k < TK; k += 4) {
+            float4 a[RI];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
+            for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const float4*>(&As[buf][ty + 16 * i][k]);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                b0[j] = B0s[k][tx * 4 + j];
-                b1[j] = DUAL ? B1s[k][tx * 4 + j] : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int b = 0; b < NB; ++b)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    acc0[i][j] = fmaf(a[i], b0[j], acc0[i][j]);
-                    if (DUAL) acc1[i][j] = fmaf(a[i], b1[j], acc1[i][j]);
+                    const float4 v = *reinterpret_cast<const float4*>(&Ws[buf][b * TN + tx + 8 * j][k]);
+#pragma unroll
+                    for (int i = 0; i < RI; ++i) {
+                        float s = acc[b][i][j];
+                        s = fmaf(a[i].x, v.x, s);
+                        s = fmaf(a[i].y, v.y, s);
+                        s = fmaf(a[i].z, v.z, s);
+                        acc[b][i][j] = fmaf(a[i].w, v.w, s);
+                    }
                 }
         }
-        __syncthreads();
+        __syncthreads();    // the next round's fetch refills this buffer
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = ty * 4 + i;
+    for (int i = 0; i < RI; ++i) {
+        const int r = ty + 16 * i;
         if (r >= rows) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n >= N) continue;
-            const size_t o = (size_t)(row0 + r) * N + n;
-            if (DUAL) {
-                float hi, lo;
-                split_tf32(gelu_dot(acc0[i][j], acc1[i][j]), hi, lo);
-                out_hi[o] = hi;
-                out_lo[o] = lo;
-            } else {
-                out_hi[o] = resid[o] + acc0[i][j];
+            const int n = n0 + tx + 8 * j;
+            if (DUAL) {     // outputs past N are products of zero weights: the zeros the next GEMM's padding needs
+                out[(size_t)(row0 + r) * padded_row(N) + n] = gelu_dot(acc[0][i][j], acc[NB - 1][i][j]);
+            } else if (n < N) {
+                const size_t o = (size_t)(row0 + r) * N + n;
+                out[o] = resid[o] + acc[0][i][j];
             }
         }
     }
@@ -147,18 +153,22 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
 }  // namespace
 
 // Grouped FFN over experts [e_begin, e_end); T rows in expert-contiguous order.
-//   h_hi/h_lo [T][D], g_hi/g_lo [T][F] (scratch), routed [T][D], post [T][D]
+//   h [T][padded_row(D)], g [T][padded_row(F)] (scratch), routed [T][D], post [T][D]
 //   slot_of_expert (device, may be NULL = identity) maps expert -> weight slot.
 int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int* offset, const int* slot_of_expert,
-                    const float* h_hi, const float* h_lo, const float* w01, const float* wo, const float* routed,
-                    float* g_hi, float* g_lo, float* post, cudaStream_t stream) {
+                    const float* h, const float* w01, const float* wo, const float* routed, float* g, float* post,
+                    cudaStream_t stream) {
     if (T == 0 || e_begin >= e_end) return INFMOE_OK;
-    const unsigned row_tiles = (unsigned)((T + TM - 1) / TM + (e_end - e_begin));
-    dim3 g1((F + TN - 1) / TN, row_tiles), g2((D + TN - 1) / TN, row_tiles);
-    ffn_simt_kernel<true><<<g1, 256, 0, stream>>>(offset, e_begin, e_end, F, D, h_hi, h_lo, w01, slot_of_expert,
-                                                  nullptr, g_hi, g_lo);
-    ffn_simt_kernel<false><<<g2, 256, 0, stream>>>(offset, e_begin, e_end, D, F, g_hi, g_lo, wo, slot_of_expert,
-                                                   routed, post, nullptr);
+    const int experts = e_end - e_begin;
+    // 16-row tiles when an expert has about that many rows at most: a 64-row tile would multiply zeros
+    const bool few = T <= 16ll * experts;
+    const int tm = few ? 16 : 64;
+    const unsigned row_tiles = (unsigned)((T + tm - 1) / tm + experts);
+    const dim3 g1((F + TN - 1) / TN, row_tiles), g2((D + TN - 1) / TN, row_tiles);
+    auto k1 = few ? ffn_simt_kernel<true, 1> : ffn_simt_kernel<true, 4>;
+    auto k2 = few ? ffn_simt_kernel<false, 1> : ffn_simt_kernel<false, 4>;
+    k1<<<g1, SIMT_THREADS, 0, stream>>>(offset, e_begin, e_end, F, D, h, w01, slot_of_expert, nullptr, g);
+    k2<<<g2, SIMT_THREADS, 0, stream>>>(offset, e_begin, e_end, D, F, g, wo, slot_of_expert, routed, post);
     note_launch(2);
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

@@ -23,10 +23,10 @@ int launch_scatter(long long T, int D, const float* X, const float* coeff, const
                    float* rcoeff, cudaStream_t stream);
 // valid_rows (device, may be NULL): rows at or past *valid_rows are skipped (tokens without an expert sit at
 // the tail of pos[]; the dispatch kernel stores their start in offset[E]).
-// CUDA-core GEMM: routed rows and FP32 head / tail planes of the LayerNorm output.
-int launch_scatter_ln_split(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
-                            const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h_hi,
-                            float* h_lo, cudaStream_t stream);
+// CUDA-core GEMM: routed rows and the LayerNorm output h, rows padded with zeros to padded_row(D) floats.
+int launch_scatter_ln_rows(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
+                           const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h,
+                           cudaStream_t stream);
 // Tensor-core GEMM: packed FP16-pair plane `h` (pack_bytes) and two floats per row in row_info (token_row_info).
 int launch_scatter_ln_pack(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
                            const float* gamma_all, const int* valid_rows, float* rscore, void* h, float* row_info,
@@ -37,7 +37,6 @@ int launch_mix_gather(long long T, int D, const int* pos, const float* routed, c
                       const float* coeff, float* out, cudaStream_t stream, const int* valid_rows = nullptr);
 int launch_layernorm(float* out, const float* in, long long n, int D, const float* gamma, cudaStream_t stream);
 int launch_gelu_dot(const float* a, float* b, size_t len, cudaStream_t stream);
-int launch_split(const float* src, float* hi, float* lo, size_t len, cudaStream_t stream);
 int launch_fill_int(int* dst, int value, cudaStream_t stream);   // *dst = value, stream ordered
 // Tile-contiguous weight layouts (see rows.cu); src1 != NULL interleaves the rows of two matrices.
 //   launch_retile       raw FP32 tiles, for the CUDA-core GEMM (tiled_elems floats)
@@ -48,20 +47,19 @@ int launch_split_tiles(const float* src0, const float* src1, int M, int K, float
 inline size_t tiled_elems(int M, int K) { return (size_t)((M + 127) / 128) * 128 * (size_t)((K + 31) / 32) * 32; }
 inline size_t split_bound_at(int M, int K) { return tiled_elems(M, K) + (size_t)((M + 127) / 128) * 128; }
 inline size_t split_plane_elems(int M, int K) { return split_bound_at(M, K) + 32; }
-// h = LN(x; gamma) for rows already in place, as launch_scatter_ln_split / _pack write it.
-int launch_ln_split(long long n, int D, const float* in, const float* gamma, float* h_hi, float* h_lo,
-                    cudaStream_t stream);
+// h = LN(x; gamma) for rows already in place, as launch_scatter_ln_rows / _pack write it.
+int launch_ln_rows(long long n, int D, const float* in, const float* gamma, float* h, cudaStream_t stream);
 int launch_ln_pack(long long n, int D, const float* in, const float* gamma, void* h, float* row_info,
                    cudaStream_t stream);
-// Bytes of a packed FP16-pair plane [rows][K] (rows padded to whole groups of 32 values).
+// Bytes of an activation plane [rows][K], FP16 pairs or FP32 (rows padded to whole groups of 32 values).
 inline size_t pack_bytes(long long rows, int K) { return (size_t)rows * (size_t)((K + 31) / 32) * 128; }
 
 // CUDA-core GEMM.  Expert weights live in two raw FP32 planes in tile-contiguous layout (128 x 32 tiles):
 // w01 [slots] x tiled(2F x D) (row 2f = wi_0[f], row 2f+1 = wi_1[f]) and wo [slots] x tiled(D x F).
-// Activations travel as two FP32 planes: hi = value rounded to TF32, lo = value - hi.
+// Activations h [T][padded_row(D)] and g [T][padded_row(F)] are FP32 (pack_bytes).
 int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int* offset, const int* slot_of_expert,
-                    const float* h_hi, const float* h_lo, const float* w01, const float* wo, const float* routed,
-                    float* g_hi, float* g_lo, float* post, cudaStream_t stream);
+                    const float* h, const float* w01, const float* wo, const float* routed, float* g, float* post,
+                    cudaStream_t stream);
 
 // A one-warp kernel that waits, with the GEMM's bounded wait and the given limit, on a barrier nobody completes.
 int launch_wait_probe(unsigned long long limit_ns, int* status, unsigned long long* waited_ns, cudaStream_t stream);

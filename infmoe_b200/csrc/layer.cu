@@ -112,7 +112,7 @@ struct ExpertStore {
 };
 
 struct WsLayout {
-    size_t gate, pos, count, offset, slot_map, score, rscore, routed, post, h_hi, h_lo, g_hi, g_lo, row_info, part, part_count, slots,
+    size_t gate, pos, count, offset, slot_map, score, rscore, routed, post, h, g, row_info, part, part_count, slots,
         custom_slots, custom_ws, total;
     size_t part_bytes;
 };
@@ -247,12 +247,10 @@ WsLayout ws_layout(const infmoe_layer* L, long long T, bool streamed) {
     const bool row_planes = L->identity || L->custom || !uses_umma(L);
     w.routed = take(row_planes ? 4 * t * D : 0);
     w.post = take(row_planes ? 4 * t * D : 0);
-    // activations: one packed plane each on the tensor-core path (h_lo / g_lo stay empty), FP32 head and tail planes
-    // on the CUDA-core path
-    w.h_hi = take(row_planes ? 4 * t * D : pack_bytes((long long)t, L->D));
-    w.h_lo = take(row_planes ? 4 * t * D : 0);
-    w.g_hi = take(row_planes ? 4 * t * F : pack_bytes((long long)t, L->F));
-    w.g_lo = take(row_planes ? 4 * t * F : 0);
+    // activations: FP16 pairs on the tensor-core path, FP32 on the CUDA-core path (where `g` also serves as a [T][D]
+    // buffer when the result goes to per-row addresses)
+    w.h = take(pack_bytes((long long)t, L->D));
+    w.g = take(row_planes && D > F ? pack_bytes((long long)t, L->D) : pack_bytes((long long)t, L->F));
     w.row_info = take(row_planes ? 0 : 8 * t);
     w.part_bytes = row_planes ? 0 : ffn_umma_part_bytes((long long)t, L->D, L->F);
     w.part = take(w.part_bytes);
@@ -432,7 +430,7 @@ struct FfnOutput {
 
 // Workspace pieces the experts work in.
 struct FfnBuffers {
-    float *h_hi, *h_lo, *g_hi, *g_lo;   // tensor-core path: packed planes in h_hi / g_hi
+    float *h, *g;                       // FP16 pairs (tensor-core path) or FP32 (CUDA-core path)
     float* row_info;
     void* part;
     size_t part_bytes;
@@ -449,9 +447,9 @@ int run_ffn(infmoe_layer* L, long long T, int e_begin, int e_end, const int* d_o
         f.slots = slots;
         f.w01 = planes[0];
         f.wo = planes[1];
-        f.h = w.h_hi;
+        f.h = w.h;
         f.row_info = w.row_info;
-        f.g = w.g_hi;
+        f.g = w.g;
         f.resid = routed;
         f.out = o.out ? o.out : o.post;
         f.out_pos = o.out ? o.pos : nullptr;
@@ -463,8 +461,8 @@ int run_ffn(infmoe_layer* L, long long T, int e_begin, int e_end, const int* d_o
         f.status = L->d_status;
         return launch_ffn_umma(f, T, L->D, L->F, L->E, e_begin, e_end, L->num_sms, stream, mid);
     }
-    return launch_ffn_simt(T, L->D, L->F, e_begin, e_end, d_offset, d_slot_map, w.h_hi, w.h_lo, planes[0], planes[1],
-                           routed, w.g_hi, w.g_lo, o.post, stream);
+    return launch_ffn_simt(T, L->D, L->F, e_begin, e_end, d_offset, d_slot_map, w.h, planes[0], planes[1], routed, w.g,
+                           o.post, stream);
 }
 
 void free_device_state(infmoe_layer* L) {
@@ -1051,10 +1049,8 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     float* routed = (float*)(base + w.routed);
     float* post = (float*)(base + w.post);
     FfnBuffers buf;
-    buf.h_hi = (float*)(base + w.h_hi);
-    buf.h_lo = (float*)(base + w.h_lo);
-    buf.g_hi = (float*)(base + w.g_hi);
-    buf.g_lo = (float*)(base + w.g_lo);
+    buf.h = (float*)(base + w.h);
+    buf.g = (float*)(base + w.g);
     buf.row_info = (float*)(base + w.row_info);
     buf.part = w.part_bytes ? base + w.part : nullptr;
     buf.part_bytes = w.part_bytes;
@@ -1144,12 +1140,12 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
         const bool pack = uses_umma(L);   // the GEMM run_ffn picks
         // tensor-core path: no routed copy, the second GEMM's epilogue reads its residual from d_in through pos[]
         if (pack) {
-            INFMOE_TRY(launch_scatter_ln_pack(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, rscore, buf.h_hi,
+            INFMOE_TRY(launch_scatter_ln_pack(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, rscore, buf.h,
                                               buf.row_info, stream));
             routed = const_cast<float*>(d_in);   // run_ffn's residual operand
         } else {
-            INFMOE_TRY(launch_scatter_ln_split(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, routed, rscore,
-                                               buf.h_hi, buf.h_lo, stream));
+            INFMOE_TRY(launch_scatter_ln_rows(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, routed, rscore,
+                                              buf.h, stream));
         }
         INFMOE_TRY(prof_mark(L, 3, stream));
         // 4. experts (:360-402)
@@ -1239,9 +1235,8 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     // 5. combine (:407-412; the gather reads the expert output), unless the GEMM epilogue has done it
     if (fused_combine) {
     } else {
-        // with per-row addresses the rows are first combined in the caller's row order (g_hi is free by now:
-        // T x d_ff floats), then copied out
-        float* ordered = row_dst ? buf.g_hi : d_out;
+        // with per-row addresses the rows are first combined in the caller's row order (g is free by now), then copied out
+        float* ordered = row_dst ? buf.g : d_out;
         if (mix)
             INFMOE_TRY(launch_mix_gather(T, L->D, pos, routed, post, rscore, ordered, stream, valid_rows));
         else
@@ -1800,7 +1795,7 @@ namespace {
 // returns the device-side status.
 int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_w, const float* wi0, const float* wi1,
                 const float* wo, const float* x, float* y, cudaStream_t stream) {
-    const size_t r = (size_t)rows, d = (size_t)D, f = (size_t)F;
+    const size_t r = (size_t)rows;
     char* p = base;
     auto take = [&](size_t bytes) {
         char* at = p;
@@ -1809,10 +1804,8 @@ int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_
     };
     const char* path = getenv("INFMOE_FFN");
     const bool simt = (path && strcmp(path, "simt") == 0) || !ffn_umma_supported(D, F, 1);
-    float* h_hi = (float*)take(simt ? 4 * r * d : pack_bytes(rows, D));
-    float* h_lo = (float*)take(simt ? 4 * r * d : 0);
-    float* g_hi = (float*)take(simt ? 4 * r * f : pack_bytes(rows, F));
-    float* g_lo = (float*)take(simt ? 4 * r * f : 0);
+    float* h = (float*)take(pack_bytes(rows, D));
+    float* g = (float*)take(pack_bytes(rows, F));
     float* row_info = (float*)take(simt ? 0 : 8 * r);
     float* planes[2];
     planes[0] = (float*)take(4 * (simt ? tiled_elems(2 * F, D) : split_plane_elems(2 * F, D)));
@@ -1823,24 +1816,23 @@ int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_
     INFMOE_CUDA_TRY(cudaMemsetAsync(offset, 0, 4, stream));
     INFMOE_TRY(launch_fill_int(offset + 1, (int)rows, stream));
     INFMOE_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), stream));
-    if (simt) INFMOE_TRY(launch_ln_split(rows, D, x, ln_w, h_hi, h_lo, stream));
-    else INFMOE_TRY(launch_ln_pack(rows, D, x, ln_w, h_hi, row_info, stream));
+    if (simt) INFMOE_TRY(launch_ln_rows(rows, D, x, ln_w, h, stream));
+    else INFMOE_TRY(launch_ln_pack(rows, D, x, ln_w, h, row_info, stream));
     INFMOE_TRY(load_expert_planes(!simt, D, F, wi0, wi1, wo, planes[0], planes[1], false, nullptr, stream));
     int dev = 0, sms = 0;
     INFMOE_CUDA_TRY(cudaGetDevice(&dev));
     INFMOE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (simt) {
-        INFMOE_TRY(launch_ffn_simt(rows, D, F, 0, 1, offset, nullptr, h_hi, h_lo, planes[0], planes[1], x, g_hi, g_lo,
-                                   y, stream));
+        INFMOE_TRY(launch_ffn_simt(rows, D, F, 0, 1, offset, nullptr, h, planes[0], planes[1], x, g, y, stream));
     } else {
         FfnUmma u{};
         u.offset = offset;
         u.slots = 1;
         u.w01 = planes[0];
         u.wo = planes[1];
-        u.h = h_hi;
+        u.h = h;
         u.row_info = row_info;
-        u.g = g_hi;
+        u.g = g;
         u.resid = x;
         u.out = y;
         u.status = status;
@@ -1855,8 +1847,8 @@ int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_
 }  // namespace
 
 namespace {
-// Scratch of the CUDA-core form, the larger one but for the row scales and row_info of the tensor-core form (which
-// are at most 2 MB beside a scratch of 32 MB: 512 bytes per 128-row weight block, which has at least one 16 KB tile).
+// Scratch measure: two FP32 planes each of h and g and the weight tiles, more than either form needs but for the row scales and row_info of the tensor-core form (which are at most
+// 2 MB beside a scratch of 32 MB: 512 bytes per 128-row weight block, which has at least one 16 KB tile).
 // It is also the measure of what infmoe_t5ff_run_static takes.
 size_t t5ff_scratch_bytes(int64_t rows, int32_t D, int32_t F) {
     const size_t r = (size_t)rows, d = (size_t)D, f = (size_t)F;

@@ -45,43 +45,39 @@ scatter_kernel(long long T, int D, int vec, const float* __restrict__ X, const f
 // for the grouped GEMM.  gamma is [E][D]; the expert of row j is gate[pos[j]].  Rows at or past *valid_rows (tokens
 // without an expert, empty receive slots) are skipped.
 //
-// For the CUDA-core GEMM: the routed row, the routed score, and TF32 head and FP32 tail planes h_hi / h_lo [T][D].
+// For the CUDA-core GEMM: the routed row, the routed score, and h in FP32, rows padded with zeros to whole groups of 32.
+__device__ __forceinline__ void warp_ln_rows(const float* __restrict__ src, const float* __restrict__ gamma, int D,
+                                             bool vec, float* __restrict__ routed, float* __restrict__ h) {
+    const int lane = threadIdx.x & 31;
+    float mean, rstd;
+    warp_row_stats(src, D, vec, mean, rstd);
+    for (int base = 4 * lane; base < (int)padded_row(D); base += 128) {
+        float hh[4] = {0.f, 0.f, 0.f, 0.f};
+        if (base < D) {
+            const float4 v = load_row4(src, base, D, vec), g = load_row4(gamma, base, D, vec);
+            const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (base + k < D) {
+                    hh[k] = ln_apply(vv[k], mean, rstd, gg[k]);
+                    if (routed) routed[base + k] = vv[k];
+                }
+        }
+        *reinterpret_cast<float4*>(h + base) = make_float4(hh[0], hh[1], hh[2], hh[3]);
+    }
+}
+
 __global__ void __launch_bounds__(ROW_WARPS * 32)
-scatter_ln_split_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ score,
-                        const int* __restrict__ pos, const int* __restrict__ gate,
-                        const float* __restrict__ gamma_all, const int* __restrict__ valid_rows,
-                        float* __restrict__ routed, float* __restrict__ rscore, float* __restrict__ h_hi,
-                        float* __restrict__ h_lo) {
+scatter_ln_rows_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ score,
+                       const int* __restrict__ pos, const int* __restrict__ gate, const float* __restrict__ gamma_all,
+                       const int* __restrict__ valid_rows, float* __restrict__ routed, float* __restrict__ rscore,
+                       float* __restrict__ h) {
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;
     const int p = pos[j];
-    const int e = gate[p];
-    const float* src = X + (long long)p * D;
-    const float* gamma = gamma_all + (long long)e * D;
-    float mean, rstd;
-    warp_row_stats(src, D, vec != 0, mean, rstd);
-    for (int base = 4 * lane; base < D; base += 128) {
-        float hh[4] = {0.f, 0.f, 0.f, 0.f}, ll[4] = {0.f, 0.f, 0.f, 0.f};
-        const float4 v = load_row4(src, base, D, vec != 0);
-        const float4 g = load_row4(gamma, base, D, vec != 0);
-        const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (base + k < D) split_tf32(ln_apply(vv[k], mean, rstd, gg[k]), hh[k], ll[k]);
-        const long long o = j * D + base;
-        if (vec) {
-            *reinterpret_cast<float4*>(routed + o) = v;
-            *reinterpret_cast<float4*>(h_hi + o) = make_float4(hh[0], hh[1], hh[2], hh[3]);
-            *reinterpret_cast<float4*>(h_lo + o) = make_float4(ll[0], ll[1], ll[2], ll[3]);
-        } else {
-            for (int k = 0; k < 4 && base + k < D; ++k) {
-                routed[o + k] = vv[k];
-                h_hi[o + k] = hh[k];
-                h_lo[o + k] = ll[k];
-            }
-        }
-    }
+    warp_ln_rows(X + (long long)p * D, gamma_all + (long long)gate[p] * D, D, vec != 0, routed + j * D,
+                 h + j * (long long)padded_row(D));
     if (lane == 0 && rscore && score) rscore[j] = score[p];
 }
 
@@ -292,21 +288,11 @@ layernorm_kernel(long long n, int D, int vec, const float* __restrict__ in, cons
 
 // h = LN(x; gamma) for rows already in place, as the scatter kernels write it.
 __global__ void __launch_bounds__(ROW_WARPS * 32)
-ln_split_kernel(long long n, int D, int vec, const float* __restrict__ in, const float* __restrict__ gamma,
-                float* __restrict__ h_hi, float* __restrict__ h_lo) {
-    const int lane = threadIdx.x & 31;
+ln_rows_kernel(long long n, int D, int vec, const float* __restrict__ in, const float* __restrict__ gamma,
+               float* __restrict__ h) {
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= n) return;
-    const float* src = in + j * D;
-    float mean, rstd;
-    warp_row_stats(src, D, vec != 0, mean, rstd);
-    for (int base = 4 * lane; base < D; base += 128) {
-        const float4 v = load_row4(src, base, D, vec != 0);
-        const float4 g = load_row4(gamma, base, D, vec != 0);
-        const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
-        for (int k = 0; k < 4 && base + k < D; ++k)
-            split_tf32(ln_apply(vv[k], mean, rstd, gg[k]), h_hi[j * D + base + k], h_lo[j * D + base + k]);
-    }
+    warp_ln_rows(in + j * D, gamma, D, vec != 0, nullptr, h + j * (long long)padded_row(D));
 }
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 ln_pack_kernel(long long n, int D, int vec, const float* __restrict__ in, const float* __restrict__ gamma,
@@ -319,24 +305,6 @@ ln_pack_kernel(long long n, int D, int vec, const float* __restrict__ in, const 
 __global__ void gelu_dot_kernel(const float* __restrict__ a, float* __restrict__ b, size_t len) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += stride) b[i] = gelu_dot(a[i], b[i]);
-}
-
-// hi/lo planes of a raw FP32 array (weights at load time).
-__global__ void split_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo,
-                             size_t len4, size_t len) {
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < len4; i += stride) {
-        const float4 v = reinterpret_cast<const float4*>(src)[i];
-        float4 h, l;
-        split_tf32(v.x, h.x, l.x);
-        split_tf32(v.y, h.y, l.y);
-        split_tf32(v.z, h.z, l.z);
-        split_tf32(v.w, h.w, l.w);
-        reinterpret_cast<float4*>(hi)[i] = h;
-        reinterpret_cast<float4*>(lo)[i] = l;
-    }
-    for (size_t i = len4 * 4 + (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += stride)
-        split_tf32(src[i], hi[i], lo[i]);
 }
 
 // Weight matrix -> tile-contiguous layout: tiles of 128 rows x 32 values (16 KB),
@@ -439,14 +407,13 @@ int launch_scatter(long long T, int D, const float* X, const float* coeff, const
     return INFMOE_OK;
 }
 
-int launch_scatter_ln_split(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
-                            const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h_hi,
-                            float* h_lo, cudaStream_t stream) {
+int launch_scatter_ln_rows(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
+                           const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h,
+                           cudaStream_t stream) {
     if (T == 0) return INFMOE_OK;
-    const int vec = (D % 4 == 0) && aligned16(X) && aligned16(routed) && aligned16(h_hi) && aligned16(h_lo) &&
-                    aligned16(gamma_all);
-    scatter_ln_split_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, X, score, pos, gate, gamma_all,
-                                                                        valid_rows, routed, rscore, h_hi, h_lo);
+    const int vec = (D % 4 == 0) && aligned16(X) && aligned16(gamma_all);
+    scatter_ln_rows_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, X, score, pos, gate, gamma_all,
+                                                                       valid_rows, routed, rscore, h);
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
@@ -554,11 +521,10 @@ int launch_layernorm(float* out, const float* in, long long n, int D, const floa
     return INFMOE_OK;
 }
 
-int launch_ln_split(long long n, int D, const float* in, const float* gamma, float* h_hi, float* h_lo,
-                    cudaStream_t stream) {
+int launch_ln_rows(long long n, int D, const float* in, const float* gamma, float* h, cudaStream_t stream) {
     if (n == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && aligned16(in) && aligned16(gamma);
-    ln_split_kernel<<<row_grid(n), ROW_WARPS * 32, 0, stream>>>(n, D, vec, in, gamma, h_hi, h_lo);
+    ln_rows_kernel<<<row_grid(n), ROW_WARPS * 32, 0, stream>>>(n, D, vec, in, gamma, h);
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
@@ -616,18 +582,6 @@ __global__ void fill_int_kernel(int* dst, int value) { *dst = value; }
 
 int launch_fill_int(int* dst, int value, cudaStream_t stream) {
     fill_int_kernel<<<1, 1, 0, stream>>>(dst, value);
-    note_launch();
-    INFMOE_CUDA_TRY(cudaGetLastError());
-    return INFMOE_OK;
-}
-
-int launch_split(const float* src, float* hi, float* lo, size_t len, cudaStream_t stream) {
-    if (len == 0) return INFMOE_OK;
-    const bool vec = aligned16(src) && aligned16(hi) && aligned16(lo);
-    const size_t len4 = vec ? len / 4 : 0;
-    const size_t work = len4 ? len4 : len;
-    const unsigned grid = (unsigned)((work + 255) / 256 < 148 * 16 ? (work + 255) / 256 : 148 * 16);
-    split_kernel<<<grid, 256, 0, stream>>>(src, hi, lo, len4, len);
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

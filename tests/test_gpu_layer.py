@@ -504,3 +504,31 @@ def test_tiles_cut_along_k_have_the_bits_of_uncut_ones(oracle, T, D, F):
     for out in got:                                # also again: the counters of the cut tiles are back at zero
         np.testing.assert_array_equal(out, want)
     assert oracle.rel_l2(want[:4], oracle.expert_ffn_f64(x[:4], ln, wi0, wi1, wo)) <= TOL
+
+
+# CUDA-core GEMM: experts with 0, 1, 15 .. 17 and 63 .. 65 rows (its tiles are 16 rows high when the experts have at most
+# 16 on average, else 64), widths inside, at and past a block of 32 and a 128-row weight block.
+@pytest.mark.parametrize("counts", [(1, 0, 15, 16, 17), (63, 64, 65, 0, 1, 130)])
+@pytest.mark.parametrize("D,F", [(510, 1022), (33, 63), (6, 5), (129, 257)])
+def test_cuda_core_experts_against_oracle(oracle, counts, D, F):
+    import torch
+    from infmoe_b200 import MoELayer
+    rng = np.random.default_rng(D + F + len(counts))
+    E, n = len(counts), sum(counts)
+    layer = MoELayer.create(E, D, F, 2, np.ones((E, D), np.float32), None, "T5_FF", "default", None)
+    experts = []
+    for e in range(E):
+        experts.append([(1 + 0.01 * rng.standard_normal(D)).astype(np.float32)] +
+                       [(rng.standard_normal((F, D)) / np.sqrt(D)).astype(np.float32) for _ in range(2)] +
+                       [(rng.standard_normal((D, F)) / np.sqrt(F)).astype(np.float32)])
+        layer.set_expert(e, *(torch.from_numpy(a).cuda() for a in experts[e]))
+    gate = rng.permutation(np.repeat(np.arange(E, dtype=np.int32), counts))
+    x = rng.standard_normal((n, D)).astype(np.float32)
+    out = layer.expert_forward(torch.from_numpy(x).cuda(), torch.from_numpy(gate).cuda()).cpu().numpy()
+    layer.sync_status()
+    layer.terminate()
+    for e in range(E):
+        rows = gate == e
+        if rows.any():
+            want = oracle.expert_ffn_f64(x[rows], *experts[e])
+            assert oracle.rel_l2(out[rows] - x[rows], want - x[rows]) <= 2e-6   # FP32 chains of up to 1022 adds
