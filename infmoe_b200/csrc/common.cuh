@@ -47,6 +47,37 @@ extern long long g_kernel_launches;
 inline void note_launch(int n = 1) { g_kernel_launches += n; }
 
 #ifdef __CUDACC__
+// Launches a kernel that begins with pdl_wait (see there); cluster > 1: in clusters of that many blocks.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsigned threads, size_t smem, unsigned cluster,
+                                  cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, Params(args)...);
+}
+
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch.  The kernels of a pass are short next to the time between two dependent launches
+// (1-2 us on an idle GPU), so each is launched while its predecessor still runs (launch_chained): its blocks start as
+// soon as every block of the predecessor has started (pdl_trigger) and left room, do what needs no memory, and wait
+// in pdl_wait until the predecessor has completed and its writes are visible.  Every block of every kernel launched
+// this way calls pdl_wait before it touches global memory; the predecessor did the same, so all earlier kernels of the
+// stream are complete too.  (Without the launch attribute both are no-ops.)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // Canonical FP32 reductions.  Routing must agree bit for bit with the CPU
 // checker, so the summation order is fixed: lane l of a warp owns elements

@@ -84,6 +84,8 @@ dispatch_kernel(const int* __restrict__ gate, long long T, int E, const int* __r
     };
 
     for (int e = tid; e < B; e += DISPATCH_THREADS) s_count[e] = 0;
+    pdl_trigger();
+    pdl_wait();
     if (r == 0)
         for (int i = tid; i < zero_count; i += DISPATCH_THREADS) zero[i] = 0;
     __syncthreads();
@@ -173,6 +175,8 @@ dispatch_kernel(const int* __restrict__ gate, long long T, int E, const int* __r
 
 size_t dispatch_smem_bytes(int E) { return sizeof(int) * (size_t)DISPATCH_TABLES * (size_t)(E + 1); }
 
+bool dispatch_supported(int E) { return dispatch_smem_bytes(E) <= 200 * 1024; }
+
 int launch_dispatch(const int* gate, long long T, int E, int* pos, int* count, int* offset, int* status,
                     cudaStream_t stream, const int* region_count, int region_size, int* zero, int zero_count) {
     if (T < 0 || T > 0x7fffffffLL || E <= 0 || (T > 0 && (!gate || !pos)) || !count || !offset ||
@@ -181,7 +185,7 @@ int launch_dispatch(const int* gate, long long T, int E, int* pos, int* count, i
         return INFMOE_ERR_INVALID_ARGUMENT;
     }
     const size_t smem = dispatch_smem_bytes(E);
-    if (smem > 200 * 1024) {
+    if (!dispatch_supported(E)) {
         set_error("expert_count: expert_count %d exceeds the dispatch kernel's shared-memory limit", E);
         return INFMOE_ERR_UNSUPPORTED;
     }
@@ -196,20 +200,9 @@ int launch_dispatch(const int* gate, long long T, int E, int* pos, int* count, i
         return v ? atoi(v) : 0;
     }();
     if (forced == 1 || forced == 2 || forced == 4 || forced == 8) cluster = forced;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)cluster);
-    cfg.blockDim = dim3(DISPATCH_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    INFMOE_CUDA_TRY(cudaLaunchKernelEx(&cfg, dispatch_kernel, gate, T, E, region_count, region_size, pos, count, offset,
-                                       status, zero, zero ? zero_count : 0));
+    INFMOE_CUDA_TRY(launch_chained(dispatch_kernel, (unsigned)cluster, DISPATCH_THREADS, smem, (unsigned)cluster, stream,
+                                   gate, T, E, region_count, region_size, pos, count, offset, status, zero,
+                                   zero ? zero_count : 0));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

@@ -63,13 +63,14 @@ __global__ void __launch_bounds__(SIMT_THREADS)
 ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, int K, const float* __restrict__ act,
                 const float* __restrict__ w, const int* __restrict__ slot_of_expert, const float* __restrict__ resid,
                 float* __restrict__ out) {
+    const unsigned n_tiles = (unsigned)(N + TN - 1) / TN;     // grid: row tile major
     constexpr int TM = 16 * RI, WROWS = DUAL ? 2 * TN : TN, NB = DUAL ? 2 : 1;
     __shared__ __align__(16) float As[2][TM][PITCH];
     __shared__ __align__(16) float Ws[2][WROWS][PITCH];
     __shared__ int s_info[4];
     if (threadIdx.x == 0) {
         int e = 0, r0 = 0, rows = 0;
-        const bool ok = locate_tile(offset, e_begin, e_end, TM, blockIdx.y, e, r0, rows);
+        const bool ok = locate_tile(offset, e_begin, e_end, TM, blockIdx.x / n_tiles, e, r0, rows);
         s_info[0] = ok ? 1 : 0;
         s_info[1] = e;
         s_info[2] = r0;
@@ -79,7 +80,7 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
     if (!s_info[0]) return;
     const int expert = s_info[1], row0 = s_info[2], rows = s_info[3];
     const int slot = slot_of_expert ? slot_of_expert[expert] : expert;
-    const int n0 = blockIdx.x * TN, m0 = NB * n0;    // first output, first weight row (inside one 128-row block)
+    const int n0 = (int)(blockIdx.x % n_tiles) * TN, m0 = NB * n0;    // first output, first weight row (inside one 128-row block)
     const int KB = (K + TK - 1) / TK, MB = (NB * N + 127) / 128;
     const float* wt = w + (size_t)slot * (size_t)MB * KB * 4096 + ((size_t)(m0 >> 7) * KB) * 4096 + (size_t)(m0 & 127) * TK;
     const float* at = act + (size_t)row0 * KB * TK;
@@ -164,9 +165,11 @@ int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int
     const bool few = T <= 16ll * experts;
     const int tm = few ? 16 : 64;
     const unsigned row_tiles = (unsigned)((T + tm - 1) / tm + experts);
-    const dim3 g1((F + TN - 1) / TN, row_tiles), g2((D + TN - 1) / TN, row_tiles);
+    const unsigned g1 = (unsigned)((F + TN - 1) / TN) * row_tiles, g2 = (unsigned)((D + TN - 1) / TN) * row_tiles;
     auto k1 = few ? ffn_simt_kernel<true, 1> : ffn_simt_kernel<true, 4>;
     auto k2 = few ? ffn_simt_kernel<false, 1> : ffn_simt_kernel<false, 4>;
+    // Not chained (launch_chained): blocks put on the SMs while those of the kernel before are still there crowd on the
+    // idle ones, and there are only a few per SM.  The pass of 300 tokens took 195 us so, 126 with a late trigger.
     k1<<<g1, SIMT_THREADS, 0, stream>>>(offset, e_begin, e_end, F, D, h, w01, slot_of_expert, nullptr, g);
     k2<<<g2, SIMT_THREADS, 0, stream>>>(offset, e_begin, e_end, D, F, g, wo, slot_of_expert, routed, post);
     note_launch(2);

@@ -371,6 +371,27 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int MB = (args.M_total + UMMA_M - 1) / UMMA_M;
     const int KB = (args.K + BK - 1) / BK;
 
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(smem_u32(&s_full[s]), 1);
+            mbar_init(smem_u32(&s_empty[s]), 1);
+        }
+        for (int b = 0; b < C::NACC; ++b) {
+            mbar_init(smem_u32(&s_acc_full[b]), 1);
+            mbar_init(smem_u32(&s_acc_empty[b]), EPI_WARPS);
+        }
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                     "r"((uint32_t)TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    pdl_trigger();
+    pdl_wait();
+
     // ---- tile schedule: experts by falling token count, exclusive prefix of their tiles ---------
     for (int e = threadIdx.x; e < args.E; e += GEMM_THREADS)
         s_cnt[e] = (e >= args.e_begin && e < args.e_end) ? args.offset[e + 1] - args.offset[e] : 0;
@@ -405,24 +426,6 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             carry += __shfl_sync(0xffffffffu, incl, 31);
         }
         if (lane == 0) s_prefix[args.E] = carry;
-    }
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&s_full[s]), 1);
-            mbar_init(smem_u32(&s_empty[s]), 1);
-        }
-        for (int b = 0; b < C::NACC; ++b) {
-            mbar_init(smem_u32(&s_acc_full[b]), 1);
-            mbar_init(smem_u32(&s_acc_empty[b]), EPI_WARPS);
-        }
-        s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == MMA_WARP) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
-                     "r"((uint32_t)TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
@@ -783,7 +786,7 @@ int launch_one(GemmArgs args, long long T, int slots, const void* tokens, size_t
     INFMOE_TRY(token_maps(&tm, tokens, args.K, T));
     auto kern = ffn_umma_kernel<EPI, NMAX, STAGES>;
     INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-    kern<<<num_ctas, GEMM_THREADS, C::SMEM, stream>>>(map_w, tm, args);
+    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)num_ctas, GEMM_THREADS, C::SMEM, 1, stream, map_w, tm, args));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

@@ -19,6 +19,7 @@ int launch_select_top1(long long T, int E, const float* aff, int* gate, float* w
 int launch_dispatch(const int* gate, long long T, int E, int* pos, int* count, int* offset, int* status,
                     cudaStream_t stream, const int* region_count = nullptr, int region_size = 0, int* zero = nullptr,
                     int zero_count = 0);
+bool dispatch_supported(int E);   // the expert count fits the dispatch kernel
 int launch_scatter(long long T, int D, const float* X, const float* coeff, const int* pos, float* routed,
                    float* rcoeff, cudaStream_t stream);
 // valid_rows (device, may be NULL): rows at or past *valid_rows are skipped (tokens without an expert sit at
@@ -31,6 +32,12 @@ int launch_scatter_ln_rows(long long T, int D, const float* X, const float* scor
 int launch_scatter_ln_pack(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
                            const float* gamma_all, const int* valid_rows, float* rscore, void* h, float* row_info,
                            cudaStream_t stream);
+// launch_dispatch (without regions) and one of the two scatters in one kernel, where dispatch_scatter_supported.
+bool dispatch_scatter_supported(long long T, int D, int E);
+int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
+                            const float* gamma_all, int* pos, int* count, int* offset, int* status, int* zero,
+                            int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
+                            cudaStream_t stream);
 int launch_gather(long long T, int D, const float* in, const int* pos, float* out, cudaStream_t stream,
                   const int* valid_rows = nullptr);
 int launch_mix_gather(long long T, int D, const int* pos, const float* routed, const float* post,

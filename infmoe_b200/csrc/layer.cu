@@ -1070,8 +1070,14 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                                 L->D, L->E, gate, score, L->d_status, stream));
     INFMOE_TRY(prof_mark(L, 1, stream));
     // 2. dispatch metadata (:350-352)
-    INFMOE_TRY(launch_dispatch(gate_in, T, L->E, pos, count, offset, L->d_status, stream, region_count, region_size,
-                               w.part_bytes ? buf.part_count : nullptr, FFN_COUNTERS));
+    // (with few tokens the scatter kernel of step 3 computes it on the way, except when an expert count past the
+    // dispatch kernel's limit has to be refused)
+    const bool with_scatter = !L->identity && !L->custom && !region_count && dispatch_supported(L->E) &&
+                              dispatch_scatter_supported(T, L->D, L->E);
+    int* const zero = w.part_bytes ? buf.part_count : nullptr;
+    if (!with_scatter)
+        INFMOE_TRY(launch_dispatch(gate_in, T, L->E, pos, count, offset, L->d_status, stream, region_count, region_size,
+                                   zero, FFN_COUNTERS));
     const int* valid_rows = offset + L->E;   // rows past it have no expert (or are empty slots): nobody touches them
     INFMOE_TRY(prof_mark(L, 2, stream));
     // whole layer: the variant decides; experts alone: the caller asks for the mix by passing the scores
@@ -1139,7 +1145,12 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
         // 3. scatter fused with the experts' LayerNorm and the operand split (:354-355, T5FFLayer.cc:99-103)
         const bool pack = uses_umma(L);   // the GEMM run_ffn picks
         // tensor-core path: no routed copy, the second GEMM's epilogue reads its residual from d_in through pos[]
-        if (pack) {
+        if (with_scatter) {
+            INFMOE_TRY(launch_dispatch_scatter(T, L->D, L->E, d_in, score, gate_in, s->d_ln, pos, count, offset,
+                                               L->d_status, zero, FFN_COUNTERS, routed, rscore, buf.h, buf.row_info, pack,
+                                               stream));
+            if (pack) routed = const_cast<float*>(d_in);
+        } else if (pack) {
             INFMOE_TRY(launch_scatter_ln_pack(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, rscore, buf.h,
                                               buf.row_info, stream));
             routed = const_cast<float*>(d_in);   // run_ffn's residual operand

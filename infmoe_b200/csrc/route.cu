@@ -162,6 +162,8 @@ route_kernel(const float* __restrict__ X, const float* __restrict__ C, const flo
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long t0 = (long long)blockIdx.x * RT_TOKENS;
     const bool use_ln = gamma != nullptr;
+    pdl_trigger();
+    pdl_wait();
     // row statistics, four tokens per warp, two at a time (rows past the end alias the tile's first row)
     if (use_ln) {
 #pragma unroll
@@ -446,6 +448,10 @@ route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(rt_smem_u32(&s_full[i])), "r"(1u) : "memory");
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pdl_trigger();
+    pdl_wait();
+    if (tid == 0) {
         // the first two stages of the first pass are fetched while the warps compute the row statistics
         issue(0, 0, 0);
         if (nstages > 1) issue(1, 1, 0);
@@ -652,6 +658,8 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
     const long long t0 = (long long)(blockIdx.x / S) * RS_TOKENS;
     const int nt = (int)min((long long)RS_TOKENS, T - t0);
     const int chunks = (D + 127) / 128 * 32;              // float4 per staged row
+    pdl_trigger();
+    pdl_wait();
     if (gamma) {
         if (warp < nt) {
             float mean, rstd;
@@ -837,19 +845,8 @@ int launch_route_small(const float* X, const float* C, const float* gamma, long 
     auto kern = route_small_kernel<VEC>;
     if (smem > 40 * 1024)
         INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_MAX_SMEM));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((T + RS_TOKENS - 1) / RS_TOKENS * cluster));
-    cfg.blockDim = dim3(RS_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    INFMOE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, X, C, gamma, T, D, E, gate, score, status));
+    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)((T + RS_TOKENS - 1) / RS_TOKENS * cluster), RS_THREADS, smem,
+                                   (unsigned)cluster, stream, X, C, gamma, T, D, E, gate, score, status));
     return INFMOE_OK;
 }
 }  // namespace
@@ -870,14 +867,16 @@ int launch_route(const float* X, const float* C, const float* gamma, long long T
                                                                                status, stream));
     } else if (vec && !no_tma && T < (1ll << 31) && route_maps(&map_x, &map_c, X, C, T, D, E) == INFMOE_OK) {
         INFMOE_CUDA_TRY(cudaFuncSetAttribute(route_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM + 1024));
-        route_tma_kernel<<<(unsigned)grid, RT_THREADS, RT_SMEM + 1024, stream>>>(map_x, map_c, X, gamma, T, D, E, gate,
-                                                                               score, status);
+        INFMOE_CUDA_TRY(launch_chained(route_tma_kernel, (unsigned)grid, RT_THREADS, RT_SMEM + 1024, 1, stream, map_x, map_c,
+                                       X, gamma, T, D, E, gate, score, status));
     } else if (vec) {
         INFMOE_CUDA_TRY(cudaFuncSetAttribute(route_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM));
-        route_kernel<true><<<(unsigned)grid, RT_THREADS, RT_SMEM, stream>>>(X, C, gamma, T, D, E, gate, score, status);
+        INFMOE_CUDA_TRY(launch_chained(route_kernel<true>, (unsigned)grid, RT_THREADS, RT_SMEM, 1, stream, X, C, gamma, T, D,
+                                       E, gate, score, status));
     } else {
         INFMOE_CUDA_TRY(cudaFuncSetAttribute(route_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM));
-        route_kernel<false><<<(unsigned)grid, RT_THREADS, RT_SMEM, stream>>>(X, C, gamma, T, D, E, gate, score, status);
+        INFMOE_CUDA_TRY(launch_chained(route_kernel<false>, (unsigned)grid, RT_THREADS, RT_SMEM, 1, stream, X, C, gamma, T, D,
+                                       E, gate, score, status));
     }
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());

@@ -33,6 +33,8 @@ __device__ __forceinline__ void copy_row(const float* __restrict__ src, float* _
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 scatter_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ coeff,
                const int* __restrict__ pos, float* __restrict__ routed, float* __restrict__ rcoeff) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T) return;
@@ -72,6 +74,8 @@ scatter_ln_rows_kernel(long long T, int D, int vec, const float* __restrict__ X,
                        const int* __restrict__ pos, const int* __restrict__ gate, const float* __restrict__ gamma_all,
                        const int* __restrict__ valid_rows, float* __restrict__ routed, float* __restrict__ rscore,
                        float* __restrict__ h) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;
@@ -123,6 +127,8 @@ scatter_ln_pack_kernel(long long T, int D, int vec, const float* __restrict__ X,
                        const int* __restrict__ pos, const int* __restrict__ gate, const float* __restrict__ gamma_all,
                        const int* __restrict__ valid_rows, float* __restrict__ rscore, uint16_t* __restrict__ h,
                        float2* __restrict__ row_info) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;
@@ -145,6 +151,8 @@ scatter_ln_pack_reg_kernel(long long T, int D, const float* __restrict__ X, cons
                            const int* __restrict__ pos, const int* __restrict__ gate,
                            const float* __restrict__ gamma_all, const int* __restrict__ valid_rows,
                            float* __restrict__ rscore, uint16_t* __restrict__ h, float2* __restrict__ row_info) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;
@@ -224,10 +232,156 @@ scatter_ln_pack_reg_kernel(long long T, int D, const float* __restrict__ X, cons
     }
 }
 
+// Few tokens: dispatch metadata (dispatch.cu) and the scatter in one launch.  A block per token counts the tokens that
+// come before its own (smaller expert, or same expert and smaller index) while its row and the expert's LayerNorm weight
+// are on their way to shared memory, so nothing waits for a separate kernel of one cluster and then for pos[] and
+// gate[]; one more block writes count[] and offset[].  T blocks read T gates each, from L2: 4 MB for 1024 tokens, the
+// most it takes.  Results, LayerNorm bits included, are those of dispatch_kernel and the scatter kernels.
+// Layer of 32 tokens, 4 experts, 64 x 256: 36 -> 24 us together with launch_chained; 1 token, 32 experts, 4096 x 10240:
+// 149 -> 136.
+constexpr int DS_THREADS = 128;
+template <bool PACK>
+__global__ void __launch_bounds__(DS_THREADS)
+dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ X, const float* __restrict__ score,
+                        const int* __restrict__ gate, const float* __restrict__ gamma_all, int* __restrict__ pos,
+                        int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
+                        int* __restrict__ zero, int zero_count, float* __restrict__ routed, float* __restrict__ rscore,
+                        void* __restrict__ h, float2* __restrict__ row_info) {
+    extern __shared__ __align__(16) float ds_smem[];
+    __shared__ int s_before[DS_THREADS / 32];
+    __shared__ float s_top[DS_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_trigger();
+    pdl_wait();
+    if ((int)blockIdx.x == T) {      // histogram and its exclusive scan, 32 buckets at a time
+        int* hist = reinterpret_cast<int*>(ds_smem);
+        for (int e = tid; e <= E; e += DS_THREADS) hist[e] = 0;
+        for (int i = tid; i < zero_count; i += DS_THREADS) zero[i] = 0;
+        __syncthreads();
+        bool bad = false;
+        for (int t = tid; t < T; t += DS_THREADS) {
+            const int e = gate[t];
+            const bool ok = e >= 0 && e < E;
+            bad |= !ok;
+            atomicAdd(&hist[ok ? e : E], 1);
+        }
+        if (bad && status) atomicOr(status, STATUS_BAD_GATE);
+        __syncthreads();
+        if (warp == 0) {
+            int carry = 0;
+            for (int e0 = 0; e0 <= E; e0 += 32) {
+                const int e = e0 + lane, c = e <= E ? hist[e] : 0;
+                int incl = c;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const int n = __shfl_up_sync(0xffffffffu, incl, off);
+                    if (lane >= off) incl += n;
+                }
+                if (e <= E) offset[e] = carry + incl - c;     // offset[E]: tokens that have an expert
+                if (e < E) count[e] = c;
+                carry += __shfl_sync(0xffffffffu, incl, 31);
+            }
+        }
+        return;
+    }
+    const int t = (int)blockIdx.x;
+    const int P = (int)padded_row(D);
+    float *s_x = ds_smem, *s_g = ds_smem + P;
+    int e = gate[t];
+    if (e < 0 || e >= E) e = E;
+    const float* src = X + (size_t)t * D;
+    const float* gamma = gamma_all + (size_t)(e < E ? e : 0) * D;
+    if (vec) {
+        for (int k = 4 * tid; k < D; k += 4 * DS_THREADS) {
+            const uint32_t dx = (uint32_t)__cvta_generic_to_shared(s_x + k), dg = (uint32_t)__cvta_generic_to_shared(s_g + k);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dx), "l"(src + k) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dg), "l"(gamma + k) : "memory");
+        }
+    } else {
+#pragma unroll 4
+        for (int k = tid; k < D; k += DS_THREADS) {
+            s_x[k] = src[k];
+            s_g[k] = gamma[k];
+        }
+    }
+    for (int k = D + tid; k < P; k += DS_THREADS) s_x[k] = s_g[k] = 0.f;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    int before = 0;
+    for (int o = tid; o < T; o += DS_THREADS) {
+        int g = gate[o];
+        if (g < 0 || g >= E) g = E;
+        before += (g < e || (g == e && o < t)) ? 1 : 0;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) s_before[warp] = before;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    int j = 0;
+#pragma unroll
+    for (int w = 0; w < DS_THREADS / 32; ++w) j += s_before[w];
+    if (tid == 0) {
+        pos[j] = t;
+        if (e < E && rscore && score) rscore[j] = score[t];
+    }
+    if (e == E) return;              // no expert: nobody reads the row
+    float mean, rstd;
+    warp_row_stats(s_x, D, (D & 3) == 0, mean, rstd);     // every warp for itself
+    __syncthreads();
+    float top = 0.f;
+    for (int k = 4 * tid; k < P; k += 4 * DS_THREADS) {
+        float* x = s_x + k;
+        const float4 g = *reinterpret_cast<const float4*>(s_g + k);
+        float4 v = *reinterpret_cast<const float4*>(x);
+        if (!PACK)
+            for (int i = 0; i < 4 && k + i < D; ++i) routed[(size_t)j * D + k + i] = x[i];
+        v.x = k < D ? ln_apply(v.x, mean, rstd, g.x) : 0.f;
+        v.y = k + 1 < D ? ln_apply(v.y, mean, rstd, g.y) : 0.f;
+        v.z = k + 2 < D ? ln_apply(v.z, mean, rstd, g.z) : 0.f;
+        v.w = k + 3 < D ? ln_apply(v.w, mean, rstd, g.w) : 0.f;
+        if (PACK) {
+            top = fmaxf(fmaxf(fmaxf(top, fabsf(v.x)), fmaxf(fabsf(v.y), fabsf(v.z))), fabsf(v.w));
+            *reinterpret_cast<float4*>(x) = v;            // the thread's own values again below
+        } else {
+            *reinterpret_cast<float4*>(static_cast<float*>(h) + (size_t)j * P + k) = v;
+        }
+    }
+    if (!PACK) return;
+    top = warp_max(top);
+    if (lane == 0) s_top[warp] = top;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < DS_THREADS / 32; ++w) top = fmaxf(top, s_top[w]);
+    const int s = row_exponent(top);
+    const float scale = exp2_int(s);
+    uint16_t* pack_row = static_cast<uint16_t*>(h) + (size_t)j * pack_pitch(D);
+    for (int k = 4 * tid; k < P; k += 4 * DS_THREADS) {
+        float4 v = *reinterpret_cast<const float4*>(s_x + k);
+        v = make_float4(__fmul_rn(v.x, scale), __fmul_rn(v.y, scale), __fmul_rn(v.z, scale), __fmul_rn(v.w, scale));
+        *reinterpret_cast<float4*>(s_x + k) = v;
+        const float x[4] = {v.x, v.y, v.z, v.w};
+        store_pack4(pack_row, k, x);
+    }
+    __syncthreads();
+    if (warp == 0) {                 // the sum of squares in the order of the other scatter kernels
+        float squares = 0.f;
+        for (int k = 4 * lane; k < P; k += 128) {
+            const float4 v = *reinterpret_cast<const float4*>(s_x + k);
+            squares = fmaf(v.x, v.x, squares);
+            squares = fmaf(v.y, v.y, squares);
+            squares = fmaf(v.z, v.z, squares);
+            squares = fmaf(v.w, v.w, squares);
+        }
+        squares = warp_xor_sum(squares);
+        if (lane == 0) row_info[j] = token_row_info(s, squares);
+    }
+}
+
 // out[pos[j],:] = in[j,:] for the rows below *valid_rows (all rows when valid_rows is NULL)
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 gather_kernel(long long T, int D, int vec, const float* __restrict__ in, const int* __restrict__ pos,
               const int* __restrict__ valid_rows, float* __restrict__ out) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;
@@ -240,6 +394,8 @@ __global__ void __launch_bounds__(ROW_WARPS * 32)
 mix_gather_kernel(long long T, int D, int vec, const int* __restrict__ pos, const float* __restrict__ routed,
                   const float* __restrict__ post, const float* __restrict__ coeff,
                   const int* __restrict__ valid_rows, float* __restrict__ out) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;
@@ -401,7 +557,27 @@ int launch_scatter(long long T, int D, const float* X, const float* coeff, const
     }
     if (T == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && aligned16(X) && aligned16(routed);
-    scatter_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, X, coeff, pos, routed, rcoeff);
+    INFMOE_CUDA_TRY(launch_chained(scatter_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, T, D, vec, X, coeff, pos,
+                                   routed, rcoeff));
+    note_launch();
+    INFMOE_CUDA_TRY(cudaGetLastError());
+    return INFMOE_OK;
+}
+
+// Up to 1024 tokens whose row and LayerNorm weight fit into 48 KB of shared memory with the histogram's E + 1 words.
+bool dispatch_scatter_supported(long long T, int D, int E) { return T <= 1024 && D <= 6016 && E < 8192; }
+
+int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
+                            const float* gamma_all, int* pos, int* count, int* offset, int* status, int* zero,
+                            int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
+                            cudaStream_t stream) {
+    const int vec = (D % 4 == 0) && aligned16(X) && aligned16(gamma_all);
+    size_t smem = 2 * padded_row(D) * sizeof(float);
+    if (smem < sizeof(int) * (size_t)(E + 1)) smem = sizeof(int) * (size_t)(E + 1);
+    auto kern = pack ? dispatch_scatter_kernel<true> : dispatch_scatter_kernel<false>;
+    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)T + 1, DS_THREADS, smem, 1, stream, (int)T, D, E, vec, X, score, gate,
+                                   gamma_all, pos, count, offset, status, zero, zero ? zero_count : 0, routed, rscore, h,
+                                   (float2*)row_info));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
@@ -412,8 +588,8 @@ int launch_scatter_ln_rows(long long T, int D, const float* X, const float* scor
                            cudaStream_t stream) {
     if (T == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && aligned16(X) && aligned16(gamma_all);
-    scatter_ln_rows_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, X, score, pos, gate, gamma_all,
-                                                                       valid_rows, routed, rscore, h);
+    INFMOE_CUDA_TRY(launch_chained(scatter_ln_rows_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, T, D, vec, X, score,
+                                   pos, gate, gamma_all, valid_rows, routed, rscore, h));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
@@ -434,15 +610,16 @@ int launch_scatter_ln_pack(long long T, int D, const float* X, const float* scor
         constexpr int smem = 4 * NV * 32 * 16;                                                                     \
         if (smem > 48 * 1024)                                                                                      \
             INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));        \
-        kern<<<grid, 128, smem, stream>>>(T, D, X, score, pos, gate, gamma_all, valid_rows, rscore, pack, info);   \
+        INFMOE_CUDA_TRY(launch_chained(kern, grid, 128, smem, 1, stream, T, D, X, score, pos, gate, gamma_all,     \
+                                       valid_rows, rscore, pack, info));                                           \
     } while (0)
         if (D <= 1024) INFMOE_SCATTER_REG(8);
         else if (D <= 2048) INFMOE_SCATTER_REG(16);
         else INFMOE_SCATTER_REG(32);
 #undef INFMOE_SCATTER_REG
     } else {
-        scatter_ln_pack_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, X, score, pos, gate, gamma_all,
-                                                                           valid_rows, rscore, pack, info);
+        INFMOE_CUDA_TRY(launch_chained(scatter_ln_pack_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, T, D, vec, X, score,
+                                       pos, gate, gamma_all, valid_rows, rscore, pack, info));
     }
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
@@ -487,7 +664,8 @@ int launch_gather(long long T, int D, const float* in, const int* pos, float* ou
     }
     if (T == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && aligned16(in) && aligned16(out);
-    gather_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, in, pos, valid_rows, out);
+    INFMOE_CUDA_TRY(launch_chained(gather_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, T, D, vec, in, pos, valid_rows,
+                                   out));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
@@ -501,8 +679,8 @@ int launch_mix_gather(long long T, int D, const int* pos, const float* routed, c
     }
     if (T == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && aligned16(routed) && aligned16(post) && aligned16(out);
-    mix_gather_kernel<<<row_grid(T), ROW_WARPS * 32, 0, stream>>>(T, D, vec, pos, routed, post, coeff, valid_rows,
-                                                                  out);
+    INFMOE_CUDA_TRY(launch_chained(mix_gather_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, T, D, vec, pos, routed, post,
+                                   coeff, valid_rows, out));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

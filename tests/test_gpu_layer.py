@@ -532,3 +532,96 @@ def test_cuda_core_experts_against_oracle(oracle, counts, D, F):
         if rows.any():
             want = oracle.expert_ffn_f64(x[rows], *experts[e])
             assert oracle.rel_l2(out[rows] - x[rows], want - x[rows]) <= 2e-6   # FP32 chains of up to 1022 adds
+
+
+# Up to 1024 tokens one kernel computes the dispatch metadata and scatters; beyond, or with d_model > 6016, two do.
+@pytest.mark.parametrize("T,D,E,variant", [(1, 64, 4, "default"), (33, 66, 3, "base_layer"), (1023, 36, 70, "cpm_2"),
+                                           (1024, 40, 5, "base_layer"), (1025, 40, 5, "base_layer"),
+                                           (7, 6016, 2, "default"), (7, 6020, 2, "default"), (129, 130, 33, "default")])
+def test_few_and_many_tokens_dispatch_alike(oracle, T, D, E, variant):
+    import torch
+    from infmoe_b200 import MoELayer
+    from infmoe_b200.devmem import read_device
+    F = 40
+    rng = np.random.default_rng(T + D + E)
+    c = (rng.standard_normal((E, D)) * 0.02).astype(np.float32)
+    ln = (1 + 0.01 * rng.standard_normal(D)).astype(np.float32) if variant == "cpm_2" else None
+    experts = [[(1 + 0.01 * rng.standard_normal(D)).astype(np.float32)] +
+               [(rng.standard_normal((F, D)) / np.sqrt(D)).astype(np.float32) for _ in range(2)] +
+               [(rng.standard_normal((D, F)) / np.sqrt(F)).astype(np.float32)] for _ in range(E)]
+    x = rng.standard_normal((T, D)).astype(np.float32)
+    layer = MoELayer.create(E, D, F, 2, c, None, "T5_FF", variant, ln)
+    for e, ex in enumerate(experts):
+        layer.set_expert(e, *(torch.from_numpy(a).cuda() for a in ex))
+    out = layer.forward(torch.from_numpy(x).cuda()).cpu().numpy()
+    layer.sync_status()
+    gate_p, _, pos_p, count_p, offset_p = layer.last_routing()
+    gate, score = oracle.route(x, c, ln)
+    count, offset, pos = oracle.dispatch(gate, E)
+    np.testing.assert_array_equal(read_device(gate_p, T, np.int32), gate)
+    np.testing.assert_array_equal(read_device(pos_p, T, np.int32), pos)
+    np.testing.assert_array_equal(read_device(count_p, E, np.int32), count)
+    np.testing.assert_array_equal(read_device(offset_p, E + 1, np.int32), offset)
+    assert oracle.rel_l2(out, oracle.layer_forward_f64(x, variant, gate, score, experts)) <= TOL
+    # the experts alone, every seventh token without one: its row stays as it was
+    bad = gate.copy()
+    bad[::7] = -1
+    keep = torch.full((T, D), -7.0, device="cuda")
+    layer.expert_forward(torch.from_numpy(x).cuda(), torch.from_numpy(bad).cuda(), out=keep)
+    with pytest.raises(Exception):
+        layer.sync_status()
+    keep = keep.cpu().numpy()
+    assert np.all(keep[::7] == -7.0)
+    good = bad >= 0
+    if good.any() and variant != "base_layer":
+        np.testing.assert_array_equal(keep[good], out[good])
+    layer.terminate()
+
+
+def test_pass_under_capture_between_other_kernels():
+    """Kernels of a pass start before their predecessors have ended; their reads and writes still follow them: the
+    input is filled by the kernel before the pass and the output overwritten by the one after it, eagerly and in a graph."""
+    import torch
+    from infmoe_b200 import MoELayer
+    g = torch.Generator(device="cuda").manual_seed(3)
+    E, D, F = 4, 256, 512
+    layer = MoELayer.create(E, D, F, 2, torch.randn(E, D, generator=g, device="cuda").cpu().numpy(), None, "T5_FF",
+                            "default", None)
+    for e in range(E):
+        layer.set_expert(e, torch.ones(D, device="cuda"), torch.randn(F, D, generator=g, device="cuda") / 16,
+                         torch.randn(F, D, generator=g, device="cuda") / 16, torch.randn(D, F, generator=g, device="cuda") / 22)
+    for T in (3, 1500):
+        src = torch.randn(4, T, D, generator=g, device="cuda")
+        want = [layer.forward(src[i].contiguous()).clone() for i in range(4)]
+        torch.cuda.synchronize()
+        x, out, acc = torch.zeros(T, D, device="cuda"), torch.zeros(T, D, device="cuda"), torch.zeros(T, D, device="cuda")
+        side = torch.cuda.Stream()
+        graph = torch.cuda.CUDAGraph()
+
+        def step(i):
+            x.copy_(src[i] * 1.0)
+            layer.forward(x, out)
+            acc.add_(out)
+            out.fill_(-1.0)
+            x.fill_(5.0)
+
+        with torch.cuda.stream(side):
+            for _ in range(3):
+                acc.zero_()
+                for i in range(4):
+                    step(i)
+        side.synchronize()
+        ref = torch.zeros(T, D, device="cuda")
+        for w in want:
+            ref.add_(w)
+        assert torch.equal(acc, ref)
+        with torch.cuda.graph(graph, stream=side):
+            acc.zero_()
+            for i in range(4):
+                step(i)
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(acc, ref)
+    layer.sync_status()
+    layer.terminate()
