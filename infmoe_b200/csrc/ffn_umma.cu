@@ -39,13 +39,18 @@
 // round-to-nearest adds, in ascending k.  That order is the same for every tile,
 // whatever the launch, so a token's result does not depend on its neighbours.
 //
-// Pipeline per CTA (persistent, one CTA per SM, 12 warps):
+// Pipeline per CTA (persistent, one CTA per SM, 20 warps):
 //   warp 0        TMA producer: a stage is one weight tile (16 KB) and the token tile of the same k block
 //   warp 1        MMA issuer (and owner of the TMEM allocation): one commit per k block frees the stage, one per chunk
-//                 hands its accumulator to the accumulate warps.  Chunks rotate over NACC accumulators
-//   warps 4..11   accumulate + epilogue: tcgen05.ld the chunk (one TMEM lane quarter and every other
+//                 hands its accumulator to the accumulate warps.  Chunks rotate over as many accumulators as fit into
+//                 TMEM at the width of the launch's widest token tile (2 at 192 columns, 4 at 128, at most 8)
+//   warps 4..19   accumulate + epilogue: tcgen05.ld the chunk (one TMEM lane quarter and every fourth
 //                 16-column slice per warp), add into registers; after the last chunk gelu*dot and its
-//                 split (lane pairs exchange a and b by shuffle) or residual add
+//                 split (lane pairs exchange a and b by shuffle) or residual add.  The epilogue is a chain of
+//                 shuffles, loads and stores, so warps in flight set its speed, and with K = 1024 or less it sets the
+//                 kernel's: 8 -> 16 warps (and 8 residual values in flight per thread instead of 16, which spilled)
+//                 took 8 experts x 256 x 1024 with 16384 tokens from 296 to 209 us per layer, three layers of 8 x 1024 x
+//                 4096 with 4096 tokens from 1446 to 1284, 777 tokens x 12 x 1000 x 2724 from 154 to 132
 //
 // Tiles are (expert, 128-row weight block, token chunk); the list is derived in
 // the kernel from offset[E+1], so no host synchronisation is needed.
@@ -205,7 +210,8 @@ enum { EPI_GELU_PAIR = 0, EPI_RESIDUAL = 1 };
 constexpr int TMA_WARP = 0;
 constexpr int MMA_WARP = 1;                           // issues all MMAs; owns the TMEM allocation
 constexpr int EPI_WARP0 = 4;
-constexpr int EPI_WARPS = 8;                          // two warps per TMEM lane quarter
+constexpr int EPI_GROUPS = 4;                         // warps per TMEM lane quarter
+constexpr int EPI_WARPS = 4 * EPI_GROUPS;
 constexpr int GEMM_THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
 constexpr int TMEM_COLS = 512;
 constexpr int CHUNK_BLOCKS = 8;                       // k blocks (of 6 MMAs) an accumulator takes between two drains
@@ -215,9 +221,9 @@ template <int NMAX, int STAGES>
 struct Cfg {
     static constexpr int STAGE = W_TILE + NMAX * ROW_BYTES;         // weight tile, then token tile
     static constexpr int SMEM = STAGES * STAGE + 1024;              // + slack for 1024-byte alignment
-    static constexpr int NACC = TMEM_COLS / NMAX;                   // accumulators
-    static constexpr int SLICES = (NMAX / 16 + 1) / 2;              // 16-column slices owned by one epilogue thread
-    static_assert(NMAX % 16 == 0 && NACC >= 2, "token chunk");
+    static constexpr int MAX_ACC = 8;                                // accumulators, at most
+    static constexpr int SLICES = (NMAX / 16 + EPI_GROUPS - 1) / EPI_GROUPS;   // 16-column slices owned by one epilogue thread
+    static_assert(NMAX % 16 == 0 && 2 * NMAX <= TMEM_COLS, "token chunk");
     static_assert((NMAX * ROW_BYTES) % 1024 == 0, "tiles must keep 1024-byte alignment");
 };
 
@@ -354,13 +360,14 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const GemmArgs args) {
     using C = Cfg<NMAX, STAGES>;
     extern __shared__ uint8_t smem_raw[];
-    // k block `it` (counted over all items of the CTA) uses stage it % STAGES, chunk `cc` accumulator cc % NACC
+    // k block `it` (counted over all items of the CTA) uses stage it % STAGES; chunks rotate over the accumulators
     __shared__ __align__(8) uint64_t s_full[STAGES];        // TMA -> MMA: stage filled
     __shared__ __align__(8) uint64_t s_empty[STAGES];       // MMA -> TMA: stage consumed
-    __shared__ __align__(8) uint64_t s_acc_full[C::NACC];   // MMA -> accumulate warps: chunk done
-    __shared__ __align__(8) uint64_t s_acc_empty[C::NACC];  // accumulate warps -> MMA: chunk read out
+    __shared__ __align__(8) uint64_t s_acc_full[C::MAX_ACC];   // MMA -> accumulate warps: chunk done
+    __shared__ __align__(8) uint64_t s_acc_empty[C::MAX_ACC];  // accumulate warps -> MMA: chunk read out
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
+    __shared__ int s_widest;
     __shared__ int s_prefix[MAX_EXPERTS + 1];
     __shared__ int s_cnt[MAX_EXPERTS];
     __shared__ short s_order[MAX_EXPERTS];
@@ -376,7 +383,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             mbar_init(smem_u32(&s_full[s]), 1);
             mbar_init(smem_u32(&s_empty[s]), 1);
         }
-        for (int b = 0; b < C::NACC; ++b) {
+        for (int b = 0; b < C::MAX_ACC; ++b) {
             mbar_init(smem_u32(&s_acc_full[b]), 1);
             mbar_init(smem_u32(&s_acc_empty[b]), EPI_WARPS);
         }
@@ -407,7 +414,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
     __syncthreads();
     if (warp == 0) {
-        int carry = 0;
+        int carry = 0, widest = 16;
         for (int e0 = 0; e0 < args.E; e0 += 32) {
             const int e = e0 + lane;   // list position
             int nt = 0;
@@ -415,6 +422,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 int nch, csz;
                 chunking<NMAX>(s_cnt[s_order[e]], nch, csz);
                 nt = nch * MB;
+                widest = max(widest, csz);
             }
             int incl = nt;
 #pragma unroll
@@ -425,12 +433,18 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             if (e < args.E) s_prefix[e] = carry + incl - nt;
             carry += __shfl_sync(0xffffffffu, incl, 31);
         }
-        if (lane == 0) s_prefix[args.E] = carry;
+        widest = __reduce_max_sync(0xffffffffu, widest);
+        if (lane == 0) {
+            s_prefix[args.E] = carry;
+            s_widest = widest;
+        }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = s_tmem_base;
+    // as many accumulators as fit beside one another at the width of the widest token tile
+    const uint32_t acc_stride = (uint32_t)s_widest, nacc = min((uint32_t)C::MAX_ACC, (uint32_t)TMEM_COLS / acc_stride);
     volatile int* abort_flag = &s_abort;
     Schedule sched(s_prefix[args.E], KB, args);
     Item item;
@@ -465,15 +479,14 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // cycles per MMA whatever its N, which held a decode step of 27 experts at 1694 us of first GEMM where the
         // same bytes stream in 1269.  Elected: 1259 us (7.2 TB/s); 4096 tokens 2780 -> 2383.
         if (elect_one()) {
-            uint32_t it = 0, cc = 0;
+            uint32_t it = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             while (ok && sched.next(item) && !*abort_flag) {
                 const TileInfo t = decode_tile<NMAX>(item.tile, s_prefix, s_order, args);
                 const uint32_t idesc = make_idesc(t.n_pad);
-                for (int c = item.c0; ok && c < item.c1; ++c, ++cc) {
-                    const uint32_t acc = cc % C::NACC;
-                    const uint32_t d = tmem_base + acc * NMAX;
-                    if (!mbar_wait(smem_u32(&s_acc_empty[acc]), ((cc / C::NACC) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                for (int c = item.c0; ok && c < item.c1; ++c) {
+                    const uint32_t d = tmem_base + acc * acc_stride;
+                    if (!mbar_wait(smem_u32(&s_acc_empty[acc]), acc_phase ^ 1, abort_flag)) { ok = false; break; }
                     const int kb0 = c * CHUNK_BLOCKS, kb_end = min(KB, kb0 + CHUNK_BLOCKS);
                     for (int kb = kb0; kb < kb_end; ++kb, ++it) {
                         const uint32_t s = it % STAGES;
@@ -492,6 +505,10 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         umma_commit(smem_u32(&s_empty[s]));
                         if (kb + 1 == kb_end) umma_commit(smem_u32(&s_acc_full[acc]));
                     }
+                    if (++acc == nacc) {
+                        acc = 0;
+                        acc_phase ^= 1;
+                    }
                 }
             }
         }
@@ -502,9 +519,9 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // round-to-nearest adds in ascending k, to a running sum in registers; then the accumulator goes back to the
         // MMA issuer.
         const int q = warp & 3;                 // TMEM lane quarter this warp may access
-        const int half = (warp - EPI_WARP0) >> 2;   // even or odd 16-column slices
+        const int group = (warp - EPI_WARP0) >> 2;   // 16-column slices group, group + EPI_GROUPS, ...
         const uint32_t tlane = tmem_base + ((uint32_t)(q * 32) << 16);
-        uint32_t cc = 0;
+        uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
         while (ok && sched.next(item) && !*abort_flag) {
             const TileInfo t = decode_tile<NMAX>(item.tile, s_prefix, s_order, args);
@@ -520,7 +537,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             auto store_block = [&](int c) {     // sum[][] -> block of chunk c
 #pragma unroll
                 for (int i = 0; i < C::SLICES; ++i) {
-                    const int sl = 2 * i + half;
+                    const int sl = EPI_GROUPS * i + group;
                     if (sl >= nsl) continue;
 #pragma unroll
                     for (int v = 0; v < 4; ++v)
@@ -528,35 +545,30 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                                make_float4(sum[i][4 * v], sum[i][4 * v + 1], sum[i][4 * v + 2], sum[i][4 * v + 3]));
                 }
             };
-            for (int c = item.c0; c < item.c1; ++c, ++cc) {
-                const uint32_t acc = cc % C::NACC;
+            for (int c = item.c0; c < item.c1; ++c) {
                 // the warp stays converged for the .aligned TMEM instructions, also when a wait is abandoned
-                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_acc_full[acc]), (cc / C::NACC) & 1, abort_flag))) {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_acc_full[acc]), acc_phase, abort_flag))) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
 #pragma unroll
-                for (int i = 0; i < C::SLICES; i += 2) {
-                    const int s0 = 2 * i + half, s1 = s0 + 2;
-                    if (s0 >= nsl) continue;
-                    uint32_t r0[16], r1[16];
-                    tmem_ld16(tlane + acc * NMAX + s0 * 16, r0);
-                    const bool two = i + 1 < C::SLICES && s1 < nsl;
-                    if (two) tmem_ld16(tlane + acc * NMAX + s1 * 16, r1);
+                for (int i = 0; i < C::SLICES; ++i) {
+                    const int sl = EPI_GROUPS * i + group;
+                    if (sl >= nsl) continue;
+                    uint32_t r[16];
+                    tmem_ld16(tlane + acc * acc_stride + sl * 16, r);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int x = 0; x < 16; ++x) sum[i][x] = __fadd_rn(sum[i][x], __uint_as_float(r0[x]));
-                    if (two) {
-#pragma unroll
-                        for (int x = 0; x < 16; ++x)
-                            sum[i + 1 < C::SLICES ? i + 1 : i][x] =
-                                __fadd_rn(sum[i + 1 < C::SLICES ? i + 1 : i][x], __uint_as_float(r1[x]));
-                    }
+                    for (int x = 0; x < 16; ++x) sum[i][x] = __fadd_rn(sum[i][x], __uint_as_float(r[x]));
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&s_acc_empty[acc]));
+                if (++acc == nacc) {
+                    acc = 0;
+                    acc_phase ^= 1;
+                }
                 if (part && (item.c0 > 0 || c + 1 == item.c1)) {
                     store_block(c);
 #pragma unroll
@@ -583,7 +595,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const int first = sched.prefix_chunks(item.tail) - 1;
 #pragma unroll
                 for (int i = 0; i < C::SLICES; ++i) {
-                    const int sl = 2 * i + half;
+                    const int sl = EPI_GROUPS * i + group;
                     if (sl >= nsl) continue;
                     const float4* src = part + (size_t)(sl * 4) * UMMA_M;
 #pragma unroll 2
@@ -606,7 +618,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             const float bound = decode_bound(__ldg(args.bound + (size_t)t.slot * args.bound_stride));
 #pragma unroll
             for (int i = 0; i < C::SLICES; ++i) {
-                const int sl = 2 * i + half;
+                const int sl = EPI_GROUPS * i + group;
                 if (sl >= nsl) continue;     // uniform across the warp
                 // What belongs to the slice's 16 token columns, one column per lane (lanes 16..31 repeat them),
                 // handed out by shuffle below: 2^-s of the token row, and 2^s of g (GELU_PAIR) or the output row and
@@ -654,27 +666,29 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (lc_ok)
                     lane_ptr = args.out_row_ptr ? args.out_row_ptr[lane_row]
                                                 : (unsigned long long)(args.out + (size_t)lane_row * (size_t)args.M_total);
-                // The residual values of the slice's 16 columns are fetched first, all in flight together: issued
+                // The residual values of eight columns are fetched first, all in flight together: issued
                 // one by one between the stores (which may alias them as far as the compiler knows) each would
-                // cost a trip to L2 or HBM, 80 in a row per thread, and the next tile's first chunk would wait.
-                float xres[16];
+                // cost a trip to L2 or HBM, and the next tile's first chunk would wait.
 #pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    const int resid_row = __shfl_sync(0xffffffffu, lane_row, c);
-                    xres[c] = (sl * 16 + c < t.n_tok && m_ok)
-                                  ? args.resid[(size_t)resid_row * (size_t)args.M_total + (size_t)m] : 0.f;
-                }
+                for (int c0 = 0; c0 < 16; c0 += 8) {
+                    float xres[8];
 #pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    const int col = sl * 16 + c;
-                    const unsigned long long out_row = __shfl_sync(0xffffffffu, lane_ptr, c);
-                    const float alpha = __shfl_sync(0xffffffffu, lane_alpha, c);
-                    const float v = unscale(sum[i][c], w_inv, __shfl_sync(0xffffffffu, lane_inv, c));
-                    if (col < t.n_tok && m_ok) {
-                        const float x = xres[c];
-                        float y = __fadd_rn(x, v);
-                        if (args.mix_score) y = mix_value(alpha, 1.0f - alpha, y, x);
-                        reinterpret_cast<float*>(out_row)[m] = y;
+                    for (int c = 0; c < 8; ++c) {
+                        const int resid_row = __shfl_sync(0xffffffffu, lane_row, c0 + c);
+                        xres[c] = (sl * 16 + c0 + c < t.n_tok && m_ok)
+                                      ? args.resid[(size_t)resid_row * (size_t)args.M_total + (size_t)m] : 0.f;
+                    }
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const unsigned long long out_row = __shfl_sync(0xffffffffu, lane_ptr, c0 + c);
+                        const float alpha = __shfl_sync(0xffffffffu, lane_alpha, c0 + c);
+                        const float v = unscale(sum[i][c0 + c], w_inv, __shfl_sync(0xffffffffu, lane_inv, c0 + c));
+                        if (sl * 16 + c0 + c < t.n_tok && m_ok) {
+                            const float x = xres[c];
+                            float y = __fadd_rn(x, v);
+                            if (args.mix_score) y = mix_value(alpha, 1.0f - alpha, y, x);
+                            reinterpret_cast<float*>(out_row)[m] = y;
+                        }
                     }
                 }
             }

@@ -96,7 +96,7 @@ struct FfnUmma {
 int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_begin, int e_end, int num_sms,
                     cudaStream_t stream, cudaEvent_t mid_event = nullptr);
 constexpr int FFN_CTAS = 148;                   // most CTAs of a launch (SMs of a B200); the workspace is sized for them
-constexpr int FFN_COUNTERS = FFN_CTAS * 8;      // ints in part_count: one per cut tile and accumulate warp
+constexpr int FFN_COUNTERS = FFN_CTAS * 16;      // ints in part_count: one per cut tile and accumulate warp
 size_t ffn_umma_part_bytes(long long T, int D, int F);
 // Rows of `in` [n][D] copied to the addresses dst[i] (one per row; they may point into a peer GPU's memory).
 int launch_rows_to_ptrs(long long n, int D, const float* in, const unsigned long long* dst, cudaStream_t stream);
