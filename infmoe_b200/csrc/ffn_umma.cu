@@ -52,6 +52,11 @@
 //                 took 8 experts x 256 x 1024 with 16384 tokens from 296 to 209 us per layer, three layers of 8 x 1024 x
 //                 4096 with 4096 tokens from 1446 to 1284, 777 tokens x 12 x 1000 x 2724 from 154 to 132
 //
+// Pairs (CTAS = 2, a cluster of two).  Both CTAs walk the same items; tile rows 0..127 belong to the first one, 128..255
+// to the second.  Each fetches its own weight tile and its half of the token rows, counting on the first one's barrier;
+// the first one's issuer runs the MMAs for both (M = 256) and its commits arrive in both; both CTAs' accumulate warps
+// hand the accumulator back to it.
+//
 // Tiles are (expert, 128-row weight block, token chunk); the list is derived in
 // the kernel from offset[E+1], so no host synchronisation is needed.
 //
@@ -64,6 +69,8 @@
 // Every mbarrier wait is bounded: on expiry the CTA raises STATUS_WAIT_TIMEOUT, lets
 // copies in flight land, frees its TMEM and returns.
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -170,6 +177,48 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t adesc, uin
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same over a pair of CTAs (M = 256): each CTA's shared memory holds 128 rows of A and half the rows of B, each
+// CTA's tensor memory 128 rows of D.  Issued by the first CTA of the pair.
+__device__ __forceinline__ void umma_f16_ss_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                 uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+template <int CTAS>
+__device__ __forceinline__ void umma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    if (CTAS == 1) umma_f16_ss(d, a, b, idesc, accumulate);
+    else umma_f16_ss_pair(d, a, b, idesc, accumulate);
+}
+// Arrives on the barrier at this offset in both CTAs of the pair once all MMAs issued so far have completed.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+        ::"r"(bar), "h"((uint16_t)3)
+        : "memory");
+}
+// Address of a shared-memory location of this CTA in the first CTA of the pair.
+__device__ __forceinline__ uint32_t leader_addr(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A load into this CTA's shared memory that counts on a barrier of the pair's first CTA.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
+        : "memory");
+}
 // Arrives on the mbarrier once all MMAs issued so far by this thread have completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -200,9 +249,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
     return d;
 }
 
-// Instruction descriptor: FP16 operands (format 0), FP32 accumulate, both operands K-major, M = 128, N = n.
-__device__ __forceinline__ uint32_t make_idesc(int n) {
-    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(UMMA_M >> 4) << 24);
+// Instruction descriptor: FP16 operands (format 0), FP32 accumulate, both operands K-major, M = m, N = n.
+__device__ __forceinline__ uint32_t make_idesc(int m, int n) {
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 enum { EPI_GELU_PAIR = 0, EPI_RESIDUAL = 1 };
@@ -217,14 +266,15 @@ constexpr int TMEM_COLS = 512;
 constexpr int CHUNK_BLOCKS = 8;                       // k blocks (of 6 MMAs) an accumulator takes between two drains
 constexpr int W_TILE = UMMA_M * ROW_BYTES;            // 16 KB of weights per k block
 
-template <int NMAX, int STAGES>
+template <int NMAX, int STAGES, int CTAS>
 struct Cfg {
-    static constexpr int STAGE = W_TILE + NMAX * ROW_BYTES;         // weight tile, then token tile
+    static constexpr int STAGE = W_TILE + NMAX / CTAS * ROW_BYTES;  // weight tile, then this CTA's part of the token tile
     static constexpr int SMEM = STAGES * STAGE + 1024;              // + slack for 1024-byte alignment
     static constexpr int MAX_ACC = 8;                                // accumulators, at most
     static constexpr int SLICES = (NMAX / 16 + EPI_GROUPS - 1) / EPI_GROUPS;   // 16-column slices owned by one epilogue thread
-    static_assert(NMAX % 16 == 0 && 2 * NMAX <= TMEM_COLS, "token chunk");
-    static_assert((NMAX * ROW_BYTES) % 1024 == 0, "tiles must keep 1024-byte alignment");
+    static constexpr int N_STEP = 16 * CTAS;                        // token tiles are padded to a multiple of this
+    static_assert(NMAX % N_STEP == 0 && 2 * NMAX <= TMEM_COLS, "token chunk");
+    static_assert((NMAX / CTAS * ROW_BYTES) % 1024 == 0, "tiles must keep 1024-byte alignment");
 };
 
 struct GemmArgs {
@@ -264,16 +314,16 @@ struct TileInfo {
     int expert, slot, mb, row0, n_tok, n_pad;
 };
 
-template <int NMAX>
+template <int NMAX, int STEP>
 __device__ __forceinline__ void chunking(int cnt, int& nch, int& csz) {
     nch = (cnt + NMAX - 1) / NMAX;
-    csz = nch ? (((cnt + nch - 1) / nch + 15) & ~15) : 0;  // balanced chunks, multiple of 16, <= NMAX
+    csz = nch ? (((cnt + nch - 1) / nch + STEP - 1) & ~(STEP - 1)) : 0;  // balanced chunks, multiple of STEP, <= NMAX
 }
 
 // Tiles are listed by expert in order of falling token count (s_order: list position -> expert, s_prefix: first
 // tile of each list position), so the long tiles of the busiest experts are handed out first and the short ones
 // fill the end of the schedule.
-template <int NMAX>
+template <int NMAX, int STEP>
 __device__ __forceinline__ TileInfo decode_tile(int tile, const int* s_prefix, const short* s_order, const GemmArgs& a) {
     int lo = 0, hi = a.E - 1;  // last list position with s_prefix[.] <= tile
     while (lo < hi) {
@@ -286,13 +336,13 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, const int* s_prefix, c
     t.slot = a.slot_of_expert ? a.slot_of_expert[ex] : ex;
     const int beg = a.offset[ex], cnt = a.offset[ex + 1] - beg;
     int nch, csz;
-    chunking<NMAX>(cnt, nch, csz);
+    chunking<NMAX, STEP>(cnt, nch, csz);
     const int local = tile - s_prefix[lo];
     t.mb = local / nch;                 // chunk-minor: CTAs working side by side share the weight tile in L2
     const int c = local % nch;
     t.row0 = beg + c * csz;
     t.n_tok = min(csz, beg + cnt - t.row0);
-    t.n_pad = (t.n_tok + 15) & ~15;
+    t.n_pad = (t.n_tok + STEP - 1) & ~(STEP - 1);
     return t;
 }
 
@@ -306,11 +356,12 @@ struct Item {
     int c0, c1;        // chunks [c0, c1) of the tile
     int tail;          // index among the cut tiles, -1: this CTA holds the whole tile
 };
+template <int CTAS>
 struct Schedule {
     int total, m, full, R, U, cuts, round, u, hi;
     __device__ __forceinline__ int first_unit(int b) const { return (int)((long long)b * U / cuts); }
     __device__ __forceinline__ Schedule(int total_, int KB, const GemmArgs& a) : total(total_) {
-        const int G = (int)gridDim.x;
+        const int G = (int)gridDim.x / CTAS;
         m = (KB + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;
         full = total / G;
         R = total - full * G;
@@ -318,9 +369,9 @@ struct Schedule {
         cuts = 0;
         round = 0;
         u = hi = 0;
-        if (R > 0 && a.part && (long long)(G - R) * m >= 2ll * G && (long long)R * m <= a.part_blocks) {
+        if (R > 0 && a.part && (long long)(G - R) * m >= 2ll * G && (long long)R * m * CTAS <= a.part_blocks) {
             cuts = min(G, U);
-            const int b = (int)blockIdx.x;
+            const int b = (int)blockIdx.x / CTAS;
             if (b < cuts) {
                 u = first_unit(b);
                 hi = first_unit(b + 1);
@@ -328,7 +379,7 @@ struct Schedule {
         }
     }
     __device__ __forceinline__ bool next(Item& it) {
-        const int G = (int)gridDim.x, b = (int)blockIdx.x;
+        const int G = (int)gridDim.x / CTAS, b = (int)blockIdx.x / CTAS;
         if (round < full || (cuts == 0 && round == full)) {
             it.tile = round * G + ((round & 1) ? G - 1 - b : b);
             it.c0 = 0;
@@ -354,11 +405,11 @@ struct Schedule {
     }
 };
 
-template <int EPI, int NMAX, int STAGES>
+template <int EPI, int NMAX, int STAGES, int CTAS>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ TokenMaps token_maps,
                 const GemmArgs args) {
-    using C = Cfg<NMAX, STAGES>;
+    using C = Cfg<NMAX, STAGES, CTAS>;
     extern __shared__ uint8_t smem_raw[];
     // k block `it` (counted over all items of the CTA) uses stage it % STAGES; chunks rotate over the accumulators
     __shared__ __align__(8) uint64_t s_full[STAGES];        // TMA -> MMA: stage filled
@@ -375,7 +426,10 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int MB = (args.M_total + UMMA_M - 1) / UMMA_M;
+    const int MB1 = (args.M_total + UMMA_M - 1) / UMMA_M;    // 128-row weight blocks
+    const int MB = (MB1 + CTAS - 1) / CTAS;                  // of which a tile has CTAS
+    uint32_t rank = 0;
+    if (CTAS > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int KB = (args.K + BK - 1) / BK;
 
     if (threadIdx.x == 0) {
@@ -385,16 +439,23 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
         for (int b = 0; b < C::MAX_ACC; ++b) {
             mbar_init(smem_u32(&s_acc_full[b]), 1);
-            mbar_init(smem_u32(&s_acc_empty[b]), EPI_WARPS);
+            mbar_init(smem_u32(&s_acc_empty[b]), EPI_WARPS * CTAS);
         }
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == MMA_WARP) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
-                     "r"((uint32_t)TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CTAS == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                         "r"((uint32_t)TMEM_COLS)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                         "r"((uint32_t)TMEM_COLS)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
     }
     pdl_trigger();
     pdl_wait();
@@ -420,7 +481,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             int nt = 0;
             if (e < args.E) {
                 int nch, csz;
-                chunking<NMAX>(s_cnt[s_order[e]], nch, csz);
+                chunking<NMAX, C::N_STEP>(s_cnt[s_order[e]], nch, csz);
                 nt = nch * MB;
                 widest = max(widest, csz);
             }
@@ -441,12 +502,13 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
     tc_fence_before();
     __syncthreads();
+    if (CTAS > 1) cluster_sync();    // the barriers of both CTAs are ready
     tc_fence_after();
     const uint32_t tmem_base = s_tmem_base;
     // as many accumulators as fit beside one another at the width of the widest token tile
     const uint32_t acc_stride = (uint32_t)s_widest, nacc = min((uint32_t)C::MAX_ACC, (uint32_t)TMEM_COLS / acc_stride);
     volatile int* abort_flag = &s_abort;
-    Schedule sched(s_prefix[args.E], KB, args);
+    Schedule<CTAS> sched(s_prefix[args.E], KB, args);
     Item item;
 
     if (warp == TMA_WARP) {
@@ -455,20 +517,30 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             uint32_t it = 0;
             bool ok = true;
             while (ok && sched.next(item) && !*abort_flag) {
-                const TileInfo t = decode_tile<NMAX>(item.tile, s_prefix, s_order, args);
+                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, args);
                 // a box of n_pad token rows (rows past the chunk's tokens belong to the next expert or are
                 // zero-filled past the end; they only feed accumulator columns that are never stored)
-                const CUtensorMap* map_pk = &token_maps.pk[(t.n_pad >> 4) - 1];
-                const uint32_t bytes = W_TILE + t.n_pad * ROW_BYTES;
-                const int w_row0 = (int)(args.w_stride / BK) * t.slot + t.mb * KB * UMMA_M;
+                const int n_own = t.n_pad / CTAS;
+                const CUtensorMap* map_pk = &token_maps.pk[(n_own >> 4) - 1];
+                const uint32_t bytes = W_TILE + n_own * ROW_BYTES;
+                // a second CTA past the last weight block loads that block again and drops the result
+                const int mb = min(t.mb * CTAS + (int)rank, MB1 - 1);
+                const int w_row0 = (int)(args.w_stride / BK) * t.slot + mb * KB * UMMA_M;
                 const int kb_end = min(KB, item.c1 * CHUNK_BLOCKS);
                 for (int kb = item.c0 * CHUNK_BLOCKS; kb < kb_end; ++kb, ++it) {
                     const uint32_t s = it % STAGES;
                     if (!mbar_wait(smem_u32(&s_empty[s]), ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
                     const uint32_t bar = smem_u32(&s_full[s]), dst = ring + s * C::STAGE;
-                    mbar_expect_tx(bar, bytes);
-                    tma_load_2d(dst, &map_w, bar, 0, w_row0 + kb * UMMA_M);
-                    tma_load_2d(dst + W_TILE, map_pk, bar, kb * 2 * BK, t.row0);
+                    if (CTAS == 1) {
+                        mbar_expect_tx(bar, bytes);
+                        tma_load_2d(dst, &map_w, bar, 0, w_row0 + kb * UMMA_M);
+                        tma_load_2d(dst + W_TILE, map_pk, bar, kb * 2 * BK, t.row0);
+                    } else {
+                        if (rank == 0) mbar_expect_tx(bar, CTAS * bytes);
+                        const uint32_t lead = leader_addr(bar);
+                        tma_load_2d_pair(dst, &map_w, lead, 0, w_row0 + kb * UMMA_M);
+                        tma_load_2d_pair(dst + W_TILE, map_pk, lead, kb * 2 * BK, t.row0 + (int)rank * n_own);
+                    }
                 }
             }
         }
@@ -478,12 +550,16 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // issuing, the operands of every MMA had to be moved to uniform registers behind a divergent branch: ~148
         // cycles per MMA whatever its N, which held a decode step of 27 experts at 1694 us of first GEMM where the
         // same bytes stream in 1269.  Elected: 1259 us (7.2 TB/s); 4096 tokens 2780 -> 2383.
-        if (elect_one()) {
+        if (rank == 0 && elect_one()) {
+            auto commit = [](uint32_t bar) {
+                if (CTAS == 1) umma_commit(bar);
+                else umma_commit_pair(bar);
+            };
             uint32_t it = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             while (ok && sched.next(item) && !*abort_flag) {
-                const TileInfo t = decode_tile<NMAX>(item.tile, s_prefix, s_order, args);
-                const uint32_t idesc = make_idesc(t.n_pad);
+                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, args);
+                const uint32_t idesc = make_idesc(UMMA_M * CTAS, t.n_pad);
                 for (int c = item.c0; ok && c < item.c1; ++c) {
                     const uint32_t d = tmem_base + acc * acc_stride;
                     if (!mbar_wait(smem_u32(&s_acc_empty[acc]), acc_phase ^ 1, abort_flag)) { ok = false; break; }
@@ -495,15 +571,15 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         const uint64_t dw = make_smem_desc(ring + s * C::STAGE), dx = make_smem_desc(ring + s * C::STAGE + W_TILE);
                         // In a row hi is bytes 0..63, lo bytes 64..127; 32 bytes along K = 2 units of the descriptor
                         // address.  Corrections first (small terms).
-                        umma_f16_ss(d, dw + 4, dx, idesc, kb == kb0 ? 0u : 1u);
-                        umma_f16_ss(d, dw + 6, dx + 2, idesc, 1u);
+                        umma_f16<CTAS>(d, dw + 4, dx, idesc, kb == kb0 ? 0u : 1u);
+                        umma_f16<CTAS>(d, dw + 6, dx + 2, idesc, 1u);
 #pragma unroll
                         for (int j = 0; j < 2; ++j) {
-                            umma_f16_ss(d, dw + 2 * j, dx + 4 + 2 * j, idesc, 1u);
-                            umma_f16_ss(d, dw + 2 * j, dx + 2 * j, idesc, 1u);
+                            umma_f16<CTAS>(d, dw + 2 * j, dx + 4 + 2 * j, idesc, 1u);
+                            umma_f16<CTAS>(d, dw + 2 * j, dx + 2 * j, idesc, 1u);
                         }
-                        umma_commit(smem_u32(&s_empty[s]));
-                        if (kb + 1 == kb_end) umma_commit(smem_u32(&s_acc_full[acc]));
+                        commit(smem_u32(&s_empty[s]));
+                        if (kb + 1 == kb_end) commit(smem_u32(&s_acc_full[acc]));
                     }
                     if (++acc == nacc) {
                         acc = 0;
@@ -524,7 +600,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
         while (ok && sched.next(item) && !*abort_flag) {
-            const TileInfo t = decode_tile<NMAX>(item.tile, s_prefix, s_order, args);
+            const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, args);
             const int nsl = t.n_pad >> 4;
             float sum[C::SLICES][16];
 #pragma unroll
@@ -533,7 +609,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int c = 0; c < 16; ++c) sum[i][c] = 0.f;
             const int row = q * 32 + lane;      // row of the tile this thread works on
             const size_t block = (size_t)(args.part_cols >> 2) * UMMA_M;   // float4 per block of chunk sums
-            float4* const part = item.tail >= 0 ? args.part + (size_t)item.tail * sched.m * block + row : nullptr;
+            float4* const part = item.tail >= 0 ? args.part + ((size_t)item.tail * CTAS + rank) * sched.m * block + row : nullptr;
             auto store_block = [&](int c) {     // sum[][] -> block of chunk c
 #pragma unroll
                 for (int i = 0; i < C::SLICES; ++i) {
@@ -564,7 +640,10 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&s_acc_empty[acc]));
+                if (lane == 0) {
+                    if (CTAS == 1) mbar_arrive(smem_u32(&s_acc_empty[acc]));
+                    else mbar_arrive_cluster(leader_addr(smem_u32(&s_acc_empty[acc])));
+                }
                 if (++acc == nacc) {
                     acc = 0;
                     acc_phase ^= 1;
@@ -584,7 +663,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 __threadfence();
                 __syncwarp();
                 int done = 0;
-                int* const counter = args.part_count + item.tail * EPI_WARPS + (warp - EPI_WARP0);
+                int* const counter = args.part_count + (item.tail * CTAS + rank) * EPI_WARPS + (warp - EPI_WARP0);
                 if (lane == 0) {
                     done = atomicAdd(counter, item.c1 - item.c0) + item.c1 - item.c0;
                     if (done == sched.m) *counter = 0;    // everybody has arrived; ready for the next launch
@@ -611,10 +690,12 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     }
                 }
             }
-            const int m = t.mb * UMMA_M + row;
+            const int mb = t.mb * CTAS + (int)rank;
+            if (mb >= MB1) continue;
+            const int m = mb * UMMA_M + row;
             const bool m_ok = m < args.M_total;
             // 2^-s of the weight row (padding rows have one too)
-            const float w_inv = __ldg(args.w + (size_t)t.slot * args.w_stride + (size_t)MB * KB * (UMMA_M * BK) + m);
+            const float w_inv = __ldg(args.w + (size_t)t.slot * args.w_stride + (size_t)MB1 * KB * (UMMA_M * BK) + m);
             const float bound = decode_bound(__ldg(args.bound + (size_t)t.slot * args.bound_stride));
 #pragma unroll
             for (int i = 0; i < C::SLICES; ++i) {
@@ -705,10 +786,15 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         while (global_ns() - t0 < 200000ull) __nanosleep(1000);
         __syncthreads();
     }
+    if (CTAS > 1) cluster_sync();    // nobody touches the other CTA's shared or tensor memory any more
     if (warp == MMA_WARP) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS)
-                     : "memory");
+        if (CTAS == 1)
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS)
+                         : "memory");
+        else
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS)
+                         : "memory");
     }
 }
 
@@ -784,13 +870,13 @@ int token_maps(TokenMaps* out, const void* pack, int K, long long T) {
     return INFMOE_OK;
 }
 
-template <int EPI, int NMAX, int STAGES>
+template <int EPI, int NMAX, int STAGES, int CTAS>
 int launch_one(GemmArgs args, long long T, int slots, const void* tokens, size_t part_bytes, int num_ctas,
                cudaStream_t stream) {
-    using C = Cfg<NMAX, STAGES>;
+    using C = Cfg<NMAX, STAGES, CTAS>;
     static_assert(C::SMEM + 12288 <= 227 * 1024, "shared-memory ring too large");
-    static_assert(NMAX <= 16 * TOKEN_BOXES, "a token tile needs a tensor map of its height");
-    args.part_cols = (int)(T < NMAX ? (T + 15) / 16 * 16 : NMAX);
+    static_assert(NMAX / CTAS <= 16 * TOKEN_BOXES, "a token tile needs a tensor map of its height");
+    args.part_cols = (int)(T < NMAX ? (T + C::N_STEP - 1) / C::N_STEP * C::N_STEP : NMAX);
     const size_t blocks = part_bytes / ((size_t)args.part_cols * UMMA_M * sizeof(float));
     args.part_blocks = (int)(blocks < 0x7fffffff ? blocks : 0x7fffffff);
     CUtensorMap map_w;
@@ -798,9 +884,9 @@ int launch_one(GemmArgs args, long long T, int slots, const void* tokens, size_t
     // weights: the plane as a [rows][32] matrix of 128-byte rows, one 16 KB tile per box
     INFMOE_TRY(make_map(&map_w, args.w, BK, (uint64_t)slots * (args.w_stride / BK), UMMA_M));
     INFMOE_TRY(token_maps(&tm, tokens, args.K, T));
-    auto kern = ffn_umma_kernel<EPI, NMAX, STAGES>;
+    auto kern = ffn_umma_kernel<EPI, NMAX, STAGES, CTAS>;
     INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)num_ctas, GEMM_THREADS, C::SMEM, 1, stream, map_w, tm, args));
+    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)(num_ctas / CTAS * CTAS), GEMM_THREADS, C::SMEM, CTAS, stream, map_w, tm, args));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
@@ -883,18 +969,27 @@ int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_be
     a2.out_pos = f.out_pos;
     a2.mix_score = f.mix_score;
     a2.out_row_ptr = f.out_row_ptr;
-    // Token chunk and ring.  With few tokens per expert the token tiles are small, so the ring holds more, smaller
-    // stages: 128 KB of weights on their way per SM instead of 80 KB.
+    // Token chunk, ring and CTAs per tile.
+    //   few tokens per expert   64 columns, so that the ring holds more, smaller stages: 128 KB of weights on their way
+    //                           per SM instead of 80 KB
+    //   K from 2048             pairs of CTAs on tiles of 256 weight rows (cta_group::2).  Each CTA fetches and holds half of
+    //                           the token tile, so shared memory takes 63 instead of 78 KB of traffic per k block of 144
+    //                           tokens and L2 half the token reads; where the GPU is at its power cap that is time.
+    //                           Layer, us, one CTA / pairs: 4096 tokens 32 x 4096 x 10240 4173 / 3900, 16384 tokens
+    //                           12485 / 11651; second GEMM of 777 x 12 x 1000 x 2724 (K = 2724) 52 / 47
+    //   shorter K               one CTA: token tiles of a pair are multiples of 32, and the epilogue, not the MMAs, is in
+    //                           front; first GEMM, us: K = 1024, 16 experts x 4096, 1000 tokens 104 / 112, K = 680, 6
+    //                           experts, 4640 tokens 65 / 80
     const bool small = T <= 64 || T <= 16ll * (e_end - e_begin);
-#define INFMOE_LAUNCH_PAIR(NMAX, STAGES)                                                                             \
-    do {                                                                                                             \
-        INFMOE_TRY((launch_one<EPI_GELU_PAIR, NMAX, STAGES>(a1, T, f.slots, f.h, f.part_bytes, num_sms, stream)));   \
-        if (mid_event) INFMOE_CUDA_TRY(cudaEventRecord(mid_event, stream));                                          \
-        INFMOE_TRY((launch_one<EPI_RESIDUAL, NMAX, STAGES>(a2, T, f.slots, f.g, f.part_bytes, num_sms, stream)));    \
-    } while (0)
-    if (small) INFMOE_LAUNCH_PAIR(64, 8);
-    else INFMOE_LAUNCH_PAIR(192, 5);
-#undef INFMOE_LAUNCH_PAIR
+    const auto pick = [&](auto epi, const GemmArgs& a, const void* tokens) -> int {
+        constexpr int EPI = decltype(epi)::value;
+        if (small) return launch_one<EPI, 64, 8, 1>(a, T, f.slots, tokens, f.part_bytes, num_sms, stream);
+        if (a.K >= 2048) return launch_one<EPI, 192, 7, 2>(a, T, f.slots, tokens, f.part_bytes, num_sms, stream);
+        return launch_one<EPI, 192, 5, 1>(a, T, f.slots, tokens, f.part_bytes, num_sms, stream);
+    };
+    INFMOE_TRY(pick(std::integral_constant<int, EPI_GELU_PAIR>(), a1, f.h));
+    if (mid_event) INFMOE_CUDA_TRY(cudaEventRecord(mid_event, stream));
+    INFMOE_TRY(pick(std::integral_constant<int, EPI_RESIDUAL>(), a2, f.g));
     return INFMOE_OK;
 }
 
@@ -903,7 +998,7 @@ int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_be
 size_t ffn_umma_part_bytes(long long T, int D, int F) {
     const int K = D > F ? D : F;
     const size_t chunks = (size_t)((K + BK - 1) / BK + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;
-    const size_t cols = (size_t)(T < 192 ? (T + 15) / 16 * 16 : 192);
+    const size_t cols = (size_t)(T < 256 ? (T + 31) / 32 * 32 : 256);
     const size_t need = (size_t)FFN_CTAS * chunks * cols * UMMA_M * sizeof(float);
     return need < (64u << 20) ? need : (size_t)(64u << 20);
 }

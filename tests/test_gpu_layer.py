@@ -625,3 +625,40 @@ def test_pass_under_capture_between_other_kernels():
         assert torch.equal(acc, ref)
     layer.sync_status()
     layer.terminate()
+
+
+# Second GEMM (K = d_ff >= 2048) and first GEMM (K = d_model >= 2048) on pairs of CTAs: an odd number of 128-row weight
+# blocks (the pair's second CTA has nothing to write), token tiles of 32, 64 and 192 columns with remainders, experts
+# without tokens, and the K just below the line.
+@pytest.mark.parametrize("D,F", [(640, 2048), (2048, 192), (132, 2044), (2080, 2080)])
+def test_paired_tiles_against_oracle(oracle, D, F):
+    import torch
+    from infmoe_b200 import MoELayer
+    counts = (0, 1, 31, 33, 192, 193, 0, 70)
+    rng = np.random.default_rng(D + F)
+    E, n = len(counts), sum(counts)
+    layer = MoELayer.create(E, D, F, 2, np.ones((E, D), np.float32), None, "T5_FF", "default", None)
+    experts = []
+    for e in range(E):
+        experts.append([(1 + 0.01 * rng.standard_normal(D)).astype(np.float32)] +
+                       [(rng.standard_normal((F, D)) / np.sqrt(D)).astype(np.float32) for _ in range(2)] +
+                       [(rng.standard_normal((D, F)) / np.sqrt(F)).astype(np.float32)])
+        layer.set_expert(e, *(torch.from_numpy(a).cuda() for a in experts[e]))
+    gate = rng.permutation(np.repeat(np.arange(E, dtype=np.int32), counts))
+    x = rng.standard_normal((n, D)).astype(np.float32)
+    dx, dg = torch.from_numpy(x).cuda(), torch.from_numpy(gate).cuda()
+    out = [layer.expert_forward(dx, dg).cpu().numpy() for _ in range(3)]
+    layer.sync_status()
+    # the same rows among fewer: one CTA per tile, 64 columns, with the same additions
+    few = np.sort(rng.choice(n, 60, replace=False))
+    alone = layer.expert_forward(dx[few].contiguous(), dg[few].contiguous()).cpu().numpy()
+    layer.sync_status()
+    layer.terminate()
+    np.testing.assert_array_equal(out[1], out[0])
+    np.testing.assert_array_equal(out[2], out[0])
+    np.testing.assert_array_equal(alone, out[0][few])
+    for e in range(E):
+        rows = np.flatnonzero(gate == e)[:24]
+        if rows.size:
+            want = oracle.expert_ffn_f64(x[rows], *experts[e])
+            assert oracle.rel_l2(out[0][rows], want) <= TOL
