@@ -74,7 +74,8 @@ inline cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsign
 // soon as every block of the predecessor has started (pdl_trigger) and left room, do what needs no memory, and wait
 // in pdl_wait until the predecessor has completed and its writes are visible.  Every block of every kernel launched
 // this way calls pdl_wait before it touches global memory; the predecessor did the same, so all earlier kernels of the
-// stream are complete too.  (Without the launch attribute both are no-ops.)
+// stream are complete too.  (Without the launch attribute both are no-ops.)  One kernel reads memory before its wait, the
+// second expert GEMM; see there.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
