@@ -630,7 +630,7 @@ route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // normalised token rows in shared memory, and the butterfly over the lanes is the canonical reduction.  The CTAs' best
 // candidates meet in the first one through distributed shared memory.  Same additions in the same order as above.
 // Each centroid is read once per RS_TOKENS tokens, from L2, and a shared-memory load feeds only four multiply-adds:
-// past the line in use_small_route the kernels above win.
+// past the line in use_small_route the other kernels win.
 // One token, d_model 4096, 32 experts: 47 -> 9.6 us; 64 tokens 52 -> 12.5; d_model 1024, 8 experts: 13 -> 3.5.
 constexpr int RS_TOKENS = 4;
 constexpr int RS_THREADS = 256;
@@ -757,6 +757,171 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Many tokens, rows of up to 2048 floats.  A warp keeps TOKENS rows in registers (the 32 lanes are the 32 partial
+// indices l, 128 registers of row values per lane whatever the row length), so a row crosses HBM once, its statistics and
+// LayerNorm need no shared memory, and all that moves is the centroids: staged into shared memory 8 experts at a time
+// (cp.async, two buffers) and read by every warp, one 128-bit load for 4 TOKENS multiply-adds.  32 scores (tokens x
+// experts) at a time end in a transposed butterfly: in the step over bit b of l a lane hands half of its values to its
+// partner and adds the other half, so 31 shuffles reduce 32 values, each over the canonical pairs of lanes, and lane i
+// ends up with score i.
+// Bound by shared-memory reads and FMA issue about equally with four rows per warp, by the reads with two.  The tiled
+// kernel above reads a row twice and normalises it in shared memory, and multiplies 32 experts at a time however few
+// there are.  us, tiled / this: (D, E, tokens) (1024, 8, 4096) 18.7 / 8.5, (1024, 8, 16384) 72 / 28, (1024, 16, 4096)
+// 19.2 / 11.1, (256, 8, 16384) 24.5 / 9.5, (1024, 64, 16384) 93 / 82.
+constexpr int RR_THREADS = 256;
+constexpr int RR_STAGE_EXPERTS = 8;
+
+template <int TOKENS, int NV>
+__global__ void __launch_bounds__(RR_THREADS, 1)
+route_rows_kernel(const float* __restrict__ X, const float* __restrict__ C, const float* __restrict__ gamma,
+                  long long T, int D, int E, int* __restrict__ gate, float* __restrict__ score,
+                  int* __restrict__ status) {
+    constexpr int EB = 32 / TOKENS;                            // experts per reduction
+    constexpr int SUBS = EB / RR_STAGE_EXPERTS;                // of RR_STAGE_EXPERTS experts each
+    constexpr int PITCH = NV * 32;                             // float4 per staged centroid
+    extern __shared__ __align__(16) float4 rr_c[];             // [2][RR_STAGE_EXPERTS][PITCH]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long t0 = ((long long)blockIdx.x * (RR_THREADS / 32) + warp) * TOKENS;
+    const int stages = (E + RR_STAGE_EXPERTS - 1) / RR_STAGE_EXPERTS;
+    auto fetch = [&](int stage) {
+        float4* buf = rr_c + (stage & 1) * RR_STAGE_EXPERTS * PITCH;
+        for (int i = tid; i < RR_STAGE_EXPERTS * PITCH; i += RR_THREADS) {
+            const int e = stage * RR_STAGE_EXPERTS + i / PITCH, k = 4 * (i % PITCH);
+            const bool ok = e < E && k < D;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(buf + i);
+            const int bytes = ok ? 16 : 0;                     // the rest of the 16 bytes is zero-filled
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                         ::"r"(dst), "l"(C + (ok ? (long long)e * D + k : 0)), "r"(bytes)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    pdl_trigger();
+    pdl_wait();
+    fetch(0);
+    float4 x[TOKENS][NV];
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int k = 4 * lane + 128 * i;
+            x[t][i] = (t0 + t < T && k < D) ? *reinterpret_cast<const float4*>(X + (t0 + t) * (long long)D + k)
+                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    if (gamma) {                 // the additions of warp_row_stats, from registers
+        float mean[TOKENS], rstd[TOKENS];
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t) {
+            float s = 0.f;
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                if (4 * lane + 128 * i < D)
+                    s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[t][i].x), x[t][i].y), x[t][i].z), x[t][i].w);
+            mean[t] = __fdiv_rn(warp_xor_sum(s), (float)D);
+        }
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t) {
+            float q = 0.f;
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                if (4 * lane + 128 * i < D) {
+                    float d = __fsub_rn(x[t][i].x, mean[t]);
+                    q = __fmaf_rn(d, d, q);
+                    d = __fsub_rn(x[t][i].y, mean[t]);
+                    q = __fmaf_rn(d, d, q);
+                    d = __fsub_rn(x[t][i].z, mean[t]);
+                    q = __fmaf_rn(d, d, q);
+                    d = __fsub_rn(x[t][i].w, mean[t]);
+                    q = __fmaf_rn(d, d, q);
+                }
+            rstd[t] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(warp_xor_sum(q), (float)D), 1e-6f)));
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int k = 4 * lane + 128 * i;
+            if (k >= D) continue;
+            const float4 g = *reinterpret_cast<const float4*>(gamma + k);
+#pragma unroll
+            for (int t = 0; t < TOKENS; ++t) {
+                x[t][i].x = ln_apply(x[t][i].x, mean[t], rstd[t], g.x);
+                x[t][i].y = ln_apply(x[t][i].y, mean[t], rstd[t], g.y);
+                x[t][i].z = ln_apply(x[t][i].z, mean[t], rstd[t], g.z);
+                x[t][i].w = ln_apply(x[t][i].w, mean[t], rstd[t], g.w);
+            }
+        }
+    }
+
+    float best = -FLT_MAX;       // reference plugin/cuda/moe.cu:26-27; this lane's token is lane % TOKENS
+    int best_e = -1;
+    for (int e0 = 0; e0 < E; e0 += EB) {
+        float acc[32];           // [expert][token]
+#pragma unroll
+        for (int v = 0; v < 32; ++v) acc[v] = 0.f;
+#pragma unroll
+        for (int sub = 0; sub < SUBS; ++sub) {
+            const int stage = e0 / RR_STAGE_EXPERTS + sub;
+            if (stage >= stages) break;
+            if (stage + 1 < stages) {
+                fetch(stage + 1);    // its buffer was left by everybody before the barrier that ended stage - 1
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            const float4* buf = rr_c + (stage & 1) * RR_STAGE_EXPERTS * PITCH + lane;
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                if (128 * i >= D) break;
+#pragma unroll
+                for (int e = 0; e < RR_STAGE_EXPERTS; ++e) {
+                    const float4 c = buf[e * PITCH + 32 * i];
+#pragma unroll
+                    for (int t = 0; t < TOKENS; ++t) {
+                        float& a = acc[(sub * RR_STAGE_EXPERTS + e) * TOKENS + t];
+                        a = __fmaf_rn(x[t][i].x, c.x, a);
+                        a = __fmaf_rn(x[t][i].y, c.y, a);
+                        a = __fmaf_rn(x[t][i].z, c.z, a);
+                        a = __fmaf_rn(x[t][i].w, c.w, a);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) {
+            const bool upper = lane & off;
+#pragma unroll
+            for (int v = 0; v < off; ++v) {
+                const float keep = upper ? acc[v + off] : acc[v], give = upper ? acc[v] : acc[v + off];
+                acc[v] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, off));
+            }
+        }
+        // lane = (expert e0 + lane / TOKENS, token lane % TOKENS); candidates and ties as in the kernels above
+        float cand = acc[0];
+        int cand_e = e0 + lane / TOKENS;
+        if (cand_e >= E || !(cand > best)) cand_e = -1;
+#pragma unroll
+        for (int off = 16; off >= TOKENS; off >>= 1) {
+            const float os = __shfl_xor_sync(0xffffffffu, cand, off);
+            const int oe = __shfl_xor_sync(0xffffffffu, cand_e, off);
+            if (rs_better(os, oe, cand, cand_e)) {
+                cand = os;
+                cand_e = oe;
+            }
+        }
+        if (cand_e >= 0) {
+            best = cand;
+            best_e = cand_e;
+        }
+    }
+    if (lane < TOKENS && t0 + lane < T) {
+        gate[t0 + lane] = best_e;
+        if (score) score[t0 + lane] = best;
+        if (best_e < 0 && status) atomicOr(status, STATUS_NO_EXPERT);
+    }
+}
+
 // Top-1 over a materialised score matrix (one warp per token; lanes scan
 // strided expert indices and the lowest index wins ties, which equals the
 // reference's sequential strict '>' scan).
@@ -829,12 +994,18 @@ int route_maps(CUtensorMap* mx, CUtensorMap* mc, const float* X, const float* C,
 
 namespace {
 inline size_t rs_smem(int D) { return (size_t)RS_TOKENS * (size_t)((D + 127) / 128) * 512; }
-// The small kernel's time grows with T E once its clusters fill the chip, the tiled kernels' (up to 32 tokens per SM)
-// with D alone.  Measured, small against tiled, us (D, E; T): (4096, 32) 512: 35 / 52, 1024: 52 / 52; (1024, 64) 256:
-// 10.5 / 24, 512: 14.6 / 24, 1024: 27 / 24.5; (2048, 16) 1024: 17 / 29, 2048: 26 / 30; (1000, 12) 1024: 8.8 / 13.3, 2048:
-// 13.9 / 13.5; (1024, 8) 2048: 9.6 / 13.5, 4096: 14.6 / 14.1; (64, 4) 2048: 5.4 / 6.3, 4096: 7.6 / 6.7.
-bool use_small_route(long long T, int D, int E) {
-    return T * (E < 8 ? 8 : E) < 24576 && rs_smem(D) <= RS_MAX_SMEM;
+// Two rows per warp instead of four make the rows kernel wait for shared memory: with 32 experts and 2048 floats it takes
+// 39 us for 4096 tokens, where the tiled one multiplies all 32 at the price of one (31 us with 16).
+bool route_rows_supported(int D, int E, bool vec) { return vec && (D <= 1024 || (D <= 2048 && E <= 16)); }
+// The small kernel's time grows with T E once its clusters fill the chip, that of the others with a CTA's (32 tokens or
+// 16) until those do.  Measured, us (D, E; T).  Small against rows in registers: (1024, 8) 1024: 6.5 / 8.1, 2048: 11.2 /
+// 8.0; (2048, 8) 512: 5.9 / 6.0, 1024: 7.6 / 6.0; (1024, 16) 512: 6.8 / 10.3, 1024: 10.9 / 10.3; (512, 32) 512: 10.7 / 11.1;
+// (1024, 64) 256: 9.8 / 21, 512: 14.2 / 21, 1024: 27 / 21.  Small against tiled: (4096, 32) 512: 35 / 52, 1024: 52 / 52;
+// (4096, 8) 4096: 49 / 55, 16384: 185 / 233.
+bool use_small_route(long long T, int D, int E, bool rows) {
+    const long long e = E < 8 ? 8 : E;
+    if (rs_smem(D) > RS_MAX_SMEM) return false;
+    return rows ? T < 256 + 8192 / e : T * e < 24576 || E <= 8;
 }
 template <bool VEC>
 int launch_route_small(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
@@ -847,6 +1018,17 @@ int launch_route_small(const float* X, const float* C, const float* gamma, long 
         INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_MAX_SMEM));
     INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)((T + RS_TOKENS - 1) / RS_TOKENS * cluster), RS_THREADS, smem,
                                    (unsigned)cluster, stream, X, C, gamma, T, D, E, gate, score, status));
+    return INFMOE_OK;
+}
+template <int TOKENS, int NV>
+int launch_route_rows(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
+                      float* score, int* status, cudaStream_t stream) {
+    constexpr int smem = 2 * RR_STAGE_EXPERTS * NV * 32 * 16;
+    auto kern = route_rows_kernel<TOKENS, NV>;
+    INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const long long per_cta = RR_THREADS / 32 * TOKENS;
+    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)((T + per_cta - 1) / per_cta), RR_THREADS, smem, 1, stream, X, C, gamma, T,
+                                   D, E, gate, score, status));
     return INFMOE_OK;
 }
 }  // namespace
@@ -862,9 +1044,13 @@ int launch_route(const float* X, const float* C, const float* gamma, long long T
     const long long grid = (T + RT_TOKENS - 1) / RT_TOKENS;
     static const bool no_tma = [] { const char* v = getenv("INFMOE_ROUTE"); return v && !strcmp(v, "cp_async"); }();
     CUtensorMap map_x, map_c;
-    if (use_small_route(T, D, E)) {
+    const bool rows = route_rows_supported(D, E, vec);
+    if (use_small_route(T, D, E, rows)) {
         INFMOE_TRY((vec ? launch_route_small<true> : launch_route_small<false>)(X, C, gamma, T, D, E, gate, score,
                                                                                status, stream));
+    } else if (rows) {
+        INFMOE_TRY((D <= 1024 ? launch_route_rows<4, 8> : launch_route_rows<2, 16>)(X, C, gamma, T, D, E, gate, score,
+                                                                                    status, stream));
     } else if (vec && !no_tma && T < (1ll << 31) && route_maps(&map_x, &map_c, X, C, T, D, E) == INFMOE_OK) {
         INFMOE_CUDA_TRY(cudaFuncSetAttribute(route_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM + 1024));
         INFMOE_CUDA_TRY(launch_chained(route_tma_kernel, (unsigned)grid, RT_THREADS, RT_SMEM + 1024, 1, stream, map_x, map_c,

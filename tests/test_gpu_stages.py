@@ -51,12 +51,18 @@ def test_route_bit_exact(g, oracle, T, D, E, ln):
 
 
 # The few-token kernel: tokens per cluster (4), experts per CTA and warp (8), a centroid row of one, just under and just
-# over 128 floats, its longest row (12800 floats) and one past it; and the tiled kernels, which now start at
-# T * max(E, 8) = 24576, aligned and unaligned.
+# over 128 floats, its longest row (12800 floats) and one past it; and the other kernels from where they start on,
+# aligned and unaligned.
 @pytest.mark.parametrize("T,D,E,ln", [(1, 4, 1, False), (3, 127, 7, True), (4, 128, 8, True), (5, 132, 9, False),
                                       (9, 510, 65, True), (2, 64, 300, True), (6, 12800, 3, True), (6, 12804, 3, True),
-                                      (3071, 36, 8, True), (3072, 36, 8, True), (3100, 510, 5, True),
-                                      (800, 516, 33, False)])
+                                      (1279, 36, 8, True), (1280, 36, 8, True), (3100, 510, 9, True),
+                                      (800, 516, 33, False),
+                                      # rows in registers: four rows of up to 1024 floats or two of up to 2048 per
+                                      # warp, 8 or 16 experts per reduction; one expert or one float4 past, the tiled
+                                      # kernel
+                                      (4001, 1024, 9, True), (3075, 4, 8, False), (900, 1028, 16, True),
+                                      (1000, 2048, 16, True), (2500, 1500, 15, False), (1500, 2048, 17, True),
+                                      (700, 2052, 40, True)])
 def test_route_few_and_many_tokens(g, oracle, T, D, E, ln):
     test_route_bit_exact(g, oracle, T, D, E, ln)
 
