@@ -49,7 +49,7 @@ from infmoe_b200 import synth  # noqa: E402
 # capture of workload cpm2_profile (profiles/ffn_umma_kernel_cpm2_profile.md) divided by the weight elements that
 # launch streams; 4 = each raw FP32 weight crosses HBM once.  It is a figure from that capture, scaled by the
 # elements this launch streams -- it is not measured by this run.
-TRAFFIC_BYTES_PER_WEIGHT = 4.27
+TRAFFIC_BYTES_PER_WEIGHT = 4.16
 TRAFFIC_SOURCE = "ncu capture of cpm2_profile (profiles/ffn_umma_kernel_cpm2_profile.md), bytes per weight element x elements streamed"
 
 METRIC = "moe_layer_tokens_per_s"
@@ -244,20 +244,20 @@ def ref_gpu_baseline(w, torch, sample_experts=8, reps=3):
 def gemm_roofline(kernel, achieved_tflops, kernel_ms, peaks, clock_summary, timed_s):
     """Roofline object of the grouped expert GEMM.
 
-    `peak` is the ceiling of the MMAs this kernel actually issues: per product one TF32 MMA (half the bf16 rate) and
-    two BF16 MMAs with K = 16 (the bf16 rate), i.e. measured bf16 / 4.  The burst figure is the denominator while the
+    `peak` is the ceiling of the MMAs this kernel actually issues: per product three FP16 MMAs with K = 16 (the bf16
+    rate), i.e. measured bf16 / 3.  The burst figure is the denominator while the
     timed region is short and the SM clock sampled during it stays near its maximum; a long region that runs into
     the power cap is held against the sustained figure.  `frac_3xtf32` is against what plain 3xTF32 (three TF32 MMAs
-    per product, the arithmetic the kernel replaces) could reach: bf16 / 6."""
+    per product) could reach: bf16 / 6."""
     sm, mx = clock_summary.get("sm_mhz"), clock_summary.get("sm_max_mhz")
     burst = timed_s < 1.0 and sm is not None and mx and sm >= 0.9 * mx
     bf16 = peaks["bf16_tflops"] if burst else peaks["bf16_sustained"]
     regime = "burst" if burst else "sustained"
-    return {"kernel": kernel, "bound": "tensor", "achieved": achieved_tflops, "peak": bf16 / 4.0, "unit": "TFLOP/s",
-            "frac": achieved_tflops / (bf16 / 4.0), "peak_3xtf32": bf16 / 6.0,
+    return {"kernel": kernel, "bound": "tensor", "achieved": achieved_tflops, "peak": bf16 / 3.0, "unit": "TFLOP/s",
+            "frac": achieved_tflops / (bf16 / 3.0), "peak_3xtf32": bf16 / 6.0,
             "frac_3xtf32": achieved_tflops / (bf16 / 6.0),
-            "peak_source": f"bf16 {regime} {bf16} TFLOP/s of {peaks['source']} / 4 (per product 1 TF32 MMA at half the "
-                           f"bf16 rate + 2 BF16 K=16 MMAs); 3xTF32 = bf16 / 6; regime chosen from the timed region "
+            "peak_source": f"bf16 {regime} {bf16} TFLOP/s of {peaks['source']} / 3 (per product 3 FP16 K=16 "
+                           f"MMAs at the bf16 rate); 3xTF32 = bf16 / 6; regime chosen from the timed region "
                            f"({timed_s:.2f} s) and the sampled SM clock ({sm} of {mx} MHz)",
             "ms": kernel_ms}
 
@@ -409,7 +409,7 @@ def run_single(args, w):
     roofline = None
     if g1_ms:
         achieved = useful_flops / (g1_ms * 1e-3) / 1e12
-        weight_bytes = (2 * D * F * 4.0) * active      # raw FP32 interleaved wi_0/wi_1 matrix of every active expert
+        weight_bytes = (2 * D * F * 4.0) * active      # interleaved wi_0/wi_1 matrix, 4 bytes a weight, of every active expert
         traffic = TRAFFIC_BYTES_PER_WEIGHT * active * 2.0 * F * D if not w.streamed else None
         roofline = gemm_roofline("ffn_umma_kernel<EPI_GELU_PAIR>", achieved, g1_ms, peaks, clock_summary,
                                  timed_s=ms * 1e-3 * args.steps)
@@ -434,7 +434,7 @@ def run_single(args, w):
     line = {
         "metric": METRIC, "value": T / (ms * 1e-3), "unit": UNIT, "n_gpus": 1, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f32 (split-operand tensor-core products: TF32 head + BF16 corrections, FP32 accumulate)", "data": "synthetic",
+        "dtype": "f32 (split-operand tensor-core products: FP16 pairs, FP32 accumulate)", "data": "synthetic",
         "config": dict(workload_config(w, 1), **({"expert_cache_slots": args.cache_slots} if args.cache_slots else {})),
         "e2e": {"value": T / e2e_s, "unit": UNIT, "h2d_bytes_per_step": int(hx.numel() * 4),
                 "d2h_bytes_per_step": int(hout.numel() * 4), "ms_per_step": 1e3 * e2e_s,

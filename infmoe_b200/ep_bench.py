@@ -270,7 +270,7 @@ def run(args, total, scaling, metric, unit, clock_sampler_cls, peaks_fn, workloa
             "metric": metric, "value": T_total / (main["ms"] * 1e-3), "unit": unit, "n_gpus": world,
             "steps": args.steps, "warmup": warmup, "ms_per_step": main["ms"],
             "higher_is_better": True, "scaling": scaling, "vs_baseline": None,
-            "dtype": "f32 (split-operand tensor-core products: TF32 head + BF16 corrections, FP32 accumulate)",
+            "dtype": "f32 (split-operand tensor-core products: FP16 pairs, FP32 accumulate)",
             "data": "synthetic", "config": cfg,
             "e2e": {"value": T_total / (e2e["ms"] * 1e-3), "unit": unit,
                     "h2d_bytes_per_step": main["hx_bytes"] * world, "d2h_bytes_per_step": main["hx_bytes"] * world,

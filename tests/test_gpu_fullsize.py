@@ -130,9 +130,9 @@ def test_offload_decode_full_size(oracle):
 
 @pytest.mark.parametrize("case", ["row_scales", "outliers", "large_magnitude"])
 def test_split_operand_products_with_wide_value_ranges(oracle, case):
-    """The expert GEMMs add two BF16 correction products to a TF32 head product.  Inputs drawn from N(0, 1) never
-    test what 8-bit correction operands do to weights with a wide exponent spread, with outliers, or to the
-    integer TF32 rounding at large magnitudes (where a mantissa carry moves the exponent): these cases do."""
+    """The expert GEMMs work on FP16 pairs scaled by a power of two per row.  Inputs drawn from N(0, 1) never test
+    what the scales do to weights with a wide exponent spread inside and between rows, with outliers, or at
+    magnitudes far outside the range of FP16: these cases do."""
     import torch
     assert torch.cuda.is_available()
     from tests import gpu_util as g
@@ -155,7 +155,7 @@ def test_split_operand_products_with_wide_value_ranges(oracle, case):
             m[idx] *= np.float32(1000.0)
         x[rng.random(x.shape) < 1e-3] *= np.float32(300.0)
     else:
-        # weights near 2^60, LayerNorm weight 2^-60: values whose TF32 rounding carries into the exponent included
+        # weights near 2^60, LayerNorm weight 2^-60: values whose rounding to 11 bits carries into the exponent included
         ln = (ln * np.float32(2.0 ** -60)).astype(np.float32)
         wi0 = (wi0 * np.float32(2.0 ** 60)).astype(np.float32)
         wi1 = (wi1 * np.float32(2.0 ** 60)).astype(np.float32)
