@@ -45,15 +45,17 @@ int launch_mix_gather(long long T, int D, const int* pos, const float* routed, c
 int launch_layernorm(float* out, const float* in, long long n, int D, const float* gamma, cudaStream_t stream);
 int launch_gelu_dot(const float* a, float* b, size_t len, cudaStream_t stream);
 int launch_fill_int(int* dst, int value, cudaStream_t stream);   // *dst = value, stream ordered
-// Tile-contiguous weight layouts (see rows.cu); src1 != NULL interleaves the rows of two matrices.
-//   launch_retile       raw FP32 tiles, for the CUDA-core GEMM (tiled_elems floats)
-//   launch_split_tiles  FP16-pair tiles, the rows' 2^-s and, of two matrices, the gate bound, for the tensor-core GEMM
-//                       (split_plane_elems floats: tiles, one float per padded row, 32 floats for the bound)
+// Tile-contiguous weight layouts (see rows.cu).
+//   launch_retile        one matrix as raw FP32 tiles, for the CUDA-core GEMM (tiled_elems floats); src1 != NULL
+//                        interleaves the rows of two matrices
+//   launch_split_expert  both planes of an expert for the tensor-core GEMM (split_plane_elems floats each: FP16-pair
+//                        tiles, 2^-s of every padded row, 32 floats for the gate bound, the norms it is taken from)
 int launch_retile(const float* src0, const float* src1, int M, int K, float* dst, cudaStream_t stream);
-int launch_split_tiles(const float* src0, const float* src1, int M, int K, float* dst, cudaStream_t stream);
+int launch_split_expert(const float* wi0, const float* wi1, const float* wo, int D, int F, float* w01, float* wo_dst,
+                        cudaStream_t stream);
 inline size_t tiled_elems(int M, int K) { return (size_t)((M + 127) / 128) * 128 * (size_t)((K + 31) / 32) * 32; }
 inline size_t split_bound_at(int M, int K) { return tiled_elems(M, K) + (size_t)((M + 127) / 128) * 128; }
-inline size_t split_plane_elems(int M, int K) { return split_bound_at(M, K) + 32; }
+inline size_t split_plane_elems(int M, int K) { return split_bound_at(M, K) + 32 + (size_t)((M + 127) / 128) * 64; }
 // h = LN(x; gamma) for rows already in place, as launch_scatter_ln_rows / _pack write it.
 int launch_ln_rows(long long n, int D, const float* in, const float* gamma, float* h, cudaStream_t stream);
 int launch_ln_pack(long long n, int D, const float* in, const float* gamma, void* h, float* row_info,
@@ -77,7 +79,7 @@ struct FfnUmma {
     const int* offset;              // [E+1] first row of each expert
     const int* slot_of_expert;      // expert -> weight slot (NULL: identity)
     int slots;                      // weight slots in the planes
-    const float *w01, *wo;          // split planes (launch_split_tiles), [slots] x split_plane_elems
+    const float *w01, *wo;          // split planes (launch_split_expert), [slots] x split_plane_elems
     const void* h;                  // packed LayerNorm output [T][D]
     const float* row_info;          // [T][2]
     void* g;                        // packed gate activations [T][F] (scratch)

@@ -73,7 +73,7 @@ struct ExpertStore {
     float* d_ln = nullptr;
     std::vector<char> ln_on_device;
     // device-resident weights in the GEMM's tile-contiguous layout: FP16 pairs with their row scales for the
-    // tensor-core GEMM (launch_split_tiles), raw FP32 for the CUDA-core one (launch_retile)
+    // tensor-core GEMM (launch_split_expert), raw FP32 for the CUDA-core one (launch_retile)
     //   [0] w01 [E] x plane(2F x D)  (row 2f = wi_0[f], row 2f+1 = wi_1[f])
     //   [1] wo  [E] x plane(D x F)
     bool split = false;
@@ -306,9 +306,9 @@ int load_expert_planes(bool split, int D, int F, const float* wi0, const float* 
         wi1 = staging + n;
         wo = staging + 2 * n;
     }
-    const auto layout = split ? launch_split_tiles : launch_retile;
-    INFMOE_TRY(layout(wi0, wi1, 2 * F, D, w01, stream));
-    INFMOE_TRY(layout(wo, nullptr, D, F, wo_dst, stream));
+    if (split) return launch_split_expert(wi0, wi1, wo, D, F, w01, wo_dst, stream);
+    INFMOE_TRY(launch_retile(wi0, wi1, 2 * F, D, w01, stream));
+    INFMOE_TRY(launch_retile(wo, nullptr, D, F, wo_dst, stream));
     return INFMOE_OK;
 }
 
@@ -1859,7 +1859,7 @@ int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_
 
 namespace {
 // Scratch measure: two FP32 planes each of h and g and the weight tiles, more than either form needs but for the row scales and row_info of the tensor-core form (which are at most
-// 2 MB beside a scratch of 32 MB: 512 bytes per 128-row weight block, which has at least one 16 KB tile).
+// 2 MB beside a scratch of 32 MB: 768 bytes per 128-row weight block, which has at least one 16 KB tile).
 // It is also the measure of what infmoe_t5ff_run_static takes.
 size_t t5ff_scratch_bytes(int64_t rows, int32_t D, int32_t F) {
     const size_t r = (size_t)rows, d = (size_t)D, f = (size_t)F;

@@ -488,60 +488,113 @@ retile_kernel(const float* __restrict__ src0, const float* __restrict__ src1, in
     dst[seg * 32 + lane] = v;
 }
 
-// Tensor-core GEMM, first pass: 2^-s of every (padded) row from its largest magnitude, and the gate bound, the largest
-// log2(|wi_0[f]| |wi_1[f]|) of the expert (g_exponent).  One warp per row of the sources, all rows read once; squares
-// are summed in 64 bits because the magnitudes may be anywhere in the FP32 range.
-__global__ void __launch_bounds__(256)
-row_scale_kernel(const float* __restrict__ src0, const float* __restrict__ src1, int M, int K, int padded,
-                 float* __restrict__ inv, uint32_t* __restrict__ bound) {
+// Tensor-core GEMM: both planes of an expert in two launches (an expert that is streamed pays for them on every call).
+struct SplitExpert {
+    const float *wi0, *wi1, *wo;
+    int D, F;
+    float *w01, *wo_dst;         // destination planes
+    int MB[2], KB[2];            // 128-row and 32-column blocks of w01 (0) and wo (1)
+    float* inv[2];               // 2^-s of every padded row
+    float* norms;                // log2(|wi_0[f]| |wi_1[f]|) of every padded f
+    uint32_t* bound;             // the largest of them, encoded
+};
+
+// First pass: 2^-s of every padded row from its largest magnitude, and log2 of the norm products behind the gate bound
+// (g_exponent).  One warp per row (w01: per f, two rows); squares are summed in 64 bits because the magnitudes may be
+// anywhere in the FP32 range.  HBM bound; vec: rows are 16-byte aligned.
+__device__ __forceinline__ void warp_row_size(const float* __restrict__ row, int K, bool vec, float& top, double& sum) {
     const int lane = threadIdx.x & 31;
-    const int step = src1 ? 2 : 1;
-    const int m0 = ((int)blockIdx.x * 8 + (int)(threadIdx.x >> 5)) * step;   // rows m0 (and m0 + 1)
-    if (m0 >= padded) return;
-    double norm[2] = {0.0, 0.0};
-    for (int i = 0; i < step; ++i) {
-        const int m = m0 + i;
-        float top = 0.f;
-        double sum = 0.0;
-        if (m < M) {
-            const float* row = src1 ? (i ? src1 : src0) + (size_t)(m >> 1) * K : src0 + (size_t)m * K;
+    top = 0.f;
+    sum = 0.0;
+    if (vec) {
 #pragma unroll 8
-            for (int k = lane; k < K; k += 32) {
-                const float v = row[k];
-                top = fmaxf(top, fabsf(v));
-                sum += (double)v * (double)v;
-            }
+        for (int k = 4 * lane; k < K; k += 128) {
+            const float4 v = *reinterpret_cast<const float4*>(row + k);
+            top = fmaxf(fmaxf(fmaxf(top, fabsf(v.x)), fmaxf(fabsf(v.y), fabsf(v.z))), fabsf(v.w));
+            sum += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
         }
-        top = warp_max(top);
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        norm[i] = sum;
-        if (lane == 0) inv[m] = exp2_int(-row_exponent(top));
+    } else {
+#pragma unroll 8
+        for (int k = lane; k < K; k += 32) {
+            const float v = row[k];
+            top = fmaxf(top, fabsf(v));
+            sum += (double)v * v;
+        }
     }
-    if (src1 && lane == 0 && m0 < M)
-        atomicMax(bound, encode_bound(0.5f * ((float)log2(norm[0]) + (float)log2(norm[1]))));
+    top = warp_max(top);
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+}
+__global__ void __launch_bounds__(256)
+row_scale_kernel(const SplitExpert a, int vec) {
+    const int lane = threadIdx.x & 31;
+    int w = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5);
+    float top;
+    double sum0 = 0.0, sum1 = 0.0;
+    if (w < a.MB[0] * 64) {      // rows 2 f and 2 f + 1 of w01
+        float top1 = top = 0.f;
+        if (w < a.F) {
+            warp_row_size(a.wi0 + (size_t)w * a.D, a.D, vec != 0, top, sum0);
+            warp_row_size(a.wi1 + (size_t)w * a.D, a.D, vec != 0, top1, sum1);
+        }
+        if (lane == 0) {
+            a.inv[0][2 * w] = exp2_int(-row_exponent(top));
+            a.inv[0][2 * w + 1] = exp2_int(-row_exponent(top1));
+            a.norms[w] = 0.5f * ((float)log2(sum0) + (float)log2(sum1));     // -inf past the matrix
+        }
+        return;
+    }
+    w -= a.MB[0] * 64;
+    if (w >= a.MB[1] * 128) return;
+    top = 0.f;
+    if (w < a.D) warp_row_size(a.wo + (size_t)w * a.F, a.F, vec != 0, top, sum0);
+    if (lane == 0) a.inv[1][w] = exp2_int(-row_exponent(top));
 }
 
-// Second pass: the tiles as FP16 pairs, a row of a tile being 32 x hi, 32 x lo of the values times 2^s.
+// Second pass: the tiles as FP16 pairs, a row of a tile being 32 x hi, 32 x lo of the values times 2^s.  A block per tile,
+// 16 lanes per row, two values each, the values of eight rows in flight.  The last block takes the maximum of the norms.
 __global__ void __launch_bounds__(256)
-split_tiles_kernel(const float* __restrict__ src0, const float* __restrict__ src1, int M, int K, int MB, int KB,
-                   const float* __restrict__ inv, uint16_t* __restrict__ dst) {
-    const int lane = threadIdx.x & 31;
-    const long long seg = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);   // (mb, kb, r) flattened
-    if (seg >= (long long)MB * KB * 128) return;
-    const int r = (int)(seg % 128);
-    const long long tile = seg / 128;
-    const int kb = (int)(tile % KB), mb = (int)(tile / KB);
-    const int m = mb * 128 + r, k = kb * 32 + lane;
-    float v = 0.f;
-    if (m < M && k < K) {
-        if (src1) v = (m & 1) ? src1[(size_t)(m >> 1) * K + k] : src0[(size_t)(m >> 1) * K + k];
-        else v = src0[(size_t)m * K + k];
+split_tiles_kernel(const SplitExpert a) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x == gridDim.x - 1) {
+        __shared__ uint32_t s_bound[8];
+        uint32_t best = 0;
+        for (int f = (int)threadIdx.x; f < a.MB[0] * 64; f += 256) best = max(best, encode_bound(a.norms[f]));
+        best = __reduce_max_sync(0xffffffffu, best);
+        if (lane == 0) s_bound[warp] = best;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int i = 1; i < 8; ++i) best = max(best, s_bound[i]);
+            *a.bound = best;
+        }
+        return;
     }
-    // 2^s = 1 / 2^-s exactly (both are normal)
-    const uint32_t p = split_f16(__fmul_rn(v, __fdiv_rn(1.0f, inv[m])));
-    dst[seg * 64 + lane] = (uint16_t)p;
-    dst[seg * 64 + 32 + lane] = (uint16_t)(p >> 16);
+    int tile = (int)blockIdx.x;                    // tiles of w01, then of wo
+    const int which = tile >= a.MB[0] * a.KB[0] ? 1 : 0;
+    if (which) tile -= a.MB[0] * a.KB[0];
+    const int mb = tile / a.KB[which], kb = tile % a.KB[which];
+    const int M = which ? a.D : 2 * a.F, K = which ? a.F : a.D, k = kb * 32 + 2 * (lane & 15);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(which ? a.wo_dst : a.w01) + (size_t)tile * 4096 + (lane & 15);
+    const float* inv = a.inv[which] + mb * 128;
+    float v[8][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {                  // rows warp * 16 + 2 i (+ 1 in the upper half of the warp)
+        const int m = mb * 128 + warp * 16 + 2 * i + (lane >> 4);
+        v[i][0] = v[i][1] = 0.f;
+        if (m < M) {
+            const float* row = which ? a.wo + (size_t)m * K : ((m & 1) ? a.wi1 : a.wi0) + (size_t)(m >> 1) * K;
+            if (k < K) v[i][0] = row[k];
+            if (k + 1 < K) v[i][1] = row[k + 1];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = warp * 16 + 2 * i + (lane >> 4);
+        const float scale = __fdiv_rn(1.0f, inv[r]);     // 2^s exactly (both are normal)
+        const uint32_t p0 = split_f16(__fmul_rn(v[i][0], scale)), p1 = split_f16(__fmul_rn(v[i][1], scale));
+        dst[r * 32] = __byte_perm(p0, p1, 0x5410);
+        dst[r * 32 + 16] = __byte_perm(p0, p1, 0x7632);
+    }
 }
 
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
@@ -718,15 +771,28 @@ int launch_ln_pack(long long n, int D, const float* in, const float* gamma, void
     return INFMOE_OK;
 }
 
-int launch_split_tiles(const float* src0, const float* src1, int M, int K, float* dst, cudaStream_t stream) {
-    const int MB = (M + 127) / 128, KB = (K + 31) / 32, padded = MB * 128;
-    float* inv = dst + tiled_elems(M, K);
-    uint32_t* bound = (uint32_t*)(dst + split_bound_at(M, K));
-    INFMOE_CUDA_TRY(cudaMemsetAsync(bound, 0, 32 * sizeof(float), stream));
-    const int warps = src1 ? padded / 2 : padded;
-    row_scale_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(src0, src1, M, K, padded, inv, bound);
-    const long long segs = (long long)MB * KB * 128;
-    split_tiles_kernel<<<(unsigned)((segs + 7) / 8), 256, 0, stream>>>(src0, src1, M, K, MB, KB, inv, (uint16_t*)dst);
+int launch_split_expert(const float* wi0, const float* wi1, const float* wo, int D, int F, float* w01, float* wo_dst,
+                        cudaStream_t stream) {
+    SplitExpert a;
+    a.wi0 = wi0;
+    a.wi1 = wi1;
+    a.wo = wo;
+    a.D = D;
+    a.F = F;
+    a.w01 = w01;
+    a.wo_dst = wo_dst;
+    a.MB[0] = (2 * F + 127) / 128;
+    a.KB[0] = (D + 31) / 32;
+    a.MB[1] = (D + 127) / 128;
+    a.KB[1] = (F + 31) / 32;
+    a.inv[0] = w01 + tiled_elems(2 * F, D);
+    a.inv[1] = wo_dst + tiled_elems(D, F);
+    a.bound = (uint32_t*)(w01 + split_bound_at(2 * F, D));
+    a.norms = w01 + split_bound_at(2 * F, D) + 32;
+    const int vec = D % 4 == 0 && F % 4 == 0 && aligned16(wi0) && aligned16(wi1) && aligned16(wo);
+    const int warps = a.MB[0] * 64 + a.MB[1] * 128;
+    row_scale_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(a, vec);
+    split_tiles_kernel<<<(unsigned)(a.MB[0] * a.KB[0] + a.MB[1] * a.KB[1] + 1), 256, 0, stream>>>(a);
     note_launch(2);
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
