@@ -628,7 +628,9 @@ route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // cluster owns RS_TOKENS tokens and its CTAs share the experts: a warp computes one expert's scores at a time, lane l
 // being partial index l (its float4 loads of the centroid row are one coalesced run, eight in flight), against the
 // normalised token rows in shared memory, and the butterfly over the lanes is the canonical reduction.  The CTAs' best
-// candidates meet in the first one through distributed shared memory.  Same additions in the same order as above.
+// candidates meet in the first one through distributed shared memory, behind the second half of a cluster barrier whose
+// first half every CTA passes on entry: a CTA's shared memory may be written only once that CTA is known to run.  Same
+// additions in the same order as above.
 // Each centroid is read once per RS_TOKENS tokens, from L2, and a shared-memory load feeds only four multiply-adds:
 // past the line in use_small_route the other kernels win.
 // One token, d_model 4096, 32 experts: 47 -> 9.6 us; 64 tokens 52 -> 12.5; d_model 1024, 8 experts: 13 -> 3.5.
@@ -658,6 +660,7 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
     const long long t0 = (long long)(blockIdx.x / S) * RS_TOKENS;
     const int nt = (int)min((long long)RS_TOKENS, T - t0);
     const int chunks = (D + 127) / 128 * 32;              // float4 per staged row
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     pdl_trigger();
     pdl_wait();
     if (gamma) {
@@ -731,6 +734,7 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
         }
     }
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // the first CTA has started
     if (tid < RS_TOKENS) {
         float b = -FLT_MAX;
         int be = -1;

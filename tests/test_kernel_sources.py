@@ -1,0 +1,41 @@
+"""Orderings inside kernels that no run on a GPU can be relied on to show, checked in the source."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "infmoe_b200", "csrc")
+
+
+def _kernels():
+    """(file, name, body) of every __global__ function, comments removed."""
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        with open(path) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\(", text):
+            if m.group(1) == "__launch_bounds__":
+                m = re.compile(r"\)\s*(\w+)\s*\(").search(text, m.end())
+            start = text.index("{", m.end())
+            depth, i = 0, start
+            while True:
+                depth += {"{": 1, "}": -1}.get(text[i], 0)
+                i += 1
+                if depth == 0:
+                    break
+            yield os.path.basename(path), m.group(1), text[start:i]
+
+
+def test_kernels_are_found():
+    names = {name for _, name, _ in _kernels()}
+    assert {"route_small_kernel", "dispatch_kernel", "ffn_umma_kernel", "gather_kernel"} <= names
+
+
+@pytest.mark.parametrize("file,name,body", [k for k in _kernels() if re.search(r"map_shared_rank|leader_addr\(", k[2])],
+                         ids=lambda v: v if len(v) < 40 else "")
+def test_other_blocks_memory_is_touched_only_behind_a_cluster_barrier(file, name, body):
+    """Distributed shared memory may be accessed once the target block is known to have started, which only a
+    cluster-wide barrier establishes."""
+    remote = re.search(r"map_shared_rank|leader_addr\(", body).start()
+    barrier = re.search(r"cluster\.sync\(\)|cluster_sync\(\)|barrier\.cluster\.wait", body)
+    assert barrier and barrier.start() < remote, f"{file}: {name} reaches another block's memory before any cluster barrier"
