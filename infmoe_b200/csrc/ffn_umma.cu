@@ -689,6 +689,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     __threadfence();
                 }
                 done = __shfl_sync(0xffffffffu, done, 0);
+                __syncwarp();    // orders lane 0's fence before the other lanes' reads of the sums; a shuffle does not
                 if (done != sched.m) continue;
                 const int first = sched.prefix_chunks(item.tail) - 1;
 #pragma unroll

@@ -39,3 +39,13 @@ def test_other_blocks_memory_is_touched_only_behind_a_cluster_barrier(file, name
     remote = re.search(r"map_shared_rank|leader_addr\(", body).start()
     barrier = re.search(r"cluster\.sync\(\)|cluster_sync\(\)|barrier\.cluster\.wait", body)
     assert barrier and barrier.start() < remote, f"{file}: {name} reaches another block's memory before any cluster barrier"
+
+
+def test_sums_of_a_cut_tile_are_read_behind_a_warp_barrier():
+    """Lane 0 counts the arrivals and fences; a shuffle hands the count to the other lanes but orders no memory, so a
+    warp barrier has to stand between it and their reads of what other blocks stored."""
+    body = next(b for _, n, b in _kernels() if n == "ffn_umma_kernel")
+    counted, read = body.index("atomicAdd(counter"), body.index("__ldcg(src")
+    handed_on = body.rindex("__shfl_sync(0xffffffffu, done", counted, read)
+    assert "__threadfence();" in body[counted:handed_on]
+    assert "__syncwarp();" in body[handed_on:read]
