@@ -166,10 +166,11 @@ __device__ __forceinline__ float ln_apply(float x, float mean, float rstd, float
     return __fmul_rn(gamma, __fmul_rn(__fsub_rn(x, mean), rstd));
 }
 
-// Operand of the tensor-core GEMM: an FP32 value, scaled by a power of two of its row, as a pair of FP16 values,
+// Operand of the tensor-core GEMM: an FP32 value, scaled by powers of two of its row and column, as a pair of FP16 values,
 // hi = x rounded to 11 significant bits, lo = x - hi rounded to 11 (in the lower / upper half of the word).  |lo| is at
 // most half a unit of hi, so together they hold x to within 2^-23 relative (the last bit of an FP32 value) down to
-// |x| = 2^-3, and to within 2^-25 absolute below that.
+// |x| = 2^-2, which is 2^-17 of the row's largest value.  Below that FP16's smallest step sets an absolute limit, 2^-25, so
+// rows have to be even; see the weight layout in rows.cu.
 __device__ __forceinline__ uint32_t split_f16(float x) {
     const __half hi = __float2half_rn(x);
     const __half lo = __float2half_rn(__fsub_rn(x, __half2float(hi)));
@@ -196,23 +197,14 @@ __device__ __forceinline__ int row_exponent(float max_abs) {
     return min(126, 14 - ((__float_as_int(max_abs) >> 23) - 127));
 }
 // Exponent of the gate activations g of one token.  |g_f| = |gelu(a_f) b_f| <= |a_f| |b_f| <= |h|^2 |wi_0[f]| |wi_1[f]|
-// (2-norms), so with h2 = log2 |h|^2 and w = max_f log2(|wi_0[f]| |wi_1[f]|) no g 2^s exceeds 2^15.  The bound is about
-// 2^13 above a typical g at d_model 4096, which leaves typical values near 2^2 and their lo parts well inside the
-// normal range of FP16.  Both GEMMs compute it from the same two numbers.
+// (2-norms), and the weight layout scales neuron f by 2^a_f so that |wi_0[f]| |wi_1[f]| 2^a_f <= 2^w for all of them.  So
+// with h2 = log2 |h|^2 no g 2^a_f 2^s exceeds 2^15.  The bound is about 2^13 above a typical g at d_model 4096, which
+// leaves typical values near 2^2, with all their bits.  Both GEMMs compute it from the same two numbers.
 __device__ __forceinline__ int g_exponent(float h2, float w) {
     float b = h2 + w + 0.01f;
     if (!(b > -111.f)) b = -111.f;
     if (!(b < 141.f)) b = 141.f;
     return 15 - (int)ceilf(b);
-}
-// Order-preserving map of floats onto unsigned integers above 0, for atomicMax.
-__device__ __forceinline__ uint32_t encode_bound(float x) {
-    const uint32_t u = __float_as_uint(x);
-    return (u & 0x80000000u) ? ~u : u | 0x80000000u;
-}
-__device__ __forceinline__ float decode_bound(float stored) {
-    const uint32_t u = __float_as_uint(stored);
-    return __uint_as_float((u & 0x80000000u) ? u & 0x7fffffffu : ~u);
 }
 // sum 2^-s of the weight row 2^-s of the token row; the smaller factor first, so that nothing overflows on the way.
 __device__ __forceinline__ float unscale(float sum, float w_inv, float x_inv) {

@@ -23,7 +23,8 @@
 // w * x = lo(w) hi(x) + hi(w) lo(x) + hi(w) hi(x) + (a term below 2^-22): three kind::f16 products, six K = 16 MMAs
 // per k block of 32.  s is a power of two per weight row (its largest value lands in [2^14, 2^15), chosen when the
 // weights are laid out) and per token row (from the row itself for h, from a bound that cannot be exceeded for g,
-// see g_exponent); the epilogues multiply the sums by 2^-s, which is exact.
+// see g_exponent); the epilogues multiply the sums by 2^-s, which is exact.  Powers of two per column, which cancel between
+// the operands, even the rows out beforehand (rows.cu, SplitExpert).
 // The pair takes the four bytes of the FP32 value in HBM, L2 and shared memory, and nothing has to be converted on
 // the way to the tensor cores.  What it replaced, a TF32 head product with BF16 corrections of weights that four
 // warps split between shared memory and TMEM, took 8 MMAs and about 1000 cycles per k block (of 144 tokens), held
@@ -285,8 +286,8 @@ struct GemmArgs {
     int K;
     const float* w;             // weight plane: per slot the tiles, then the rows' 2^-s (see split_plane_elems)
     size_t w_stride;            // floats per slot
-    const float* bound;         // log2 bound of the experts' gates, encoded (see decode_bound): first slot ...
-    size_t bound_stride;        // ... and floats from one slot to the next
+    const int* bound;           // w of g_exponent: first slot ...
+    size_t bound_stride;        // ... and words from one slot to the next
     const float2* row_info;     // [T] of the h rows: 2^-s and log2 of the squared norm
     void* out_pack;             // GELU_PAIR: packed plane of g
     float* out;                 // RESIDUAL: y [T][M_total]
@@ -716,7 +717,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             const bool m_ok = m < args.M_total;
             // 2^-s of the weight row (padding rows have one too)
             const float w_inv = __ldg(args.w + (size_t)t.slot * args.w_stride + (size_t)MB1 * KB * (UMMA_M * BK) + m);
-            const float bound = decode_bound(__ldg(args.bound + (size_t)t.slot * args.bound_stride));
+            const float bound = (float)__ldg(args.bound + (size_t)t.slot * args.bound_stride);
 #pragma unroll
             for (int i = 0; i < C::SLICES; ++i) {
                 const int sl = EPI_GROUPS * i + group;
@@ -971,7 +972,7 @@ int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_be
     a1.K = D;
     a1.w = f.w01;
     a1.w_stride = split_plane_elems(2 * F, D);
-    a1.bound = f.w01 + split_bound_at(2 * F, D);
+    a1.bound = reinterpret_cast<const int*>(f.w01 + split_range_at(2 * F, D));
     a1.bound_stride = a1.w_stride;
     a1.row_info = reinterpret_cast<const float2*>(f.row_info);
     a1.out_pack = f.g;

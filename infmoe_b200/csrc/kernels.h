@@ -28,15 +28,18 @@ int launch_scatter(long long T, int D, const float* X, const float* coeff, const
 int launch_scatter_ln_rows(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
                            const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h,
                            cudaStream_t stream);
-// Tensor-core GEMM: packed FP16-pair plane `h` (pack_bytes) and two floats per row in row_info (token_row_info).
-int launch_scatter_ln_pack(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
-                           const float* gamma_all, const int* valid_rows, float* rscore, void* h, float* row_info,
-                           cudaStream_t stream);
-// launch_dispatch (without regions) and one of the two scatters in one kernel, where dispatch_scatter_supported.
+// Tensor-core GEMM: packed FP16-pair plane `h` (pack_bytes) and two floats per row in row_info (token_row_info), of rows
+// row0 .. row0 + T - 1.  gamma: the LayerNorm weights that launch_split_expert left in the first weight slot, gamma_stride
+// floats from one slot to the next.
+int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, const float* score, const int* pos,
+                           const int* gate, const float* gamma, size_t gamma_stride, const int* slot_of_expert,
+                           const int* valid_rows, float* rscore, void* h, float* row_info, cudaStream_t stream);
+// launch_dispatch (without regions) and one of the two scatters in one kernel, where dispatch_scatter_supported.  gamma is
+// what the scatter takes: with `pack` that of the weight slots (experts in order), else the LayerNorm weights [E][D].
 bool dispatch_scatter_supported(long long T, int D, int E);
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
-                            const float* gamma_all, int* pos, int* count, int* offset, int* status, int* zero,
-                            int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
+                            const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,
+                            int* zero, int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
                             cudaStream_t stream);
 int launch_gather(long long T, int D, const float* in, const int* pos, float* out, cudaStream_t stream,
                   const int* valid_rows = nullptr);
@@ -49,14 +52,17 @@ int launch_fill_int(int* dst, int value, cudaStream_t stream);   // *dst = value
 //   launch_retile        one matrix as raw FP32 tiles, for the CUDA-core GEMM (tiled_elems floats); src1 != NULL
 //                        interleaves the rows of two matrices
 //   launch_split_expert  both planes of an expert for the tensor-core GEMM (split_plane_elems floats each: FP16-pair
-//                        tiles, 2^-s of every padded row, 32 floats for the gate bound, the norms it is taken from)
+//                        tiles, 2^-s of every padded row, 32 words for the largest of the numbers behind them, one per
+//                        neuron, column exponents, LayerNorm weights gamma' to use with the plane, see rows.cu)
 int launch_retile(const float* src0, const float* src1, int M, int K, float* dst, cudaStream_t stream);
-int launch_split_expert(const float* wi0, const float* wi1, const float* wo, int D, int F, float* w01, float* wo_dst,
-                        cudaStream_t stream);
+int launch_split_expert(const float* gamma, const float* wi0, const float* wi1, const float* wo, int D, int F, float* w01,
+                        float* wo_dst, cudaStream_t stream);
 inline size_t tiled_elems(int M, int K) { return (size_t)((M + 127) / 128) * 128 * (size_t)((K + 31) / 32) * 32; }
-inline size_t split_bound_at(int M, int K) { return tiled_elems(M, K) + (size_t)((M + 127) / 128) * 128; }
-inline size_t split_plane_elems(int M, int K) { return split_bound_at(M, K) + 32 + (size_t)((M + 127) / 128) * 64; }
-// h = LN(x; gamma) for rows already in place, as launch_scatter_ln_rows / _pack write it.
+inline size_t split_range_at(int M, int K) { return tiled_elems(M, K) + (size_t)((M + 127) / 128) * 128; }
+inline size_t split_columns_at(int M, int K) { return split_range_at(M, K) + 32 + (size_t)((M + 127) / 128) * 64; }
+inline size_t split_gamma_at(int M, int K) { return split_columns_at(M, K) + (size_t)((K + 31) / 32) * 32; }
+inline size_t split_plane_elems(int M, int K) { return split_gamma_at(M, K) + (size_t)((K + 31) / 32) * 32; }
+// h = LN(x; gamma) for rows already in place, as launch_scatter_ln_rows / _pack write it (_pack: gamma' of the slot).
 int launch_ln_rows(long long n, int D, const float* in, const float* gamma, float* h, cudaStream_t stream);
 int launch_ln_pack(long long n, int D, const float* in, const float* gamma, void* h, float* row_info,
                    cudaStream_t stream);

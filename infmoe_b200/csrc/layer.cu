@@ -291,8 +291,9 @@ int ensure_resident_planes(ExpertStore* s) {
 
 // Puts one expert's matrices into its two planes (tile-contiguous, wi_0 / wi_1 rows interleaved; FP16 pairs with
 // `split`, else raw FP32).  Host sources first land in `staging` (device, 3*D*F floats).
-int load_expert_planes(bool split, int D, int F, const float* wi0, const float* wi1, const float* wo, float* w01, float* wo_dst,
-                       bool src_on_host, float* staging, cudaStream_t stream) {
+// `split` takes the expert's LayerNorm weight too (on the device) and leaves what the scatter applies in w01.
+int load_expert_planes(bool split, int D, int F, const float* ln, const float* wi0, const float* wi1, const float* wo,
+                       float* w01, float* wo_dst, bool src_on_host, float* staging, cudaStream_t stream) {
     const size_t n = (size_t)D * F;
     if (src_on_host) {
         if (!staging) {
@@ -306,7 +307,7 @@ int load_expert_planes(bool split, int D, int F, const float* wi0, const float* 
         wi1 = staging + n;
         wo = staging + 2 * n;
     }
-    if (split) return launch_split_expert(wi0, wi1, wo, D, F, w01, wo_dst, stream);
+    if (split) return launch_split_expert(ln, wi0, wi1, wo, D, F, w01, wo_dst, stream);
     INFMOE_TRY(launch_retile(wi0, wi1, 2 * F, D, w01, stream));
     INFMOE_TRY(launch_retile(wo, nullptr, D, F, wo_dst, stream));
     return INFMOE_OK;
@@ -323,7 +324,7 @@ int upload_resident(ExpertStore* s, cudaStream_t stream) {
     for (int e = 0; e < s->E; ++e) {
         if (s->on_device[e] || !s->on_host[e]) continue;
         if (!s->d_staging) INFMOE_CUDA_TRY(cudaMalloc(&s->d_staging, sizeof(float) * 3 * s->matrix_elems()));
-        INFMOE_TRY(load_expert_planes(s->split, s->D, s->F, s->h_wi0[e], s->h_wi1[e], s->h_wo[e],
+        INFMOE_TRY(load_expert_planes(s->split, s->D, s->F, s->d_ln + (size_t)e * s->D, s->h_wi0[e], s->h_wi1[e], s->h_wo[e],
                                       s->d_plane[0] + s->plane_elems(0) * e, s->d_plane[1] + s->plane_elems(1) * e,
                                       true, s->d_staging, stream));
         s->on_device[e] = 1;
@@ -768,8 +769,9 @@ int infmoe_layer_set_expert(infmoe_layer* L, int32_t e, const float* ln_w, const
         INFMOE_TRY(ensure_resident_planes(s));
         INFMOE_CUDA_TRY(cudaMemcpy(s->d_ln + (size_t)e * s->D, ln_w, sizeof(float) * s->D, cudaMemcpyDeviceToDevice));
         s->ln_on_device[e] = 1;
-        INFMOE_TRY(load_expert_planes(s->split, s->D, s->F, wi0, wi1, wo, s->d_plane[0] + s->plane_elems(0) * e,
-                                      s->d_plane[1] + s->plane_elems(1) * e, false, nullptr, 0));
+        INFMOE_TRY(load_expert_planes(s->split, s->D, s->F, s->d_ln + (size_t)e * s->D, wi0, wi1, wo,
+                                      s->d_plane[0] + s->plane_elems(0) * e, s->d_plane[1] + s->plane_elems(1) * e, false,
+                                      nullptr, 0));
         INFMOE_CUDA_TRY(cudaStreamSynchronize(0));
         s->on_device[e] = 1;
     } else {
@@ -1071,9 +1073,10 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     INFMOE_TRY(prof_mark(L, 1, stream));
     // 2. dispatch metadata (:350-352)
     // (with few tokens the scatter kernel of step 3 computes it on the way, except when an expert count past the
-    // dispatch kernel's limit has to be refused)
+    // dispatch kernel's limit has to be refused, and for streamed experts on the tensor-core path, see there)
+    const bool pack = !L->identity && !L->custom && uses_umma(L);   // the GEMM run_ffn picks
     const bool with_scatter = !L->identity && !L->custom && !region_count && dispatch_supported(L->E) &&
-                              dispatch_scatter_supported(T, L->D, L->E);
+                              dispatch_scatter_supported(T, L->D, L->E) && !(pack && streamed);
     int* const zero = w.part_bytes ? buf.part_count : nullptr;
     if (!with_scatter)
         INFMOE_TRY(launch_dispatch(gate_in, T, L->E, pos, count, offset, L->d_status, stream, region_count, region_size,
@@ -1083,7 +1086,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     // whole layer: the variant decides; experts alone: the caller asks for the mix by passing the scores
     const bool mix = given_gate ? row_score != nullptr : L->flags.base_layer_mix;
     // the tensor-core GEMM writes the layer output itself (combine fused into its epilogue)
-    const bool fused_combine = !L->identity && !L->custom && uses_umma(L);
+    const bool fused_combine = pack;
     FfnOutput ffn_out;
     ffn_out.post = post;
     if (fused_combine) {
@@ -1143,21 +1146,25 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
         }
     } else {
         // 3. scatter fused with the experts' LayerNorm and the operand split (:354-355, T5FFLayer.cc:99-103)
-        const bool pack = uses_umma(L);   // the GEMM run_ffn picks
-        // tensor-core path: no routed copy, the second GEMM's epilogue reads its residual from d_in through pos[]
+        // Tensor-core path: no routed copy, the second GEMM's epilogue reads its residual from d_in through pos[].  The
+        // LayerNorm weights to apply lie in the weight slots (launch_split_expert), so the rows of an expert that is
+        // streamed are scattered once it has arrived.
+        const size_t gamma_at = pack ? split_gamma_at(2 * L->F, L->D) : 0;
+        const auto scatter_pack = [&](long long row0, long long rows, const float* plane, const int* slots) {
+            return launch_scatter_ln_pack(row0, rows, L->D, d_in, score, pos, gate_in, plane + gamma_at, s->plane_elems(0), slots,
+                                          valid_rows, rscore, buf.h, buf.row_info, stream);
+        };
         if (with_scatter) {
-            INFMOE_TRY(launch_dispatch_scatter(T, L->D, L->E, d_in, score, gate_in, s->d_ln, pos, count, offset,
-                                               L->d_status, zero, FFN_COUNTERS, routed, rscore, buf.h, buf.row_info, pack,
-                                               stream));
-            if (pack) routed = const_cast<float*>(d_in);
+            INFMOE_TRY(launch_dispatch_scatter(T, L->D, L->E, d_in, score, gate_in, pack ? s->d_plane[0] + gamma_at : s->d_ln,
+                                               pack ? s->plane_elems(0) : (size_t)L->D, pos, count, offset, L->d_status, zero,
+                                               FFN_COUNTERS, routed, rscore, buf.h, buf.row_info, pack, stream));
         } else if (pack) {
-            INFMOE_TRY(launch_scatter_ln_pack(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, rscore, buf.h,
-                                              buf.row_info, stream));
-            routed = const_cast<float*>(d_in);   // run_ffn's residual operand
+            if (!streamed) INFMOE_TRY(scatter_pack(0, T, s->d_plane[0], nullptr));
         } else {
             INFMOE_TRY(launch_scatter_ln_rows(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, routed, rscore,
                                               buf.h, stream));
         }
+        if (pack) routed = const_cast<float*>(d_in);   // run_ffn's residual operand
         INFMOE_TRY(prof_mark(L, 3, stream));
         // 4. experts (:360-402)
         if (!streamed) {
@@ -1212,9 +1219,11 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
             if (all_cached) {
                 // nothing to copy: one grouped launch over all experts, as in resident mode
                 for (const CachePlan& pl : plan) INFMOE_CUDA_TRY(cudaStreamWaitEvent(stream, L->ev_ready[pl.slot], 0));
+                if (pack) INFMOE_TRY(scatter_pack(0, T, planes[0], slot_map));
                 INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, slot_map, nslots, planes, buf, routed, ffn_out, stream));
                 for (const CachePlan& pl : plan) INFMOE_CUDA_TRY(cudaEventRecord(L->ev_freed[pl.slot], stream));
             }
+            long long row0 = 0;      // rows are in expert order
             for (size_t j = 0; j < active.size() && !all_cached; ++j) {
                 const int e = active[j];
                 const int slot = plan[j].slot;
@@ -1227,8 +1236,8 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                     // rotation for the cache, each reusable once its retile kernels are done
                     const int area = cached ? (int)(loads % (size_t)L->mc) : slot;
                     if (cached) INFMOE_CUDA_TRY(cudaStreamWaitEvent(cs, L->ev_stage[area], 0));
-                    INFMOE_TRY(load_expert_planes(s->split, L->D, L->F, s->h_wi0[e], s->h_wi1[e], s->h_wo[e],
-                                                  planes[0] + n0 * slot, planes[1] + n1 * slot, true,
+                    INFMOE_TRY(load_expert_planes(s->split, L->D, L->F, s->d_ln + (size_t)e * L->D, s->h_wi0[e],
+                                                  s->h_wi1[e], s->h_wo[e], planes[0] + n0 * slot, planes[1] + n1 * slot, true,
                                                   staging + 3 * n * area, cs));
                     if (cached) INFMOE_CUDA_TRY(cudaEventRecord(L->ev_stage[area], cs));
                     INFMOE_CUDA_TRY(cudaEventRecord(L->ev_ready[slot], cs));
@@ -1236,6 +1245,8 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                     ++loads;
                 }
                 INFMOE_CUDA_TRY(cudaStreamWaitEvent(stream, L->ev_ready[slot], 0));
+                if (pack) INFMOE_TRY(scatter_pack(row0, L->h_count[e], planes[0], slot_map));
+                row0 += L->h_count[e];
                 INFMOE_TRY(run_ffn(L, T, e, e + 1, offset, slot_map, nslots, planes, buf, routed, ffn_out, stream));
                 INFMOE_CUDA_TRY(cudaEventRecord(L->ev_freed[slot], stream));
             }
@@ -1827,9 +1838,9 @@ int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_
     INFMOE_CUDA_TRY(cudaMemsetAsync(offset, 0, 4, stream));
     INFMOE_TRY(launch_fill_int(offset + 1, (int)rows, stream));
     INFMOE_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), stream));
+    INFMOE_TRY(load_expert_planes(!simt, D, F, ln_w, wi0, wi1, wo, planes[0], planes[1], false, nullptr, stream));
     if (simt) INFMOE_TRY(launch_ln_rows(rows, D, x, ln_w, h, stream));
-    else INFMOE_TRY(launch_ln_pack(rows, D, x, ln_w, h, row_info, stream));
-    INFMOE_TRY(load_expert_planes(!simt, D, F, wi0, wi1, wo, planes[0], planes[1], false, nullptr, stream));
+    else INFMOE_TRY(launch_ln_pack(rows, D, x, planes[0] + split_gamma_at(2 * F, D), h, row_info, stream));
     int dev = 0, sms = 0;
     INFMOE_CUDA_TRY(cudaGetDevice(&dev));
     INFMOE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1858,9 +1869,10 @@ int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_
 }  // namespace
 
 namespace {
-// Scratch measure: two FP32 planes each of h and g and the weight tiles, more than either form needs but for the row scales and row_info of the tensor-core form (which are at most
-// 2 MB beside a scratch of 32 MB: 768 bytes per 128-row weight block, which has at least one 16 KB tile).
-// It is also the measure of what infmoe_t5ff_run_static takes.
+// Scratch measure: two FP32 planes each of h and g and the weight tiles.  That is more than either form needs, but for
+// what lies behind the tensor-core form's weight tiles: 768 bytes per 128-row block and 256 per 32-column block (a block has
+// at least one 16 KB tile), so at most 2 MB beside a scratch of 32 MB, and 128 bytes.  row_info, 8 bytes per row, takes
+// the place of the second planes.  It is also the measure of what infmoe_t5ff_run_static takes.
 size_t t5ff_scratch_bytes(int64_t rows, int32_t D, int32_t F) {
     const size_t r = (size_t)rows, d = (size_t)D, f = (size_t)F;
     return align_up(4 * r * d) + align_up(pack_bytes(rows, D)) + align_up(4 * r * f) + align_up(pack_bytes(rows, F)) +
@@ -1914,7 +1926,7 @@ int infmoe_t5ff_run(int64_t rows, int32_t D, int32_t F, const float* ln_w, const
 // larger problems are rejected and belong to infmoe_t5ff_run.  Like infmoe_t5ff_run the call
 // blocks the host until the result is there.
 #define INFMOE_STATIC_SCRATCH_BYTES (32u << 20)
-#define INFMOE_STATIC_SCALE_BYTES (2u << 20)   // row scales beside the scratch, see t5ff_scratch_bytes
+#define INFMOE_STATIC_SCALE_BYTES (3u << 20)   // scales beside the scratch, see t5ff_scratch_bytes
 static __device__ __align__(256) unsigned char g_static_scratch[INFMOE_STATIC_SCRATCH_BYTES + INFMOE_STATIC_SCALE_BYTES];
 
 namespace {

@@ -9,8 +9,14 @@
 //   fused_batch_mix_and_gather_kernel        plugin/cuda/moe.cu:115-127
 //   cuApplyLayerNorm                         plugin/cuda/ops/layernorm.cu:136-174
 //   gelu_dot functor via thrust::transform   plugin/cuda/ops/gelu.cu:6-25
+#include <cooperative_groups.h>
+
+#include <climits>
+
 #include "common.cuh"
 #include "kernels.h"
+
+namespace cg = cooperative_groups;
 
 namespace infmoe {
 
@@ -44,8 +50,8 @@ scatter_kernel(long long T, int D, int vec, const float* __restrict__ X, const f
 }
 
 // The layer's fused scatter: X[pos[j],:] -> its per-expert LayerNorm h = LN(x; gamma_e) (T5FFLayer.cc:99-103), ready
-// for the grouped GEMM.  gamma is [E][D]; the expert of row j is gate[pos[j]].  Rows at or past *valid_rows (tokens
-// without an expert, empty receive slots) are skipped.
+// for the grouped GEMM.  The expert of row j is gate[pos[j]].  Rows at or past *valid_rows (tokens without an expert,
+// empty receive slots) are skipped.
 //
 // For the CUDA-core GEMM: the routed row, the routed score, and h in FP32, rows padded with zeros to whole groups of 32.
 __device__ __forceinline__ void warp_ln_rows(const float* __restrict__ src, const float* __restrict__ gamma, int D,
@@ -121,19 +127,28 @@ __device__ __forceinline__ void warp_ln_pack(const float* __restrict__ src, cons
     if (lane == 0) *info = token_row_info(s, squares);
 }
 
-// The scatter for the tensor-core GEMM (which reads its residual from X through pos[], so no routed row is written).
+// The scatter for the tensor-core GEMM (which reads its residual from X through pos[], so no routed row is written), of
+// rows j0 .. j0 + T - 1.  The LayerNorm weights are those of the experts' weight slots (gamma', see SplitExpert).
+struct SlotGamma {
+    const float* base;              // first slot
+    size_t stride;                  // floats between slots
+    const int* slot_of_expert;      // NULL: identity
+    __device__ __forceinline__ const float* of(int e) const {
+        return base + stride * (size_t)(slot_of_expert ? slot_of_expert[e] : e);
+    }
+};
 __global__ void __launch_bounds__(ROW_WARPS * 32)
-scatter_ln_pack_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ score,
-                       const int* __restrict__ pos, const int* __restrict__ gate, const float* __restrict__ gamma_all,
-                       const int* __restrict__ valid_rows, float* __restrict__ rscore, uint16_t* __restrict__ h,
-                       float2* __restrict__ row_info) {
+scatter_ln_pack_kernel(long long j0, long long T, int D, int vec, const float* __restrict__ X,
+                       const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
+                       const SlotGamma gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
+                       uint16_t* __restrict__ h, float2* __restrict__ row_info) {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
-    if (j >= T || (valid_rows && j >= *valid_rows)) return;
+    const long long j = j0 + (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
+    if (j >= j0 + T || (valid_rows && j >= *valid_rows)) return;
     const int p = pos[j];
-    warp_ln_pack(X + (long long)p * D, gamma_all + (long long)gate[p] * D, D, vec != 0,
+    warp_ln_pack(X + (long long)p * D, gamma.of(gate[p]), D, vec != 0,
                  h + j * (long long)pack_pitch(D), row_info + j);
     if (lane == 0 && rscore && score) rscore[j] = score[p];
 }
@@ -147,21 +162,21 @@ scatter_ln_pack_kernel(long long T, int D, int vec, const float* __restrict__ X,
 // Bound by HBM: reads 4 D and writes 4 D bytes per row (a third less than the two planes it wrote before).
 template <int NV>
 __global__ void __launch_bounds__(128)
-scatter_ln_pack_reg_kernel(long long T, int D, const float* __restrict__ X, const float* __restrict__ score,
-                           const int* __restrict__ pos, const int* __restrict__ gate,
-                           const float* __restrict__ gamma_all, const int* __restrict__ valid_rows,
-                           float* __restrict__ rscore, uint16_t* __restrict__ h, float2* __restrict__ row_info) {
+scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __restrict__ X,
+                           const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
+                           const SlotGamma slot_gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
+                           uint16_t* __restrict__ h, float2* __restrict__ row_info) {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const long long j = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (j >= T || (valid_rows && j >= *valid_rows)) return;
+    const long long j = j0 + (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (j >= j0 + T || (valid_rows && j >= *valid_rows)) return;
     extern __shared__ __align__(16) float4 s_gamma_all[];     // [4 warps][NV * 32]
     float4* s_gamma = s_gamma_all + (threadIdx.x >> 5) * (NV * 32);
     const int p = pos[j];
     const int e = gate[p];
     const float4* src = reinterpret_cast<const float4*>(X + (long long)p * D);
-    const float4* gamma = reinterpret_cast<const float4*>(gamma_all + (long long)e * D);
+    const float4* gamma = reinterpret_cast<const float4*>(slot_gamma.of(e));
     float4 v[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -243,7 +258,7 @@ constexpr int DS_THREADS = 128;
 template <bool PACK>
 __global__ void __launch_bounds__(DS_THREADS)
 dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ X, const float* __restrict__ score,
-                        const int* __restrict__ gate, const float* __restrict__ gamma_all, int* __restrict__ pos,
+                        const int* __restrict__ gate, const SlotGamma slot_gamma, int* __restrict__ pos,
                         int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
                         int* __restrict__ zero, int zero_count, float* __restrict__ routed, float* __restrict__ rscore,
                         void* __restrict__ h, float2* __restrict__ row_info) {
@@ -290,7 +305,7 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
     int e = gate[t];
     if (e < 0 || e >= E) e = E;
     const float* src = X + (size_t)t * D;
-    const float* gamma = gamma_all + (size_t)(e < E ? e : 0) * D;
+    const float* gamma = slot_gamma.of(e < E ? e : 0);
     if (vec) {
         for (int k = 4 * tid; k < D; k += 4 * DS_THREADS) {
             const uint32_t dx = (uint32_t)__cvta_generic_to_shared(s_x + k), dg = (uint32_t)__cvta_generic_to_shared(s_g + k);
@@ -488,113 +503,281 @@ retile_kernel(const float* __restrict__ src0, const float* __restrict__ src1, in
     dst[seg * 32 + lane] = v;
 }
 
-// Tensor-core GEMM: both planes of an expert in two launches (an expert that is streamed pays for them on every call).
+// Tensor-core GEMM: both planes of an expert in three launches (an expert that is streamed pays for them on every call).
+//
+// An FP16 pair holds an FP32 value to its last bit only down to 2^-17 of the largest value under the same power of two
+// (split_f16), and there is one power of two per row of an operand.  A layer whose values are uneven inside a row, one
+// neuron with large weights or LayerNorm weights of many magnitudes, would lose its small values.  So the layout evens
+// the rows out by powers of two that cancel in the products, all exact:
+//   per column k of wi_0 / wi_1   2^E_k, E_k the exponent of the column's largest weight, moves from both matrices into
+//                                 the LayerNorm weight: gamma'[k] = gamma[k] 2^E_k is what the scatter kernels apply.  h'
+//                                 then holds every feature at the size at which it counts in the product, so features
+//                                 and columns of any magnitudes that make up for one another are even again
+//   per neuron f                  2^a_f moves from column f of wo into g: a_f = max ω - ω_f (+ share), ω_f = log2(|wi_0'[f]|
+//                                 |wi_1'[f]|) (2-norms, rounded up).  g_f 2^a_f is at most |h'|^2 2^(max ω) whichever neuron it is
+//                                 (g_exponent), and a neuron with large weights no longer sets the scale of all the others.
+//                                 2^a_f is part of the 2^-s kept for the rows of wi_1, so the GEMM kernels do nothing for it
+//   share                         where neurons remain uneven, ω_f plus the exponent of wo's column f being more than 2^14
+//                                 below the largest, half of what is beyond that (at most 2^8) goes back to g: g has a few
+//                                 bits to spare, wo 17, and so both keep about the same
+// Error against 64 bits of the expert term, worst token, d_model 1024 to 4096 (operands emulated on the CPU; before = one
+// scale per row without this; tf32 = TF32 head and BF16 tails): ordinary weights 1.8e-7 (before 1.8e-7, tf32 1.3e-6); one neuron
+// x 1000, its wo column / 10^6, 1.8e-7 (1.0e-3, 1.3e-6); LayerNorm weights over 2^-8..2^8, wi inverse, 1.8e-7 (5.9e-2, 1.3e-6); over
+// 2^-24..2^24 1.7e-7 (1.0, 1.3e-6); one neuron x 4096, nothing making up for it, 1e-6 to 2e-5 (3e-2 to 1e-1, 3e-5 to 5e-5).
+// What remains out of reach: a value more than 2^20 below the largest of its row after all this, in a product to which
+// the larger ones contribute nothing (their weights being zero).
+constexpr int SHARE_FROM = 14, SHARE_MOST = 8, GAIN_MOST = 64;   // limits of a_f, as exponents
+constexpr int W01_EXPONENT_MOST = 110;                           // of a row of wi: 2^-s 2^a_f stays a normal float
+
 struct SplitExpert {
-    const float *wi0, *wi1, *wo;
+    const float *gamma, *wi0, *wi1, *wo;
     int D, F;
-    float *w01, *wo_dst;         // destination planes
-    int MB[2], KB[2];            // 128-row and 32-column blocks of w01 (0) and wo (1)
-    float* inv[2];               // 2^-s of every padded row
-    float* norms;                // log2(|wi_0[f]| |wi_1[f]|) of every padded f
-    uint32_t* bound;             // the largest of them, encoded
+    float *w01, *wo_dst;         // destination planes; behind their tiles:
+    float *inv01, *inv_wo;       // 2^-s of every padded row (wi_1 rows: times 2^a_f)
+    int* range;                  // max over f of ω_f and of ω_f + exponent of wo's column f
+    int* omega;                  // ω_f
+    int *col01, *col_wo;         // exponent of the largest weight of every padded column
+    float* gamma_out;            // gamma'
+    int KB01, KBwo;              // 32-column blocks
 };
 
-// First pass: 2^-s of every padded row from its largest magnitude, and log2 of the norm products behind the gate bound
-// (g_exponent).  One warp per row (w01: per f, two rows); squares are summed in 64 bits because the magnitudes may be
-// anywhere in the FP32 range.  HBM bound; vec: rows are 16-byte aligned.
-__device__ __forceinline__ void warp_row_size(const float* __restrict__ row, int K, bool vec, float& top, double& sum) {
-    const int lane = threadIdx.x & 31;
-    top = 0.f;
-    sum = 0.0;
-    if (vec) {
-#pragma unroll 8
-        for (int k = 4 * lane; k < K; k += 128) {
-            const float4 v = *reinterpret_cast<const float4*>(row + k);
-            top = fmaxf(fmaxf(fmaxf(top, fabsf(v.x)), fmaxf(fabsf(v.y), fabsf(v.z))), fabsf(v.w));
-            sum += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
-        }
-    } else {
-#pragma unroll 8
-        for (int k = lane; k < K; k += 32) {
-            const float v = row[k];
-            top = fmaxf(top, fabsf(v));
-            sum += (double)v * v;
-        }
-    }
-    top = warp_max(top);
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+// biased exponent; of a zero: below that of any other value under any shift
+__device__ __forceinline__ int exponent_field(float x) {
+    const int u = __float_as_int(x) & 0x7fffffff;
+    return u ? u >> 23 : -4000;
 }
-__global__ void __launch_bounds__(256)
-row_scale_kernel(const SplitExpert a, int vec) {
-    const int lane = threadIdx.x & 31;
-    int w = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5);
-    float top;
-    double sum0 = 0.0, sum1 = 0.0;
-    if (w < a.MB[0] * 64) {      // rows 2 f and 2 f + 1 of w01
-        float top1 = top = 0.f;
-        if (w < a.F) {
-            warp_row_size(a.wi0 + (size_t)w * a.D, a.D, vec != 0, top, sum0);
-            warp_row_size(a.wi1 + (size_t)w * a.D, a.D, vec != 0, top1, sum1);
-        }
-        if (lane == 0) {
-            a.inv[0][2 * w] = exp2_int(-row_exponent(top));
-            a.inv[0][2 * w + 1] = exp2_int(-row_exponent(top1));
-            a.norms[w] = 0.5f * ((float)log2(sum0) + (float)log2(sum1));     // -inf past the matrix
-        }
-        return;
-    }
-    w -= a.MB[0] * 64;
-    if (w >= a.MB[1] * 128) return;
-    top = 0.f;
-    if (w < a.D) warp_row_size(a.wo + (size_t)w * a.F, a.F, vec != 0, top, sum0);
-    if (lane == 0) a.inv[1][w] = exp2_int(-row_exponent(top));
+// x 2^e for any e that two normal factors make up; exact unless the result is below the normal range
+__device__ __forceinline__ float scale_by(float x, int e) {
+    const int half = e >> 1;
+    return __fmul_rn(__fmul_rn(x, exp2_int(half)), exp2_int(e - half));
+}
+__device__ __forceinline__ float4 load4(const float* __restrict__ p, bool vec) {
+    return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
 }
 
-// Second pass: the tiles as FP16 pairs, a row of a tile being 32 x hi, 32 x lo of the values times 2^s.  A block per tile,
-// 16 lanes per row, two values each, the values of eight rows in flight.  The last block takes the maximum of the norms.
-__global__ void __launch_bounds__(256)
-split_tiles_kernel(const SplitExpert a) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (blockIdx.x == gridDim.x - 1) {
-        __shared__ uint32_t s_bound[8];
-        uint32_t best = 0;
-        for (int f = (int)threadIdx.x; f < a.MB[0] * 64; f += 256) best = max(best, encode_bound(a.norms[f]));
-        best = __reduce_max_sync(0xffffffffu, best);
-        if (lane == 0) s_bound[warp] = best;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int i = 1; i < 8; ++i) best = max(best, s_bound[i]);
-            *a.bound = best;
+// Column exponents.  A cluster of eight blocks per 32 columns, eight lanes to a row (four columns each), the rows dealt out
+// over the cluster's 256 such groups; the blocks' maxima meet in the first one through distributed shared memory, so
+// nothing has to be zeroed first.  Bound by HBM (each weight is read once).  Magnitudes are compared as integers, so
+// NaN counts as the largest.
+constexpr int COL_CLUSTER = 8;
+__global__ void __launch_bounds__(256) __cluster_dims__(COL_CLUSTER, 1, 1)
+column_exponent_kernel(const SplitExpert a, int vec) {
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ uint32_t s_warp[8][32];
+    __shared__ uint32_t s_block[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = (int)cluster.block_rank();
+    int slab = (int)blockIdx.x / COL_CLUSTER;
+    const bool wo = slab >= a.KB01;
+    if (wo) slab -= a.KB01;
+    const int K = wo ? a.F : a.D, rows = wo ? a.D : a.F, k = slab * 32 + 4 * (lane & 7);
+    const int first = (rank * 256 + (int)threadIdx.x) >> 3;
+    uint32_t top[4] = {0, 0, 0, 0};
+    const auto take = [&](const float4 v) {
+        top[0] = max(top[0], __float_as_uint(v.x) & 0x7fffffffu);
+        top[1] = max(top[1], __float_as_uint(v.y) & 0x7fffffffu);
+        top[2] = max(top[2], __float_as_uint(v.z) & 0x7fffffffu);
+        top[3] = max(top[3], __float_as_uint(v.w) & 0x7fffffffu);
+    };
+    pdl_trigger();
+    if (k < K) {                                               // K is a multiple of 4
+        if (wo) {
+#pragma unroll 8
+            for (int r = first; r < rows; r += 32 * COL_CLUSTER) take(load4(a.wo + (size_t)r * K + k, vec != 0));
+        } else {
+#pragma unroll 4
+            for (int r = first; r < rows; r += 32 * COL_CLUSTER) {
+                const float4 v0 = load4(a.wi0 + (size_t)r * K + k, vec != 0), v1 = load4(a.wi1 + (size_t)r * K + k, vec != 0);
+                take(v0);
+                take(v1);
+            }
         }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        top[i] = max(top[i], __shfl_xor_sync(0xffffffffu, top[i], 8));
+        top[i] = max(top[i], __shfl_xor_sync(0xffffffffu, top[i], 16));
+        if (lane < 8) s_warp[warp][4 * lane + i] = top[i];
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        uint32_t best = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) best = max(best, s_warp[w][lane]);
+        s_block[lane] = best;
+    }
+    cluster.sync();
+    if (rank == 0 && threadIdx.x < 32) {
+        const int column = slab * 32 + lane;
+        uint32_t best = 0;
+#pragma unroll
+        for (int q = 0; q < COL_CLUSTER; ++q) best = max(best, cluster.map_shared_rank(s_block, q)[lane]);
+        const int field = (int)(best >> 23);
+        const int e = column < K && field < 255 ? max(field - 127, -126) : 0;     // infinities and NaN move nothing
+        (wo ? a.col_wo : a.col01)[column] = e;
+        if (!wo) a.gamma_out[column] = column < K ? __fmul_rn(a.gamma[column], exp2_int(e)) : 0.f;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 2) a.range[threadIdx.x] = INT_MIN;
+    cluster.sync();                                            // no block leaves while its maxima can still be read
+}
+
+// a_f from ω_f, the exponent of wo's column f and the two maxima.
+__device__ __forceinline__ int neuron_gain(int omega, int column, int max_omega, int max_reach) {
+    const int below = max_reach - (omega + column);
+    const int share = below > SHARE_FROM ? min((below - SHARE_FROM + 1) / 2, SHARE_MOST) : 0;
+    return min(max(max_omega - omega - share, -SHARE_MOST), GAIN_MOST);
+}
+
+// ROWS weight rows side by side, their elements times 2^-shift[k], to FP16 pairs in their rows of the tiles (a row of a tile
+// being 32 x hi, 32 x lo), each scaled by 2^s so that its largest magnitude lands in [2^14, 2^15).  `squares` are the sums
+// of squares of the scaled rows.  WARPS warps of the block share the rows, 128 columns at a time: a lane holds four
+// neighbouring values, so a warp reads 512 bytes and writes four whole 128-byte rows.  The rows are read twice, the second
+// time from L1 or L2.  in = false: rows of zeros.  Bound by HBM for large experts, by latency for small ones.  Rows are few and
+// long or many and short, and WARPS makes up about as many warps either way.  Columns, w01, wo, us: 4096 x 10240 85, 168, 112;
+// 1024 x 4096 14, 17, 15; 160 x 600 5.7, 4.6, 5.3.  A whole set_expert at 1024 x 4096: 103 with one warp per row and eight
+// blocks per 128 columns, now 63 (60 without the column scales).
+template <int ROWS, int WARPS, typename Shift>
+__device__ __forceinline__ void split_rows(const float* const (&row)[ROWS], bool in, int K, int KB, bool vec, int most,
+                                           uint32_t* const (&dst)[ROWS], const Shift& shift, int (&s)[ROWS],
+                                           float (&squares)[ROWS]) {
+    __shared__ int s_top[8][ROWS];
+    __shared__ float s_squares[8][ROWS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % WARPS, group = warp / WARPS * WARPS;
+    constexpr int INFINITE = 4000;
+    int top[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) top[i] = -4000;
+    if (in) {
+#pragma unroll 4
+        for (int k = 4 * lane + 128 * part; k < K; k += 128 * WARPS) {
+            float4 v[ROWS];
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) v[i] = load4(row[i] + k, vec);
+            const int4 c = shift(k);
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                const int f0 = exponent_field(v[i].x), f1 = exponent_field(v[i].y), f2 = exponent_field(v[i].z),
+                          f3 = exponent_field(v[i].w);
+                top[i] = max(max(max(top[i], f0 - c.x), max(f1 - c.y, f2 - c.z)), f3 - c.w);
+                if (max(max(f0, f1), max(f2, f3)) == 255) top[i] = INFINITE;
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        top[i] = __reduce_max_sync(0xffffffffu, top[i]);
+        if (WARPS > 1 && lane == 0) s_top[warp][i] = top[i];
+    }
+    if (WARPS > 1) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) top[i] = max(top[i], s_top[group + w][i]);
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        // a row with an infinity or a NaN only has to hand it on; a row of zeros takes any scale
+        s[i] = !in || top[i] == INFINITE ? 0 : min(max(14 + 127 - top[i], -126), most);
+        squares[i] = 0.f;
+    }
+#pragma unroll 2
+    for (int k = 4 * lane + 128 * part; k < KB * 32; k += 128 * WARPS) {
+        float4 w[ROWS];
+        int4 c = make_int4(0, 0, 0, 0);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) w[i] = in && k < K ? load4(row[i] + k, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (in && k < K) c = shift(k);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            const float v[4] = {scale_by(w[i].x, s[i] - c.x), scale_by(w[i].y, s[i] - c.y), scale_by(w[i].z, s[i] - c.z),
+                                scale_by(w[i].w, s[i] - c.w)};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) squares[i] = fmaf(v[j], v[j], squares[i]);
+            store_pack4(reinterpret_cast<uint16_t*>(dst[i] + (size_t)(k >> 5) * 4096), k & 31, v);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        squares[i] = warp_xor_sum(squares[i]);
+        if (WARPS > 1 && lane == 0) s_squares[warp][i] = squares[i];
+    }
+    if (WARPS > 1) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            squares[i] = 0.f;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) squares[i] += s_squares[group + w][i];
+        }
+    }
+}
+
+// w01: WARPS warps per neuron f, the rows 2 f = wi_0[f] and 2 f + 1 = wi_1[f].
+template <int WARPS>
+__global__ void __launch_bounds__(256)
+split_w01_kernel(const SplitExpert a, int vec) {
+    __shared__ int s_omega[8], s_reach[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int f = ((int)blockIdx.x * 8 + warp) / WARPS;        // the grid covers the padded rows exactly
+    pdl_trigger();
+    pdl_wait();
+    const auto shift = [&](int k) { return *reinterpret_cast<const int4*>(a.col01 + k); };
+    const bool in = f < a.F;
+    const float* const row[2] = {a.wi0 + (size_t)f * a.D, a.wi1 + (size_t)f * a.D};
+    uint32_t* const dst0 = reinterpret_cast<uint32_t*>(a.w01) + (size_t)(f >> 6) * a.KB01 * 4096 + (size_t)(f & 63) * 64;
+    uint32_t* const dst[2] = {dst0, dst0 + 32};
+    float squares[2];
+    int s[2];
+    split_rows<2, WARPS>(row, in, a.D, a.KB01, vec != 0, W01_EXPONENT_MOST, dst, shift, s, squares);
+    if (lane == 0) {
+        int omega = -1000, reach = -1000;
+        if (in) {
+            const float w = 0.5f * (log2f(squares[0]) + log2f(squares[1])) - (float)(s[0] + s[1]) + 0.01f;
+            omega = w > -400.f ? (int)ceilf(fminf(w, 400.f)) : -400;    // a row of zeros, or a NaN
+            reach = omega + a.col_wo[f];
+            a.omega[f] = omega;
+        }
+        a.inv01[2 * f] = exp2_int(-s[0]);
+        a.inv01[2 * f + 1] = exp2_int(-s[1]);                  // times 2^a_f in the next launch
+        s_omega[warp] = omega;
+        s_reach[warp] = reach;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; ++i) {
+            s_omega[0] = max(s_omega[0], s_omega[i]);
+            s_reach[0] = max(s_reach[0], s_reach[i]);
+        }
+        atomicMax(a.range, s_omega[0]);
+        atomicMax(a.range + 1, s_reach[0]);
+    }
+}
+
+// wo: WARPS warps per row; the blocks behind those of the rows multiply 2^a_f into 2^-s of wi_1's rows.
+template <int WARPS>
+__global__ void __launch_bounds__(256)
+split_wo_kernel(const SplitExpert a, int vec, int row_blocks) {
+    pdl_trigger();
+    pdl_wait();
+    const int max_omega = a.range[0], max_reach = a.range[1];
+    if ((int)blockIdx.x >= row_blocks) {
+        const int f = ((int)blockIdx.x - row_blocks) * 256 + (int)threadIdx.x;
+        if (f < a.F)
+            a.inv01[2 * f + 1] = __fmul_rn(a.inv01[2 * f + 1], exp2_int(neuron_gain(a.omega[f], a.col_wo[f], max_omega, max_reach)));
         return;
     }
-    int tile = (int)blockIdx.x;                    // tiles of w01, then of wo
-    const int which = tile >= a.MB[0] * a.KB[0] ? 1 : 0;
-    if (which) tile -= a.MB[0] * a.KB[0];
-    const int mb = tile / a.KB[which], kb = tile % a.KB[which];
-    const int M = which ? a.D : 2 * a.F, K = which ? a.F : a.D, k = kb * 32 + 2 * (lane & 15);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(which ? a.wo_dst : a.w01) + (size_t)tile * 4096 + (lane & 15);
-    const float* inv = a.inv[which] + mb * 128;
-    float v[8][2];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {                  // rows warp * 16 + 2 i (+ 1 in the upper half of the warp)
-        const int m = mb * 128 + warp * 16 + 2 * i + (lane >> 4);
-        v[i][0] = v[i][1] = 0.f;
-        if (m < M) {
-            const float* row = which ? a.wo + (size_t)m * K : ((m & 1) ? a.wi1 : a.wi0) + (size_t)(m >> 1) * K;
-            if (k < K) v[i][0] = row[k];
-            if (k + 1 < K) v[i][1] = row[k + 1];
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = warp * 16 + 2 * i + (lane >> 4);
-        const float scale = __fdiv_rn(1.0f, inv[r]);     // 2^s exactly (both are normal)
-        const uint32_t p0 = split_f16(__fmul_rn(v[i][0], scale)), p1 = split_f16(__fmul_rn(v[i][1], scale));
-        dst[r * 32] = __byte_perm(p0, p1, 0x5410);
-        dst[r * 32 + 16] = __byte_perm(p0, p1, 0x7632);
-    }
+    const int r = ((int)blockIdx.x * 8 + (int)(threadIdx.x >> 5)) / WARPS;
+    const auto shift = [&](int k) {
+        const int4 w = *reinterpret_cast<const int4*>(a.omega + k), c = *reinterpret_cast<const int4*>(a.col_wo + k);
+        return make_int4(neuron_gain(w.x, c.x, max_omega, max_reach), neuron_gain(w.y, c.y, max_omega, max_reach),
+                         neuron_gain(w.z, c.z, max_omega, max_reach), neuron_gain(w.w, c.w, max_omega, max_reach));
+    };
+    const float* const row[1] = {a.wo + (size_t)r * a.F};
+    uint32_t* const dst[1] = {reinterpret_cast<uint32_t*>(a.wo_dst) + (size_t)(r >> 7) * a.KBwo * 4096 + (size_t)(r & 127) * 32};
+    float unused[1];
+    int s[1];
+    split_rows<1, WARPS>(row, r < a.D, a.F, a.KBwo, vec != 0, 126, dst, shift, s, unused);
+    if ((threadIdx.x & 31) == 0) a.inv_wo[r] = exp2_int(-s[0]);
 }
 
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
@@ -621,15 +804,16 @@ int launch_scatter(long long T, int D, const float* X, const float* coeff, const
 bool dispatch_scatter_supported(long long T, int D, int E) { return T <= 1024 && D <= 6016 && E < 8192; }
 
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
-                            const float* gamma_all, int* pos, int* count, int* offset, int* status, int* zero,
-                            int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
+                            const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,
+                            int* zero, int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
                             cudaStream_t stream) {
-    const int vec = (D % 4 == 0) && aligned16(X) && aligned16(gamma_all);
+    const int vec = (D % 4 == 0) && (gamma_stride % 4 == 0) && aligned16(X) && aligned16(gamma);
     size_t smem = 2 * padded_row(D) * sizeof(float);
     if (smem < sizeof(int) * (size_t)(E + 1)) smem = sizeof(int) * (size_t)(E + 1);
     auto kern = pack ? dispatch_scatter_kernel<true> : dispatch_scatter_kernel<false>;
     INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)T + 1, DS_THREADS, smem, 1, stream, (int)T, D, E, vec, X, score, gate,
-                                   gamma_all, pos, count, offset, status, zero, zero ? zero_count : 0, routed, rscore, h,
+                                   SlotGamma{gamma, gamma_stride, nullptr}, pos, count, offset, status, zero,
+                                   zero ? zero_count : 0, routed, rscore, h,
                                    (float2*)row_info));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
@@ -648,11 +832,12 @@ int launch_scatter_ln_rows(long long T, int D, const float* X, const float* scor
     return INFMOE_OK;
 }
 
-int launch_scatter_ln_pack(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
-                           const float* gamma_all, const int* valid_rows, float* rscore, void* h, float* row_info,
-                           cudaStream_t stream) {
+int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, const float* score, const int* pos,
+                           const int* gate, const float* gamma, size_t gamma_stride, const int* slot_of_expert,
+                           const int* valid_rows, float* rscore, void* h, float* row_info, cudaStream_t stream) {
     if (T == 0) return INFMOE_OK;
-    const int vec = (D % 4 == 0) && aligned16(X) && aligned16(gamma_all);
+    const int vec = (D % 4 == 0) && (gamma_stride % 4 == 0) && aligned16(X) && aligned16(gamma);
+    const SlotGamma slots{gamma, gamma_stride, slot_of_expert};
     uint16_t* pack = (uint16_t*)h;
     float2* info = (float2*)row_info;
     if (vec && D <= 4096) {
@@ -663,7 +848,7 @@ int launch_scatter_ln_pack(long long T, int D, const float* X, const float* scor
         constexpr int smem = 4 * NV * 32 * 16;                                                                     \
         if (smem > 48 * 1024)                                                                                      \
             INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));        \
-        INFMOE_CUDA_TRY(launch_chained(kern, grid, 128, smem, 1, stream, T, D, X, score, pos, gate, gamma_all,     \
+        INFMOE_CUDA_TRY(launch_chained(kern, grid, 128, smem, 1, stream, row0, T, D, X, score, pos, gate, slots,   \
                                        valid_rows, rscore, pack, info));                                           \
     } while (0)
         if (D <= 1024) INFMOE_SCATTER_REG(8);
@@ -671,8 +856,8 @@ int launch_scatter_ln_pack(long long T, int D, const float* X, const float* scor
         else INFMOE_SCATTER_REG(32);
 #undef INFMOE_SCATTER_REG
     } else {
-        INFMOE_CUDA_TRY(launch_chained(scatter_ln_pack_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, T, D, vec, X, score,
-                                       pos, gate, gamma_all, valid_rows, rscore, pack, info));
+        INFMOE_CUDA_TRY(launch_chained(scatter_ln_pack_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, row0, T, D, vec, X,
+                                       score, pos, gate, slots, valid_rows, rscore, pack, info));
     }
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
@@ -771,9 +956,10 @@ int launch_ln_pack(long long n, int D, const float* in, const float* gamma, void
     return INFMOE_OK;
 }
 
-int launch_split_expert(const float* wi0, const float* wi1, const float* wo, int D, int F, float* w01, float* wo_dst,
-                        cudaStream_t stream) {
+int launch_split_expert(const float* gamma, const float* wi0, const float* wi1, const float* wo, int D, int F, float* w01,
+                        float* wo_dst, cudaStream_t stream) {
     SplitExpert a;
+    a.gamma = gamma;
     a.wi0 = wi0;
     a.wi1 = wi1;
     a.wo = wo;
@@ -781,19 +967,31 @@ int launch_split_expert(const float* wi0, const float* wi1, const float* wo, int
     a.F = F;
     a.w01 = w01;
     a.wo_dst = wo_dst;
-    a.MB[0] = (2 * F + 127) / 128;
-    a.KB[0] = (D + 31) / 32;
-    a.MB[1] = (D + 127) / 128;
-    a.KB[1] = (F + 31) / 32;
-    a.inv[0] = w01 + tiled_elems(2 * F, D);
-    a.inv[1] = wo_dst + tiled_elems(D, F);
-    a.bound = (uint32_t*)(w01 + split_bound_at(2 * F, D));
-    a.norms = w01 + split_bound_at(2 * F, D) + 32;
-    const int vec = D % 4 == 0 && F % 4 == 0 && aligned16(wi0) && aligned16(wi1) && aligned16(wo);
-    const int warps = a.MB[0] * 64 + a.MB[1] * 128;
-    row_scale_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(a, vec);
-    split_tiles_kernel<<<(unsigned)(a.MB[0] * a.KB[0] + a.MB[1] * a.KB[1] + 1), 256, 0, stream>>>(a);
-    note_launch(2);
+    a.inv01 = w01 + tiled_elems(2 * F, D);
+    a.inv_wo = wo_dst + tiled_elems(D, F);
+    a.range = (int*)(w01 + split_range_at(2 * F, D));
+    a.omega = a.range + 32;
+    a.col01 = (int*)(w01 + split_columns_at(2 * F, D));
+    a.col_wo = (int*)(wo_dst + split_columns_at(D, F));
+    a.gamma_out = w01 + split_gamma_at(2 * F, D);
+    a.KB01 = (D + 31) / 32;
+    a.KBwo = (F + 31) / 32;
+    const int vec = aligned16(wi0) && aligned16(wi1) && aligned16(wo);     // D and F are multiples of 4
+    column_exponent_kernel<<<(unsigned)((a.KB01 + a.KBwo) * COL_CLUSTER), 256, 0, stream>>>(a, vec);
+    INFMOE_CUDA_TRY(cudaGetLastError());
+    // one to eight warps per row: up to about 8000 of them, at least one step of 128 columns each
+    const auto warps_per_row = [](int rows, int K) {
+        int w = 1;
+        while (w < 8 && rows * w * 2 <= 8192 && w * 2 * 128 <= K + 127) w *= 2;
+        return w;
+    };
+    const int neurons = (2 * F + 127) / 128 * 64, rows = (D + 127) / 128 * 128;
+    const int w1 = warps_per_row(neurons, D), w2 = warps_per_row(rows, F), row_blocks = rows * w2 / 8;
+    auto k1 = w1 == 1 ? split_w01_kernel<1> : w1 == 2 ? split_w01_kernel<2> : w1 == 4 ? split_w01_kernel<4> : split_w01_kernel<8>;
+    auto k2 = w2 == 1 ? split_wo_kernel<1> : w2 == 2 ? split_wo_kernel<2> : w2 == 4 ? split_wo_kernel<4> : split_wo_kernel<8>;
+    INFMOE_CUDA_TRY(launch_chained(k1, (unsigned)(neurons * w1 / 8), 256, 0, 1, stream, a, vec));
+    INFMOE_CUDA_TRY(launch_chained(k2, (unsigned)(row_blocks + (F + 255) / 256), 256, 0, 1, stream, a, vec, row_blocks));
+    note_launch(3);
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
 }
