@@ -1001,21 +1001,42 @@ inline size_t rs_smem(int D) { return (size_t)RS_TOKENS * (size_t)((D + 127) / 1
 // Two rows per warp instead of four make the rows kernel wait for shared memory: with 32 experts and 2048 floats it takes
 // 39 us for 4096 tokens, where the tiled one multiplies all 32 at the price of one (31 us with 16).
 bool route_rows_supported(int D, int E, bool vec) { return vec && (D <= 1024 || (D <= 2048 && E <= 16)); }
-// The small kernel's time grows with T E once its clusters fill the chip, that of the others with a CTA's (32 tokens or
-// 16) until those do.  Measured, us (D, E; T).  Small against rows in registers: (1024, 8) 1024: 6.5 / 8.1, 2048: 11.2 /
-// 8.0; (2048, 8) 512: 5.9 / 6.0, 1024: 7.6 / 6.0; (1024, 16) 512: 6.8 / 10.3, 1024: 10.9 / 10.3; (512, 32) 512: 10.7 / 11.1;
-// (1024, 64) 256: 9.8 / 21, 512: 14.2 / 21, 1024: 27 / 21.  Small against tiled: (4096, 32) 512: 35 / 52, 1024: 52 / 52;
-// (4096, 8) 4096: 49 / 55, 16384: 185 / 233.
-bool use_small_route(long long T, int D, int E, bool rows) {
-    const long long e = E < 8 ? 8 : E;
+int rs_cluster(int E) {
+    int cluster = 1;
+    while (cluster < 8 && cluster * RS_WARPS < E) cluster *= 2;
+    return cluster;
+}
+// The small kernel's time grows with its blocks (T / 4 clusters) once these fill the chip, that of the others with a CTA's
+// (32 tokens or 16) until those do.  Measured, us, without the LayerNorm / with it.
+// Against rows in registers (D, E; T): (1024, 8) 1024: 6.5 / 8.1, 2048: 11.2 / 8.0; (2048, 8) 512: 5.9 / 6.0, 1024: 7.6 / 6.0;
+// (1024, 16) 512: 6.8 / 10.3, 1024: 10.9 / 10.3; (512, 32) 512: 10.7 / 11.1; (1024, 64) 256: 9.8 / 21, 512: 14.2 / 21, 1024:
+// 27 / 21 (all without the LayerNorm, warm caches).  Clusters of two step up where a fourth block comes to an SM, at 888
+// tokens, small | rows with cold caches: (1024, 9) 800: 11 | 12 and 13 | 17, 1000: 15 | 12 and 17 | 16; (512, 9) 1000: 13 | 10 and 19 | 14.
+// Against the tiled kernel, small | tiled, each with cold caches:
+//   two or more blocks on an SM (D <= 7168)
+//     E <= 8       any T: (4096, 8) 3500: 39 | 44 and 51 | 68, 4900: 53 | 80 and 72 | 128, 16384 0.91 and 0.79 of tiled.  Only
+//                  where the tiled kernel fills its first wave of 148 x 32 tokens nearly whole, and seven or eight experts
+//                  are scored without the LayerNorm, is it ahead: (4096, 8) 3700: 45 | 44, 4736: 53 | 45, (6400, 8) 4096: 76 | 64
+//     more         experts by the cluster's warps, T times those: (4096, 16) 1535: 35 | 43 and 47 | 62, (6144, 32) 767: 45 | 59,
+//                  (2560, 9) 2048 1.06 and 1.12 of tiled; rows of any alignment: (4095, 9) 2700 0.90 and 1.19
+//   one block      its eight warps wait for every row they load, and four waves of blocks (of 148; 128 in clusters of four
+//                  and more) is what pays: (8192, 8) 2304: 59 | 78 and 102 | 121, 2600: 72 | 78 and 121 | 125, 4096: 96 | 78 and
+//                  168 | 139; (12800, 16) 1152: 84 | 113 and 168 | 170; (12800, 32) 500: 80 | 113 and 164 | 165, 576: 96 | 113 and
+//                  201 | 166; (8191, 8) 4096: 258 | 227.  With up to four experts, aligned and without the LayerNorm, any T as
+//                  above: (8192, 1) 3072 0.87 of tiled, 4096 1.03, 16384 0.83, (12800, 4) 0.97, 1.13, 0.98
+bool use_small_route(long long T, int D, int E, bool rows, bool vec, bool ln) {
     if (rs_smem(D) > RS_MAX_SMEM) return false;
-    return rows ? T < 256 + 8192 / e : T * e < 24576 || E <= 8;
+    const int cluster = rs_cluster(E), e = cluster * RS_WARPS < E ? E : cluster * RS_WARPS;   // experts scored, idle warps too
+    if (rows) return T < (cluster == 2 ? 888 : 256 + 8192 / (E < 8 ? 8 : E));
+    const bool one_block = rs_smem(D) > 112 * 1024, whole_wave = T > 3600 && T <= 148 * RT_TOKENS;
+    if (one_block && !(vec && !ln && E <= 4)) return T * e <= 4 * (cluster <= 2 ? 148 : 128) * 32;
+    if (E <= 8) return !(vec && !ln && (E > 6 || one_block) && whole_wave);
+    return T * e < 24576;
 }
 template <bool VEC>
 int launch_route_small(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
                        float* score, int* status, cudaStream_t stream) {
-    int cluster = 1;
-    while (cluster < 8 && cluster * RS_WARPS < E) cluster *= 2;
+    const int cluster = rs_cluster(E);
     const size_t smem = rs_smem(D);
     auto kern = route_small_kernel<VEC>;
     if (smem > 40 * 1024)
@@ -1049,7 +1070,7 @@ int launch_route(const float* X, const float* C, const float* gamma, long long T
     static const bool no_tma = [] { const char* v = getenv("INFMOE_ROUTE"); return v && !strcmp(v, "cp_async"); }();
     CUtensorMap map_x, map_c;
     const bool rows = route_rows_supported(D, E, vec);
-    if (use_small_route(T, D, E, rows)) {
+    if (use_small_route(T, D, E, rows, vec, gamma != nullptr)) {
         INFMOE_TRY((vec ? launch_route_small<true> : launch_route_small<false>)(X, C, gamma, T, D, E, gate, score,
                                                                                status, stream));
     } else if (rows) {

@@ -67,6 +67,18 @@ def test_route_few_and_many_tokens(g, oracle, T, D, E, ln):
     test_route_bit_exact(g, oracle, T, D, E, ln)
 
 
+# Both sides of the lines between the few-token kernel and the tiled one: its rows two blocks to an SM or one (more than
+# 7168 floats), a nearly whole wave of the tiled kernel, experts rounded up to a cluster's warps.
+@pytest.mark.parametrize("T,D,E,ln", [(3600, 2052, 8, False), (3601, 2052, 8, False), (4736, 2052, 7, False),
+                                      (4737, 2052, 7, False), (3700, 2052, 8, True), (1535, 2052, 9, True),
+                                      (1536, 2052, 9, True), (2368, 7172, 8, True), (2369, 7172, 8, False),
+                                      (2369, 7168, 8, True), (2369, 7171, 5, True), (3700, 7172, 4, False),
+                                      (1184, 7300, 9, False), (1185, 7300, 9, True), (513, 7300, 17, True),
+                                      (887, 516, 9, True), (888, 516, 16, False), (737, 516, 17, False)])
+def test_route_lines_between_the_kernels(g, oracle, T, D, E, ln):
+    test_route_bit_exact(g, oracle, T, D, E, ln)
+
+
 def test_route_ties_and_nan(g, oracle):
     x = np.ones((5, 16), np.float32)
     c = np.ones((6, 16), np.float32)
