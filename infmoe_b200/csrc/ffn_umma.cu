@@ -1019,7 +1019,7 @@ int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_be
 size_t ffn_umma_part_bytes(long long T, int D, int F) {
     const int K = D > F ? D : F;
     const size_t chunks = (size_t)((K + BK - 1) / BK + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;
-    const size_t cols = (size_t)(T < 256 ? (T + 31) / 32 * 32 : 256);
+    const size_t cols = (size_t)(T < 192 ? (T + 31) / 32 * 32 : 192);    // the widest token tile
     const size_t need = (size_t)FFN_CTAS * chunks * cols * UMMA_M * sizeof(float);
     return need < (64u << 20) ? need : (size_t)(64u << 20);
 }

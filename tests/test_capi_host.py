@@ -77,8 +77,48 @@ def test_workspace_size_formula():
     layer = _layer()
     small, big = layer.get_workspace_size(1), layer.get_workspace_size(100)
     assert 0 < small < big
-    # activations: routed, post, h_hi, h_lo [T][D] and g_hi, g_lo [T][F]; slots: mc x 3 matrices of D x F
-    assert big >= 4 * 100 * (4 * 8 + 2 * 16) + 3 * 2 * 8 * 16 * 4
+
+
+def _up(*sizes):
+    return sum((n + 255) // 256 * 256 for n in sizes)
+
+
+def _blocks(n, of):
+    return (n + of - 1) // of
+
+
+@pytest.mark.parametrize("T,D,F", [(1, 8, 16), (100, 8, 16), (191, 40, 2052), (1000, 64, 256), (300, 256, 1000), (4096, 1024, 4096), (16384, 4096, 10240)])
+def test_workspace_of_the_tensor_core_path(T, D, F):
+    """What the layer works in: routing and dispatch arrays, h and g as FP16 pairs (four bytes a value, rows padded to 32),
+    two floats per row, the chunk sums of cut tiles and their counters, and max_concurrency streamed slots of two weight planes
+    and the raw matrices."""
+    E, mc, ctas = 3, 2, 148
+    layer = _layer(embedding_size=D, hidden_size=F, max_concurrency=mc,
+                   expert_centroids=np.zeros((E, D), np.float32))
+
+    def plane(M, K):     # tiles, 2^-s per padded row, 32 words, a word per neuron, column exponents and gamma'
+        return _blocks(M, 128) * 128 * _blocks(K, 32) * 32 + _blocks(M, 128) * (128 + 64) + 32 + 2 * _blocks(K, 32) * 32
+
+    chunks = _blocks(max(D, F), 256)
+    sums = min(ctas * chunks * min(_blocks(T, 32) * 32, 192) * 128 * 4, 64 << 20)   # 192: the widest token tile
+    want = _up(4 * T, 4 * T, 4 * E, 4 * (E + 1), 4 * E, 4 * T, 4 * T)
+    want += _up(T * _blocks(D, 32) * 128, T * _blocks(F, 32) * 128, 8 * T, sums, ctas * 16 * 4)
+    want += _up(4 * mc * (plane(2 * F, D) + plane(D, F) + 3 * D * F)) + 256
+    assert layer.get_workspace_size(T) == want
+
+
+@pytest.mark.parametrize("T,D,F", [(1, 7, 9), (100, 130, 50), (300, 510, 1022)])
+def test_workspace_of_the_cuda_core_path(T, D, F):
+    """Routed rows and results in expert order, h and g in FP32 rows padded to 32 (g also holds a row of d_model), and streamed
+    slots of raw tiles."""
+    E, mc = 3, 2
+    layer = _layer(embedding_size=D, hidden_size=F, max_concurrency=mc,
+                   expert_centroids=np.zeros((E, D), np.float32))
+    tiles = (_blocks(2 * F, 128) * _blocks(D, 32) + _blocks(D, 128) * _blocks(F, 32)) * 4096
+    want = _up(4 * T, 4 * T, 4 * E, 4 * (E + 1), 4 * E, 4 * T, 4 * T, 4 * T * D, 4 * T * D)
+    want += _up(T * _blocks(D, 32) * 128, T * _blocks(max(D, F), 32) * 128)
+    want += _up(4 * mc * (tiles + 3 * D * F)) + 256
+    assert layer.get_workspace_size(T) == want
 
 
 def test_python_binding_surface(tmp_path):
