@@ -25,8 +25,8 @@ is the CPU restatement of the reference's math timed on this box's host cores on
 a bounded sample.  N > 1 adds `per_rank` (expert time, wait time, received rows
 and SM clock of every rank) and the fixed-size 128-expert case under `ep_cpm2`.
 
---impl reference times that CPU restatement alone (the reference itself has no CPU
-path and its TensorRT plugin cannot be built here), on all host threads.
+--impl reference prints that the reference is unavailable: it is a TensorRT plugin, and neither
+TensorRT nor its build system is there to build it, and it has no CPU path.
 """
 from __future__ import annotations
 
@@ -139,30 +139,11 @@ def cpu_step(oracle, ws, x, cent, ln, experts):
     return time.perf_counter() - t0
 
 
-def run_reference_arm(args, w, scaling="weak"):
-    rank = int(os.environ.get("RANK", "0"))
-    if rank != 0:
-        return
-    sample_experts = 2 if w.embedding_size * w.hidden_size > (1 << 24) else min(w.expert_count, 4)
-    tpe = max(1, min(w.tokens // w.expert_count, 128))
-    oracle, ws, x, cent, ln, experts = cpu_sample_setup(w, sample_experts, tpe)
-    for _ in range(args.warmup):
-        cpu_step(oracle, ws, x, cent, ln, experts)
-    t = sum(cpu_step(oracle, ws, x, cent, ln, experts) for _ in range(args.steps))
-    value = ws.tokens * args.steps / t
-    sample = (f"{sample_experts} of {w.expert_count} experts x {tpe} tokens of workload {w.name} per step, "
-              f"weights in host memory")
-    line = {
-        "impl": "reference", "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": args.gpus, "steps": args.steps,
-        "warmup": args.warmup, "ms_per_step": 1e3 * t / args.steps, "higher_is_better": True, "scaling": scaling,
-        "vs_baseline": None, "dtype": "f32", "data": "synthetic",
-        "config": workload_config(w, args.gpus),
-        "cpu_baseline": {"value": value, "unit": UNIT, "cores": oracle.num_threads(), "kind": "port", "sample": sample},
-        "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-        "note": "CPU restatement of the reference's math (oracle/oracle.c, OpenMP + AVX2); the reference has no CPU "
-                "path and its TensorRT plugin cannot be built on this box",
-    }
-    print(json.dumps(line), flush=True)
+def run_reference_arm():
+    """The reference's own code is the only thing this arm may time, and it cannot be built here."""
+    if int(os.environ.get("RANK", "0")) == 0:
+        print(json.dumps({"impl": "reference", "unavailable": "a TensorRT plugin built with meson: TensorRT, pycuda and "
+                          "meson are absent here, and it has no CPU path"}), flush=True)
 
 
 def workload_config(w, n_gpus):
@@ -473,7 +454,7 @@ def main():
     if args.seq_len:
         w = synth.scaled(w, seq_len=args.seq_len)
     if args.impl == "reference":
-        run_reference_arm(args, w, scaling)
+        run_reference_arm()
         return
     if args.gpus == 1 and int(os.environ.get("WORLD_SIZE", "1")) == 1:
         run_single(args, w)
