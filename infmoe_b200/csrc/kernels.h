@@ -29,13 +29,13 @@ int launch_scatter_ln_rows(long long T, int D, const float* X, const float* scor
                            const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h,
                            cudaStream_t stream);
 // Tensor-core GEMM: packed FP16-pair plane `h` (pack_bytes) and two floats per row in row_info (token_row_info), of rows
-// row0 .. row0 + T - 1.  gamma: the LayerNorm weights that launch_split_expert left in the first weight slot, gamma_stride
-// floats from one slot to the next.
+// row0 .. row0 + T - 1.  gamma: the LayerNorm weights that launch_split_expert left for the first expert, or a copy of them,
+// gamma_stride floats from one expert to the next.
 int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, const float* score, const int* pos,
-                           const int* gate, const float* gamma, size_t gamma_stride, const int* slot_of_expert,
-                           const int* valid_rows, float* rscore, void* h, float* row_info, cudaStream_t stream);
+                           const int* gate, const float* gamma, size_t gamma_stride, const int* valid_rows, float* rscore,
+                           void* h, float* row_info, cudaStream_t stream);
 // launch_dispatch (without regions) and one of the two scatters in one kernel, where dispatch_scatter_supported.  gamma is
-// what the scatter takes: with `pack` that of the weight slots (experts in order), else the LayerNorm weights [E][D].
+// what the scatter takes: with `pack` that of launch_split_expert, else the experts' LayerNorm weights.
 bool dispatch_scatter_supported(long long T, int D, int E);
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
                             const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,

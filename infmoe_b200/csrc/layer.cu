@@ -196,6 +196,13 @@ struct infmoe_layer {
     std::vector<long long> cache_used;          // slot -> tick of the last use
     long long cache_tick = 0;
     std::vector<cudaEvent_t> ev_stage;          // landing area k has been retiled and may be overwritten
+    // Streamed experts on the tensor-core path: the LayerNorm weights that launch_split_expert makes for an expert depend on
+    // its matrices, so they are there only once it has been on the device.  They are kept [E][D] from then on, so that a
+    // later pass scatters its rows before the experts arrive; gamma_version: the expert's version they belong to, 0: none.
+    float* d_gamma = nullptr;
+    std::vector<unsigned> gamma_version;
+    cudaEvent_t ev_gamma = nullptr;             // behind the newest of them
+    bool gamma_recorded = false;
     unsigned long long weight_h2d_bytes = 0;    // expert weight bytes copied host -> device by enqueue so far
 
     long long launches_at_create = 0;
@@ -482,6 +489,8 @@ void free_device_state(infmoe_layer* L) {
     for (float* p : L->d_cache)
         if (p) cudaFree(p);
     if (L->d_cache_staging) cudaFree(L->d_cache_staging);
+    if (L->d_gamma) cudaFree(L->d_gamma);
+    if (L->ev_gamma) cudaEventDestroy(L->ev_gamma);
     if (L->own_in) cudaFree(L->own_in);
     if (L->own_out) cudaFree(L->own_out);
     if (L->own_ws) cudaFree(L->own_ws);
@@ -871,6 +880,19 @@ int ensure_cache(infmoe_layer* L) {
     return INFMOE_OK;
 }
 
+// The kept LayerNorm weights of streamed experts; a pass on another stream than the one that wrote them waits for them.
+int ensure_kept_gamma(infmoe_layer* L, cudaStream_t stream) {
+    if (!L->d_gamma) {
+        const size_t bytes = sizeof(float) * (size_t)L->E * L->D;
+        INFMOE_CUDA_TRY(cudaMalloc(&L->d_gamma, bytes));
+        INFMOE_CUDA_TRY(cudaMemsetAsync(L->d_gamma, 0, bytes, stream));
+        L->gamma_version.assign(L->E, 0);
+    }
+    if (!L->ev_gamma) INFMOE_CUDA_TRY(cudaEventCreateWithFlags(&L->ev_gamma, cudaEventDisableTiming));
+    if (L->gamma_recorded) INFMOE_CUDA_TRY(cudaStreamWaitEvent(stream, L->ev_gamma, 0));
+    return INFMOE_OK;
+}
+
 struct CachePlan {
     int slot;
     bool load;
@@ -1073,10 +1095,10 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     INFMOE_TRY(prof_mark(L, 1, stream));
     // 2. dispatch metadata (:350-352)
     // (with few tokens the scatter kernel of step 3 computes it on the way, except when an expert count past the
-    // dispatch kernel's limit has to be refused, and for streamed experts on the tensor-core path, see there)
+    // dispatch kernel's limit has to be refused)
     const bool pack = !L->identity && !L->custom && uses_umma(L);   // the GEMM run_ffn picks
     const bool with_scatter = !L->identity && !L->custom && !region_count && dispatch_supported(L->E) &&
-                              dispatch_scatter_supported(T, L->D, L->E) && !(pack && streamed);
+                              dispatch_scatter_supported(T, L->D, L->E);
     int* const zero = w.part_bytes ? buf.part_count : nullptr;
     if (!with_scatter)
         INFMOE_TRY(launch_dispatch(gate_in, T, L->E, pos, count, offset, L->d_status, stream, region_count, region_size,
@@ -1147,19 +1169,25 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     } else {
         // 3. scatter fused with the experts' LayerNorm and the operand split (:354-355, T5FFLayer.cc:99-103)
         // Tensor-core path: no routed copy, the second GEMM's epilogue reads its residual from d_in through pos[].  The
-        // LayerNorm weights to apply lie in the weight slots (launch_split_expert), so the rows of an expert that is
-        // streamed are scattered once it has arrived.
+        // LayerNorm weights to apply are those launch_split_expert left in the weight slots, or for streamed experts the
+        // ones kept from earlier passes (rows of experts that have none yet are scattered again further down).
         const size_t gamma_at = pack ? split_gamma_at(2 * L->F, L->D) : 0;
-        const auto scatter_pack = [&](long long row0, long long rows, const float* plane, const int* slots) {
-            return launch_scatter_ln_pack(row0, rows, L->D, d_in, score, pos, gate_in, plane + gamma_at, s->plane_elems(0), slots,
-                                          valid_rows, rscore, buf.h, buf.row_info, stream);
-        };
-        if (with_scatter) {
-            INFMOE_TRY(launch_dispatch_scatter(T, L->D, L->E, d_in, score, gate_in, pack ? s->d_plane[0] + gamma_at : s->d_ln,
-                                               pack ? s->plane_elems(0) : (size_t)L->D, pos, count, offset, L->d_status, zero,
-                                               FFN_COUNTERS, routed, rscore, buf.h, buf.row_info, pack, stream));
+        const float* gamma = s->d_ln;
+        size_t gamma_stride = (size_t)L->D;
+        if (pack && streamed) {
+            INFMOE_TRY(ensure_kept_gamma(L, stream));
+            gamma = L->d_gamma;
         } else if (pack) {
-            if (!streamed) INFMOE_TRY(scatter_pack(0, T, s->d_plane[0], nullptr));
+            gamma = s->d_plane[0] + gamma_at;
+            gamma_stride = s->plane_elems(0);
+        }
+        if (with_scatter) {
+            INFMOE_TRY(launch_dispatch_scatter(T, L->D, L->E, d_in, score, gate_in, gamma, gamma_stride, pos, count, offset,
+                                               L->d_status, zero, FFN_COUNTERS, routed, rscore, buf.h, buf.row_info, pack,
+                                               stream));
+        } else if (pack) {
+            INFMOE_TRY(launch_scatter_ln_pack(0, T, L->D, d_in, score, pos, gate_in, gamma, gamma_stride, valid_rows,
+                                              rscore, buf.h, buf.row_info, stream));
         } else {
             INFMOE_TRY(launch_scatter_ln_rows(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, routed, rscore,
                                               buf.h, stream));
@@ -1216,10 +1244,25 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
             size_t loads = 0;
             bool all_cached = cached && !active.empty();
             for (const CachePlan& pl : plan) all_cached = all_cached && !pl.load;
+            // Once expert e is in its slot: on its first pass, its LayerNorm weights are kept and its rows scattered with them.
+            bool kept = false;
+            const auto scatter_first = [&](int e, int slot, long long row0) -> int {
+                if (!pack || L->gamma_version[e] == s->version[e]) return INFMOE_OK;
+                const float* slot_gamma = planes[0] + n0 * slot + gamma_at;
+                INFMOE_CUDA_TRY(cudaMemcpyAsync(L->d_gamma + (size_t)e * L->D, slot_gamma, sizeof(float) * L->D,
+                                                cudaMemcpyDeviceToDevice, stream));
+                INFMOE_TRY(launch_scatter_ln_pack(row0, L->h_count[e], L->D, d_in, score, pos, gate_in, L->d_gamma,
+                                                  (size_t)L->D, valid_rows, rscore, buf.h, buf.row_info, stream));
+                L->gamma_version[e] = s->version[e];
+                kept = true;
+                return INFMOE_OK;
+            };
             if (all_cached) {
                 // nothing to copy: one grouped launch over all experts, as in resident mode
                 for (const CachePlan& pl : plan) INFMOE_CUDA_TRY(cudaStreamWaitEvent(stream, L->ev_ready[pl.slot], 0));
-                if (pack) INFMOE_TRY(scatter_pack(0, T, planes[0], slot_map));
+                long long row0 = 0;
+                for (size_t j = 0; j < active.size(); row0 += L->h_count[active[j++]])
+                    INFMOE_TRY(scatter_first(active[j], plan[j].slot, row0));
                 INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, slot_map, nslots, planes, buf, routed, ffn_out, stream));
                 for (const CachePlan& pl : plan) INFMOE_CUDA_TRY(cudaEventRecord(L->ev_freed[pl.slot], stream));
             }
@@ -1245,10 +1288,14 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                     ++loads;
                 }
                 INFMOE_CUDA_TRY(cudaStreamWaitEvent(stream, L->ev_ready[slot], 0));
-                if (pack) INFMOE_TRY(scatter_pack(row0, L->h_count[e], planes[0], slot_map));
+                INFMOE_TRY(scatter_first(e, slot, row0));
                 row0 += L->h_count[e];
                 INFMOE_TRY(run_ffn(L, T, e, e + 1, offset, slot_map, nslots, planes, buf, routed, ffn_out, stream));
                 INFMOE_CUDA_TRY(cudaEventRecord(L->ev_freed[slot], stream));
+            }
+            if (kept) {
+                INFMOE_CUDA_TRY(cudaEventRecord(L->ev_gamma, stream));
+                L->gamma_recorded = true;
             }
             INFMOE_TRY(prof_mark(L, 4, stream));   // streamed: copies and both GEMMs are timed together
         }

@@ -128,19 +128,16 @@ __device__ __forceinline__ void warp_ln_pack(const float* __restrict__ src, cons
 }
 
 // The scatter for the tensor-core GEMM (which reads its residual from X through pos[], so no routed row is written), of
-// rows j0 .. j0 + T - 1.  The LayerNorm weights are those of the experts' weight slots (gamma', see SplitExpert).
-struct SlotGamma {
-    const float* base;              // first slot
-    size_t stride;                  // floats between slots
-    const int* slot_of_expert;      // NULL: identity
-    __device__ __forceinline__ const float* of(int e) const {
-        return base + stride * (size_t)(slot_of_expert ? slot_of_expert[e] : e);
-    }
+// rows j0 .. j0 + T - 1.  The LayerNorm weights are gamma' (see SplitExpert), which lies with the experts' planes.
+struct ExpertGamma {
+    const float* base;              // first expert
+    size_t stride;                  // floats from one expert to the next
+    __device__ __forceinline__ const float* of(int e) const { return base + stride * (size_t)e; }
 };
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 scatter_ln_pack_kernel(long long j0, long long T, int D, int vec, const float* __restrict__ X,
                        const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
-                       const SlotGamma gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
+                       const ExpertGamma gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
                        uint16_t* __restrict__ h, float2* __restrict__ row_info) {
     pdl_trigger();
     pdl_wait();
@@ -164,7 +161,7 @@ template <int NV>
 __global__ void __launch_bounds__(128)
 scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __restrict__ X,
                            const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
-                           const SlotGamma slot_gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
+                           const ExpertGamma expert_gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
                            uint16_t* __restrict__ h, float2* __restrict__ row_info) {
     pdl_trigger();
     pdl_wait();
@@ -176,7 +173,7 @@ scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __rest
     const int p = pos[j];
     const int e = gate[p];
     const float4* src = reinterpret_cast<const float4*>(X + (long long)p * D);
-    const float4* gamma = reinterpret_cast<const float4*>(slot_gamma.of(e));
+    const float4* gamma = reinterpret_cast<const float4*>(expert_gamma.of(e));
     float4 v[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -258,7 +255,7 @@ constexpr int DS_THREADS = 128;
 template <bool PACK>
 __global__ void __launch_bounds__(DS_THREADS)
 dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ X, const float* __restrict__ score,
-                        const int* __restrict__ gate, const SlotGamma slot_gamma, int* __restrict__ pos,
+                        const int* __restrict__ gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
                         int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
                         int* __restrict__ zero, int zero_count, float* __restrict__ routed, float* __restrict__ rscore,
                         void* __restrict__ h, float2* __restrict__ row_info) {
@@ -305,7 +302,7 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
     int e = gate[t];
     if (e < 0 || e >= E) e = E;
     const float* src = X + (size_t)t * D;
-    const float* gamma = slot_gamma.of(e < E ? e : 0);
+    const float* gamma = expert_gamma.of(e < E ? e : 0);
     if (vec) {
         for (int k = 4 * tid; k < D; k += 4 * DS_THREADS) {
             const uint32_t dx = (uint32_t)__cvta_generic_to_shared(s_x + k), dg = (uint32_t)__cvta_generic_to_shared(s_g + k);
@@ -812,7 +809,7 @@ int launch_dispatch_scatter(long long T, int D, int E, const float* X, const flo
     if (smem < sizeof(int) * (size_t)(E + 1)) smem = sizeof(int) * (size_t)(E + 1);
     auto kern = pack ? dispatch_scatter_kernel<true> : dispatch_scatter_kernel<false>;
     INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)T + 1, DS_THREADS, smem, 1, stream, (int)T, D, E, vec, X, score, gate,
-                                   SlotGamma{gamma, gamma_stride, nullptr}, pos, count, offset, status, zero,
+                                   ExpertGamma{gamma, gamma_stride}, pos, count, offset, status, zero,
                                    zero ? zero_count : 0, routed, rscore, h,
                                    (float2*)row_info));
     note_launch();
@@ -833,11 +830,11 @@ int launch_scatter_ln_rows(long long T, int D, const float* X, const float* scor
 }
 
 int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, const float* score, const int* pos,
-                           const int* gate, const float* gamma, size_t gamma_stride, const int* slot_of_expert,
-                           const int* valid_rows, float* rscore, void* h, float* row_info, cudaStream_t stream) {
+                           const int* gate, const float* gamma, size_t gamma_stride, const int* valid_rows, float* rscore,
+                           void* h, float* row_info, cudaStream_t stream) {
     if (T == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && (gamma_stride % 4 == 0) && aligned16(X) && aligned16(gamma);
-    const SlotGamma slots{gamma, gamma_stride, slot_of_expert};
+    const ExpertGamma gammas{gamma, gamma_stride};
     uint16_t* pack = (uint16_t*)h;
     float2* info = (float2*)row_info;
     if (vec && D <= 4096) {
@@ -848,7 +845,7 @@ int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, c
         constexpr int smem = 4 * NV * 32 * 16;                                                                     \
         if (smem > 48 * 1024)                                                                                      \
             INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));        \
-        INFMOE_CUDA_TRY(launch_chained(kern, grid, 128, smem, 1, stream, row0, T, D, X, score, pos, gate, slots,   \
+        INFMOE_CUDA_TRY(launch_chained(kern, grid, 128, smem, 1, stream, row0, T, D, X, score, pos, gate, gammas,  \
                                        valid_rows, rscore, pack, info));                                           \
     } while (0)
         if (D <= 1024) INFMOE_SCATTER_REG(8);
@@ -857,7 +854,7 @@ int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, c
 #undef INFMOE_SCATTER_REG
     } else {
         INFMOE_CUDA_TRY(launch_chained(scatter_ln_pack_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, row0, T, D, vec, X,
-                                       score, pos, gate, slots, valid_rows, rscore, pack, info));
+                                       score, pos, gate, gammas, valid_rows, rscore, pack, info));
     }
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());

@@ -155,7 +155,8 @@ def _layer(experts, centroids, D, F, host, cache):
     return layer
 
 
-# few and many tokens take different scatter kernels, and so do the widths; streamed experts are scattered one by one
+# few and many tokens take different scatter kernels, and so do the widths; the rows of a streamed expert are scattered once
+# it has arrived on its first pass, with all others from then on
 @pytest.mark.parametrize("T,D,F", [(1, 256, 512), (200, 256, 512), (1500, 256, 512), (1300, 4100, 64), (100, 6020, 64)])
 def test_layer_resident_streamed_and_cached(oracle, T, D, F):
     import torch
@@ -179,6 +180,16 @@ def test_layer_resident_streamed_and_cached(oracle, T, D, F):
         layer = _layer(experts, centroids, D, F, True, cache)
         for _ in range(2):                           # the second call finds the slots, or the cache, filled
             np.testing.assert_array_equal(layer.forward(torch.from_numpy(x).cuda()).cpu().numpy(), out)
+        # other weights with another LayerNorm weight in the place of one expert's, and the next pass on another stream
+        layer.set_expert(1, *experts[3])
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+            replaced = layer.forward(torch.from_numpy(x).cuda())
+            torch.cuda.current_stream().synchronize()
+        layer.terminate()
+        same = [experts[0], experts[3], experts[2], experts[3]]
+        layer = _layer(same, centroids, D, F, False, 0)
+        np.testing.assert_array_equal(replaced.cpu().numpy(), layer.forward(torch.from_numpy(x).cuda()).cpu().numpy())
         layer.terminate()
 
 
