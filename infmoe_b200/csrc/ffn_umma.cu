@@ -113,8 +113,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Same with a suspend-time hint: the thread may sleep in hardware for up to `ns` nanoseconds and is woken when
-// the phase completes, instead of polling.  Polling warps take issue slots from the working warps of their
-// scheduler: with every waiting role polling, the transform warps ran 2-3x slower than alone.
+// the phase completes, instead of polling: polling warps take issue slots from the working warps of their scheduler.
 __device__ __forceinline__ bool mbar_try_wait_sleep(uint32_t bar, uint32_t parity, uint32_t ns) {
     uint32_t ok;
     asm volatile(
@@ -127,8 +126,7 @@ __device__ __forceinline__ bool mbar_try_wait_sleep(uint32_t bar, uint32_t parit
     return ok != 0;
 }
 // Bounded wait.  Returns false when the wait was abandoned (limit reached here or in another role).
-// The slow path is a real function call (about 200 cycles on B200); the common case, a barrier
-// that is already complete, is a single inlined try_wait (about 17 cycles).
+// The common case, a barrier that is already complete, is a single try_wait (about 17 cycles).
 static __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                unsigned long long limit_ns) {
     const unsigned long long t0 = global_ns();
@@ -997,9 +995,12 @@ int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_be
     //                           the token tile, so shared memory takes 63 instead of 78 KB of traffic per k block of 144
     //                           tokens and L2 half the token reads; where the GPU is at its power cap that is time.
     //                           Layer, us, one CTA / pairs: 4096 tokens 32 x 4096 x 10240 4173 / 3900, 16384 tokens
-    //                           12485 / 11651; second GEMM of 777 x 12 x 1000 x 2724 (K = 2724) 52 / 47
-    //   shorter K               one CTA: token tiles of a pair are multiples of 32, and the epilogue, not the MMAs, is in
-    //                           front; first GEMM, us: K = 1024, 16 experts x 4096, 1000 tokens 104 / 112, K = 680, 6
+    //                           12485 / 11651; second GEMM of 777 x 12 x 1000 x 2724 (K = 2724) 52 / 47.  Token tiles of a pair
+    //                           are padded to 32; 18, 24, 33, 40 tokens per expert, 32 x 2048 x 4096: 565 / 557, 567 / 570,
+    //                           579 / 585, 583 / 591, 32 x 4096 x 10240 20 and 36: 2389 / 2366, 2440 / 2466; the most it costs is
+    //                           what 20 tokens cost at 64 x 2048 x 2048, 600 / 632.  With one 128-row weight block, of which
+    //                           the second CTA has none: 4 x 128 x 4096, 1024 tokens 86 / 83, 8 x 128 x 2048, 4096 108 / 113
+    //   shorter K               one CTA: the epilogue, not the MMAs, is in front; first GEMM, us: K = 1024, 16 experts x 4096, 1000 tokens 104 / 112, K = 680, 6
     //                           experts, 4640 tokens 65 / 80
     const bool small = T <= 64 || T <= 16ll * (e_end - e_begin);
     const auto pick = [&](auto epi, const GemmArgs& a, const void* tokens) -> int {

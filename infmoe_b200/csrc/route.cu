@@ -1016,7 +1016,8 @@ int rs_cluster(int E) {
 //   two or more blocks on an SM (D <= 7168)
 //     E <= 8       any T: (4096, 8) 3500: 39 | 44 and 51 | 68, 4900: 53 | 80 and 72 | 128, 16384 0.91 and 0.79 of tiled.  Only
 //                  where the tiled kernel fills its first wave of 148 x 32 tokens nearly whole, and seven or eight experts
-//                  are scored without the LayerNorm, is it ahead: (4096, 8) 3700: 45 | 44, 4736: 53 | 45, (6400, 8) 4096: 76 | 64
+//                  are scored without the LayerNorm, is it ahead: (4096, 8) 3700: 45 | 44, 4736: 53 | 45, (6400, 8) 4096: 76 | 64.
+//                  Unaligned rows: (510, 6) 4096: 18 | 25 and 19 | 27, 16384: 46 | 76 and 48 | 88, (4095, 8) 4096: 86 | 122 and 103 | 116
 //     more         experts by the cluster's warps, T times those: (4096, 16) 1535: 35 | 43 and 47 | 62, (6144, 32) 767: 45 | 59,
 //                  (2560, 9) 2048 1.06 and 1.12 of tiled; rows of any alignment: (4095, 9) 2700 0.90 and 1.19
 //   one block      its eight warps wait for every row they load, and four waves of blocks (of 148; 128 in clusters of four

@@ -328,7 +328,9 @@ class MoELayer:
     STAGES = ("route", "dispatch", "scatter", "ffn_gemm1", "ffn_gemm2", "combine")
 
     def stage_ms(self):
-        """Average device milliseconds per stage over the calls since the last read -> (dict, calls)."""
+        """Average device milliseconds per stage over the calls since the last read -> (dict, calls).
+
+        Up to 1024 tokens "scatter" holds the dispatch too (one kernel does both)."""
         ms = (ctypes.c_float * 6)()
         n = ctypes.c_int32()
         capi.check(capi.lib().infmoe_layer_stage_ms(self._h, ms, ctypes.byref(n)))

@@ -130,9 +130,10 @@ def test_offload_decode_full_size(oracle):
 
 @pytest.mark.parametrize("case", ["row_scales", "outliers", "large_magnitude"])
 def test_split_operand_products_with_wide_value_ranges(oracle, case):
-    """The expert GEMMs work on FP16 pairs scaled by a power of two per row.  Inputs drawn from N(0, 1) never test
-    what the scales do to weights with a wide exponent spread inside and between rows, with outliers, or at
-    magnitudes far outside the range of FP16: these cases do."""
+    """The expert GEMMs work on FP16 pairs scaled by powers of two per row and column.  Inputs drawn from N(0, 1) never
+    test what the scales do to weights whose rows differ in magnitude, with outliers, or at magnitudes far outside the
+    range of FP16: these cases do.  They look at the whole output in one norm, in which the largest rows count most;
+    the expert term of every token is looked at in test_gpu_operand_range.py."""
     import torch
     assert torch.cuda.is_available()
     from tests import gpu_util as g
