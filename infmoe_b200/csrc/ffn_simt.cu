@@ -11,15 +11,23 @@
 // 32 values (launch_retile), wi_0 and wi_1 sharing one matrix with interleaved rows (row 2f = wi_0[f], row
 // 2f+1 = wi_1[f]).  So whatever the widths are, every row of a k block is 128 aligned bytes.
 //
-// Bound by FP32 FMA issue for many rows per expert, by the number of CTAs for few.  A CTA computes 16 RI token rows x 32
-// outputs; a thread RI x 4 (x 2 when both matrices are multiplied) of them.  K blocks of 32 are fetched by 16-byte
-// cp.async into two buffers.  Both operands stay row-major in shared memory at a pitch of 36 floats, and a thread reads
+// Bound by FP32 FMA issue for many rows per expert, by the number of CTAs for few.  A cluster of up to four CTAs computes 16
+// RI token rows x 32 outputs, each CTA a part of the k blocks, and adds the parts up through distributed shared memory; a
+// thread has RI x 4 (x 2 when both matrices are multiplied) outputs.  K blocks of 32 are fetched by 16-byte cp.async into two
+// buffers.  Both operands stay row-major in shared memory at a pitch of 36 floats, and a thread reads
 // four k of a row at a time: 4 + 8 128-bit loads for 128 multiply-adds, without bank conflicts (the eight weight rows a
-// warp reads at once start 4 banks apart; token rows are broadcasts).  Every output is one chain of FMAs in ascending k.
+// warp reads at once start 4 banks apart; token rows are broadcasts).  Every output is up to four chains of FMAs in
+// ascending k, cut by K alone, so a row's result does not depend on the other rows of the call.
 // Layer of 300 tokens, 6 experts, 510 x 1022: 423 -> 103 us (it was 64 x 64 tiles of scalar loads, one buffer, TF32 head
-// and tail planes added on the fly).
+// and tail planes added on the fly), 88 with the dispatch and scatter in one kernel, 67 with the clusters: 96 to 192 CTAs of
+// one chain each had left two or three of four schedulers of an SM without a warp, now 384 to 768 are in flight, five to an
+// SM.  The shorter chains also halve the error against 64 bits, 4.6e-7 -> 2.4e-7.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "kernels.h"
+
+namespace cg = cooperative_groups;
 
 namespace infmoe {
 
@@ -30,21 +38,33 @@ constexpr int TN = 32;       // outputs per CTA
 constexpr int TK = 32;       // one k block of the weight tiles
 constexpr int PITCH = TK + 4;
 
-// Finds the (expert, first row, valid rows) of row tile `tile` when every expert's rows are tiled separately by `tm`.
-// Returns false when `tile` is past the end.
+// Finds the (expert, first row, valid rows) of row tile `tile` when every expert's rows are tiled separately by `tm`: one
+// warp, 32 experts at a time.  Returns false when `tile` is past the end.
 __device__ bool locate_tile(const int* __restrict__ offset, int e_begin, int e_end, int tm, int tile, int& expert,
                             int& row0, int& rows) {
+    const int lane = threadIdx.x & 31;
     int seen = 0;
-    for (int e = e_begin; e < e_end; ++e) {
-        const int beg = offset[e], cnt = offset[e + 1] - beg;
+    for (int e0 = e_begin; e0 < e_end; e0 += 32) {
+        const int e = e0 + lane;
+        const int beg = e < e_end ? offset[e] : 0, cnt = e < e_end ? offset[e + 1] - beg : 0;
         const int nt = (cnt + tm - 1) / tm;
-        if (tile < seen + nt) {
-            expert = e;
-            row0 = beg + (tile - seen) * tm;
-            rows = min(tm, beg + cnt - row0);
+        int incl = nt;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int n = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += n;
+        }
+        const int first = seen + incl - nt;
+        const unsigned hit = __ballot_sync(0xffffffffu, tile >= first && tile < first + nt);
+        if (hit) {
+            const int src = __ffs(hit) - 1;
+            const int skip = (tile - __shfl_sync(0xffffffffu, first, src)) * tm;
+            expert = e0 + src;
+            row0 = __shfl_sync(0xffffffffu, beg, src) + skip;
+            rows = min(tm, __shfl_sync(0xffffffffu, cnt, src) - skip);
             return true;
         }
-        seen += nt;
+        seen += __shfl_sync(0xffffffffu, incl, 31);
     }
     return false;
 }
@@ -58,43 +78,52 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid)
 
 // DUAL = true : out[j][n] = gelu(A W0^T) * (A W1^T), padded rows of N outputs   (N = d_ff, K = d_model)
 // DUAL = false: out[j][n] = resid[j][n] + A W0^T, dense rows                    (N = d_model, K = d_ff)
+// Grid: clusters of S CTAs, one per (row tile, output tile), row tile major; CTA r of a cluster takes the r-th S-th of the
+// k blocks.
 template <bool DUAL, int RI>
 __global__ void __launch_bounds__(SIMT_THREADS)
 ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, int K, const float* __restrict__ act,
                 const float* __restrict__ w, const int* __restrict__ slot_of_expert, const float* __restrict__ resid,
                 float* __restrict__ out) {
-    const unsigned n_tiles = (unsigned)(N + TN - 1) / TN;     // grid: row tile major
+    cg::cluster_group cluster = cg::this_cluster();
+    const int S = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
+    const unsigned n_tiles = (unsigned)(N + TN - 1) / TN, tile = blockIdx.x / (unsigned)S;
     constexpr int TM = 16 * RI, WROWS = DUAL ? 2 * TN : TN, NB = DUAL ? 2 : 1;
-    __shared__ __align__(16) float As[2][TM][PITCH];
-    __shared__ __align__(16) float Ws[2][WROWS][PITCH];
+    constexpr int BUF = (TM + WROWS) * PITCH;                 // floats of one buffer: token rows, then weight rows
+    __shared__ __align__(16) float smem[2 * BUF];
+    static_assert(NB * RI * SIMT_THREADS * 4 <= 2 * BUF, "the partial sums reuse the buffers");
     __shared__ int s_info[4];
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         int e = 0, r0 = 0, rows = 0;
-        const bool ok = locate_tile(offset, e_begin, e_end, TM, blockIdx.x / n_tiles, e, r0, rows);
-        s_info[0] = ok ? 1 : 0;
-        s_info[1] = e;
-        s_info[2] = r0;
-        s_info[3] = rows;
+        const bool ok = locate_tile(offset, e_begin, e_end, TM, (int)(tile / n_tiles), e, r0, rows);
+        if (threadIdx.x == 0) {
+            s_info[0] = ok ? 1 : 0;
+            s_info[1] = e;
+            s_info[2] = r0;
+            s_info[3] = rows;
+        }
     }
     __syncthreads();
-    if (!s_info[0]) return;
+    if (!s_info[0]) return;      // the same in every CTA of the cluster
     const int expert = s_info[1], row0 = s_info[2], rows = s_info[3];
     const int slot = slot_of_expert ? slot_of_expert[expert] : expert;
-    const int n0 = (int)(blockIdx.x % n_tiles) * TN, m0 = NB * n0;    // first output, first weight row (inside one 128-row block)
+    const int n0 = (int)(tile % n_tiles) * TN, m0 = NB * n0;    // first output, first weight row (inside one 128-row block)
     const int KB = (K + TK - 1) / TK, MB = (NB * N + 127) / 128;
     const float* wt = w + (size_t)slot * (size_t)MB * KB * 4096 + ((size_t)(m0 >> 7) * KB) * 4096 + (size_t)(m0 & 127) * TK;
     const float* at = act + (size_t)row0 * KB * TK;
+    const auto As = [&](int buf, int r) { return smem + buf * BUF + r * PITCH; };
+    const auto Ws = [&](int buf, int r) { return smem + buf * BUF + (TM + r) * PITCH; };
 
     auto fetch = [&](int kb, int buf) {
         for (int i = threadIdx.x; i < TM * 8; i += SIMT_THREADS) {
             const int r = i >> 3, c = (i & 7) * 4;
             const bool valid = r < rows;
-            copy16(&As[buf][r][c], at + (size_t)(valid ? r : 0) * KB * TK + kb * TK + c, valid);
+            copy16(As(buf, r) + c, at + (size_t)(valid ? r : 0) * KB * TK + kb * TK + c, valid);
         }
         for (int i = threadIdx.x; i < WROWS * 8; i += SIMT_THREADS) {
             const int r = i >> 3, c = (i & 7) * 4;
             // wi_0 and wi_1 rows apart, so that neighbouring outputs are neighbouring rows
-            copy16(&Ws[buf][DUAL ? (r & 1) * TN + (r >> 1) : r][c], wt + (size_t)kb * 4096 + r * TK + c, true);
+            copy16(Ws(buf, DUAL ? (r & 1) * TN + (r >> 1) : r) + c, wt + (size_t)kb * 4096 + r * TK + c, true);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -102,10 +131,11 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
     // token rows ty + 16 i, outputs tx + 8 j
     const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
     float acc[NB][RI][4] = {};
-    fetch(0, 0);
-    for (int kb = 0; kb < KB; ++kb) {
+    const int kb0 = KB * part / S, kb_end = KB * (part + 1) / S;
+    fetch(kb0, kb0 & 1);
+    for (int kb = kb0; kb < kb_end; ++kb) {
         const int buf = kb & 1;
-        if (kb + 1 < KB) {
+        if (kb + 1 < kb_end) {
             fetch(kb + 1, buf ^ 1);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
@@ -116,12 +146,12 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
         for (int k = 0; k < TK; k += 4) {
             float4 a[RI];
 #pragma unroll
-            for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const float4*>(&As[buf][ty + 16 * i][k]);
+            for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const float4*>(As(buf, ty + 16 * i) + k);
 #pragma unroll
             for (int b = 0; b < NB; ++b)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float4 v = *reinterpret_cast<const float4*>(&Ws[buf][b * TN + tx + 8 * j][k]);
+                    const float4 v = *reinterpret_cast<const float4*>(Ws(buf, b * TN + tx + 8 * j) + k);
 #pragma unroll
                     for (int i = 0; i < RI; ++i) {
                         float s = acc[b][i][j];
@@ -134,21 +164,43 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
         }
         __syncthreads();    // the next round's fetch refills this buffer
     }
+    // Sums of the cluster's CTAs, added in ascending k.  Item (i, t): the four outputs of thread t in its row i; the CTAs share
+    // the items out.
+    float4* const red = reinterpret_cast<float4*>(smem);          // [NB][RI][thread]
 #pragma unroll
-    for (int i = 0; i < RI; ++i) {
-        const int r = ty + 16 * i;
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+            red[(b * RI + i) * SIMT_THREADS + threadIdx.x] = make_float4(acc[b][i][0], acc[b][i][1], acc[b][i][2], acc[b][i][3]);
+    cluster.sync();
+    constexpr int ITEMS = RI * SIMT_THREADS;
+    for (int it = ITEMS * part / S + (int)threadIdx.x; it < ITEMS * (part + 1) / S; it += SIMT_THREADS) {
+        const int t = it % SIMT_THREADS, r = (t >> 3) + 16 * (it / SIMT_THREADS);
         if (r >= rows) continue;
+        float sum[NB][4] = {};
+        for (int q = 0; q < S; ++q) {
+            const float4* from = cluster.map_shared_rank(red, q);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const float4 v = from[b * ITEMS + it];
+                sum[b][0] += v.x;
+                sum[b][1] += v.y;
+                sum[b][2] += v.z;
+                sum[b][3] += v.w;
+            }
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx + 8 * j;
+            const int n = n0 + (t & 7) + 8 * j;
             if (DUAL) {     // outputs past N are products of zero weights: the zeros the next GEMM's padding needs
-                out[(size_t)(row0 + r) * padded_row(N) + n] = gelu_dot(acc[0][i][j], acc[NB - 1][i][j]);
+                out[(size_t)(row0 + r) * padded_row(N) + n] = gelu_dot(sum[0][j], sum[NB - 1][j]);
             } else if (n < N) {
                 const size_t o = (size_t)(row0 + r) * N + n;
-                out[o] = resid[o] + acc[0][i][j];
+                out[o] = resid[o] + sum[0][j];
             }
         }
     }
+    cluster.sync();      // nobody leaves while its sums are being read
 }
 
 }  // namespace
@@ -165,13 +217,25 @@ int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int
     const bool few = T <= 16ll * experts;
     const int tm = few ? 16 : 64;
     const unsigned row_tiles = (unsigned)((T + tm - 1) / tm + experts);
-    const unsigned g1 = (unsigned)((F + TN - 1) / TN) * row_tiles, g2 = (unsigned)((D + TN - 1) / TN) * row_tiles;
-    auto k1 = few ? ffn_simt_kernel<true, 1> : ffn_simt_kernel<true, 4>;
-    auto k2 = few ? ffn_simt_kernel<false, 1> : ffn_simt_kernel<false, 4>;
     // Not chained (launch_chained): blocks put on the SMs while those of the kernel before are still there crowd on the
     // idle ones, and there are only a few per SM.  The pass of 300 tokens took 195 us so, 126 with a late trigger.
-    k1<<<g1, SIMT_THREADS, 0, stream>>>(offset, e_begin, e_end, F, D, h, w01, slot_of_expert, nullptr, g);
-    k2<<<g2, SIMT_THREADS, 0, stream>>>(offset, e_begin, e_end, D, F, g, wo, slot_of_expert, routed, post);
+    const auto launch = [&](auto kern, int N, int K, const float* act, const float* w, const float* resid, float* out) {
+        // CTAs per tile: by K alone, so that a row's additions do not depend on the other rows of the call
+        const unsigned S = K > 7 * TK ? 4 : K > 3 * TK ? 2 : 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)((N + TN - 1) / TN) * row_tiles * S);
+        cfg.blockDim = dim3(SIMT_THREADS);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = S;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, kern, offset, e_begin, e_end, N, K, act, w, slot_of_expert, resid, out);
+    };
+    INFMOE_CUDA_TRY(launch(few ? ffn_simt_kernel<true, 1> : ffn_simt_kernel<true, 4>, F, D, h, w01, (const float*)nullptr, g));
+    INFMOE_CUDA_TRY(launch(few ? ffn_simt_kernel<false, 1> : ffn_simt_kernel<false, 4>, D, F, (const float*)g, wo, routed, post));
     note_launch(2);
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

@@ -534,6 +534,29 @@ def test_cuda_core_experts_against_oracle(oracle, counts, D, F):
             assert oracle.rel_l2(out[rows] - x[rows], want - x[rows]) <= 2e-6   # FP32 chains of up to 1022 adds
 
 
+# A row's outputs are summed over one, two or four CTAs that share the k blocks, by K alone: the edges between them (96 | 97,
+# 224 | 225 values), and the same rows in calls with 16-row and 64-row tiles have the same bits.
+@pytest.mark.parametrize("D,F", [(95, 97), (225, 223), (97, 226), (450, 161)])
+def test_cuda_core_experts_with_k_shared_by_a_cluster(oracle, D, F):
+    import torch
+    from infmoe_b200 import MoELayer
+    rng = np.random.default_rng(D * F)
+    layer = MoELayer.create(1, D, F, 2, np.ones((1, D), np.float32), None, "T5_FF", "default", None)
+    expert = [(1 + 0.01 * rng.standard_normal(D)).astype(np.float32)] + \
+             [(rng.standard_normal((F, D)) / np.sqrt(D)).astype(np.float32) for _ in range(2)] + \
+             [(rng.standard_normal((D, F)) / np.sqrt(F)).astype(np.float32)]
+    layer.set_expert(0, *(torch.from_numpy(a).cuda() for a in expert))
+    x = rng.standard_normal((130, D)).astype(np.float32)
+    run = lambda n: layer.expert_forward(torch.from_numpy(x[:n]).cuda(),
+                                         torch.zeros(n, dtype=torch.int32, device="cuda")).cpu().numpy()
+    out, few = run(130), run(16)
+    layer.sync_status()
+    layer.terminate()
+    np.testing.assert_array_equal(few, out[:16])
+    want = oracle.expert_ffn_f64(x, *expert)
+    assert oracle.rel_l2(out - x, want - x) <= 2e-6     # FP32 chains of up to 450 adds
+
+
 # Up to 1024 tokens one kernel computes the dispatch metadata and scatters; beyond, or with d_model > 6016, two do.
 @pytest.mark.parametrize("T,D,E,variant", [(1, 64, 4, "default"), (33, 66, 3, "base_layer"), (1023, 36, 70, "cpm_2"),
                                            (1024, 40, 5, "base_layer"), (1025, 40, 5, "base_layer"),
