@@ -84,8 +84,8 @@ dispatch_kernel(const int* __restrict__ gate, long long T, int E, const int* __r
     };
 
     for (int e = tid; e < B; e += DISPATCH_THREADS) s_count[e] = 0;
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     if (r == 0)
         for (int i = tid; i < zero_count; i += DISPATCH_THREADS) zero[i] = 0;
     __syncthreads();

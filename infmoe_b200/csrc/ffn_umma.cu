@@ -278,6 +278,9 @@ struct Cfg {
 
 struct GemmArgs {
     const int* offset;          // [E+1] first routed row of each expert
+    const int* gate;            // [tokens] experts of the tokens, to count instead of reading offset[] (NULL: read it)
+    int tokens;
+    int early;                  // GELU_PAIR: what offset or gate points to is complete when the kernel starts
     const int* slot_of_expert;  // expert -> weight slot (NULL: identity)
     int E, e_begin, e_end;      // experts [e_begin, e_end) are processed
     int M_total;                // weight rows: 2 * d_ff (wi_0 / wi_1 rows interleaved) or d_model
@@ -323,7 +326,8 @@ __device__ __forceinline__ void chunking(int cnt, int& nch, int& csz) {
 // tile of each list position), so the long tiles of the busiest experts are handed out first and the short ones
 // fill the end of the schedule.
 template <int NMAX, int STEP>
-__device__ __forceinline__ TileInfo decode_tile(int tile, const int* s_prefix, const short* s_order, const GemmArgs& a) {
+__device__ __forceinline__ TileInfo decode_tile(int tile, const int* s_prefix, const short* s_order, const int* s_beg,
+                                                const int* s_cnt, const GemmArgs& a) {
     int lo = 0, hi = a.E - 1;  // last list position with s_prefix[.] <= tile
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -333,7 +337,7 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, const int* s_prefix, c
     const int ex = s_order[lo];
     t.expert = ex;
     t.slot = a.slot_of_expert ? a.slot_of_expert[ex] : ex;
-    const int beg = a.offset[ex], cnt = a.offset[ex + 1] - beg;
+    const int beg = s_beg[ex], cnt = s_cnt[ex];
     int nch, csz;
     chunking<NMAX, STEP>(cnt, nch, csz);
     const int local = tile - s_prefix[lo];
@@ -420,6 +424,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     __shared__ int s_widest;
     __shared__ int s_prefix[MAX_EXPERTS + 1];
     __shared__ int s_cnt[MAX_EXPERTS];
+    __shared__ int s_beg[MAX_EXPERTS];
     __shared__ short s_order[MAX_EXPERTS];
 
     const int warp = threadIdx.x >> 5;
@@ -456,17 +461,49 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
         }
     }
-    // The first GEMM lets the second one's blocks start only after its own wait.  So when they start, everything before
-    // the first GEMM is complete, and they can read offset[], make their schedule and fetch weights while the first one's
-    // last tiles are still running.  What the first GEMM writes they touch after their own wait, further down.
-    // Layer, us: 32 tokens 64 x 256 24.5 -> 22.3, one token 4096 x 10240 138.5 -> 133.7, 777 x 12 x 1000 x 2724 124 -> 120.
-    if (EPI == EPI_GELU_PAIR) pdl_wait();
-    pdl_trigger();
+    // Work before the wait.  The scatter kernels and the first GEMM let their successor's blocks start only after their own
+    // wait.  So when a block of the second GEMM starts, everything before the first one is complete, and it can read
+    // offset[], make its schedule and fetch weights while the first one's last tiles are still running; what the first one
+    // writes it touches after its own wait, further down.  In the same way the first GEMM (`early`) starts while the
+    // scatter is still running: offset[] is complete when a kernel of its own has made it, and the gates are when the scatter
+    // makes offset[] itself.
+    // Layer, us, second GEMM: 32 tokens 64 x 256 24.5 -> 22.3, one token 4096 x 10240 138.5 -> 133.7, 777 x 12 x 1000 x 2724
+    // 124 -> 120.
+    const bool early = EPI == EPI_RESIDUAL || args.early;
+    if (!early) pdl_wait();
+    if (EPI == EPI_RESIDUAL || !early) pdl_trigger();
 
     // ---- tile schedule: experts by falling token count, exclusive prefix of their tiles ---------
-    for (int e = threadIdx.x; e < args.E; e += GEMM_THREADS)
-        s_cnt[e] = (e >= args.e_begin && e < args.e_end) ? args.offset[e + 1] - args.offset[e] : 0;
-    __syncthreads();
+    if (EPI == EPI_GELU_PAIR && args.gate) {
+        for (int e = threadIdx.x; e < args.E; e += GEMM_THREADS) s_cnt[e] = 0;
+        __syncthreads();
+        for (int t = threadIdx.x; t < args.tokens; t += GEMM_THREADS) {
+            const int e = __ldcg(args.gate + t);
+            if (e >= 0 && e < args.E) atomicAdd(&s_cnt[e], 1);
+        }
+        __syncthreads();
+        if (warp == 2) {
+            int carry = 0;
+            for (int e0 = 0; e0 < args.E; e0 += 32) {
+                const int e = e0 + lane, c = e < args.E ? s_cnt[e] : 0;
+                int incl = c;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const int n = __shfl_up_sync(0xffffffffu, incl, off);
+                    if (lane >= off) incl += n;
+                }
+                if (e < args.E) s_beg[e] = carry + incl - c;
+                carry += __shfl_sync(0xffffffffu, incl, 31);
+            }
+        }
+    } else {
+        for (int e = threadIdx.x; e < args.E; e += GEMM_THREADS) {
+            const int beg = __ldcg(args.offset + e);
+            s_beg[e] = beg;
+            s_cnt[e] = (e >= args.e_begin && e < args.e_end) ? __ldcg(args.offset + e + 1) - beg : 0;
+        }
+        __syncthreads();
+    }
     for (int e = threadIdx.x; e < args.E; e += GEMM_THREADS) {
         const int c = s_cnt[e];
         int rank = 0;   // experts that come before e: more tokens, or as many and a lower index
@@ -514,13 +551,25 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     Schedule<CTAS> sched(s_prefix[args.E], KB, args);
     Item item;
 
+    // every thread of an early first GEMM passes here once, its producer when it has fetched its first weights
+    const auto wait_then_trigger = [&]() {
+        if (EPI == EPI_GELU_PAIR && early) {
+            pdl_wait();
+            pdl_trigger();
+        }
+    };
     if (warp == TMA_WARP) {
         // ================= TMA producer =================
         if (lane == 0) {
             uint32_t it = 0, ahead = 0;    // ahead: k blocks whose weights were fetched before the wait
-            bool ok = true, waited = EPI == EPI_GELU_PAIR;
+            bool ok = true, waited = !early;
+            const auto wait = [&]() {
+                if (EPI == EPI_RESIDUAL) pdl_wait();
+                wait_then_trigger();
+                waited = true;
+            };
             while (ok && sched.next(item) && !*abort_flag) {
-                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, args);
+                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, s_beg, s_cnt, args);
                 // a box of n_pad token rows (rows past the chunk's tokens belong to the next expert or are
                 // zero-filled past the end; they only feed accumulator columns that are never stored)
                 const int n_own = t.n_pad / CTAS;
@@ -547,8 +596,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 };
                 if (!waited) {
                     for (int kb = item.c0 * CHUNK_BLOCKS; kb < kb_end && ahead < STAGES; ++kb, ++ahead) fetch_weights(ahead, kb);
-                    pdl_wait();
-                    waited = true;
+                    wait();
                 }
                 for (int kb = item.c0 * CHUNK_BLOCKS; kb < kb_end; ++kb, ++it) {
                     const uint32_t s = it % STAGES;
@@ -559,7 +607,9 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     fetch_tokens(s, kb);
                 }
             }
-            if (!waited) pdl_wait();
+            if (!waited) wait();
+        } else {
+            wait_then_trigger();
         }
     } else if (warp == MMA_WARP) {
         // ================= MMA issuer =================
@@ -567,6 +617,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // issuing, the operands of every MMA had to be moved to uniform registers behind a divergent branch: ~148
         // cycles per MMA whatever its N, which held a decode step of 27 experts at 1694 us of first GEMM where the
         // same bytes stream in 1269.  Elected: 1259 us (7.2 TB/s); 4096 tokens 2780 -> 2383.
+        wait_then_trigger();
         if (rank == 0 && elect_one()) {
             auto commit = [](uint32_t bar) {
                 if (CTAS == 1) umma_commit(bar);
@@ -575,7 +626,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             uint32_t it = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             while (ok && sched.next(item) && !*abort_flag) {
-                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, args);
+                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, s_beg, s_cnt, args);
                 const uint32_t idesc = make_idesc(UMMA_M * CTAS, t.n_pad);
                 for (int c = item.c0; ok && c < item.c1; ++c) {
                     const uint32_t d = tmem_base + acc * acc_stride;
@@ -617,8 +668,9 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
         if (EPI == EPI_RESIDUAL) pdl_wait();
+        wait_then_trigger();
         while (ok && sched.next(item) && !*abort_flag) {
-            const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, args);
+            const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, s_beg, s_cnt, args);
             const int nsl = t.n_pad >> 4;
             float sum[C::SLICES][16];
 #pragma unroll
@@ -793,6 +845,8 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 }
             }
         }
+    } else {
+        wait_then_trigger();
     }
 
     // ---- teardown ---------------------------------------------------------------------------
@@ -893,7 +947,7 @@ template <int EPI, int NMAX, int STAGES, int CTAS>
 int launch_one(GemmArgs args, long long T, int slots, const void* tokens, size_t part_bytes, int num_ctas,
                cudaStream_t stream) {
     using C = Cfg<NMAX, STAGES, CTAS>;
-    static_assert(C::SMEM + 12288 <= 227 * 1024, "shared-memory ring too large");
+    static_assert(C::SMEM + 16384 <= 227 * 1024, "shared-memory ring too large");
     static_assert(NMAX / CTAS <= 16 * TOKEN_BOXES, "a token tile needs a tensor map of its height");
     args.part_cols = (int)(T < NMAX ? (T + C::N_STEP - 1) / C::N_STEP * C::N_STEP : NMAX);
     const size_t blocks = part_bytes / ((size_t)args.part_cols * UMMA_M * sizeof(float));
@@ -962,6 +1016,9 @@ int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_be
     if (num_sms > FFN_CTAS) num_sms = FFN_CTAS;
     GemmArgs a1{};
     a1.offset = f.offset;
+    a1.gate = f.gate;
+    a1.tokens = (int)T;
+    a1.early = f.early ? 1 : 0;
     a1.slot_of_expert = f.slot_of_expert;
     a1.E = E;
     a1.e_begin = e_begin;

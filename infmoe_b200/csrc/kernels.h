@@ -35,12 +35,13 @@ int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, c
                            const int* gate, const float* gamma, size_t gamma_stride, const int* valid_rows, float* rscore,
                            void* h, float* row_info, cudaStream_t stream);
 // launch_dispatch (without regions) and one of the two scatters in one kernel, where dispatch_scatter_supported.  gamma is
-// what the scatter takes: with `pack` that of launch_split_expert, else the experts' LayerNorm weights.
+// what the scatter takes: with `pack` that of launch_split_expert, else the experts' LayerNorm weights.  early: the launch
+// follows launch_route on this stream.
 bool dispatch_scatter_supported(long long T, int D, int E);
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
                             const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,
                             int* zero, int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
-                            cudaStream_t stream);
+                            bool early, cudaStream_t stream);
 int launch_gather(long long T, int D, const float* in, const int* pos, float* out, cudaStream_t stream,
                   const int* valid_rows = nullptr);
 int launch_mix_gather(long long T, int D, const int* pos, const float* routed, const float* post,
@@ -83,6 +84,8 @@ bool ffn_umma_supported(int D, int F, int E);
 // Buffers of one tensor-core FFN call (all on the device).
 struct FfnUmma {
     const int* offset;              // [E+1] first row of each expert
+    bool early;                     // the launch follows launch_dispatch and launch_scatter_ln_pack, or, with `gate`,
+    const int* gate;                // launch_dispatch_scatter on these gates: the first GEMM starts before the scatter ends
     const int* slot_of_expert;      // expert -> weight slot (NULL: identity)
     int slots;                      // weight slots in the planes
     const float *w01, *wo;          // split planes (launch_split_expert), [slots] x split_plane_elems

@@ -447,9 +447,11 @@ struct FfnBuffers {
 
 int run_ffn(infmoe_layer* L, long long T, int e_begin, int e_end, const int* d_offset, const int* d_slot_map,
             int slots, float* const planes[2], const FfnBuffers& w, const float* routed, const FfnOutput& o,
-            cudaStream_t stream, cudaEvent_t mid = nullptr) {
+            cudaStream_t stream, cudaEvent_t mid = nullptr, bool early = false, const int* d_gate = nullptr) {
     if (uses_umma(L)) {
         FfnUmma f{};
+        f.early = early;
+        f.gate = d_gate;
         f.offset = d_offset;
         f.slot_of_expert = d_slot_map;
         f.slots = slots;
@@ -1184,7 +1186,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
         if (with_scatter) {
             INFMOE_TRY(launch_dispatch_scatter(T, L->D, L->E, d_in, score, gate_in, gamma, gamma_stride, pos, count, offset,
                                                L->d_status, zero, FFN_COUNTERS, routed, rscore, buf.h, buf.row_info, pack,
-                                               stream));
+                                               !given_gate, stream));
         } else if (pack) {
             INFMOE_TRY(launch_scatter_ln_pack(0, T, L->D, d_in, score, pos, gate_in, gamma, gamma_stride, valid_rows,
                                               rscore, buf.h, buf.row_info, stream));
@@ -1198,7 +1200,8 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
         if (!streamed) {
             cudaEvent_t mid = nullptr;
             if (L->profiling) mid = L->prof_events[(size_t)(L->prof_calls % PROF_CALLS) * PROF_MARKS + 4];
-            INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, nullptr, L->E, s->d_plane, buf, routed, ffn_out, stream, mid));
+            INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, nullptr, L->E, s->d_plane, buf, routed, ffn_out, stream, mid, true,
+                               with_scatter ? gate_in : nullptr));
         } else {
             const size_t n = s->matrix_elems();
             // slot planes: w01 [mc], wo [mc], then one raw landing area per slot

@@ -162,8 +162,8 @@ route_kernel(const float* __restrict__ X, const float* __restrict__ C, const flo
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long t0 = (long long)blockIdx.x * RT_TOKENS;
     const bool use_ln = gamma != nullptr;
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     // row statistics, four tokens per warp, two at a time (rows past the end alias the tile's first row)
     if (use_ln) {
 #pragma unroll
@@ -449,8 +449,8 @@ route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     if (tid == 0) {
         // the first two stages of the first pass are fetched while the warps compute the row statistics
         issue(0, 0, 0);
@@ -661,8 +661,8 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
     const int nt = (int)min((long long)RS_TOKENS, T - t0);
     const int chunks = (D + 127) / 128 * 32;              // float4 per staged row
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     if (gamma) {
         if (warp < nt) {
             float mean, rstd;
@@ -801,8 +801,8 @@ route_rows_kernel(const float* __restrict__ X, const float* __restrict__ C, cons
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     fetch(0);
     float4 x[TOKENS][NV];
 #pragma unroll

@@ -139,8 +139,8 @@ scatter_ln_pack_kernel(long long j0, long long T, int D, int vec, const float* _
                        const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
                        const ExpertGamma gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
                        uint16_t* __restrict__ h, float2* __restrict__ row_info) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const long long j = j0 + (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= j0 + T || (valid_rows && j >= *valid_rows)) return;
@@ -163,8 +163,8 @@ scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __rest
                            const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
                            const ExpertGamma expert_gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
                            uint16_t* __restrict__ h, float2* __restrict__ row_info) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const long long j = j0 + (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (j >= j0 + T || (valid_rows && j >= *valid_rows)) return;
@@ -251,6 +251,9 @@ scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __rest
 // most it takes.  Results, LayerNorm bits included, are those of dispatch_kernel and the scatter kernels.
 // Layer of 32 tokens, 4 experts, 64 x 256: 36 -> 24 us together with launch_chained; 1 token, 32 experts, 4096 x 10240:
 // 149 -> 136.
+// early: the kernel before is the routing, whose blocks start their successor only after their own wait.  So all that was
+// enqueued before the routing is complete, the tokens are there, and a block fetches its row and computes the row's
+// statistics while the routing is still running.
 constexpr int DS_THREADS = 128;
 template <bool PACK>
 __global__ void __launch_bounds__(DS_THREADS)
@@ -258,13 +261,15 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
                         const int* __restrict__ gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
                         int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
                         int* __restrict__ zero, int zero_count, float* __restrict__ routed, float* __restrict__ rscore,
-                        void* __restrict__ h, float2* __restrict__ row_info) {
+                        void* __restrict__ h, float2* __restrict__ row_info, int early) {
     extern __shared__ __align__(16) float ds_smem[];
     __shared__ int s_before[DS_THREADS / 32];
     __shared__ float s_top[DS_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    pdl_trigger();
-    pdl_wait();
+    if (!early || (int)blockIdx.x == T) {
+        pdl_wait();
+        pdl_trigger();
+    }
     if ((int)blockIdx.x == T) {      // histogram and its exclusive scan, 32 buckets at a time
         int* hist = reinterpret_cast<int*>(ds_smem);
         for (int e = tid; e <= E; e += DS_THREADS) hist[e] = 0;
@@ -299,25 +304,32 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
     const int t = (int)blockIdx.x;
     const int P = (int)padded_row(D);
     float *s_x = ds_smem, *s_g = ds_smem + P;
+    const auto fetch = [&](float* dst, const float* src) {
+        if (vec) {
+            for (int k = 4 * tid; k < D; k += 4 * DS_THREADS) {
+                const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + k);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + k) : "memory");
+            }
+        } else {
+#pragma unroll 4
+            for (int k = tid; k < D; k += DS_THREADS) dst[k] = src[k];
+        }
+        for (int k = D + tid; k < P; k += DS_THREADS) dst[k] = 0.f;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(s_x, X + (size_t)t * D);
+    float mean, rstd;
+    const auto stats = [&]() { warp_row_stats(s_x, D, (D & 3) == 0, mean, rstd); };     // every warp for itself
+    if (early) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        stats();
+        pdl_wait();
+        pdl_trigger();
+    }
     int e = gate[t];
     if (e < 0 || e >= E) e = E;
-    const float* src = X + (size_t)t * D;
-    const float* gamma = expert_gamma.of(e < E ? e : 0);
-    if (vec) {
-        for (int k = 4 * tid; k < D; k += 4 * DS_THREADS) {
-            const uint32_t dx = (uint32_t)__cvta_generic_to_shared(s_x + k), dg = (uint32_t)__cvta_generic_to_shared(s_g + k);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dx), "l"(src + k) : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dg), "l"(gamma + k) : "memory");
-        }
-    } else {
-#pragma unroll 4
-        for (int k = tid; k < D; k += DS_THREADS) {
-            s_x[k] = src[k];
-            s_g[k] = gamma[k];
-        }
-    }
-    for (int k = D + tid; k < P; k += DS_THREADS) s_x[k] = s_g[k] = 0.f;
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    fetch(s_g, expert_gamma.of(e < E ? e : 0));
     int before = 0;
     for (int o = tid; o < T; o += DS_THREADS) {
         int g = gate[o];
@@ -336,9 +348,10 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
         if (e < E && rscore && score) rscore[j] = score[t];
     }
     if (e == E) return;              // no expert: nobody reads the row
-    float mean, rstd;
-    warp_row_stats(s_x, D, (D & 3) == 0, mean, rstd);     // every warp for itself
-    __syncthreads();
+    if (!early) {
+        stats();
+        __syncthreads();
+    }
     float top = 0.f;
     for (int k = 4 * tid; k < P; k += 4 * DS_THREADS) {
         float* x = s_x + k;
@@ -804,15 +817,14 @@ bool dispatch_scatter_supported(long long T, int D, int E) { return T <= 1024 &&
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
                             const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,
                             int* zero, int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
-                            cudaStream_t stream) {
+                            bool early, cudaStream_t stream) {
     const int vec = (D % 4 == 0) && (gamma_stride % 4 == 0) && aligned16(X) && aligned16(gamma);
     size_t smem = 2 * padded_row(D) * sizeof(float);
     if (smem < sizeof(int) * (size_t)(E + 1)) smem = sizeof(int) * (size_t)(E + 1);
     auto kern = pack ? dispatch_scatter_kernel<true> : dispatch_scatter_kernel<false>;
     INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)T + 1, DS_THREADS, smem, 1, stream, (int)T, D, E, vec, X, score, gate,
                                    ExpertGamma{gamma, gamma_stride}, pos, count, offset, status, zero,
-                                   zero ? zero_count : 0, routed, rscore, h,
-                                   (float2*)row_info));
+                                   zero ? zero_count : 0, routed, rscore, h, (float2*)row_info, early ? 1 : 0));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
