@@ -634,16 +634,21 @@ route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // Each centroid is read once per RS_TOKENS tokens, from L2, and a shared-memory load feeds only four multiply-adds:
 // past the line in use_small_route the other kernels win.
 // One token, d_model 4096, 32 experts: 47 -> 9.6 us; 64 tokens 52 -> 12.5; d_model 1024, 8 experts: 13 -> 3.5.
+// Behind a pass that has streamed its weights through L2 the same call took 17 us: the rows (twice, for their statistics), the
+// LayerNorm weights and the centroids (eight loads at a time) were one trip to HBM after the other.  While the blocks all
+// fit on the chip (AHEAD) everything is requested on entry, by cp.async into shared memory: 10 us.  (The centroid in 32 registers
+// per lane, fetched by unrolled loads, took 22: the code has to come from HBM too.)
 constexpr int RS_TOKENS = 4;
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_MAX_SMEM = 200 * 1024;
+constexpr int RS_AHEAD_SMEM = 216 * 1024;
 
 __device__ __forceinline__ bool rs_better(float s, int e, float best, int best_e) {
     return e >= 0 && (best_e < 0 || s > best || (s == best && e < best_e));
 }
 
-template <bool VEC>
+template <bool VEC, bool AHEAD>
 __global__ void __launch_bounds__(RS_THREADS)
 route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, const float* __restrict__ gamma,
                    long long T, int D, int E, int* __restrict__ gate, float* __restrict__ score,
@@ -660,40 +665,59 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
     const long long t0 = (long long)(blockIdx.x / S) * RS_TOKENS;
     const int nt = (int)min((long long)RS_TOKENS, T - t0);
     const int chunks = (D + 127) / 128 * 32;              // float4 per staged row
+    float4* const rs_g = rs_x + RS_TOKENS * chunks;       // AHEAD: LayerNorm weights, then the first centroid of each warp
+    float4* const rs_c = rs_g + (1 + warp) * chunks;
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     pdl_wait();
     pdl_trigger();
+    // All that the block needs from memory is requested at once.
+    for (int i = tid; i < chunks; i += RS_THREADS) {
+        const int k = 4 * i;
+#pragma unroll
+        for (int t = 0; t < RS_TOKENS; ++t) {
+            const float* src = X + (t0 + t) * (long long)D;
+            if (VEC && t < nt && k < D) cp_async16(rs_x + t * chunks + i, src + k);
+            else rs_x[t * chunks + i] = t < nt && k < D ? load_row4(src, k, D, false) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (AHEAD && gamma && k < D) cp_async16(rs_g + i, gamma + k);
+    }
+    cp_async_commit();
+    const int first_e = r * RS_WARPS + warp;
+    if (AHEAD && first_e < E)
+        for (int i = lane; i < chunks; i += 32) {
+            if (4 * i < D) cp_async16(rs_c + i, C + (long long)first_e * D + 4 * i);
+            else rs_c[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
     if (gamma) {
         if (warp < nt) {
             float mean, rstd;
-            warp_row_stats(X + (t0 + warp) * (long long)D, D, VEC, mean, rstd);
+            warp_row_stats(reinterpret_cast<const float*>(rs_x + warp * chunks), D, VEC, mean, rstd);
             if (lane == 0) {
                 s_mean[warp] = mean;
                 s_rstd[warp] = rstd;
             }
         }
         __syncthreads();
-    }
-    for (int i = tid; i < chunks; i += RS_THREADS) {
-        const int k = 4 * i;
-        const float4 g = (gamma && k < D) ? load_row4(gamma, k, D, VEC) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = tid; 4 * i < D; i += RS_THREADS) {
+            const int k = 4 * i;
+            const float4 w = AHEAD ? rs_g[i] : load_row4(gamma, k, D, VEC);    // AHEAD: what this thread fetched itself
 #pragma unroll
-        for (int t = 0; t < RS_TOKENS; ++t) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (t < nt && k < D) {
-                v = load_row4(X + (t0 + t) * (long long)D, k, D, VEC);
-                if (gamma) {
-                    const float mean = s_mean[t], rstd = s_rstd[t];
-                    v.x = ln_apply(v.x, mean, rstd, g.x);
-                    v.y = k + 1 < D ? ln_apply(v.y, mean, rstd, g.y) : 0.f;
-                    v.z = k + 2 < D ? ln_apply(v.z, mean, rstd, g.z) : 0.f;
-                    v.w = k + 3 < D ? ln_apply(v.w, mean, rstd, g.w) : 0.f;
-                }
+            for (int t = 0; t < RS_TOKENS; ++t) {
+                if (t >= nt) continue;
+                float4 v = rs_x[t * chunks + i];
+                const float mean = s_mean[t], rstd = s_rstd[t];
+                v.x = ln_apply(v.x, mean, rstd, w.x);
+                v.y = k + 1 < D ? ln_apply(v.y, mean, rstd, w.y) : 0.f;
+                v.z = k + 2 < D ? ln_apply(v.z, mean, rstd, w.z) : 0.f;
+                v.w = k + 3 < D ? ln_apply(v.w, mean, rstd, w.w) : 0.f;
+                rs_x[t * chunks + i] = v;
             }
-            rs_x[t * chunks + i] = v;
         }
+        __syncthreads();
     }
-    __syncthreads();
 
     float best[RS_TOKENS];
     int best_e[RS_TOKENS];
@@ -702,12 +726,10 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
         best[t] = -FLT_MAX;               // reference plugin/cuda/moe.cu:26-27
         best_e[t] = -1;
     }
-    for (int e = r * RS_WARPS + warp; e < E; e += S * RS_WARPS) {
+    for (int e = first_e; e < E; e += S * RS_WARPS) {
         const float* row = C + (long long)e * D;
         float acc[RS_TOKENS] = {};
-#pragma unroll 8
-        for (int i = lane; i < chunks; i += 32) {
-            const float4 c = 4 * i < D ? load_row4(row, 4 * i, D, VEC) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const auto multiply = [&](int i, const float4& c) {
 #pragma unroll
             for (int t = 0; t < RS_TOKENS; ++t) {
                 const float4 x = rs_x[t * chunks + i];
@@ -716,6 +738,15 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
                 acc[t] = __fmaf_rn(x.z, c.z, acc[t]);
                 acc[t] = __fmaf_rn(x.w, c.w, acc[t]);
             }
+        };
+        if (AHEAD && e == first_e) {
+            cp_async_wait<0>();           // every lane reads back only what it fetched itself
+#pragma unroll 2
+            for (int i = lane; i < chunks; i += 32) multiply(i, rs_c[i]);
+        } else {
+#pragma unroll 8
+            for (int i = lane; i < chunks; i += 32)
+                multiply(i, 4 * i < D ? load_row4(row, 4 * i, D, VEC) : make_float4(0.f, 0.f, 0.f, 0.f));
         }
 #pragma unroll
         for (int t = 0; t < RS_TOKENS; ++t) {
@@ -1038,11 +1069,15 @@ template <bool VEC>
 int launch_route_small(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
                        float* score, int* status, cudaStream_t stream) {
     const int cluster = rs_cluster(E);
-    const size_t smem = rs_smem(D);
-    auto kern = route_small_kernel<VEC>;
+    size_t smem = rs_smem(D);
+    const long long blocks = (T + RS_TOKENS - 1) / RS_TOKENS * cluster;
+    const size_t all = smem / RS_TOKENS * (RS_TOKENS + 1 + RS_WARPS);     // rows, LayerNorm weights, a centroid per warp
+    const bool ahead = VEC && blocks <= 148 && all <= RS_AHEAD_SMEM;
+    auto kern = ahead ? route_small_kernel<VEC, VEC> : route_small_kernel<VEC, false>;
+    if (ahead) smem = all;
     if (smem > 40 * 1024)
-        INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_MAX_SMEM));
-    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)((T + RS_TOKENS - 1) / RS_TOKENS * cluster), RS_THREADS, smem,
+        INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ahead ? RS_AHEAD_SMEM : RS_MAX_SMEM));
+    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)blocks, RS_THREADS, smem,
                                    (unsigned)cluster, stream, X, C, gamma, T, D, E, gate, score, status));
     return INFMOE_OK;
 }
