@@ -76,22 +76,31 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
 
+// Where the outputs go: g (DUAL), or row j to row out_pos[j] (or j) of `out`, or to the address out_row_ptr[out_pos[j]]; the
+// residual is the same row of `resid`; mix_score != NULL applies the base_layer output mix.  With the combine step in here no
+// routed copy of x and no result in expert order are written and read back: 300 tokens, 6 experts, 510 x 1022 one kernel of 3.6 us less.
+struct SimtOutput {
+    float* out;
+    const float* resid;
+    const int* out_pos;
+    const float* mix_score;
+    const unsigned long long* out_row_ptr;
+};
+
 // DUAL = true : out[j][n] = gelu(A W0^T) * (A W1^T), padded rows of N outputs   (N = d_ff, K = d_model)
-// DUAL = false: out[j][n] = resid[j][n] + A W0^T, dense rows                    (N = d_model, K = d_ff)
+// DUAL = false: out[.][n] = resid[.][n] + A W0^T, dense rows                    (N = d_model, K = d_ff)
 // Grid: clusters of S CTAs, one per (row tile, output tile), row tile major; CTA r of a cluster takes the r-th S-th of the
 // k blocks.
 template <bool DUAL, int RI>
 __global__ void __launch_bounds__(SIMT_THREADS)
 ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, int K, const float* __restrict__ act,
-                const float* __restrict__ w, const int* __restrict__ slot_of_expert, const float* __restrict__ resid,
-                float* __restrict__ out) {
+                const float* __restrict__ w, const int* __restrict__ slot_of_expert, const SimtOutput o) {
     cg::cluster_group cluster = cg::this_cluster();
     const int S = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
     const unsigned n_tiles = (unsigned)(N + TN - 1) / TN, tile = blockIdx.x / (unsigned)S;
     constexpr int TM = 16 * RI, WROWS = DUAL ? 2 * TN : TN, NB = DUAL ? 2 : 1;
     constexpr int BUF = (TM + WROWS) * PITCH;                 // floats of one buffer: token rows, then weight rows
     __shared__ __align__(16) float smem[2 * BUF];
-    static_assert(NB * RI * SIMT_THREADS * 4 <= 2 * BUF, "the partial sums reuse the buffers");
     __shared__ int s_info[4];
     if (threadIdx.x < 32) {
         int e = 0, r0 = 0, rows = 0;
@@ -164,40 +173,39 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
         }
         __syncthreads();    // the next round's fetch refills this buffer
     }
-    // Sums of the cluster's CTAs, added in ascending k.  Item (i, t): the four outputs of thread t in its row i; the CTAs share
-    // the items out.
-    float4* const red = reinterpret_cast<float4*>(smem);          // [NB][RI][thread]
+    // Sums of the cluster's CTAs, added in ascending k; the CTAs share the outputs out.  A warp takes 32 consecutive outputs of a
+    // row, so that what it stores is one run (the rows may lie in host memory).
+    constexpr int RED = TN + 8;                 // floats per row: the four rows a warp stores to end in different banks
+    static_assert(NB * TM * RED <= 2 * BUF, "the partial sums reuse the buffers");
+    float* const red = smem;                    // [NB][TM][RED]
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
         for (int i = 0; i < RI; ++i)
-            red[(b * RI + i) * SIMT_THREADS + threadIdx.x] = make_float4(acc[b][i][0], acc[b][i][1], acc[b][i][2], acc[b][i][3]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) red[(b * TM + ty + 16 * i) * RED + tx + 8 * j] = acc[b][i][j];
     cluster.sync();
-    constexpr int ITEMS = RI * SIMT_THREADS;
-    for (int it = ITEMS * part / S + (int)threadIdx.x; it < ITEMS * (part + 1) / S; it += SIMT_THREADS) {
-        const int t = it % SIMT_THREADS, r = (t >> 3) + 16 * (it / SIMT_THREADS);
-        if (r >= rows) continue;
-        float sum[NB][4] = {};
+    const int lane = threadIdx.x & 31, n = n0 + lane;
+    for (int r = TM * part / S + (int)(threadIdx.x >> 5); r < min(rows, TM * (part + 1) / S); r += SIMT_THREADS / 32) {
+        float sum[NB] = {};
         for (int q = 0; q < S; ++q) {
-            const float4* from = cluster.map_shared_rank(red, q);
+            const float* from = cluster.map_shared_rank(red, q);
 #pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                const float4 v = from[b * ITEMS + it];
-                sum[b][0] += v.x;
-                sum[b][1] += v.y;
-                sum[b][2] += v.z;
-                sum[b][3] += v.w;
-            }
+            for (int b = 0; b < NB; ++b) sum[b] += from[(b * TM + r) * RED + lane];
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + (t & 7) + 8 * j;
-            if (DUAL) {     // outputs past N are products of zero weights: the zeros the next GEMM's padding needs
-                out[(size_t)(row0 + r) * padded_row(N) + n] = gelu_dot(sum[0][j], sum[NB - 1][j]);
-            } else if (n < N) {
-                const size_t o = (size_t)(row0 + r) * N + n;
-                out[o] = resid[o] + sum[0][j];
+        const int j = row0 + r;
+        if (DUAL) {     // outputs past N are products of zero weights: the zeros the next GEMM's padding needs
+            o.out[(size_t)j * padded_row(N) + n] = gelu_dot(sum[0], sum[NB - 1]);
+        } else if (n < N) {
+            const int row = o.out_pos ? o.out_pos[j] : j;
+            float* const dst = o.out_row_ptr ? reinterpret_cast<float*>(o.out_row_ptr[row]) : o.out + (size_t)row * N;
+            const float x = o.resid[(size_t)row * N + n];
+            float y = x + sum[0];
+            if (o.mix_score) {
+                const float alpha = mix_alpha(o.mix_score[j]);
+                y = mix_value(alpha, 1.0f - alpha, y, x);
             }
+            dst[n] = y;
         }
     }
     cluster.sync();      // nobody leaves while its sums are being read
@@ -206,11 +214,11 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
 }  // namespace
 
 // Grouped FFN over experts [e_begin, e_end); T rows in expert-contiguous order.
-//   h [T][padded_row(D)], g [T][padded_row(F)] (scratch), routed [T][D], post [T][D]
+//   h [T][padded_row(D)], g [T][padded_row(F)] (scratch); output as in FfnUmma
 //   slot_of_expert (device, may be NULL = identity) maps expert -> weight slot.
 int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int* offset, const int* slot_of_expert,
-                    const float* h, const float* w01, const float* wo, const float* routed, float* g, float* post,
-                    cudaStream_t stream) {
+                    const float* h, const float* w01, const float* wo, float* g, const float* resid, float* out,
+                    const int* out_pos, const float* mix_score, const unsigned long long* out_row_ptr, cudaStream_t stream) {
     if (T == 0 || e_begin >= e_end) return INFMOE_OK;
     const int experts = e_end - e_begin;
     // 16-row tiles when an expert has about that many rows at most: a 64-row tile would multiply zeros
@@ -219,7 +227,7 @@ int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int
     const unsigned row_tiles = (unsigned)((T + tm - 1) / tm + experts);
     // Not chained (launch_chained): blocks put on the SMs while those of the kernel before are still there crowd on the
     // idle ones, and there are only a few per SM.  The pass of 300 tokens took 195 us so, 126 with a late trigger.
-    const auto launch = [&](auto kern, int N, int K, const float* act, const float* w, const float* resid, float* out) {
+    const auto launch = [&](auto kern, int N, int K, const float* act, const float* w, const SimtOutput& o) {
         // CTAs per tile: by K alone, so that a row's additions do not depend on the other rows of the call
         const unsigned S = K > 7 * TK ? 4 : K > 3 * TK ? 2 : 1;
         cudaLaunchConfig_t cfg = {};
@@ -232,10 +240,11 @@ int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kern, offset, e_begin, e_end, N, K, act, w, slot_of_expert, resid, out);
+        return cudaLaunchKernelEx(&cfg, kern, offset, e_begin, e_end, N, K, act, w, slot_of_expert, o);
     };
-    INFMOE_CUDA_TRY(launch(few ? ffn_simt_kernel<true, 1> : ffn_simt_kernel<true, 4>, F, D, h, w01, (const float*)nullptr, g));
-    INFMOE_CUDA_TRY(launch(few ? ffn_simt_kernel<false, 1> : ffn_simt_kernel<false, 4>, D, F, (const float*)g, wo, routed, post));
+    INFMOE_CUDA_TRY(launch(few ? ffn_simt_kernel<true, 1> : ffn_simt_kernel<true, 4>, F, D, h, w01, SimtOutput{g, nullptr, nullptr, nullptr, nullptr}));
+    INFMOE_CUDA_TRY(launch(few ? ffn_simt_kernel<false, 1> : ffn_simt_kernel<false, 4>, D, F, (const float*)g, wo,
+                           SimtOutput{out, resid, out_pos, mix_score, out_row_ptr}));
     note_launch(2);
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

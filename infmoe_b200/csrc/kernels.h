@@ -24,10 +24,9 @@ int launch_scatter(long long T, int D, const float* X, const float* coeff, const
                    float* rcoeff, cudaStream_t stream);
 // valid_rows (device, may be NULL): rows at or past *valid_rows are skipped (tokens without an expert sit at
 // the tail of pos[]; the dispatch kernel stores their start in offset[E]).
-// CUDA-core GEMM: routed rows and the LayerNorm output h, rows padded with zeros to padded_row(D) floats.
+// CUDA-core GEMM: the LayerNorm output h, rows padded with zeros to padded_row(D) floats.
 int launch_scatter_ln_rows(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
-                           const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h,
-                           cudaStream_t stream);
+                           const float* gamma_all, const int* valid_rows, float* rscore, float* h, cudaStream_t stream);
 // Tensor-core GEMM: packed FP16-pair plane `h` (pack_bytes) and two floats per row in row_info (token_row_info), of rows
 // row0 .. row0 + T - 1.  gamma: the LayerNorm weights that launch_split_expert left for the first expert, or a copy of them,
 // gamma_stride floats from one expert to the next.
@@ -40,8 +39,8 @@ int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, c
 bool dispatch_scatter_supported(long long T, int D, int E);
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
                             const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,
-                            int* zero, int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
-                            bool early, cudaStream_t stream);
+                            int* zero, int zero_count, float* rscore, void* h, float* row_info, bool pack, bool early,
+                            cudaStream_t stream);
 int launch_gather(long long T, int D, const float* in, const int* pos, float* out, cudaStream_t stream,
                   const int* valid_rows = nullptr);
 int launch_mix_gather(long long T, int D, const int* pos, const float* routed, const float* post,
@@ -74,8 +73,8 @@ inline size_t pack_bytes(long long rows, int K) { return (size_t)rows * (size_t)
 // w01 [slots] x tiled(2F x D) (row 2f = wi_0[f], row 2f+1 = wi_1[f]) and wo [slots] x tiled(D x F).
 // Activations h [T][padded_row(D)] and g [T][padded_row(F)] are FP32 (pack_bytes).
 int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int* offset, const int* slot_of_expert,
-                    const float* h, const float* w01, const float* wo, const float* routed, float* g, float* post,
-                    cudaStream_t stream);
+                    const float* h, const float* w01, const float* wo, float* g, const float* resid, float* out,
+                    const int* out_pos, const float* mix_score, const unsigned long long* out_row_ptr, cudaStream_t stream);
 
 // A one-warp kernel that waits, with the GEMM's bounded wait and the given limit, on a barrier nobody completes.
 int launch_wait_probe(unsigned long long limit_ns, int* status, unsigned long long* waited_ns, cudaStream_t stream);

@@ -249,8 +249,8 @@ WsLayout ws_layout(const infmoe_layer* L, long long T, bool streamed) {
     w.slot_map = take(4 * E);
     w.score = take(4 * t);
     w.rscore = take(4 * t);
-    // The tensor-core GEMM reads its residual from the input through pos[] and writes the layer output from its
-    // epilogue; only the CUDA-core path and the Identity sublayer keep routed rows and expert-ordered results.
+    // The GEMMs read their residual from the input through pos[] and write the layer output from their epilogue; routed rows
+    // and expert-ordered results are kept by the Identity and registered sublayers (and have room on the CUDA-core path).
     const bool row_planes = L->identity || L->custom || !uses_umma(L);
     w.routed = take(row_planes ? 4 * t * D : 0);
     w.post = take(row_planes ? 4 * t * D : 0);
@@ -426,10 +426,9 @@ int status_to_rc(int status) {
     return INFMOE_OK;
 }
 
-// Where the experts' result goes: `post` in expert order (a combine kernel follows), or, on the tensor-core path,
-// straight into the layer output in token order (`out` with the row map `pos`, optionally the base_layer mix).
+// Where the experts' result goes: into the layer output in token order (`out` with the row map `pos`, optionally the
+// base_layer mix).
 struct FfnOutput {
-    float* post;
     float* out = nullptr;
     const int* pos = nullptr;
     const float* mix_score = nullptr;
@@ -446,7 +445,7 @@ struct FfnBuffers {
 };
 
 int run_ffn(infmoe_layer* L, long long T, int e_begin, int e_end, const int* d_offset, const int* d_slot_map,
-            int slots, float* const planes[2], const FfnBuffers& w, const float* routed, const FfnOutput& o,
+            int slots, float* const planes[2], const FfnBuffers& w, const float* resid, const FfnOutput& o,
             cudaStream_t stream, cudaEvent_t mid = nullptr, bool early = false, const int* d_gate = nullptr) {
     if (uses_umma(L)) {
         FfnUmma f{};
@@ -460,19 +459,19 @@ int run_ffn(infmoe_layer* L, long long T, int e_begin, int e_end, const int* d_o
         f.h = w.h;
         f.row_info = w.row_info;
         f.g = w.g;
-        f.resid = routed;
-        f.out = o.out ? o.out : o.post;
-        f.out_pos = o.out ? o.pos : nullptr;
-        f.mix_score = o.out ? o.mix_score : nullptr;
-        f.out_row_ptr = o.out ? o.row_ptr : nullptr;
+        f.resid = resid;
+        f.out = o.out;
+        f.out_pos = o.pos;
+        f.mix_score = o.mix_score;
+        f.out_row_ptr = o.row_ptr;
         f.part = w.part;
         f.part_bytes = w.part_bytes;
         f.part_count = w.part_count;
         f.status = L->d_status;
         return launch_ffn_umma(f, T, L->D, L->F, L->E, e_begin, e_end, L->num_sms, stream, mid);
     }
-    return launch_ffn_simt(T, L->D, L->F, e_begin, e_end, d_offset, d_slot_map, w.h, planes[0], planes[1], routed, w.g,
-                           o.post, stream);
+    return launch_ffn_simt(T, L->D, L->F, e_begin, e_end, d_offset, d_slot_map, w.h, planes[0], planes[1], w.g, resid, o.out,
+                           o.pos, o.mix_score, o.row_ptr, stream);
 }
 
 void free_device_state(infmoe_layer* L) {
@@ -1109,16 +1108,13 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     INFMOE_TRY(prof_mark(L, 2, stream));
     // whole layer: the variant decides; experts alone: the caller asks for the mix by passing the scores
     const bool mix = given_gate ? row_score != nullptr : L->flags.base_layer_mix;
-    // the tensor-core GEMM writes the layer output itself (combine fused into its epilogue)
-    const bool fused_combine = pack;
+    // the GEMMs write the layer output themselves (combine fused into the epilogue)
+    const bool fused_combine = !L->identity && !L->custom;
     FfnOutput ffn_out;
-    ffn_out.post = post;
-    if (fused_combine) {
-        ffn_out.out = row_dst ? post : d_out;   // with per-row addresses `out` only switches the fused path on
-        ffn_out.pos = pos;
-        ffn_out.mix_score = mix ? rscore : nullptr;
-        ffn_out.row_ptr = row_dst;
-    }
+    ffn_out.out = d_out;
+    ffn_out.pos = pos;
+    ffn_out.mix_score = mix ? rscore : nullptr;
+    ffn_out.row_ptr = row_dst;
     if (L->identity) {
         // Identity expert (plugin/sublayers/IdentityLayer.hh): post = routed
         INFMOE_TRY(launch_scatter(T, L->D, d_in, score, pos, routed, rscore, stream));
@@ -1170,7 +1166,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
         }
     } else {
         // 3. scatter fused with the experts' LayerNorm and the operand split (:354-355, T5FFLayer.cc:99-103)
-        // Tensor-core path: no routed copy, the second GEMM's epilogue reads its residual from d_in through pos[].  The
+        // No routed copy, the second GEMM's epilogue reads its residual from d_in through pos[].  Tensor-core path: the
         // LayerNorm weights to apply are those launch_split_expert left in the weight slots, or for streamed experts the
         // ones kept from earlier passes (rows of experts that have none yet are scattered again further down).
         const size_t gamma_at = pack ? split_gamma_at(2 * L->F, L->D) : 0;
@@ -1185,22 +1181,21 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
         }
         if (with_scatter) {
             INFMOE_TRY(launch_dispatch_scatter(T, L->D, L->E, d_in, score, gate_in, gamma, gamma_stride, pos, count, offset,
-                                               L->d_status, zero, FFN_COUNTERS, routed, rscore, buf.h, buf.row_info, pack,
+                                               L->d_status, zero, FFN_COUNTERS, rscore, buf.h, buf.row_info, pack,
                                                !given_gate, stream));
         } else if (pack) {
             INFMOE_TRY(launch_scatter_ln_pack(0, T, L->D, d_in, score, pos, gate_in, gamma, gamma_stride, valid_rows,
                                               rscore, buf.h, buf.row_info, stream));
         } else {
-            INFMOE_TRY(launch_scatter_ln_rows(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, routed, rscore,
-                                              buf.h, stream));
+            INFMOE_TRY(launch_scatter_ln_rows(T, L->D, d_in, score, pos, gate_in, s->d_ln, valid_rows, rscore, buf.h,
+                                              stream));
         }
-        if (pack) routed = const_cast<float*>(d_in);   // run_ffn's residual operand
         INFMOE_TRY(prof_mark(L, 3, stream));
         // 4. experts (:360-402)
         if (!streamed) {
             cudaEvent_t mid = nullptr;
             if (L->profiling) mid = L->prof_events[(size_t)(L->prof_calls % PROF_CALLS) * PROF_MARKS + 4];
-            INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, nullptr, L->E, s->d_plane, buf, routed, ffn_out, stream, mid, true,
+            INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, nullptr, L->E, s->d_plane, buf, d_in, ffn_out, stream, mid, true,
                                with_scatter ? gate_in : nullptr));
         } else {
             const size_t n = s->matrix_elems();
@@ -1266,7 +1261,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                 long long row0 = 0;
                 for (size_t j = 0; j < active.size(); row0 += L->h_count[active[j++]])
                     INFMOE_TRY(scatter_first(active[j], plan[j].slot, row0));
-                INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, slot_map, nslots, planes, buf, routed, ffn_out, stream));
+                INFMOE_TRY(run_ffn(L, T, 0, L->E, offset, slot_map, nslots, planes, buf, d_in, ffn_out, stream));
                 for (const CachePlan& pl : plan) INFMOE_CUDA_TRY(cudaEventRecord(L->ev_freed[pl.slot], stream));
             }
             long long row0 = 0;      // rows are in expert order
@@ -1293,7 +1288,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
                 INFMOE_CUDA_TRY(cudaStreamWaitEvent(stream, L->ev_ready[slot], 0));
                 INFMOE_TRY(scatter_first(e, slot, row0));
                 row0 += L->h_count[e];
-                INFMOE_TRY(run_ffn(L, T, e, e + 1, offset, slot_map, nslots, planes, buf, routed, ffn_out, stream));
+                INFMOE_TRY(run_ffn(L, T, e, e + 1, offset, slot_map, nslots, planes, buf, d_in, ffn_out, stream));
                 INFMOE_CUDA_TRY(cudaEventRecord(L->ev_freed[slot], stream));
             }
             if (kept) {
@@ -1305,8 +1300,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     }
     INFMOE_TRY(prof_mark(L, 5, stream));
     // 5. combine (:407-412; the gather reads the expert output), unless the GEMM epilogue has done it
-    if (fused_combine) {
-    } else {
+    if (!fused_combine) {
         // with per-row addresses the rows are first combined in the caller's row order (g is free by now), then copied out
         float* ordered = row_dst ? buf.g : d_out;
         if (mix)
@@ -1895,7 +1889,8 @@ int t5ff_run_in(char* base, int64_t rows, int32_t D, int32_t F, const float* ln_
     INFMOE_CUDA_TRY(cudaGetDevice(&dev));
     INFMOE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (simt) {
-        INFMOE_TRY(launch_ffn_simt(rows, D, F, 0, 1, offset, nullptr, h, planes[0], planes[1], x, g, y, stream));
+        INFMOE_TRY(launch_ffn_simt(rows, D, F, 0, 1, offset, nullptr, h, planes[0], planes[1], g, x, y, nullptr, nullptr,
+                                   nullptr, stream));
     } else {
         FfnUmma u{};
         u.offset = offset;

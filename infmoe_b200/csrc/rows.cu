@@ -53,9 +53,9 @@ scatter_kernel(long long T, int D, int vec, const float* __restrict__ X, const f
 // for the grouped GEMM.  The expert of row j is gate[pos[j]].  Rows at or past *valid_rows (tokens without an expert,
 // empty receive slots) are skipped.
 //
-// For the CUDA-core GEMM: the routed row, the routed score, and h in FP32, rows padded with zeros to whole groups of 32.
+// For the CUDA-core GEMM: the routed score, and h in FP32, rows padded with zeros to whole groups of 32.
 __device__ __forceinline__ void warp_ln_rows(const float* __restrict__ src, const float* __restrict__ gamma, int D,
-                                             bool vec, float* __restrict__ routed, float* __restrict__ h) {
+                                             bool vec, float* __restrict__ h) {
     const int lane = threadIdx.x & 31;
     float mean, rstd;
     warp_row_stats(src, D, vec, mean, rstd);
@@ -66,10 +66,7 @@ __device__ __forceinline__ void warp_ln_rows(const float* __restrict__ src, cons
             const float vv[4] = {v.x, v.y, v.z, v.w}, gg[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (base + k < D) {
-                    hh[k] = ln_apply(vv[k], mean, rstd, gg[k]);
-                    if (routed) routed[base + k] = vv[k];
-                }
+                if (base + k < D) hh[k] = ln_apply(vv[k], mean, rstd, gg[k]);
         }
         *reinterpret_cast<float4*>(h + base) = make_float4(hh[0], hh[1], hh[2], hh[3]);
     }
@@ -78,16 +75,14 @@ __device__ __forceinline__ void warp_ln_rows(const float* __restrict__ src, cons
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 scatter_ln_rows_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ score,
                        const int* __restrict__ pos, const int* __restrict__ gate, const float* __restrict__ gamma_all,
-                       const int* __restrict__ valid_rows, float* __restrict__ routed, float* __restrict__ rscore,
-                       float* __restrict__ h) {
+                       const int* __restrict__ valid_rows, float* __restrict__ rscore, float* __restrict__ h) {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;
     const int p = pos[j];
-    warp_ln_rows(X + (long long)p * D, gamma_all + (long long)gate[p] * D, D, vec != 0, routed + j * D,
-                 h + j * (long long)padded_row(D));
+    warp_ln_rows(X + (long long)p * D, gamma_all + (long long)gate[p] * D, D, vec != 0, h + j * (long long)padded_row(D));
     if (lane == 0 && rscore && score) rscore[j] = score[p];
 }
 
@@ -127,8 +122,7 @@ __device__ __forceinline__ void warp_ln_pack(const float* __restrict__ src, cons
     if (lane == 0) *info = token_row_info(s, squares);
 }
 
-// The scatter for the tensor-core GEMM (which reads its residual from X through pos[], so no routed row is written), of
-// rows j0 .. j0 + T - 1.  The LayerNorm weights are gamma' (see SplitExpert), which lies with the experts' planes.
+// The scatter for the tensor-core GEMM, of rows j0 .. j0 + T - 1.  The LayerNorm weights are gamma' (see SplitExpert), which lies with the experts' planes.
 struct ExpertGamma {
     const float* base;              // first expert
     size_t stride;                  // floats from one expert to the next
@@ -260,8 +254,8 @@ __global__ void __launch_bounds__(DS_THREADS)
 dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ X, const float* __restrict__ score,
                         const int* __restrict__ gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
                         int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
-                        int* __restrict__ zero, int zero_count, float* __restrict__ routed, float* __restrict__ rscore,
-                        void* __restrict__ h, float2* __restrict__ row_info, int early) {
+                        int* __restrict__ zero, int zero_count, float* __restrict__ rscore, void* __restrict__ h,
+                        float2* __restrict__ row_info, int early) {
     extern __shared__ __align__(16) float ds_smem[];
     __shared__ int s_before[DS_THREADS / 32];
     __shared__ float s_top[DS_THREADS / 32];
@@ -357,8 +351,6 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
         float* x = s_x + k;
         const float4 g = *reinterpret_cast<const float4*>(s_g + k);
         float4 v = *reinterpret_cast<const float4*>(x);
-        if (!PACK)
-            for (int i = 0; i < 4 && k + i < D; ++i) routed[(size_t)j * D + k + i] = x[i];
         v.x = k < D ? ln_apply(v.x, mean, rstd, g.x) : 0.f;
         v.y = k + 1 < D ? ln_apply(v.y, mean, rstd, g.y) : 0.f;
         v.z = k + 2 < D ? ln_apply(v.z, mean, rstd, g.z) : 0.f;
@@ -473,7 +465,7 @@ ln_rows_kernel(long long n, int D, int vec, const float* __restrict__ in, const 
                float* __restrict__ h) {
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= n) return;
-    warp_ln_rows(in + j * D, gamma, D, vec != 0, nullptr, h + j * (long long)padded_row(D));
+    warp_ln_rows(in + j * D, gamma, D, vec != 0, h + j * (long long)padded_row(D));
 }
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 ln_pack_kernel(long long n, int D, int vec, const float* __restrict__ in, const float* __restrict__ gamma,
@@ -816,27 +808,26 @@ bool dispatch_scatter_supported(long long T, int D, int E) { return T <= 1024 &&
 
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
                             const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,
-                            int* zero, int zero_count, float* routed, float* rscore, void* h, float* row_info, bool pack,
-                            bool early, cudaStream_t stream) {
+                            int* zero, int zero_count, float* rscore, void* h, float* row_info, bool pack, bool early,
+                            cudaStream_t stream) {
     const int vec = (D % 4 == 0) && (gamma_stride % 4 == 0) && aligned16(X) && aligned16(gamma);
     size_t smem = 2 * padded_row(D) * sizeof(float);
     if (smem < sizeof(int) * (size_t)(E + 1)) smem = sizeof(int) * (size_t)(E + 1);
     auto kern = pack ? dispatch_scatter_kernel<true> : dispatch_scatter_kernel<false>;
     INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)T + 1, DS_THREADS, smem, 1, stream, (int)T, D, E, vec, X, score, gate,
                                    ExpertGamma{gamma, gamma_stride}, pos, count, offset, status, zero,
-                                   zero ? zero_count : 0, routed, rscore, h, (float2*)row_info, early ? 1 : 0));
+                                   zero ? zero_count : 0, rscore, h, (float2*)row_info, early ? 1 : 0));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
 }
 
 int launch_scatter_ln_rows(long long T, int D, const float* X, const float* score, const int* pos, const int* gate,
-                           const float* gamma_all, const int* valid_rows, float* routed, float* rscore, float* h,
-                           cudaStream_t stream) {
+                           const float* gamma_all, const int* valid_rows, float* rscore, float* h, cudaStream_t stream) {
     if (T == 0) return INFMOE_OK;
     const int vec = (D % 4 == 0) && aligned16(X) && aligned16(gamma_all);
     INFMOE_CUDA_TRY(launch_chained(scatter_ln_rows_kernel, row_grid(T), ROW_WARPS * 32, 0, 1, stream, T, D, vec, X, score,
-                                   pos, gate, gamma_all, valid_rows, routed, rscore, h));
+                                   pos, gate, gamma_all, valid_rows, rscore, h));
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;
