@@ -45,8 +45,8 @@
 //   warp 1        MMA issuer (and owner of the TMEM allocation): one commit per k block frees the stage, one per chunk
 //                 hands its accumulator to the accumulate warps.  Chunks rotate over as many accumulators as fit into
 //                 TMEM at the width of the launch's widest token tile (2 at 192 columns, 4 at 128, at most 8)
-//   warps 4..19   accumulate + epilogue: tcgen05.ld the chunk (one TMEM lane quarter and every fourth
-//                 16-column slice per warp), add into registers; after the last chunk gelu*dot and its
+//   warps 4..19   accumulate + epilogue: tcgen05.ld the chunk (one TMEM lane quarter and a quarter of the
+//                 columns per warp, 4 of 16 to 48 of 192), add into registers; after the last chunk gelu*dot and its
 //                 split (lane pairs exchange a and b by shuffle) or residual add.  The epilogue is a chain of
 //                 shuffles, loads and stores, so warps in flight set its speed, and with K = 1024 or less it sets the
 //                 kernel's: 8 -> 16 warps (and 8 residual values in flight per thread instead of 16, which spilled)
@@ -232,6 +232,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 constexpr int BK = 32;                     // k block: 32 values = one 128-byte swizzled row (32 x hi, 32 x lo)
@@ -263,6 +269,7 @@ constexpr int EPI_WARPS = 4 * EPI_GROUPS;
 constexpr int GEMM_THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
 constexpr int TMEM_COLS = 512;
 constexpr int CHUNK_BLOCKS = 8;                       // k blocks (of 6 MMAs) an accumulator takes between two drains
+constexpr int SUM_FLIGHT = 10;                        // chunk sums a thread fetches at a time (narrow tiles)
 constexpr int W_TILE = UMMA_M * ROW_BYTES;            // 16 KB of weights per k block
 
 template <int NMAX, int STAGES, int CTAS>
@@ -270,7 +277,7 @@ struct Cfg {
     static constexpr int STAGE = W_TILE + NMAX / CTAS * ROW_BYTES;  // weight tile, then this CTA's part of the token tile
     static constexpr int SMEM = STAGES * STAGE + 1024;              // + slack for 1024-byte alignment
     static constexpr int MAX_ACC = 8;                                // accumulators, at most
-    static constexpr int SLICES = (NMAX / 16 + EPI_GROUPS - 1) / EPI_GROUPS;   // 16-column slices owned by one epilogue thread
+    static constexpr int SLICES = (NMAX / EPI_GROUPS + 15) / 16;     // 16-column slices owned by one epilogue thread
     static constexpr int N_STEP = 16 * CTAS;                        // token tiles are padded to a multiple of this
     static_assert(NMAX % N_STEP == 0 && 2 * NMAX <= TMEM_COLS, "token chunk");
     static_assert((NMAX / CTAS * ROW_BYTES) % 1024 == 0, "tiles must keep 1024-byte alignment");
@@ -663,7 +670,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // round-to-nearest adds in ascending k, to a running sum in registers; then the accumulator goes back to the
         // MMA issuer.
         const int q = warp & 3;                 // TMEM lane quarter this warp may access
-        const int group = (warp - EPI_WARP0) >> 2;   // 16-column slices group, group + EPI_GROUPS, ...
+        const int group = (warp - EPI_WARP0) >> 2;   // columns [group, group + 1) / EPI_GROUPS of the tile
         const uint32_t tlane = tmem_base + ((uint32_t)(q * 32) << 16);
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
@@ -671,7 +678,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         wait_then_trigger();
         while (ok && sched.next(item) && !*abort_flag) {
             const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, s_beg, s_cnt, args);
-            const int nsl = t.n_pad >> 4;
+            const int width = t.n_pad / EPI_GROUPS, col0 = group * width;    // this warp's columns; a multiple of 4
             float sum[C::SLICES][16];
 #pragma unroll
             for (int i = 0; i < C::SLICES; ++i)
@@ -682,14 +689,13 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             float4* const part = item.tail >= 0 ? args.part + ((size_t)item.tail * CTAS + rank) * sched.m * block + row : nullptr;
             auto store_block = [&](int c) {     // sum[][] -> block of chunk c
 #pragma unroll
-                for (int i = 0; i < C::SLICES; ++i) {
-                    const int sl = EPI_GROUPS * i + group;
-                    if (sl >= nsl) continue;
+                for (int i = 0; i < C::SLICES; ++i)
 #pragma unroll
-                    for (int v = 0; v < 4; ++v)
-                        __stcg(part + c * block + (size_t)(sl * 4 + v) * UMMA_M,
+                    for (int v = 0; v < 4; ++v) {
+                        if (16 * i + 4 * v >= width) continue;
+                        __stcg(part + c * block + (size_t)((col0 >> 2) + 4 * i + v) * UMMA_M,
                                make_float4(sum[i][4 * v], sum[i][4 * v + 1], sum[i][4 * v + 2], sum[i][4 * v + 3]));
-                }
+                    }
             };
             for (int c = item.c0; c < item.c1; ++c) {
                 // the warp stays converged for the .aligned TMEM instructions, also when a wait is abandoned
@@ -700,10 +706,18 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 tc_fence_after();
 #pragma unroll
                 for (int i = 0; i < C::SLICES; ++i) {
-                    const int sl = EPI_GROUPS * i + group;
-                    if (sl >= nsl) continue;
+                    if (16 * i >= width) continue;       // uniform across the warp
+                    const uint32_t at = tlane + acc * acc_stride + col0 + 16 * i;
                     uint32_t r[16];
-                    tmem_ld16(tlane + acc * acc_stride + sl * 16, r);
+                    if (16 * i + 16 <= width) {
+                        tmem_ld16(at, r);
+                    } else {
+#pragma unroll
+                        for (int x = 0; x < 16; ++x) r[x] = 0;
+#pragma unroll
+                        for (int v = 0; v < 3; ++v)
+                            if (16 * i + 4 * v < width) tmem_ld4(at + 4 * v, r + 4 * v);
+                    }
                     tmem_ld_wait();
 #pragma unroll
                     for (int x = 0; x < 16; ++x) sum[i][x] = __fadd_rn(sum[i][x], __uint_as_float(r[x]));
@@ -743,20 +757,51 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 __syncwarp();    // orders lane 0's fence before the other lanes' reads of the sums; a shuffle does not
                 if (done != sched.m) continue;
                 const int first = sched.prefix_chunks(item.tail) - 1;
+                if constexpr (C::SLICES == 1) {
+                    // few columns: one of the thread's float4 at a time, SUM_FLIGHT chunks of it on their way together (a trip is
+                    // 1.4 us; one token through 4096 x 10240 has 40 chunk sums per tile)
 #pragma unroll
-                for (int i = 0; i < C::SLICES; ++i) {
-                    const int sl = EPI_GROUPS * i + group;
-                    if (sl >= nsl) continue;
-                    const float4* src = part + (size_t)(sl * 4) * UMMA_M;
+                    for (int v = 0; v < 4; ++v) {
+                        if (4 * v >= width) continue;
+                        const float4* src = part + (size_t)((col0 >> 2) + v) * UMMA_M;
+                        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+                        for (int c0 = first; c0 < sched.m; c0 += SUM_FLIGHT) {
+                            float4 x[SUM_FLIGHT];
+#pragma unroll
+                            for (int c = 0; c < SUM_FLIGHT; ++c)
+                                if (c0 + c < sched.m) x[c] = __ldcg(src + (c0 + c) * block);
+#pragma unroll
+                            for (int c = 0; c < SUM_FLIGHT; ++c) {
+                                if (c0 + c >= sched.m) break;
+                                y.x = __fadd_rn(y.x, x[c].x);
+                                y.y = __fadd_rn(y.y, x[c].y);
+                                y.z = __fadd_rn(y.z, x[c].z);
+                                y.w = __fadd_rn(y.w, x[c].w);
+                            }
+                        }
+                        sum[0][4 * v] = y.x;
+                        sum[0][4 * v + 1] = y.y;
+                        sum[0][4 * v + 2] = y.z;
+                        sum[0][4 * v + 3] = y.w;
+                    }
+                } else {
+                    // eight float4 in flight; more of them spill
+#pragma unroll
+                    for (int i = 0; i < C::SLICES; ++i) {
+                        if (16 * i >= width) continue;
+                        const float4* src = part + (size_t)((col0 >> 2) + 4 * i) * UMMA_M;
 #pragma unroll 2
-                    for (int c = first; c < sched.m; ++c) {
+                        for (int c = first; c < sched.m; ++c) {
 #pragma unroll
-                        for (int v = 0; v < 4; ++v) {
-                            const float4 x = __ldcg(src + c * block + (size_t)v * UMMA_M);
-                            sum[i][4 * v] = __fadd_rn(sum[i][4 * v], x.x);
-                            sum[i][4 * v + 1] = __fadd_rn(sum[i][4 * v + 1], x.y);
-                            sum[i][4 * v + 2] = __fadd_rn(sum[i][4 * v + 2], x.z);
-                            sum[i][4 * v + 3] = __fadd_rn(sum[i][4 * v + 3], x.w);
+                            for (int v = 0; v < 4; ++v) {
+                                if (16 * i + 4 * v >= width) continue;
+                                const float4 x = __ldcg(src + c * block + (size_t)v * UMMA_M);
+                                sum[i][4 * v] = __fadd_rn(sum[i][4 * v], x.x);
+                                sum[i][4 * v + 1] = __fadd_rn(sum[i][4 * v + 1], x.y);
+                                sum[i][4 * v + 2] = __fadd_rn(sum[i][4 * v + 2], x.z);
+                                sum[i][4 * v + 3] = __fadd_rn(sum[i][4 * v + 3], x.w);
+                            }
                         }
                     }
                 }
@@ -770,12 +815,12 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             const float bound = (float)__ldg(args.bound + (size_t)t.slot * args.bound_stride);
 #pragma unroll
             for (int i = 0; i < C::SLICES; ++i) {
-                const int sl = EPI_GROUPS * i + group;
-                if (sl >= nsl) continue;     // uniform across the warp
+                if (16 * i >= width) continue;     // uniform across the warp
+                const int sl0 = col0 + 16 * i;
                 // What belongs to the slice's 16 token columns, one column per lane (lanes 16..31 repeat them),
                 // handed out by shuffle below: 2^-s of the token row, and 2^s of g (GELU_PAIR) or the output row and
                 // the mix coefficient (RESIDUAL).
-                const int lc = sl * 16 + (lane & 15);
+                const int lc = sl0 + (lane & 15);
                 const int r = t.row0 + lc;
                 const bool lc_ok = lc < t.n_tok;
                 const float2 info = lc_ok ? __ldg(args.row_info + r) : make_float2(1.f, 0.f);
@@ -791,12 +836,13 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     const float lane_scale = exp2_int(g_exp);
 #pragma unroll
                     for (int c = 0; c < 16; c += 2) {
+                        if (16 * i + c >= width) continue;
                         const float v0 = unscale(sum[i][c], w_inv, __shfl_sync(0xffffffffu, lane_inv, c));
                         const float v1 = unscale(sum[i][c + 1], w_inv, __shfl_sync(0xffffffffu, lane_inv, c + 1));
                         const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
                         const float a = odd ? got : v0, b = odd ? v1 : got;
                         const float g = gelu_dot_fast(a, b) * __shfl_sync(0xffffffffu, lane_scale, c + odd);
-                        const int col = sl * 16 + c + odd;
+                        const int col = sl0 + c + odd;
                         // Packed plane: neighbouring f (lanes two apart, same column) exchange their halves so that
                         // every lane stores one 32-bit word, even f the pair of hi, odd f the pair of lo.
                         const uint32_t hl = split_f16(g);
@@ -823,11 +869,13 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 // cost a trip to L2 or HBM, and the next tile's first chunk would wait.
 #pragma unroll
                 for (int c0 = 0; c0 < 16; c0 += 8) {
+                    if (16 * i + c0 >= width) continue;
+                    const int end = min(t.n_tok, col0 + width) - (sl0 + c0);    // columns of these eight that are this warp's
                     float xres[8];
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         const int resid_row = __shfl_sync(0xffffffffu, lane_row, c0 + c);
-                        xres[c] = (sl * 16 + c0 + c < t.n_tok && m_ok)
+                        xres[c] = (c < end && m_ok)
                                       ? args.resid[(size_t)resid_row * (size_t)args.M_total + (size_t)m] : 0.f;
                     }
 #pragma unroll
@@ -835,7 +883,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         const unsigned long long out_row = __shfl_sync(0xffffffffu, lane_ptr, c0 + c);
                         const float alpha = __shfl_sync(0xffffffffu, lane_alpha, c0 + c);
                         const float v = unscale(sum[i][c0 + c], w_inv, __shfl_sync(0xffffffffu, lane_inv, c0 + c));
-                        if (sl * 16 + c0 + c < t.n_tok && m_ok) {
+                        if (c < end && m_ok) {
                             const float x = xres[c];
                             float y = __fadd_rn(x, v);
                             if (args.mix_score) y = mix_value(alpha, 1.0f - alpha, y, x);

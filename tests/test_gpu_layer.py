@@ -685,3 +685,30 @@ def test_paired_tiles_against_oracle(oracle, D, F):
         if rows.size:
             want = oracle.expert_ffn_f64(x[rows], *experts[e])
             assert oracle.rel_l2(out[0][rows], want) <= TOL
+
+
+# A tile's columns are shared out evenly over four warps per row quarter, 4 to 48 columns each: every width from 16 to 192,
+# full and with one token less, tiles of one CTA (K < 2048) and of two.
+@pytest.mark.parametrize("D,F", [(260, 516), (2052, 132)])
+def test_token_tiles_of_every_width(oracle, D, F):
+    import torch
+    from infmoe_b200 import MoELayer
+    counts = tuple(range(16, 193, 16)) + tuple(range(15, 192, 16))
+    rng = np.random.default_rng(D)
+    E, n = len(counts), sum(counts)
+    layer = MoELayer.create(E, D, F, 2, np.ones((E, D), np.float32), None, "T5_FF", "default", None)
+    expert = [(1 + 0.01 * rng.standard_normal(D)).astype(np.float32)] + \
+             [(rng.standard_normal((F, D)) / np.sqrt(D)).astype(np.float32) for _ in range(2)] + \
+             [(rng.standard_normal((D, F)) / np.sqrt(F)).astype(np.float32)]
+    for e in range(E):
+        layer.set_expert(e, *(torch.from_numpy(a).cuda() for a in expert))
+    gate = torch.from_numpy(rng.permutation(np.repeat(np.arange(E, dtype=np.int32), counts))).cuda()
+    x = rng.standard_normal((n, D)).astype(np.float32)
+    dx = torch.from_numpy(x).cuda()
+    out = layer.expert_forward(dx, gate).cpu().numpy()
+    # the same rows, all experts being alike, in one expert's tiles of 192 columns
+    same = layer.expert_forward(dx, torch.zeros_like(gate)).cpu().numpy()
+    layer.sync_status()
+    layer.terminate()
+    np.testing.assert_array_equal(same, out)
+    assert oracle.rel_l2(out[:64] - x[:64], oracle.expert_ffn_f64(x[:64], *expert) - x[:64]) <= TOL
