@@ -151,6 +151,25 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return mbar_wait_slow(bar, parity, abort_flag);
 }
 
+// L2 policies of a load: weights that one tile alone reads give way first, so that streaming them does not push out what
+// the passes come back to (activations, chunk sums, centroids, and the kernels' code).
+__device__ __forceinline__ uint64_t l2_evict_first() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ uint64_t l2_evict_normal() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
+                                                 uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
+        : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -216,6 +235,14 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair_hint(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
+                                                      uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], "
+        "[%2], %5;"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
         : "memory");
 }
 // Arrives on the mbarrier once all MMAs issued so far by this thread have completed.
@@ -570,6 +597,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (lane == 0) {
             uint32_t it = 0, ahead = 0;    // ahead: k blocks whose weights were fetched before the wait
             bool ok = true, waited = !early;
+            const uint64_t evict_first = l2_evict_first(), evict_normal = l2_evict_normal();
             const auto wait = [&]() {
                 if (EPI == EPI_RESIDUAL) pdl_wait();
                 wait_then_trigger();
@@ -586,14 +614,15 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const int mb = min(t.mb * CTAS + (int)rank, MB1 - 1);
                 const int w_row0 = (int)(args.w_stride / BK) * t.slot + mb * KB * UMMA_M;
                 const int kb_end = min(KB, item.c1 * CHUNK_BLOCKS);
+                const uint64_t policy = s_cnt[t.expert] <= NMAX ? evict_first : evict_normal;    // one token chunk: read once
                 const auto fetch_weights = [&](uint32_t s, int kb) {
                     const uint32_t bar = smem_u32(&s_full[s]), dst = ring + s * C::STAGE;
                     if (CTAS == 1) {
                         mbar_expect_tx(bar, bytes);
-                        tma_load_2d(dst, &map_w, bar, 0, w_row0 + kb * UMMA_M);
+                        tma_load_2d_hint(dst, &map_w, bar, 0, w_row0 + kb * UMMA_M, policy);
                     } else {
                         if (rank == 0) mbar_expect_tx(bar, CTAS * bytes);
-                        tma_load_2d_pair(dst, &map_w, leader_addr(bar), 0, w_row0 + kb * UMMA_M);
+                        tma_load_2d_pair_hint(dst, &map_w, leader_addr(bar), 0, w_row0 + kb * UMMA_M, policy);
                     }
                 };
                 const auto fetch_tokens = [&](uint32_t s, int kb) {
