@@ -265,6 +265,15 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
                  : "r"(taddr)
                  : "memory");
 }
+// Asynchronous copies of 4 and 8 bytes into shared memory, and the wait for all of this thread's.
+__device__ __forceinline__ void copy4_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy8_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 constexpr int BK = 32;                     // k block: 32 values = one 128-byte swizzled row (32 x hi, 32 x lo)
@@ -460,6 +469,12 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     __shared__ int s_cnt[MAX_EXPERTS];
     __shared__ int s_beg[MAX_EXPERTS];
     __shared__ short s_order[MAX_EXPERTS];
+    // what the epilogue needs of its tile, per warp: two words per column (row_info of h, later 2^-s and 2^s of g; or log2 of
+    // the squared norm and the output row, later 2^-s and the row), the scores of the mix, 2^-s of the weight rows, the bound
+    __shared__ __align__(16) float2 s_col[EPI_WARPS][C::SLICES * 16];
+    __shared__ float s_mix[EPI == EPI_RESIDUAL ? EPI_WARPS : 1][C::SLICES * 16];
+    __shared__ float s_winv[EPI_WARPS][32];
+    __shared__ int s_bound[EPI_WARPS];
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -714,6 +729,27 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 #pragma unroll
                 for (int c = 0; c < 16; ++c) sum[i][c] = 0.f;
             const int row = q * 32 + lane;      // row of the tile this thread works on
+            const int mb = t.mb * CTAS + (int)rank, m = mb * UMMA_M + row;
+            const int w16 = warp - EPI_WARP0, wm = EPI == EPI_RESIDUAL ? w16 : 0;
+            // requested now, used when the sums are complete
+            copy_async_wait();
+            __syncwarp();                       // the last tile's have landed and are not needed any more
+            if (mb < MB1) {
+                for (int c = lane; c < width && col0 + c < t.n_tok; c += 32) {
+                    const int r = t.row0 + col0 + c;
+                    if (EPI == EPI_GELU_PAIR) {
+                        copy8_async(&s_col[w16][c], args.row_info + r);
+                    } else {
+                        copy4_async(&s_col[w16][c].x, &args.row_info[r].y);
+                        if (args.out_pos) copy4_async(&s_col[w16][c].y, args.out_pos + r);
+                        if (args.mix_score) copy4_async(&s_mix[wm][c], args.mix_score + r);
+                    }
+                }
+                // 2^-s of the weight row (padding rows have one too)
+                copy4_async(&s_winv[w16][lane],
+                            args.w + (size_t)t.slot * args.w_stride + (size_t)MB1 * KB * (UMMA_M * BK) + m);
+                if (lane == 0) copy4_async(&s_bound[w16], args.bound + (size_t)t.slot * args.bound_stride);
+            }
             const size_t block = (size_t)(args.part_cols >> 2) * UMMA_M;   // float4 per block of chunk sums
             float4* const part = item.tail >= 0 ? args.part + ((size_t)item.tail * CTAS + rank) * sched.m * block + row : nullptr;
             auto store_block = [&](int c) {     // sum[][] -> block of chunk c
@@ -760,6 +796,14 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (++acc == nacc) {
                     acc = 0;
                     acc_phase ^= 1;
+                }
+                if (EPI == EPI_RESIDUAL && c == item.c0 && mb < MB1 && mb * UMMA_M + q * 32 < args.M_total) {
+                    // the residual's lines, so that they are in L2 when the sums are complete
+                    copy_async_wait();
+                    for (int x = lane; x < width && col0 + x < t.n_tok; x += 32) {
+                        const int r = args.out_pos ? __float_as_int(s_col[w16][x].y) : t.row0 + col0 + x;
+                        prefetch_l2(args.resid + (size_t)r * (size_t)args.M_total + (size_t)(mb * UMMA_M + q * 32));
+                    }
                 }
                 if (part && (item.c0 > 0 || c + 1 == item.c1)) {
                     store_block(c);
@@ -835,93 +879,91 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     }
                 }
             }
-            const int mb = t.mb * CTAS + (int)rank;
             if (mb >= MB1) continue;
-            const int m = mb * UMMA_M + row;
             const bool m_ok = m < args.M_total;
-            // 2^-s of the weight row (padding rows have one too)
-            const float w_inv = __ldg(args.w + (size_t)t.slot * args.w_stride + (size_t)MB1 * KB * (UMMA_M * BK) + m);
-            const float bound = (float)__ldg(args.bound + (size_t)t.slot * args.bound_stride);
-#pragma unroll
-            for (int i = 0; i < C::SLICES; ++i) {
-                if (16 * i >= width) continue;     // uniform across the warp
-                const int sl0 = col0 + 16 * i;
-                // What belongs to the slice's 16 token columns, one column per lane (lanes 16..31 repeat them),
-                // handed out by shuffle below: 2^-s of the token row, and 2^s of g (GELU_PAIR) or the output row and
-                // the mix coefficient (RESIDUAL).
-                const int lc = sl0 + (lane & 15);
-                const int r = t.row0 + lc;
-                const bool lc_ok = lc < t.n_tok;
-                const float2 info = lc_ok ? __ldg(args.row_info + r) : make_float2(1.f, 0.f);
-                const int g_exp = g_exponent(info.y, bound);
-                const float lane_inv = EPI == EPI_GELU_PAIR ? info.x : exp2_int(-g_exp);
+            copy_async_wait();
+            __syncwarp();
+            const float w_inv = s_winv[w16][lane], bound = (float)s_bound[w16];
+            // the columns' two words, each made by the lane that fetched it
+            for (int c = lane; c < width; c += 32) {
+                const bool ok = col0 + c < t.n_tok;
+                const float2 info = ok ? s_col[w16][c] : make_float2(1.f, 0.f);
                 if (EPI == EPI_GELU_PAIR) {
-                    // Even weight row = wi_0 (a), odd row = wi_1 (b) of the same d_ff index f, so a lane pair holds
-                    // (a, b) of f for all 16 token columns.  The pair splits the columns: the even lane takes the
-                    // even ones, the odd lane the odd ones; one shuffle per column pair hands each lane the half
-                    // it lacks, and every gelu is evaluated once.
-                    const int F = args.M_total >> 1, f = m >> 1;
-                    const int odd = lane & 1;
-                    const float lane_scale = exp2_int(g_exp);
+                    s_col[w16][c] = make_float2(info.x, exp2_int(g_exponent(info.y, bound)));
+                } else {
+                    const int r = ok && args.out_pos ? __float_as_int(info.y) : t.row0 + col0 + c;
+                    s_col[w16][c] = make_float2(exp2_int(-g_exponent(info.x, bound)), __int_as_float(r));
+                    if (args.mix_score && ok) s_mix[wm][c] = mix_alpha(s_mix[wm][c]);
+                }
+            }
+            __syncwarp();
+            if constexpr (EPI == EPI_GELU_PAIR) {
+                // Even weight row = wi_0 (a), odd row = wi_1 (b) of the same d_ff index f, so a lane pair holds (a, b) of f for
+                // all token columns.  The pair splits the columns: the even lane takes the even ones, the odd lane the odd
+                // ones; one shuffle per column pair hands each lane the half it lacks, and every gelu is evaluated once.
+                // Packed plane: neighbouring f (lanes two apart, same column) exchange their halves so that every lane stores
+                // one 32-bit word, even f the pair of hi, odd f the pair of lo.  The plane is zero padded to whole groups of
+                // 32 (weight rows past the matrix are zero, so those values are 0).
+                const int F = args.M_total >> 1, f = m >> 1, odd = lane & 1;
+                const uint32_t pitch = (uint32_t)pack_pitch(F), halves = (f & 1) ? 0x3276u : 0x5410u;
+                uint16_t* const out = reinterpret_cast<uint16_t*>(args.out_pack) + (size_t)(t.row0 + col0 + odd) * pitch +
+                                      (size_t)(f >> 5) * 64 + (f & 31) + ((f & 1) ? 31 : 0);
+                const int end = f < ((F + 31) & ~31) ? min(t.n_tok - col0, width) - odd : 0;    // columns this lane stores
+#pragma unroll
+                for (int i = 0; i < C::SLICES; ++i)
 #pragma unroll
                     for (int c = 0; c < 16; c += 2) {
-                        if (16 * i + c >= width) continue;
-                        const float v0 = unscale(sum[i][c], w_inv, __shfl_sync(0xffffffffu, lane_inv, c));
-                        const float v1 = unscale(sum[i][c + 1], w_inv, __shfl_sync(0xffffffffu, lane_inv, c + 1));
+                        if (16 * i + c >= width) continue;     // uniform across the warp
+                        const float4 col = *reinterpret_cast<const float4*>(&s_col[w16][16 * i + c]);
+                        const float v0 = unscale(sum[i][c], w_inv, col.x), v1 = unscale(sum[i][c + 1], w_inv, col.z);
                         const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
                         const float a = odd ? got : v0, b = odd ? v1 : got;
-                        const float g = gelu_dot_fast(a, b) * __shfl_sync(0xffffffffu, lane_scale, c + odd);
-                        const int col = sl0 + c + odd;
-                        // Packed plane: neighbouring f (lanes two apart, same column) exchange their halves so that
-                        // every lane stores one 32-bit word, even f the pair of hi, odd f the pair of lo.
-                        const uint32_t hl = split_f16(g);
+                        const uint32_t hl = split_f16(gelu_dot_fast(a, b) * (odd ? col.w : col.y));
                         const uint32_t nb = __shfl_xor_sync(0xffffffffu, hl, 2);
-                        // The packed plane is zero padded to whole groups of 32 (weight rows past the matrix are
-                        // zero, so those values are 0).
-                        if (col < t.n_tok && f < ((F + 31) & ~31)) {
-                            uint16_t* gp = reinterpret_cast<uint16_t*>(args.out_pack) +
-                                           (size_t)(t.row0 + col) * pack_pitch(F) + (size_t)(f >> 5) * 64 + (f & 31);
-                            if (!(f & 1)) *reinterpret_cast<uint32_t*>(gp) = __byte_perm(hl, nb, 0x5410);
-                            else *reinterpret_cast<uint32_t*>(gp + 31) = __byte_perm(nb, hl, 0x7632);
+                        if (16 * i + c < end)
+                            *reinterpret_cast<uint32_t*>(out + (size_t)(16 * i + c) * pitch) = __byte_perm(hl, nb, halves);
+                    }
+            } else {
+#pragma unroll
+                for (int i = 0; i < C::SLICES; ++i) {
+                    if (16 * i >= width) continue;     // uniform across the warp
+                    unsigned long long lane_ptr = 0;   // address of the output row of column 16 i + (lane & 15)
+                    if (args.out_row_ptr && 16 * i + (lane & 15) < min(width, t.n_tok - col0))
+                        lane_ptr = args.out_row_ptr[__float_as_int(s_col[w16][16 * i + (lane & 15)].y)];
+                    // The residual values of eight columns are fetched first, all in flight together: issued
+                    // one by one between the stores (which may alias them as far as the compiler knows) each would
+                    // cost a trip to L2, and the next tile's first chunk would wait.
+#pragma unroll
+                    for (int c0 = 0; c0 < 16; c0 += 8) {
+                        if (16 * i + c0 >= width) continue;
+                        const int end = m_ok ? min(t.n_tok - col0, width) - (16 * i + c0) : 0;    // columns of these eight to store
+                        int r[8];
+                        float y[8];
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            r[c] = __float_as_int(s_col[w16][16 * i + c0 + c].y);
+                            y[c] = c < end ? args.resid[(size_t)r[c] * (size_t)args.M_total + (size_t)m] : 0.f;
                         }
-                    }
-                    continue;
-                }
-                const int lane_row = (lc_ok && args.out_pos) ? args.out_pos[r] : r;
-                const float lane_alpha = (args.mix_score && lc_ok) ? mix_alpha(args.mix_score[r]) : 0.f;
-                unsigned long long lane_ptr = 0;
-                if (lc_ok)
-                    lane_ptr = args.out_row_ptr ? args.out_row_ptr[lane_row]
-                                                : (unsigned long long)(args.out + (size_t)lane_row * (size_t)args.M_total);
-                // The residual values of eight columns are fetched first, all in flight together: issued
-                // one by one between the stores (which may alias them as far as the compiler knows) each would
-                // cost a trip to L2 or HBM, and the next tile's first chunk would wait.
 #pragma unroll
-                for (int c0 = 0; c0 < 16; c0 += 8) {
-                    if (16 * i + c0 >= width) continue;
-                    const int end = min(t.n_tok, col0 + width) - (sl0 + c0);    // columns of these eight that are this warp's
-                    float xres[8];
+                        for (int c = 0; c < 8; ++c) {
+                            const float x = y[c];
+                            y[c] = __fadd_rn(x, unscale(sum[i][c0 + c], w_inv, s_col[w16][16 * i + c0 + c].x));
+                            if (args.mix_score) {
+                                const float alpha = s_mix[wm][16 * i + c0 + c];
+                                y[c] = mix_value(alpha, 1.0f - alpha, y[c], x);
+                            }
+                        }
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const int resid_row = __shfl_sync(0xffffffffu, lane_row, c0 + c);
-                        xres[c] = (c < end && m_ok)
-                                      ? args.resid[(size_t)resid_row * (size_t)args.M_total + (size_t)m] : 0.f;
-                    }
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const unsigned long long out_row = __shfl_sync(0xffffffffu, lane_ptr, c0 + c);
-                        const float alpha = __shfl_sync(0xffffffffu, lane_alpha, c0 + c);
-                        const float v = unscale(sum[i][c0 + c], w_inv, __shfl_sync(0xffffffffu, lane_inv, c0 + c));
-                        if (c < end && m_ok) {
-                            const float x = xres[c];
-                            float y = __fadd_rn(x, v);
-                            if (args.mix_score) y = mix_value(alpha, 1.0f - alpha, y, x);
-                            reinterpret_cast<float*>(out_row)[m] = y;
+                        for (int c = 0; c < 8; ++c) {
+                            float* out = args.out + (size_t)r[c] * (size_t)args.M_total;
+                            if (args.out_row_ptr) out = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, lane_ptr, c0 + c));
+                            if (c < end) out[m] = y[c];
                         }
                     }
                 }
             }
         }
+        copy_async_wait();
     } else {
         wait_then_trigger();
     }
@@ -931,7 +973,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     __syncthreads();
     if (s_abort) {
         if (threadIdx.x == 0 && args.status) atomicOr(args.status, STATUS_WAIT_TIMEOUT);
-        // let bulk copies that were already issued land before the shared memory is released
+        // let copies that were already issued land before the shared memory is released
         const unsigned long long t0 = global_ns();
         while (global_ns() - t0 < 200000ull) __nanosleep(1000);
         __syncthreads();
