@@ -36,7 +36,7 @@ int launch_scatter_ln_pack(long long row0, long long T, int D, const float* X, c
 // launch_dispatch (without regions) and one of the two scatters in one kernel, where dispatch_scatter_supported.  gamma is
 // what the scatter takes: with `pack` that of launch_split_expert, else the experts' LayerNorm weights.  early: the launch
 // follows launch_route on this stream.
-bool dispatch_scatter_supported(long long T, int D, int E);
+bool dispatch_scatter_supported(long long T, int D, int E, const float* X, bool pack);
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
                             const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,
                             int* zero, int zero_count, float* rscore, void* h, float* row_info, bool pack, bool early,

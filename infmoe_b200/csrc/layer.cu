@@ -1099,7 +1099,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     // dispatch kernel's limit has to be refused)
     const bool pack = !L->identity && !L->custom && uses_umma(L);   // the GEMM run_ffn picks
     const bool with_scatter = !L->identity && !L->custom && !region_count && dispatch_supported(L->E) &&
-                              dispatch_scatter_supported(T, L->D, L->E);
+                              dispatch_scatter_supported(T, L->D, L->E, d_in, pack);
     int* const zero = w.part_bytes ? buf.part_count : nullptr;
     if (!with_scatter)
         INFMOE_TRY(launch_dispatch(gate_in, T, L->E, pos, count, offset, L->d_status, stream, region_count, region_size,

@@ -152,6 +152,86 @@ scatter_ln_pack_kernel(long long j0, long long T, int D, int vec, const float* _
 // cp.async while the row is on its way, so the output loop never waits for L2.
 // Bound by HBM: reads 4 D and writes 4 D bytes per row (a third less than the two planes it wrote before).
 template <int NV>
+struct RowInRegisters {
+    float4 v[NV];
+    float mean, rstd;
+    static __device__ __forceinline__ int lane() { return threadIdx.x & 31; }
+    __device__ __forceinline__ void fetch(const float* __restrict__ row, int D) {
+        const float4* src = reinterpret_cast<const float4*>(row);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int base = 4 * lane() + 128 * i;
+            v[i] = base < D ? src[base >> 2] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    // LayerNorm weights to shared memory; every lane reads back only what it fetched itself (ln_pack waits for it)
+    static __device__ __forceinline__ void fetch_gamma(float4* s_gamma, const float* __restrict__ gamma, int D) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int base = 4 * lane() + 128 * i;
+            if (base < D) {
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_gamma + (base >> 2));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(gamma + base) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    __device__ __forceinline__ void stats(int D) {
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            if (4 * lane() + 128 * i < D) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v[i].x), v[i].y), v[i].z), v[i].w);
+        mean = __fdiv_rn(warp_xor_sum(s), (float)D);
+        float q = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            if (4 * lane() + 128 * i < D) {
+                float d = __fsub_rn(v[i].x, mean);
+                q = __fmaf_rn(d, d, q);
+                d = __fsub_rn(v[i].y, mean);
+                q = __fmaf_rn(d, d, q);
+                d = __fsub_rn(v[i].z, mean);
+                q = __fmaf_rn(d, d, q);
+                d = __fsub_rn(v[i].w, mean);
+                q = __fmaf_rn(d, d, q);
+            }
+        const float var = __fdiv_rn(warp_xor_sum(q), (float)D);
+        rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, 1e-6f)));
+    }
+    __device__ __forceinline__ void ln_pack(const float4* s_gamma, int D, uint16_t* __restrict__ pack_row, float2* info) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        float top = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int base = 4 * lane() + 128 * i;
+            if (base >= D) continue;
+            const float4 g = s_gamma[base >> 2];
+            v[i].x = ln_apply(v[i].x, mean, rstd, g.x);
+            v[i].y = ln_apply(v[i].y, mean, rstd, g.y);
+            v[i].z = ln_apply(v[i].z, mean, rstd, g.z);
+            v[i].w = ln_apply(v[i].w, mean, rstd, g.w);
+            top = fmaxf(fmaxf(fmaxf(top, fabsf(v[i].x)), fmaxf(fabsf(v[i].y), fabsf(v[i].z))), fabsf(v[i].w));
+        }
+        const int exponent = row_exponent(warp_max(top));
+        const float scale = exp2_int(exponent);
+        const int k_end = (D + 31) & ~31;
+        float squares = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int base = 4 * lane() + 128 * i;
+            if (base >= k_end) continue;
+            const float x[4] = {__fmul_rn(v[i].x, scale), __fmul_rn(v[i].y, scale), __fmul_rn(v[i].z, scale),
+                                __fmul_rn(v[i].w, scale)};     // zeros past the row
+#pragma unroll
+            for (int k = 0; k < 4; ++k) squares = fmaf(x[k], x[k], squares);
+            store_pack4(pack_row, base, x);
+        }
+        squares = warp_xor_sum(squares);
+        if (lane() == 0) *info = token_row_info(exponent, squares);
+    }
+};
+
+template <int NV>
 __global__ void __launch_bounds__(128)
 scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __restrict__ X,
                            const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
@@ -159,82 +239,52 @@ scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __rest
                            uint16_t* __restrict__ h, float2* __restrict__ row_info) {
     pdl_wait();
     pdl_trigger();
-    const int lane = threadIdx.x & 31;
     const long long j = j0 + (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (j >= j0 + T || (valid_rows && j >= *valid_rows)) return;
     extern __shared__ __align__(16) float4 s_gamma_all[];     // [4 warps][NV * 32]
     float4* s_gamma = s_gamma_all + (threadIdx.x >> 5) * (NV * 32);
     const int p = pos[j];
     const int e = gate[p];
-    const float4* src = reinterpret_cast<const float4*>(X + (long long)p * D);
-    const float4* gamma = reinterpret_cast<const float4*>(expert_gamma.of(e));
-    float4 v[NV];
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int base = 4 * lane + 128 * i;
-        v[i] = base < D ? src[base >> 2] : make_float4(0.f, 0.f, 0.f, 0.f);
+    RowInRegisters<NV> row;
+    row.fetch(X + (long long)p * D, D);
+    row.fetch_gamma(s_gamma, expert_gamma.of(e), D);
+    row.stats(D);
+    row.ln_pack(s_gamma, D, h + j * (long long)pack_pitch(D), row_info + j);
+    if ((threadIdx.x & 31) == 0 && rscore && score) rscore[j] = score[p];
+}
+
+// count[] and offset[] of the T gates by one block of THREADS threads, and zero[] cleared on the way.
+template <int THREADS>
+__device__ __forceinline__ void histogram_block(int* hist, int T, int E, const int* __restrict__ gate, int* __restrict__ count,
+                                                int* __restrict__ offset, int* __restrict__ status, int* __restrict__ zero,
+                                                int zero_count) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int e = tid; e <= E; e += THREADS) hist[e] = 0;
+    for (int i = tid; i < zero_count; i += THREADS) zero[i] = 0;
+    __syncthreads();
+    bool bad = false;
+    for (int t = tid; t < T; t += THREADS) {
+        const int e = gate[t];
+        const bool ok = e >= 0 && e < E;
+        bad |= !ok;
+        atomicAdd(&hist[ok ? e : E], 1);
     }
+    if (bad && status) atomicOr(status, STATUS_BAD_GATE);
+    __syncthreads();
+    if (tid < 32) {
+        int carry = 0;
+        for (int e0 = 0; e0 <= E; e0 += 32) {     // exclusive scan, 32 buckets at a time
+            const int e = e0 + lane, c = e <= E ? hist[e] : 0;
+            int incl = c;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int base = 4 * lane + 128 * i;
-        if (base < D) {
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_gamma + (base >> 2));
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(gamma + (base >> 2)) : "memory");
+            for (int off = 1; off < 32; off <<= 1) {
+                const int n = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off) incl += n;
+            }
+            if (e <= E) offset[e] = carry + incl - c;     // offset[E]: tokens that have an expert
+            if (e < E) count[e] = c;
+            carry += __shfl_sync(0xffffffffu, incl, 31);
         }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < NV; ++i)
-        if (4 * lane + 128 * i < D) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v[i].x), v[i].y), v[i].z), v[i].w);
-    const float mean = __fdiv_rn(warp_xor_sum(s), (float)D);
-    float q = 0.f;
-#pragma unroll
-    for (int i = 0; i < NV; ++i)
-        if (4 * lane + 128 * i < D) {
-            float d = __fsub_rn(v[i].x, mean);
-            q = __fmaf_rn(d, d, q);
-            d = __fsub_rn(v[i].y, mean);
-            q = __fmaf_rn(d, d, q);
-            d = __fsub_rn(v[i].z, mean);
-            q = __fmaf_rn(d, d, q);
-            d = __fsub_rn(v[i].w, mean);
-            q = __fmaf_rn(d, d, q);
-        }
-    const float var = __fdiv_rn(warp_xor_sum(q), (float)D);
-    const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, 1e-6f)));
-    uint16_t* pack_row = h + j * (long long)pack_pitch(D);
-    asm volatile("cp.async.wait_group 0;" ::: "memory");   // every lane reads back only what it fetched itself
-    float top = 0.f;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int base = 4 * lane + 128 * i;
-        if (base >= D) continue;
-        const float4 g = s_gamma[base >> 2];
-        v[i].x = ln_apply(v[i].x, mean, rstd, g.x);
-        v[i].y = ln_apply(v[i].y, mean, rstd, g.y);
-        v[i].z = ln_apply(v[i].z, mean, rstd, g.z);
-        v[i].w = ln_apply(v[i].w, mean, rstd, g.w);
-        top = fmaxf(fmaxf(fmaxf(top, fabsf(v[i].x)), fmaxf(fabsf(v[i].y), fabsf(v[i].z))), fabsf(v[i].w));
-    }
-    const int exponent = row_exponent(warp_max(top));
-    const float scale = exp2_int(exponent);
-    const int k_end = (D + 31) & ~31;
-    float squares = 0.f;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int base = 4 * lane + 128 * i;
-        if (base >= k_end) continue;
-        const float x[4] = {__fmul_rn(v[i].x, scale), __fmul_rn(v[i].y, scale), __fmul_rn(v[i].z, scale),
-                            __fmul_rn(v[i].w, scale)};     // zeros past the row
-#pragma unroll
-        for (int k = 0; k < 4; ++k) squares = fmaf(x[k], x[k], squares);
-        store_pack4(pack_row, base, x);
-    }
-    squares = warp_xor_sum(squares);
-    if (lane == 0) {
-        row_info[j] = token_row_info(exponent, squares);
-        if (rscore && score) rscore[j] = score[p];
     }
 }
 
@@ -264,35 +314,8 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
         pdl_wait();
         pdl_trigger();
     }
-    if ((int)blockIdx.x == T) {      // histogram and its exclusive scan, 32 buckets at a time
-        int* hist = reinterpret_cast<int*>(ds_smem);
-        for (int e = tid; e <= E; e += DS_THREADS) hist[e] = 0;
-        for (int i = tid; i < zero_count; i += DS_THREADS) zero[i] = 0;
-        __syncthreads();
-        bool bad = false;
-        for (int t = tid; t < T; t += DS_THREADS) {
-            const int e = gate[t];
-            const bool ok = e >= 0 && e < E;
-            bad |= !ok;
-            atomicAdd(&hist[ok ? e : E], 1);
-        }
-        if (bad && status) atomicOr(status, STATUS_BAD_GATE);
-        __syncthreads();
-        if (warp == 0) {
-            int carry = 0;
-            for (int e0 = 0; e0 <= E; e0 += 32) {
-                const int e = e0 + lane, c = e <= E ? hist[e] : 0;
-                int incl = c;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const int n = __shfl_up_sync(0xffffffffu, incl, off);
-                    if (lane >= off) incl += n;
-                }
-                if (e <= E) offset[e] = carry + incl - c;     // offset[E]: tokens that have an expert
-                if (e < E) count[e] = c;
-                carry += __shfl_sync(0xffffffffu, incl, 31);
-            }
-        }
+    if ((int)blockIdx.x == T) {
+        histogram_block<DS_THREADS>(reinterpret_cast<int*>(ds_smem), T, E, gate, count, offset, status, zero, zero_count);
         return;
     }
     const int t = (int)blockIdx.x;
@@ -391,6 +414,71 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
         squares = warp_xor_sum(squares);
         if (lane == 0) row_info[j] = token_row_info(s, squares);
     }
+}
+
+// The same for more tokens, aligned rows of up to 128 NV floats: eight tokens per block, a warp and its registers for each.
+// The blocks read T / 8 x T gates, from L2, and compare each with eight: key (gate, token) below the own one.  4096
+// tokens are the most it takes: 8 MB and about 1.5 us of comparisons, against a kernel of one cluster between routing and
+// scatter.  Dispatch and scatter, us, each timed by itself: 4096 tokens of 512 floats 12 + 10 -> 19, 1024 floats 11 + 12 -> 21, 2500 tokens
+// of 512 floats 11 + 10 -> 12; in a pass the row's half of it runs under the routing.
+constexpr int DM_THREADS = 256;
+constexpr int DM_TOKENS = DM_THREADS / 32;
+constexpr int DM_MAX_TOKENS = 4096;
+template <int NV>
+__global__ void __launch_bounds__(DM_THREADS)
+dispatch_scatter_reg_kernel(int T, int D, int E, const float* __restrict__ X, const float* __restrict__ score,
+                            const int* __restrict__ gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
+                            int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
+                            int* __restrict__ zero, int zero_count, float* __restrict__ rscore, uint16_t* __restrict__ h,
+                            float2* __restrict__ row_info, int early) {
+    extern __shared__ __align__(16) float4 dm_gamma[];     // [warp][NV * 32]; histogram block: E + 1 words
+    __shared__ int s_before[DM_TOKENS][DM_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int t0 = (int)blockIdx.x * DM_TOKENS, t = t0 + warp;
+    if (t0 >= T) {
+        pdl_wait();
+        pdl_trigger();
+        histogram_block<DM_THREADS>(reinterpret_cast<int*>(dm_gamma), T, E, gate, count, offset, status, zero, zero_count);
+        return;
+    }
+    RowInRegisters<NV> row;
+    if (!early) pdl_wait();
+    row.fetch(X + (size_t)min(t, T - 1) * D, D);
+    row.stats(D);
+    if (early) pdl_wait();
+    pdl_trigger();
+    const auto key = [&](int o) {
+        const int g = gate[o];
+        return (g >= 0 && g < E ? g : E) * DM_MAX_TOKENS + o;
+    };
+    const int own = key(min(t, T - 1)), e = own / DM_MAX_TOKENS;
+    float4* const s_gamma = dm_gamma + warp * (NV * 32);
+    row.fetch_gamma(s_gamma, expert_gamma.of(e < E ? e : 0), D);
+    int keys[DM_TOKENS], before[DM_TOKENS] = {};
+#pragma unroll
+    for (int j = 0; j < DM_TOKENS; ++j) keys[j] = key(min(t0 + j, T - 1));
+#pragma unroll 4
+    for (int o = tid; o < T; o += DM_THREADS) {
+        const int k = key(o);
+#pragma unroll
+        for (int j = 0; j < DM_TOKENS; ++j) before[j] += k < keys[j] ? 1 : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < DM_TOKENS; ++j) {
+        const int n = __reduce_add_sync(0xffffffffu, before[j]);
+        if (lane == 0) s_before[j][warp] = n;
+    }
+    __syncthreads();
+    if (t >= T) return;
+    int j = 0;
+#pragma unroll
+    for (int w = 0; w < DM_THREADS / 32; ++w) j += s_before[warp][w];
+    if (lane == 0) {
+        pos[j] = t;
+        if (e < E && rscore && score) rscore[j] = score[t];
+    }
+    if (e == E) return;              // no expert: nobody reads the row
+    row.ln_pack(s_gamma, D, h + (size_t)j * pack_pitch(D), row_info + j);
 }
 
 // out[pos[j],:] = in[j,:] for the rows below *valid_rows (all rows when valid_rows is NULL)
@@ -803,20 +891,44 @@ int launch_scatter(long long T, int D, const float* X, const float* coeff, const
     return INFMOE_OK;
 }
 
-// Up to 1024 tokens whose row and LayerNorm weight fit into 48 KB of shared memory with the histogram's E + 1 words.
-bool dispatch_scatter_supported(long long T, int D, int E) { return T <= 1024 && D <= 6016 && E < 8192; }
+// Up to 1024 tokens whose row and LayerNorm weight fit into 48 KB of shared memory with the histogram's E + 1 words; up to
+// DM_MAX_TOKENS of aligned rows that eight warps hold in registers.
+bool dispatch_scatter_supported(long long T, int D, int E, const float* X, bool pack) {
+    if (E >= 8192) return false;
+    if (T <= 1024 && D <= 6016) return true;
+    return pack && T <= DM_MAX_TOKENS && D <= 2048 && D % 4 == 0 && aligned16(X);
+}
 
 int launch_dispatch_scatter(long long T, int D, int E, const float* X, const float* score, const int* gate,
                             const float* gamma, size_t gamma_stride, int* pos, int* count, int* offset, int* status,
                             int* zero, int zero_count, float* rscore, void* h, float* row_info, bool pack, bool early,
                             cudaStream_t stream) {
     const int vec = (D % 4 == 0) && (gamma_stride % 4 == 0) && aligned16(X) && aligned16(gamma);
-    size_t smem = 2 * padded_row(D) * sizeof(float);
-    if (smem < sizeof(int) * (size_t)(E + 1)) smem = sizeof(int) * (size_t)(E + 1);
-    auto kern = pack ? dispatch_scatter_kernel<true> : dispatch_scatter_kernel<false>;
-    INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)T + 1, DS_THREADS, smem, 1, stream, (int)T, D, E, vec, X, score, gate,
-                                   ExpertGamma{gamma, gamma_stride}, pos, count, offset, status, zero,
-                                   zero ? zero_count : 0, rscore, h, (float2*)row_info, early ? 1 : 0));
+    const ExpertGamma gammas{gamma, gamma_stride};
+    const size_t hist = sizeof(int) * (size_t)(E + 1);
+    if (!zero) zero_count = 0;
+    if (T <= 1024 && D <= 6016) {
+        size_t smem = 2 * padded_row(D) * sizeof(float);
+        if (smem < hist) smem = hist;
+        auto kern = pack ? dispatch_scatter_kernel<true> : dispatch_scatter_kernel<false>;
+        INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)T + 1, DS_THREADS, smem, 1, stream, (int)T, D, E, vec, X, score, gate,
+                                       gammas, pos, count, offset, status, zero, zero_count, rscore, h, (float2*)row_info,
+                                       early ? 1 : 0));
+    } else {
+        if (!vec || !pack) {
+            set_error("dispatch_scatter: unaligned rows");
+            return INFMOE_ERR_UNSUPPORTED;
+        }
+        const int nv = D <= 1024 ? 8 : 16;
+        size_t smem = (size_t)DM_TOKENS * nv * 512;
+        if (smem < hist) smem = hist;
+        auto kern = nv == 8 ? dispatch_scatter_reg_kernel<8> : dispatch_scatter_reg_kernel<16>;
+        if (smem > 48 * 1024)
+            INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)((T + DM_TOKENS - 1) / DM_TOKENS + 1), DM_THREADS, smem, 1, stream,
+                                       (int)T, D, E, X, score, gate, gammas, pos, count, offset, status, zero, zero_count,
+                                       rscore, (uint16_t*)h, (float2*)row_info, early ? 1 : 0));
+    }
     note_launch();
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

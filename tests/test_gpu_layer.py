@@ -687,6 +687,15 @@ def test_paired_tiles_against_oracle(oracle, D, F):
             assert oracle.rel_l2(out[0][rows], want) <= TOL
 
 
+# From 1025 to 4096 tokens of aligned rows of up to 2048 floats one kernel computes the dispatch metadata and scatters, eight
+# tokens to a block: its lines, a last block of one and of seven tokens, rows that end inside a register and one expert.
+@pytest.mark.parametrize("T,D,E,variant", [(1025, 36, 1, "default"), (1031, 1024, 70, "cpm_2"), (2063, 1028, 9, "default"),
+                                           (4095, 132, 33, "base_layer"), (4096, 2048, 5, "cpm_2"), (4097, 132, 5, "default"),
+                                           (1100, 2052, 6, "default")])
+def test_dispatch_of_a_few_thousand_tokens_alike(oracle, T, D, E, variant):
+    test_few_and_many_tokens_dispatch_alike(oracle, T, D, E, variant)
+
+
 # A tile's columns are shared out evenly over four warps per row quarter, 4 to 48 columns each: every width from 16 to 192,
 # full and with one token less, tiles of one CTA (K < 2048) and of two.
 @pytest.mark.parametrize("D,F", [(260, 516), (2052, 132)])
