@@ -20,8 +20,8 @@
 // ascending k, cut by K alone, so a row's result does not depend on the other rows of the call.
 // Layer of 300 tokens, 6 experts, 510 x 1022: 423 -> 103 us (it was 64 x 64 tiles of scalar loads, one buffer, TF32 head
 // and tail planes added on the fly), 88 with the dispatch and scatter in one kernel, 67 with the clusters: 96 to 192 CTAs of
-// one chain each had left two or three of four schedulers of an SM without a warp, now 384 to 768 are in flight, five to an
-// SM.  The shorter chains also halve the error against 64 bits, 4.6e-7 -> 2.4e-7.
+// one chain each had left two or three of four schedulers of an SM without a warp, now 384 to 768 are in flight, six to an
+// SM (at 80 registers; five, at 96, left 28 of 768 CTAs for a second wave: 66.8 -> 65.6).  The shorter chains also halve the error against 64 bits, 4.6e-7 -> 2.4e-7.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -92,7 +92,7 @@ struct SimtOutput {
 // Grid: clusters of S CTAs, one per (row tile, output tile), row tile major; CTA r of a cluster takes the r-th S-th of the
 // k blocks.
 template <bool DUAL, int RI>
-__global__ void __launch_bounds__(SIMT_THREADS)
+__global__ void __launch_bounds__(SIMT_THREADS, 6)
 ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, int K, const float* __restrict__ act,
                 const float* __restrict__ w, const int* __restrict__ slot_of_expert, const SimtOutput o) {
     cg::cluster_group cluster = cg::this_cluster();
