@@ -909,20 +909,36 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 uint16_t* const out = reinterpret_cast<uint16_t*>(args.out_pack) + (size_t)(t.row0 + col0 + odd) * pitch +
                                       (size_t)(f >> 5) * 64 + (f & 31) + ((f & 1) ? 31 : 0);
                 const int end = f < ((F + 31) & ~31) ? min(t.n_tok - col0, width) - odd : 0;    // columns this lane stores
+                // Eight columns at a time, every step for all of them before the next: one chain of shared-memory read, shuffle,
+                // exponential, reciprocal, conversions, shuffle and store is some 300 cycles, and a store keeps the
+                // compiler from starting the next one above it.
 #pragma unroll
-                for (int i = 0; i < C::SLICES; ++i)
+                for (int i = 0; i < 2 * C::SLICES; ++i) {
+                    if (8 * i >= width) continue;     // uniform across the warp
+                    float* const v = &sum[i >> 1][8 * (i & 1)];
+                    const float4* const cols = reinterpret_cast<const float4*>(&s_col[w16][8 * i]);
+                    float a[4], b[4];
+                    uint32_t hl[4], nb[4];
 #pragma unroll
-                    for (int c = 0; c < 16; c += 2) {
-                        if (16 * i + c >= width) continue;     // uniform across the warp
-                        const float4 col = *reinterpret_cast<const float4*>(&s_col[w16][16 * i + c]);
-                        const float v0 = unscale(sum[i][c], w_inv, col.x), v1 = unscale(sum[i][c + 1], w_inv, col.z);
+                    for (int c = 0; c < 4; ++c) {
+                        const float4 col = cols[c];
+                        const float v0 = unscale(v[2 * c], w_inv, col.x), v1 = unscale(v[2 * c + 1], w_inv, col.z);
                         const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
-                        const float a = odd ? got : v0, b = odd ? v1 : got;
-                        const uint32_t hl = split_f16(gelu_dot_fast(a, b) * (odd ? col.w : col.y));
-                        const uint32_t nb = __shfl_xor_sync(0xffffffffu, hl, 2);
-                        if (16 * i + c < end)
-                            *reinterpret_cast<uint32_t*>(out + (size_t)(16 * i + c) * pitch) = __byte_perm(hl, nb, halves);
+                        a[c] = odd ? got : v0;
+                        b[c] = odd ? v1 : got;
                     }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float4 col = cols[c];
+                        hl[c] = split_f16(gelu_dot_fast(a[c], b[c]) * (odd ? col.w : col.y));
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) nb[c] = __shfl_xor_sync(0xffffffffu, hl[c], 2);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (8 * i + 2 * c < end)
+                            *reinterpret_cast<uint32_t*>(out + (size_t)(8 * i + 2 * c) * pitch) = __byte_perm(hl[c], nb[c], halves);
+                }
             } else {
 #pragma unroll
                 for (int i = 0; i < C::SLICES; ++i) {
