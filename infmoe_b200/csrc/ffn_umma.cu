@@ -396,7 +396,8 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, const int* s_prefix, c
 // walk the (sorted) list forwards in even rounds and backwards in odd ones, so that over two rounds every CTA gets
 // one tile from each end of a stretch.  The R tiles left after the last whole round are cut into chunk units and dealt
 // out evenly when that pays: an uncut tail lasts one tile (m chunks), a cut one R m / G chunks plus storing and
-// re-reading the chunk sums, which is worth about two chunks.
+// re-reading the chunk sums, which is worth about two chunks.  A CTA whose share spans two tiles stores, fences and counts
+// twice, about as long as a chunk and a half; where shares that end with their tile are no longer than that, they are taken.
 struct Item {
     int tile;
     int c0, c1;        // chunks [c0, c1) of the tile
@@ -404,50 +405,67 @@ struct Item {
 };
 template <int CTAS>
 struct Schedule {
-    int total, m, full, R, U, cuts, round, u, hi;
-    __device__ __forceinline__ int first_unit(int b) const { return (int)((long long)b * U / cuts); }
-    __device__ __forceinline__ Schedule(int total_, int KB, const GemmArgs& a) : total(total_) {
-        const int G = (int)gridDim.x / CTAS;
+    int m, full, rounds, round;      // chunks of a tile, whole rounds, whole tiles of this CTA, those it has taken
+    int per, u, hi;                  // chunks of a holder's share where no share spans two tiles, else 0; the units it has left
+    static __device__ __forceinline__ int ctas() { return (int)gridDim.x / CTAS; }
+    static __device__ __forceinline__ int first_unit(int b, int units, int cuts) { return (int)((long long)b * units / cuts); }
+    __device__ __forceinline__ int whole_tile(int r) const {
+        const int b = (int)blockIdx.x / CTAS;
+        return r * ctas() + ((r & 1) ? ctas() - 1 - b : b);
+    }
+    __device__ __forceinline__ Schedule(int total, int KB, const GemmArgs& a) {
+        const int G = ctas(), b = (int)blockIdx.x / CTAS;
         m = (KB + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;
         full = total / G;
-        R = total - full * G;
-        U = R * m;
-        cuts = 0;
-        round = 0;
-        u = hi = 0;
-        if (R > 0 && a.part && (long long)(G - R) * m >= 2ll * G && (long long)R * m * CTAS <= a.part_blocks) {
-            cuts = min(G, U);
-            const int b = (int)blockIdx.x / CTAS;
+        rounds = full;
+        round = per = u = hi = 0;
+        const int R = total - full * G, units = R * m;
+        if (R == 0) return;
+        if (!a.part || (long long)(G - R) * m < 2ll * G || (long long)units * CTAS > a.part_blocks) {
+            if (whole_tile(full) < total) ++rounds;
+            return;
+        }
+        per = (m + G / R - 1) / (G / R);
+        if (2 * per * G <= 2 * units + 3 * G) {
+            const int holders = (m + per - 1) / per;
+            if (b < R * holders) {
+                u = b / holders * m + b % holders * per;
+                hi = min(u + per, (b / holders + 1) * m);
+            }
+        } else {
+            per = 0;
+            const int cuts = min(G, units);
             if (b < cuts) {
-                u = first_unit(b);
-                hi = first_unit(b + 1);
+                u = first_unit(b, units, cuts);
+                hi = first_unit(b + 1, units, cuts);
             }
         }
     }
     __device__ __forceinline__ bool next(Item& it) {
-        const int G = (int)gridDim.x / CTAS, b = (int)blockIdx.x / CTAS;
-        if (round < full || (cuts == 0 && round == full)) {
-            it.tile = round * G + ((round & 1) ? G - 1 - b : b);
+        if (round < rounds) {
+            it.tile = whole_tile(round);
             it.c0 = 0;
             it.c1 = m;
             it.tail = -1;
             ++round;
-            return it.tile < total;
+            return true;
         }
         if (u >= hi) return false;
         const int t = u / m;
-        it.tile = full * G + t;
+        it.tile = full * ctas() + t;
         it.c0 = u - t * m;
         it.c1 = min(m, hi - t * m);
         it.tail = (it.c0 == 0 && it.c1 == m) ? -1 : t;
         u = t * m + it.c1;
         return true;
     }
-    // chunks of cut tile t that its first holder sums up in registers
-    __device__ __forceinline__ int prefix_chunks(int t) const {
+    // chunks of cut tile t, of `total` tiles, that its first holder sums up in registers
+    __device__ __forceinline__ int prefix_chunks(int t, int total) const {
+        if (per) return per;
+        const int units = (total - full * ctas()) * m, cuts = min(ctas(), units);
         const long long u0 = (long long)t * m;
-        const int b = (int)(((u0 + 1) * cuts - 1) / U);     // holder of unit u0
-        return min(m, (int)(first_unit(b + 1) - u0));
+        const int b = (int)(((u0 + 1) * cuts - 1) / units);     // holder of unit u0
+        return min(m, (int)(first_unit(b + 1, units, cuts) - u0));
     }
 };
 
@@ -829,7 +847,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 done = __shfl_sync(0xffffffffu, done, 0);
                 __syncwarp();    // orders lane 0's fence before the other lanes' reads of the sums; a shuffle does not
                 if (done != sched.m) continue;
-                const int first = sched.prefix_chunks(item.tail) - 1;
+                const int first = sched.prefix_chunks(item.tail, s_prefix[args.E]) - 1;
                 if constexpr (C::SLICES == 1) {
                     // few columns: one of the thread's float4 at a time, SUM_FLIGHT chunks of it on their way together (a trip is
                     // 1.4 us; one token through 4096 x 10240 has 40 chunk sums per tile)
