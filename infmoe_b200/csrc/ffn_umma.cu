@@ -665,6 +665,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 };
                 if (!waited) {
                     for (int kb = item.c0 * CHUNK_BLOCKS; kb < kb_end && ahead < STAGES; ++kb, ++ahead) fetch_weights(ahead, kb);
+                    asm volatile("prefetch.tensormap [%0];" ::"l"(map_pk) : "memory");
                     wait();
                 }
                 for (int kb = item.c0 * CHUNK_BLOCKS; kb < kb_end; ++kb, ++it) {

@@ -8,8 +8,10 @@
 
 namespace infmoe {
 
+// constant: no kernel or copy that may still be running writes C or gamma, so they may be read before the stream's earlier
+// kernels have ended.
 int launch_route(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
-                 float* score, int* status, cudaStream_t stream);
+                 float* score, int* status, cudaStream_t stream, bool constant = false);
 int make_f32_row_map(CUtensorMap* map, const void* base, long long K, long long rows, int box_rows);
 int launch_select_top1(long long T, int E, const float* aff, int* gate, float* weight, int* status,
                        cudaStream_t stream);

@@ -363,6 +363,8 @@ int ensure_device(infmoe_layer* L) {
     }
     INFMOE_CUDA_TRY(cudaMalloc(&L->d_status, sizeof(int)));
     INFMOE_CUDA_TRY(cudaMemset(L->d_status, 0, sizeof(int)));
+    // passes on other streams read these without waiting for this one
+    INFMOE_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
     INFMOE_CUDA_TRY(cudaHostAlloc(&L->h_status, sizeof(int), cudaHostAllocDefault));
     *L->h_status = 0;
     INFMOE_CUDA_TRY(cudaHostAlloc(&L->h_count, sizeof(int) * (L->E + 1), cudaHostAllocDefault));
@@ -1092,7 +1094,7 @@ static int layer_run(infmoe_layer* L, const float* d_in, float* d_out, void* d_w
     // 1. routing (plugin/MoELayerPlugin.cc:312-345)
     if (!given_gate)
         INFMOE_TRY(launch_route(d_in, L->d_centroids, L->flags.layernorm_before_score ? L->d_gating_ln : nullptr, T,
-                                L->D, L->E, gate, score, L->d_status, stream));
+                                L->D, L->E, gate, score, L->d_status, stream, true));
     INFMOE_TRY(prof_mark(L, 1, stream));
     // 2. dispatch metadata (:350-352)
     // (with few tokens the scatter kernel of step 3 computes it on the way, except when an expert count past the

@@ -652,7 +652,7 @@ template <bool VEC, bool AHEAD>
 __global__ void __launch_bounds__(RS_THREADS)
 route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, const float* __restrict__ gamma,
                    long long T, int D, int E, int* __restrict__ gate, float* __restrict__ score,
-                   int* __restrict__ status) {
+                   int* __restrict__ status, int constant) {
     cg::cluster_group cluster = cg::this_cluster();
     const int S = (int)cluster.num_blocks(), r = (int)cluster.block_rank();
     extern __shared__ __align__(16) float4 rs_x[];        // [RS_TOKENS][steps * 32] normalised rows, zero past D
@@ -668,9 +668,25 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
     float4* const rs_g = rs_x + RS_TOKENS * chunks;       // AHEAD: LayerNorm weights, then the first centroid of each warp
     float4* const rs_c = rs_g + (1 + warp) * chunks;
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    const int first_e = r * RS_WARPS + warp;
+    const auto fetch_centroid = [&]() {
+        if (first_e < E)
+            for (int i = lane; i < chunks; i += 32) {
+                if (4 * i < D) cp_async16(rs_c + i, C + (long long)first_e * D + 4 * i);
+                else rs_c[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+    };
+    const auto fetch_gamma = [&](int i) {
+        if (gamma && 4 * i < D) cp_async16(rs_g + i, gamma + 4 * i);
+    };
+    // All that the block needs from memory is requested at once, and what no kernel on the stream writes (`constant`) before
+    // the wait.
+    if (AHEAD && constant) {
+        for (int i = tid; i < chunks; i += RS_THREADS) fetch_gamma(i);
+        fetch_centroid();
+    }
     pdl_wait();
     pdl_trigger();
-    // All that the block needs from memory is requested at once.
     for (int i = tid; i < chunks; i += RS_THREADS) {
         const int k = 4 * i;
 #pragma unroll
@@ -679,15 +695,10 @@ route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, con
             if (VEC && t < nt && k < D) cp_async16(rs_x + t * chunks + i, src + k);
             else rs_x[t * chunks + i] = t < nt && k < D ? load_row4(src, k, D, false) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        if (AHEAD && gamma && k < D) cp_async16(rs_g + i, gamma + k);
+        if (AHEAD && !constant) fetch_gamma(i);
     }
     cp_async_commit();
-    const int first_e = r * RS_WARPS + warp;
-    if (AHEAD && first_e < E)
-        for (int i = lane; i < chunks; i += 32) {
-            if (4 * i < D) cp_async16(rs_c + i, C + (long long)first_e * D + 4 * i);
-            else rs_c[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+    if (AHEAD && !constant) fetch_centroid();
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
@@ -1067,7 +1078,7 @@ bool use_small_route(long long T, int D, int E, bool rows, bool vec, bool ln) {
 }
 template <bool VEC>
 int launch_route_small(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
-                       float* score, int* status, cudaStream_t stream) {
+                       float* score, int* status, bool constant, cudaStream_t stream) {
     const int cluster = rs_cluster(E);
     size_t smem = rs_smem(D);
     const long long blocks = (T + RS_TOKENS - 1) / RS_TOKENS * cluster;
@@ -1078,7 +1089,8 @@ int launch_route_small(const float* X, const float* C, const float* gamma, long 
     if (smem > 40 * 1024)
         INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ahead ? RS_AHEAD_SMEM : RS_MAX_SMEM));
     INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)blocks, RS_THREADS, smem,
-                                   (unsigned)cluster, stream, X, C, gamma, T, D, E, gate, score, status));
+                                   (unsigned)cluster, stream, X, C, gamma, T, D, E, gate, score, status,
+                                   constant ? 1 : 0));
     return INFMOE_OK;
 }
 template <int TOKENS, int NV>
@@ -1095,7 +1107,7 @@ int launch_route_rows(const float* X, const float* C, const float* gamma, long l
 }  // namespace
 
 int launch_route(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
-                 float* score, int* status, cudaStream_t stream) {
+                 float* score, int* status, cudaStream_t stream, bool constant) {
     if (T < 0 || D <= 0 || E <= 0 || !X || !C || !gate) {
         set_error("route: bad argument (T=%lld D=%d E=%d)", T, D, E);
         return INFMOE_ERR_INVALID_ARGUMENT;
@@ -1108,7 +1120,7 @@ int launch_route(const float* X, const float* C, const float* gamma, long long T
     const bool rows = route_rows_supported(D, E, vec);
     if (use_small_route(T, D, E, rows, vec, gamma != nullptr)) {
         INFMOE_TRY((vec ? launch_route_small<true> : launch_route_small<false>)(X, C, gamma, T, D, E, gate, score,
-                                                                               status, stream));
+                                                                               status, constant, stream));
     } else if (rows) {
         INFMOE_TRY((D <= 1024 ? launch_route_rows<4, 8> : launch_route_rows<2, 16>)(X, C, gamma, T, D, E, gate, score,
                                                                                     status, stream));
