@@ -45,6 +45,9 @@
 //   warp 1        MMA issuer (and owner of the TMEM allocation): one commit per k block frees the stage, one per chunk
 //                 hands its accumulator to the accumulate warps.  Chunks rotate over as many accumulators as fit into
 //                 TMEM at the width of the launch's widest token tile (2 at 192 columns, 4 at 128, at most 8)
+//   warp 2        walks the schedule and lists the CTA's items (tiles, or parts of cut ones) for the others, up to four ahead
+//   warp 3        fetches what the epilogue needs of an item (scales of its rows, output rows, mix coefficients), and the
+//                 residual's lines into L2
 //   warps 4..19   accumulate + epilogue: tcgen05.ld the chunk (one TMEM lane quarter and a quarter of the
 //                 columns per warp, 4 of 16 to 48 of 192), add into registers; after the last chunk gelu*dot and its
 //                 split (lane pairs exchange a and b by shuffle) or residual add.  The epilogue is a chain of
@@ -265,14 +268,6 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
                  : "r"(taddr)
                  : "memory");
 }
-// Asynchronous copies of 4 and 8 bytes into shared memory, and the wait for all of this thread's.
-__device__ __forceinline__ void copy4_async(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy8_async(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -299,6 +294,8 @@ enum { EPI_GELU_PAIR = 0, EPI_RESIDUAL = 1 };
 
 constexpr int TMA_WARP = 0;
 constexpr int MMA_WARP = 1;                           // issues all MMAs; owns the TMEM allocation
+constexpr int ITEM_WARP = 2;                          // walks the schedule ahead of the others
+constexpr int COLUMN_WARP = 3;                        // fetches what the epilogue needs of each tile
 constexpr int EPI_WARP0 = 4;
 constexpr int EPI_GROUPS = 4;                         // warps per TMEM lane quarter
 constexpr int EPI_WARPS = 4 * EPI_GROUPS;
@@ -358,6 +355,16 @@ struct TokenMaps {
 struct TileInfo {
     int expert, slot, mb, row0, n_tok, n_pad;
 };
+
+// An entry of the list that the item warp writes and the others read: chunks [c0, c1) of a tile (c1 = 0: no more items).
+// tail: index among the cut tiles (-1: this CTA holds the whole tile), prefix: chunks that the tile's first holder sums up;
+// alone: the expert's weights are read by this token tile only.
+struct __align__(16) ListItem {
+    int c0, c1, tail, prefix;
+    int row0, n_tok, n_pad, slot;
+    int mb, alone, unused[2];
+};
+constexpr int ITEM_SLOTS = 4;
 
 template <int NMAX, int STEP>
 __device__ __forceinline__ void chunking(int cnt, int& nch, int& csz) {
@@ -487,12 +494,15 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     __shared__ int s_cnt[MAX_EXPERTS];
     __shared__ int s_beg[MAX_EXPERTS];
     __shared__ short s_order[MAX_EXPERTS];
-    // what the epilogue needs of its tile, per warp: two words per column (row_info of h, later 2^-s and 2^s of g; or log2 of
-    // the squared norm and the output row, later 2^-s and the row), the scores of the mix, 2^-s of the weight rows, the bound
-    __shared__ __align__(16) float2 s_col[EPI_WARPS][C::SLICES * 16];
-    __shared__ float s_mix[EPI == EPI_RESIDUAL ? EPI_WARPS : 1][C::SLICES * 16];
-    __shared__ float s_winv[EPI_WARPS][32];
-    __shared__ int s_bound[EPI_WARPS];
+    // the next items, and what the epilogue needs of each: two words per column (2^-s of the token row and 2^s of g, or 2^-s of
+    // the row of g and the output row), the mix coefficients, 2^-s of the weight rows
+    __shared__ ListItem s_item[ITEM_SLOTS];
+    __shared__ __align__(16) float2 s_col[ITEM_SLOTS][NMAX];
+    __shared__ float s_mix[EPI == EPI_RESIDUAL ? ITEM_SLOTS : 1][NMAX];
+    __shared__ __align__(16) float s_winv[ITEM_SLOTS][UMMA_M];
+    __shared__ __align__(8) uint64_t s_item_full[ITEM_SLOTS];   // item warp -> all others
+    __shared__ __align__(8) uint64_t s_col_full[ITEM_SLOTS];    // column warp -> accumulate warps
+    __shared__ __align__(8) uint64_t s_item_empty[ITEM_SLOTS];  // all others -> item warp
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -511,6 +521,11 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         for (int b = 0; b < C::MAX_ACC; ++b) {
             mbar_init(smem_u32(&s_acc_full[b]), 1);
             mbar_init(smem_u32(&s_acc_empty[b]), EPI_WARPS * CTAS);
+        }
+        for (int i = 0; i < ITEM_SLOTS; ++i) {      // an item's readers: producer, column warp, issuer, accumulate warps
+            mbar_init(smem_u32(&s_item_full[i]), 1);
+            mbar_init(smem_u32(&s_col_full[i]), 32);
+            mbar_init(smem_u32(&s_item_empty[i]), 2 + (rank == 0 ? 1 : 0) + EPI_WARPS);
         }
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -615,8 +630,17 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     // as many accumulators as fit beside one another at the width of the widest token tile
     const uint32_t acc_stride = (uint32_t)s_widest, nacc = min((uint32_t)C::MAX_ACC, (uint32_t)TMEM_COLS / acc_stride);
     volatile int* abort_flag = &s_abort;
-    Schedule<CTAS> sched(s_prefix[args.E], KB, args);
-    Item item;
+    const int m_chunks = (KB + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;
+    // A reader's place in the list of items.
+    struct Place {
+        uint32_t slot = 0, phase = 0;
+        __device__ __forceinline__ void advance() {
+            if (++slot == ITEM_SLOTS) {
+                slot = 0;
+                phase ^= 1;
+            }
+        }
+    };
 
     // every thread of an early first GEMM passes here once, its producer when it has fetched its first weights
     const auto wait_then_trigger = [&]() {
@@ -636,8 +660,11 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 wait_then_trigger();
                 waited = true;
             };
-            while (ok && sched.next(item) && !*abort_flag) {
-                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, s_beg, s_cnt, args);
+            for (Place at; ok; at.advance()) {
+                if (!mbar_wait(smem_u32(&s_item_full[at.slot]), at.phase, abort_flag)) break;
+                const ListItem t = s_item[at.slot];
+                if (t.c1 == 0) break;
+                mbar_arrive(smem_u32(&s_item_empty[at.slot]));
                 // a box of n_pad token rows (rows past the chunk's tokens belong to the next expert or are
                 // zero-filled past the end; they only feed accumulator columns that are never stored)
                 const int n_own = t.n_pad / CTAS;
@@ -646,8 +673,8 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 // a second CTA past the last weight block loads that block again and drops the result
                 const int mb = min(t.mb * CTAS + (int)rank, MB1 - 1);
                 const int w_row0 = (int)(args.w_stride / BK) * t.slot + mb * KB * UMMA_M;
-                const int kb_end = min(KB, item.c1 * CHUNK_BLOCKS);
-                const uint64_t policy = s_cnt[t.expert] <= NMAX ? evict_first : evict_normal;    // one token chunk: read once
+                const int kb_begin = t.c0 * CHUNK_BLOCKS, kb_end = min(KB, t.c1 * CHUNK_BLOCKS);
+                const uint64_t policy = t.alone ? evict_first : evict_normal;
                 const auto fetch_weights = [&](uint32_t s, int kb) {
                     const uint32_t bar = smem_u32(&s_full[s]), dst = ring + s * C::STAGE;
                     if (CTAS == 1) {
@@ -664,11 +691,11 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     else tma_load_2d_pair(dst, map_pk, leader_addr(bar), kb * 2 * BK, t.row0 + (int)rank * n_own);
                 };
                 if (!waited) {
-                    for (int kb = item.c0 * CHUNK_BLOCKS; kb < kb_end && ahead < STAGES; ++kb, ++ahead) fetch_weights(ahead, kb);
+                    for (int kb = kb_begin; kb < kb_end && ahead < STAGES; ++kb, ++ahead) fetch_weights(ahead, kb);
                     asm volatile("prefetch.tensormap [%0];" ::"l"(map_pk) : "memory");
                     wait();
                 }
-                for (int kb = item.c0 * CHUNK_BLOCKS; kb < kb_end; ++kb, ++it) {
+                for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
                     const uint32_t s = it % STAGES;
                     if (it >= ahead) {
                         if (!mbar_wait(smem_u32(&s_empty[s]), ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
@@ -695,10 +722,13 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             };
             uint32_t it = 0, acc = 0, acc_phase = 0;
             bool ok = true;
-            while (ok && sched.next(item) && !*abort_flag) {
-                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, s_beg, s_cnt, args);
-                const uint32_t idesc = make_idesc(UMMA_M * CTAS, t.n_pad);
-                for (int c = item.c0; ok && c < item.c1; ++c) {
+            for (Place at; ok; at.advance()) {
+                if (!mbar_wait(smem_u32(&s_item_full[at.slot]), at.phase, abort_flag)) break;
+                const int c0 = s_item[at.slot].c0, c1 = s_item[at.slot].c1;
+                const uint32_t idesc = make_idesc(UMMA_M * CTAS, s_item[at.slot].n_pad);
+                if (c1 == 0) break;
+                mbar_arrive(smem_u32(&s_item_empty[at.slot]));
+                for (int c = c0; ok && c < c1; ++c) {
                     const uint32_t d = tmem_base + acc * acc_stride;
                     if (!mbar_wait(smem_u32(&s_acc_empty[acc]), acc_phase ^ 1, abort_flag)) { ok = false; break; }
                     const int kb0 = c * CHUNK_BLOCKS, kb_end = min(KB, kb0 + CHUNK_BLOCKS);
@@ -739,8 +769,15 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         bool ok = true;
         if (EPI == EPI_RESIDUAL) pdl_wait();
         wait_then_trigger();
-        while (ok && sched.next(item) && !*abort_flag) {
-            const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, s_beg, s_cnt, args);
+        for (Place at; ok; at.advance()) {
+            // the warp stays converged for the .aligned TMEM instructions, also when a wait is abandoned
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_item_full[at.slot]), at.phase, abort_flag))) break;
+            const ListItem t = s_item[at.slot];
+            if (t.c1 == 0) break;
+            const auto done_with_item = [&]() {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&s_item_empty[at.slot]));
+            };
             const int width = t.n_pad / EPI_GROUPS, col0 = group * width;    // this warp's columns; a multiple of 4
             float sum[C::SLICES][16];
 #pragma unroll
@@ -749,28 +786,8 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int c = 0; c < 16; ++c) sum[i][c] = 0.f;
             const int row = q * 32 + lane;      // row of the tile this thread works on
             const int mb = t.mb * CTAS + (int)rank, m = mb * UMMA_M + row;
-            const int w16 = warp - EPI_WARP0, wm = EPI == EPI_RESIDUAL ? w16 : 0;
-            // requested now, used when the sums are complete
-            copy_async_wait();
-            __syncwarp();                       // the last tile's have landed and are not needed any more
-            if (mb < MB1) {
-                for (int c = lane; c < width && col0 + c < t.n_tok; c += 32) {
-                    const int r = t.row0 + col0 + c;
-                    if (EPI == EPI_GELU_PAIR) {
-                        copy8_async(&s_col[w16][c], args.row_info + r);
-                    } else {
-                        copy4_async(&s_col[w16][c].x, &args.row_info[r].y);
-                        if (args.out_pos) copy4_async(&s_col[w16][c].y, args.out_pos + r);
-                        if (args.mix_score) copy4_async(&s_mix[wm][c], args.mix_score + r);
-                    }
-                }
-                // 2^-s of the weight row (padding rows have one too)
-                copy4_async(&s_winv[w16][lane],
-                            args.w + (size_t)t.slot * args.w_stride + (size_t)MB1 * KB * (UMMA_M * BK) + m);
-                if (lane == 0) copy4_async(&s_bound[w16], args.bound + (size_t)t.slot * args.bound_stride);
-            }
             const size_t block = (size_t)(args.part_cols >> 2) * UMMA_M;   // float4 per block of chunk sums
-            float4* const part = item.tail >= 0 ? args.part + ((size_t)item.tail * CTAS + rank) * sched.m * block + row : nullptr;
+            float4* const part = t.tail >= 0 ? args.part + ((size_t)t.tail * CTAS + rank) * m_chunks * block + row : nullptr;
             auto store_block = [&](int c) {     // sum[][] -> block of chunk c
 #pragma unroll
                 for (int i = 0; i < C::SLICES; ++i)
@@ -781,8 +798,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                                make_float4(sum[i][4 * v], sum[i][4 * v + 1], sum[i][4 * v + 2], sum[i][4 * v + 3]));
                     }
             };
-            for (int c = item.c0; c < item.c1; ++c) {
-                // the warp stays converged for the .aligned TMEM instructions, also when a wait is abandoned
+            for (int c = t.c0; c < t.c1; ++c) {
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_acc_full[acc]), acc_phase, abort_flag))) {
                     ok = false;
                     break;
@@ -816,15 +832,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     acc = 0;
                     acc_phase ^= 1;
                 }
-                if (EPI == EPI_RESIDUAL && c == item.c0 && mb < MB1 && mb * UMMA_M + q * 32 < args.M_total) {
-                    // the residual's lines, so that they are in L2 when the sums are complete
-                    copy_async_wait();
-                    for (int x = lane; x < width && col0 + x < t.n_tok; x += 32) {
-                        const int r = args.out_pos ? __float_as_int(s_col[w16][x].y) : t.row0 + col0 + x;
-                        prefetch_l2(args.resid + (size_t)r * (size_t)args.M_total + (size_t)(mb * UMMA_M + q * 32));
-                    }
-                }
-                if (part && (item.c0 > 0 || c + 1 == item.c1)) {
+                if (part && (t.c0 > 0 || c + 1 == t.c1)) {
                     store_block(c);
 #pragma unroll
                     for (int i = 0; i < C::SLICES; ++i)
@@ -839,16 +847,19 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 __threadfence();
                 __syncwarp();
                 int done = 0;
-                int* const counter = args.part_count + (item.tail * CTAS + rank) * EPI_WARPS + (warp - EPI_WARP0);
+                int* const counter = args.part_count + (t.tail * CTAS + rank) * EPI_WARPS + (warp - EPI_WARP0);
                 if (lane == 0) {
-                    done = atomicAdd(counter, item.c1 - item.c0) + item.c1 - item.c0;
-                    if (done == sched.m) *counter = 0;    // everybody has arrived; ready for the next launch
+                    done = atomicAdd(counter, t.c1 - t.c0) + t.c1 - t.c0;
+                    if (done == m_chunks) *counter = 0;    // everybody has arrived; ready for the next launch
                     __threadfence();
                 }
                 done = __shfl_sync(0xffffffffu, done, 0);
                 __syncwarp();    // orders lane 0's fence before the other lanes' reads of the sums; a shuffle does not
-                if (done != sched.m) continue;
-                const int first = sched.prefix_chunks(item.tail, s_prefix[args.E]) - 1;
+                if (done != m_chunks) {
+                    done_with_item();
+                    continue;
+                }
+                const int first = t.prefix - 1;
                 if constexpr (C::SLICES == 1) {
                     // few columns: one of the thread's float4 at a time, SUM_FLIGHT chunks of it on their way together (a trip is
                     // 1.4 us; one token through 4096 x 10240 has 40 chunk sums per tile)
@@ -858,14 +869,14 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         const float4* src = part + (size_t)((col0 >> 2) + v) * UMMA_M;
                         float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
-                        for (int c0 = first; c0 < sched.m; c0 += SUM_FLIGHT) {
+                        for (int c0 = first; c0 < m_chunks; c0 += SUM_FLIGHT) {
                             float4 x[SUM_FLIGHT];
 #pragma unroll
                             for (int c = 0; c < SUM_FLIGHT; ++c)
-                                if (c0 + c < sched.m) x[c] = __ldcg(src + (c0 + c) * block);
+                                if (c0 + c < m_chunks) x[c] = __ldcg(src + (c0 + c) * block);
 #pragma unroll
                             for (int c = 0; c < SUM_FLIGHT; ++c) {
-                                if (c0 + c >= sched.m) break;
+                                if (c0 + c >= m_chunks) break;
                                 y.x = __fadd_rn(y.x, x[c].x);
                                 y.y = __fadd_rn(y.y, x[c].y);
                                 y.z = __fadd_rn(y.z, x[c].z);
@@ -884,7 +895,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         if (16 * i >= width) continue;
                         const float4* src = part + (size_t)((col0 >> 2) + 4 * i) * UMMA_M;
 #pragma unroll 2
-                        for (int c = first; c < sched.m; ++c) {
+                        for (int c = first; c < m_chunks; ++c) {
 #pragma unroll
                             for (int v = 0; v < 4; ++v) {
                                 if (16 * i + 4 * v >= width) continue;
@@ -898,24 +909,15 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     }
                 }
             }
-            if (mb >= MB1) continue;
-            const bool m_ok = m < args.M_total;
-            copy_async_wait();
-            __syncwarp();
-            const float w_inv = s_winv[w16][lane], bound = (float)s_bound[w16];
-            // the columns' two words, each made by the lane that fetched it
-            for (int c = lane; c < width; c += 32) {
-                const bool ok = col0 + c < t.n_tok;
-                const float2 info = ok ? s_col[w16][c] : make_float2(1.f, 0.f);
-                if (EPI == EPI_GELU_PAIR) {
-                    s_col[w16][c] = make_float2(info.x, exp2_int(g_exponent(info.y, bound)));
-                } else {
-                    const int r = ok && args.out_pos ? __float_as_int(info.y) : t.row0 + col0 + c;
-                    s_col[w16][c] = make_float2(exp2_int(-g_exponent(info.x, bound)), __int_as_float(r));
-                    if (args.mix_score && ok) s_mix[wm][c] = mix_alpha(s_mix[wm][c]);
-                }
+            if (mb >= MB1) {
+                done_with_item();
+                continue;
             }
-            __syncwarp();
+            const bool m_ok = m < args.M_total;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_col_full[at.slot]), at.phase, abort_flag))) break;
+            const float w_inv = s_winv[at.slot][row];
+            const float2* const s_tab = &s_col[at.slot][col0];      // this warp's columns
+            const float* const s_alpha = &s_mix[EPI == EPI_RESIDUAL ? at.slot : 0][col0];
             if constexpr (EPI == EPI_GELU_PAIR) {
                 // Even weight row = wi_0 (a), odd row = wi_1 (b) of the same d_ff index f, so a lane pair holds (a, b) of f for
                 // all token columns.  The pair splits the columns: the even lane takes the even ones, the odd lane the odd
@@ -935,7 +937,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int i = 0; i < 2 * C::SLICES; ++i) {
                     if (8 * i >= width) continue;     // uniform across the warp
                     float* const v = &sum[i >> 1][8 * (i & 1)];
-                    const float4* const cols = reinterpret_cast<const float4*>(&s_col[w16][8 * i]);
+                    const float4* const cols = reinterpret_cast<const float4*>(s_tab + 8 * i);
                     float a[4], b[4];
                     uint32_t hl[4], nb[4];
 #pragma unroll
@@ -964,7 +966,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     if (16 * i >= width) continue;     // uniform across the warp
                     unsigned long long lane_ptr = 0;   // address of the output row of column 16 i + (lane & 15)
                     if (args.out_row_ptr && 16 * i + (lane & 15) < min(width, t.n_tok - col0))
-                        lane_ptr = args.out_row_ptr[__float_as_int(s_col[w16][16 * i + (lane & 15)].y)];
+                        lane_ptr = args.out_row_ptr[__float_as_int(s_tab[16 * i + (lane & 15)].y)];
                     // The residual values of eight columns are fetched first, all in flight together: issued
                     // one by one between the stores (which may alias them as far as the compiler knows) each would
                     // cost a trip to L2, and the next tile's first chunk would wait.
@@ -976,15 +978,15 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         float y[8];
 #pragma unroll
                         for (int c = 0; c < 8; ++c) {
-                            r[c] = __float_as_int(s_col[w16][16 * i + c0 + c].y);
+                            r[c] = __float_as_int(s_tab[16 * i + c0 + c].y);
                             y[c] = c < end ? args.resid[(size_t)r[c] * (size_t)args.M_total + (size_t)m] : 0.f;
                         }
 #pragma unroll
                         for (int c = 0; c < 8; ++c) {
                             const float x = y[c];
-                            y[c] = __fadd_rn(x, unscale(sum[i][c0 + c], w_inv, s_col[w16][16 * i + c0 + c].x));
+                            y[c] = __fadd_rn(x, unscale(sum[i][c0 + c], w_inv, s_tab[16 * i + c0 + c].x));
                             if (args.mix_score) {
-                                const float alpha = s_mix[wm][16 * i + c0 + c];
+                                const float alpha = s_alpha[16 * i + c0 + c];
                                 y[c] = mix_value(alpha, 1.0f - alpha, y[c], x);
                             }
                         }
@@ -997,10 +999,78 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     }
                 }
             }
+            done_with_item();
         }
-        copy_async_wait();
-    } else {
+    } else if (warp == ITEM_WARP) {
+        // ================= list of items =================
+        // The schedule and the place of a tile (searches, divisions) take one to two thousand cycles, and every role took them
+        // at each tile, the issuer and the accumulate warps while nothing else went on in their part.
+        Schedule<CTAS> sched(s_prefix[args.E], KB, args);
+        Place at;
+        bool more = true, first = true;
+        while (more) {
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_item_empty[at.slot]), at.phase ^ 1, abort_flag))) break;
+            Item item;
+            more = sched.next(item);
+            ListItem e = {};
+            if (more) {
+                const TileInfo t = decode_tile<NMAX, C::N_STEP>(item.tile, s_prefix, s_order, s_beg, s_cnt, args);
+                e.c0 = item.c0;
+                e.c1 = item.c1;
+                e.tail = item.tail;
+                e.prefix = item.tail >= 0 ? sched.prefix_chunks(item.tail, s_prefix[args.E]) : 0;
+                e.row0 = t.row0;
+                e.n_tok = t.n_tok;
+                e.n_pad = t.n_pad;
+                e.slot = t.slot;
+                e.mb = t.mb;
+                e.alone = s_cnt[t.expert] <= NMAX ? 1 : 0;
+            }
+            if (lane == 0) {
+                s_item[at.slot] = e;
+                mbar_arrive(smem_u32(&s_item_full[at.slot]));
+            }
+            __syncwarp();
+            at.advance();
+            if (first) wait_then_trigger();
+            first = false;
+        }
+    } else if (warp == COLUMN_WARP) {
+        // ================= columns of the items =================
+        if (EPI == EPI_RESIDUAL) pdl_wait();
         wait_then_trigger();
+        for (Place at;; at.advance()) {
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_item_full[at.slot]), at.phase, abort_flag))) break;
+            const ListItem t = s_item[at.slot];
+            if (t.c1 == 0) break;
+            const int mb = t.mb * CTAS + (int)rank;
+            if (mb < MB1) {
+                // 2^-s of the weight rows (padding rows have one too)
+                const float* const scales = args.w + (size_t)t.slot * args.w_stride + (size_t)MB1 * KB * (UMMA_M * BK);
+                const float4 inv = __ldg(reinterpret_cast<const float4*>(scales + mb * UMMA_M) + lane);
+                const float bound = (float)__ldg(args.bound + (size_t)t.slot * args.bound_stride);
+                for (int c = lane; c < t.n_pad; c += 32) {
+                    const bool ok = c < t.n_tok;
+                    const float2 info = ok ? __ldg(args.row_info + t.row0 + c) : make_float2(1.f, 0.f);
+                    const int g_exp = g_exponent(info.y, bound);
+                    if (EPI == EPI_GELU_PAIR) {
+                        s_col[at.slot][c] = make_float2(info.x, exp2_int(g_exp));
+                    } else {
+                        const int r = ok && args.out_pos ? __ldg(args.out_pos + t.row0 + c) : t.row0 + c;
+                        s_col[at.slot][c] = make_float2(exp2_int(-g_exp), __int_as_float(r));
+                        if (args.mix_score && ok) s_mix[EPI == EPI_RESIDUAL ? at.slot : 0][c] = mix_alpha(__ldg(args.mix_score + t.row0 + c));
+                        // the residual's lines, so that they are in L2 when the sums are complete
+                        if (ok)
+                            for (int x = mb * UMMA_M; x < min(args.M_total, (mb + 1) * UMMA_M); x += 32)
+                                prefetch_l2(args.resid + (size_t)r * (size_t)args.M_total + (size_t)x);
+                    }
+                }
+                reinterpret_cast<float4*>(s_winv[at.slot])[lane] = inv;
+            }
+            mbar_arrive(smem_u32(&s_col_full[at.slot]));
+            __syncwarp();      // the slot is used again only after this phase of its columns, also where nobody waits for them
+            if (lane == 0) mbar_arrive(smem_u32(&s_item_empty[at.slot]));
+        }
     }
 
     // ---- teardown ---------------------------------------------------------------------------
@@ -1101,7 +1171,7 @@ template <int EPI, int NMAX, int STAGES, int CTAS>
 int launch_one(GemmArgs args, long long T, int slots, const void* tokens, size_t part_bytes, int num_ctas,
                cudaStream_t stream) {
     using C = Cfg<NMAX, STAGES, CTAS>;
-    static_assert(C::SMEM + 16384 <= 227 * 1024, "shared-memory ring too large");
+    static_assert(C::SMEM + 26 * 1024 <= 227 * 1024, "shared-memory ring too large");
     static_assert(NMAX / CTAS <= 16 * TOKEN_BOXES, "a token tile needs a tensor map of its height");
     args.part_cols = (int)(T < NMAX ? (T + C::N_STEP - 1) / C::N_STEP * C::N_STEP : NMAX);
     const size_t blocks = part_bytes / ((size_t)args.part_cols * UMMA_M * sizeof(float));
