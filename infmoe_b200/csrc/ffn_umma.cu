@@ -46,8 +46,7 @@
 //                 hands its accumulator to the accumulate warps.  Chunks rotate over as many accumulators as fit into
 //                 TMEM at the width of the launch's widest token tile (2 at 192 columns, 4 at 128, at most 8)
 //   warp 2        walks the schedule and lists the CTA's items (tiles, or parts of cut ones) for the others, up to four ahead
-//   warp 3        fetches what the epilogue needs of an item (scales of its rows, output rows, mix coefficients), and the
-//                 residual's lines into L2
+//   warp 3        fetches what the epilogue needs of an item (scales of its rows, output rows, mix coefficients)
 //   warps 4..19   accumulate + epilogue: tcgen05.ld the chunk (one TMEM lane quarter and a quarter of the
 //                 columns per warp, 4 of 16 to 48 of 192), add into registers; after the last chunk gelu*dot and its
 //                 split (lane pairs exchange a and b by shuffle) or residual add.  The epilogue is a chain of
@@ -268,7 +267,6 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
                  : "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 constexpr int BK = 32;                     // k block: 32 values = one 128-byte swizzled row (32 x hi, 32 x lo)
@@ -302,7 +300,7 @@ constexpr int EPI_WARPS = 4 * EPI_GROUPS;
 constexpr int GEMM_THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
 constexpr int TMEM_COLS = 512;
 constexpr int CHUNK_BLOCKS = 8;                       // k blocks (of 6 MMAs) an accumulator takes between two drains
-constexpr int SUM_FLIGHT = 10;                        // chunk sums a thread fetches at a time (narrow tiles)
+constexpr int SUM_FLIGHT = 8;                         // chunk sums a thread fetches at a time (narrow tiles)
 constexpr int W_TILE = UMMA_M * ROW_BYTES;            // 16 KB of weights per k block
 
 template <int NMAX, int STAGES, int CTAS>
@@ -772,7 +770,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         for (Place at; ok; at.advance()) {
             // the warp stays converged for the .aligned TMEM instructions, also when a wait is abandoned
             if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_item_full[at.slot]), at.phase, abort_flag))) break;
-            const ListItem t = s_item[at.slot];
+            const ListItem& t = s_item[at.slot];     // read where it is used: a copy would take registers from the sums
             if (t.c1 == 0) break;
             const auto done_with_item = [&]() {
                 __syncwarp();
@@ -786,15 +784,16 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int c = 0; c < 16; ++c) sum[i][c] = 0.f;
             const int row = q * 32 + lane;      // row of the tile this thread works on
             const int mb = t.mb * CTAS + (int)rank, m = mb * UMMA_M + row;
-            const size_t block = (size_t)(args.part_cols >> 2) * UMMA_M;   // float4 per block of chunk sums
-            float4* const part = t.tail >= 0 ? args.part + ((size_t)t.tail * CTAS + rank) * m_chunks * block + row : nullptr;
+            const int block = (args.part_cols >> 2) * UMMA_M;   // float4 per block of chunk sums
+            const auto part_of_tile = [&]() { return args.part + ((size_t)t.tail * CTAS + rank) * m_chunks * (size_t)block + row; };
             auto store_block = [&](int c) {     // sum[][] -> block of chunk c
+                float4* const dst = part_of_tile() + (size_t)c * block;
 #pragma unroll
                 for (int i = 0; i < C::SLICES; ++i)
 #pragma unroll
                     for (int v = 0; v < 4; ++v) {
                         if (16 * i + 4 * v >= width) continue;
-                        __stcg(part + c * block + (size_t)((col0 >> 2) + 4 * i + v) * UMMA_M,
+                        __stcg(dst + ((col0 >> 2) + 4 * i + v) * UMMA_M,
                                make_float4(sum[i][4 * v], sum[i][4 * v + 1], sum[i][4 * v + 2], sum[i][4 * v + 3]));
                     }
             };
@@ -832,7 +831,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     acc = 0;
                     acc_phase ^= 1;
                 }
-                if (part && (t.c0 > 0 || c + 1 == t.c1)) {
+                if (t.tail >= 0 && (t.c0 > 0 || c + 1 == t.c1)) {
                     store_block(c);
 #pragma unroll
                     for (int i = 0; i < C::SLICES; ++i)
@@ -841,7 +840,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 }
             }
             if (!ok) break;
-            if (part) {
+            if (t.tail >= 0) {
                 // Each warp of the CTAs that share a tile owns the same rows and columns of it; the last of them to
                 // arrive here finishes them.
                 __threadfence();
@@ -862,18 +861,19 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const int first = t.prefix - 1;
                 if constexpr (C::SLICES == 1) {
                     // few columns: one of the thread's float4 at a time, SUM_FLIGHT chunks of it on their way together (a trip is
-                    // 1.4 us; one token through 4096 x 10240 has 40 chunk sums per tile)
+                    // 1.4 us; one token through 4096 x 10240 has 40 chunk sums per tile).  Eight: ten spill, which every drain pays
+                    // for (decode of 8 tokens 533 -> 547 us, 128 tokens 11 x 512 x 1408 42.2 -> 45.0)
 #pragma unroll
                     for (int v = 0; v < 4; ++v) {
                         if (4 * v >= width) continue;
-                        const float4* src = part + (size_t)((col0 >> 2) + v) * UMMA_M;
+                        const float4* src = part_of_tile() + ((col0 >> 2) + v) * UMMA_M;
                         float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
                         for (int c0 = first; c0 < m_chunks; c0 += SUM_FLIGHT) {
                             float4 x[SUM_FLIGHT];
 #pragma unroll
                             for (int c = 0; c < SUM_FLIGHT; ++c)
-                                if (c0 + c < m_chunks) x[c] = __ldcg(src + (c0 + c) * block);
+                                if (c0 + c < m_chunks) x[c] = __ldcg(src + (size_t)(c0 + c) * block);
 #pragma unroll
                             for (int c = 0; c < SUM_FLIGHT; ++c) {
                                 if (c0 + c >= m_chunks) break;
@@ -893,13 +893,13 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 #pragma unroll
                     for (int i = 0; i < C::SLICES; ++i) {
                         if (16 * i >= width) continue;
-                        const float4* src = part + (size_t)((col0 >> 2) + 4 * i) * UMMA_M;
+                        const float4* src = part_of_tile() + ((col0 >> 2) + 4 * i) * UMMA_M;
 #pragma unroll 2
                         for (int c = first; c < m_chunks; ++c) {
 #pragma unroll
                             for (int v = 0; v < 4; ++v) {
                                 if (16 * i + 4 * v >= width) continue;
-                                const float4 x = __ldcg(src + c * block + (size_t)v * UMMA_M);
+                                const float4 x = __ldcg(src + (size_t)c * block + v * UMMA_M);
                                 sum[i][4 * v] = __fadd_rn(sum[i][4 * v], x.x);
                                 sum[i][4 * v + 1] = __fadd_rn(sum[i][4 * v + 1], x.y);
                                 sum[i][4 * v + 2] = __fadd_rn(sum[i][4 * v + 2], x.z);
@@ -1059,10 +1059,6 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         const int r = ok && args.out_pos ? __ldg(args.out_pos + t.row0 + c) : t.row0 + c;
                         s_col[at.slot][c] = make_float2(exp2_int(-g_exp), __int_as_float(r));
                         if (args.mix_score && ok) s_mix[EPI == EPI_RESIDUAL ? at.slot : 0][c] = mix_alpha(__ldg(args.mix_score + t.row0 + c));
-                        // the residual's lines, so that they are in L2 when the sums are complete
-                        if (ok)
-                            for (int x = mb * UMMA_M; x < min(args.M_total, (mb + 1) * UMMA_M); x += 32)
-                                prefetch_l2(args.resid + (size_t)r * (size_t)args.M_total + (size_t)x);
                     }
                 }
                 reinterpret_cast<float4*>(s_winv[at.slot])[lane] = inv;
