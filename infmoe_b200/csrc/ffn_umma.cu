@@ -557,9 +557,13 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     if (EPI == EPI_GELU_PAIR && args.gate) {
         for (int e = threadIdx.x; e < args.E; e += GEMM_THREADS) s_cnt[e] = 0;
         __syncthreads();
-        for (int t = threadIdx.x; t < args.tokens; t += GEMM_THREADS) {
-            const int e = __ldcg(args.gate + t);
-            if (e >= 0 && e < args.E) atomicAdd(&s_cnt[e], 1);
+        for (int t0 = threadIdx.x; t0 < args.tokens; t0 += 8 * GEMM_THREADS) {
+            int e[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) e[i] = t0 + i * GEMM_THREADS < args.tokens ? __ldcg(args.gate + t0 + i * GEMM_THREADS) : -1;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (e[i] >= 0 && e[i] < args.E) atomicAdd(&s_cnt[e[i]], 1);
         }
         __syncthreads();
         if (warp == 2) {

@@ -822,11 +822,12 @@ template <int TOKENS, int NV>
 __global__ void __launch_bounds__(RR_THREADS, 1)
 route_rows_kernel(const float* __restrict__ X, const float* __restrict__ C, const float* __restrict__ gamma,
                   long long T, int D, int E, int* __restrict__ gate, float* __restrict__ score,
-                  int* __restrict__ status) {
+                  int* __restrict__ status, int constant) {
     constexpr int EB = 32 / TOKENS;                            // experts per reduction
     constexpr int SUBS = EB / RR_STAGE_EXPERTS;                // of RR_STAGE_EXPERTS experts each
     constexpr int PITCH = NV * 32;                             // float4 per staged centroid
-    extern __shared__ __align__(16) float4 rr_c[];             // [2][RR_STAGE_EXPERTS][PITCH]
+    extern __shared__ __align__(16) float4 rr_c[];             // [2][RR_STAGE_EXPERTS][PITCH], then LayerNorm weights [PITCH]
+    float4* const rr_g = rr_c + 2 * RR_STAGE_EXPERTS * PITCH;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long t0 = ((long long)blockIdx.x * (RR_THREADS / 32) + warp) * TOKENS;
     const int stages = (E + RR_STAGE_EXPERTS - 1) / RR_STAGE_EXPERTS;
@@ -843,9 +844,16 @@ route_rows_kernel(const float* __restrict__ X, const float* __restrict__ C, cons
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // what no kernel on the stream writes (`constant`) is requested before the wait
+    const auto fetch_first = [&]() {
+        if (gamma)
+            for (int i = tid; 4 * i < D; i += RR_THREADS) cp_async16(rr_g + i, gamma + 4 * i);
+        fetch(0);
+    };
+    if (constant) fetch_first();
     pdl_wait();
     pdl_trigger();
-    fetch(0);
+    if (!constant) fetch_first();
     float4 x[TOKENS][NV];
 #pragma unroll
     for (int t = 0; t < TOKENS; ++t)
@@ -883,11 +891,13 @@ route_rows_kernel(const float* __restrict__ X, const float* __restrict__ C, cons
                 }
             rstd[t] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(warp_xor_sum(q), (float)D), 1e-6f)));
         }
+        cp_async_wait<0>();
+        __syncthreads();
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int k = 4 * lane + 128 * i;
             if (k >= D) continue;
-            const float4 g = *reinterpret_cast<const float4*>(gamma + k);
+            const float4 g = rr_g[k >> 2];
 #pragma unroll
             for (int t = 0; t < TOKENS; ++t) {
                 x[t][i].x = ln_apply(x[t][i].x, mean[t], rstd[t], g.x);
@@ -1095,13 +1105,13 @@ int launch_route_small(const float* X, const float* C, const float* gamma, long 
 }
 template <int TOKENS, int NV>
 int launch_route_rows(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
-                      float* score, int* status, cudaStream_t stream) {
-    constexpr int smem = 2 * RR_STAGE_EXPERTS * NV * 32 * 16;
+                      float* score, int* status, bool constant, cudaStream_t stream) {
+    constexpr int smem = (2 * RR_STAGE_EXPERTS + 1) * NV * 32 * 16;
     auto kern = route_rows_kernel<TOKENS, NV>;
     INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const long long per_cta = RR_THREADS / 32 * TOKENS;
     INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)((T + per_cta - 1) / per_cta), RR_THREADS, smem, 1, stream, X, C, gamma, T,
-                                   D, E, gate, score, status));
+                                   D, E, gate, score, status, constant ? 1 : 0));
     return INFMOE_OK;
 }
 }  // namespace
@@ -1123,7 +1133,7 @@ int launch_route(const float* X, const float* C, const float* gamma, long long T
                                                                                status, constant, stream));
     } else if (rows) {
         INFMOE_TRY((D <= 1024 ? launch_route_rows<4, 8> : launch_route_rows<2, 16>)(X, C, gamma, T, D, E, gate, score,
-                                                                                    status, stream));
+                                                                                    status, constant, stream));
     } else if (vec && !no_tma && T < (1ll << 31) && route_maps(&map_x, &map_c, X, C, T, D, E) == INFMOE_OK) {
         INFMOE_CUDA_TRY(cudaFuncSetAttribute(route_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM + 1024));
         INFMOE_CUDA_TRY(launch_chained(route_tma_kernel, (unsigned)grid, RT_THREADS, RT_SMEM + 1024, 1, stream, map_x, map_c,

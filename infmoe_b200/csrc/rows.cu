@@ -253,6 +253,20 @@ scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __rest
     if ((threadIdx.x & 31) == 0 && rscore && score) rscore[j] = score[p];
 }
 
+// f(t, gate[t]) for t = threadIdx.x, + THREADS, ... below T, with eight loads on their way together (one by one they are a trip
+// to L2 each, 0.7 us, sixteen of them for a block that looks at 4096 gates).
+template <int THREADS, typename F>
+__device__ __forceinline__ void for_gates(const int* __restrict__ gate, int T, const F& f) {
+    for (int t0 = threadIdx.x; t0 < T; t0 += 8 * THREADS) {
+        int g[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) g[i] = t0 + i * THREADS < T ? gate[t0 + i * THREADS] : 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (t0 + i * THREADS < T) f(t0 + i * THREADS, g[i]);
+    }
+}
+
 // count[] and offset[] of the T gates by one block of THREADS threads, and zero[] cleared on the way.
 template <int THREADS>
 __device__ __forceinline__ void histogram_block(int* hist, int T, int E, const int* __restrict__ gate, int* __restrict__ count,
@@ -263,12 +277,11 @@ __device__ __forceinline__ void histogram_block(int* hist, int T, int E, const i
     for (int i = tid; i < zero_count; i += THREADS) zero[i] = 0;
     __syncthreads();
     bool bad = false;
-    for (int t = tid; t < T; t += THREADS) {
-        const int e = gate[t];
+    for_gates<THREADS>(gate, T, [&](int, int e) {
         const bool ok = e >= 0 && e < E;
         bad |= !ok;
         atomicAdd(&hist[ok ? e : E], 1);
-    }
+    });
     if (bad && status) atomicOr(status, STATUS_BAD_GATE);
     __syncthreads();
     if (tid < 32) {
@@ -419,13 +432,14 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ 
 // The same for more tokens, aligned rows of up to 128 NV floats: eight tokens per block, a warp and its registers for each.
 // The blocks read T / 8 x T gates, from L2, and compare each with eight: key (gate, token) below the own one.  4096
 // tokens are the most it takes: 8 MB and about 1.5 us of comparisons, against a kernel of one cluster between routing and
-// scatter.  Dispatch and scatter, us, each timed by itself: 4096 tokens of 512 floats 12 + 10 -> 19, 1024 floats 11 + 12 -> 21, 2500 tokens
-// of 512 floats 11 + 10 -> 12; in a pass the row's half of it runs under the routing.
+// scatter.  Bound by latency: the gates' trips to L2, then the LayerNorm weights', in one to two rounds of blocks (three or four
+// to an SM by registers).  Dispatch and scatter, us, each timed by itself: 4096 tokens of 512 floats 12 + 10 -> 14.7, 1024 floats 11
+// + 12 -> 16.8, 2500 tokens of 512 floats 11 + 10 -> 10.9.
 constexpr int DM_THREADS = 256;
 constexpr int DM_TOKENS = DM_THREADS / 32;
 constexpr int DM_MAX_TOKENS = 4096;
 template <int NV>
-__global__ void __launch_bounds__(DM_THREADS)
+__global__ void __launch_bounds__(DM_THREADS, NV <= 4 ? 4 : NV <= 8 ? 3 : 2)
 dispatch_scatter_reg_kernel(int T, int D, int E, const float* __restrict__ X, const float* __restrict__ score,
                             const int* __restrict__ gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
                             int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
@@ -434,8 +448,8 @@ dispatch_scatter_reg_kernel(int T, int D, int E, const float* __restrict__ X, co
     extern __shared__ __align__(16) float4 dm_gamma[];     // [warp][NV * 32]; histogram block: E + 1 words
     __shared__ int s_before[DM_TOKENS][DM_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int t0 = (int)blockIdx.x * DM_TOKENS, t = t0 + warp;
-    if (t0 >= T) {
+    const int t0 = ((int)blockIdx.x - 1) * DM_TOKENS, t = t0 + warp;
+    if (blockIdx.x == 0) {      // first, because it takes as long as any
         pdl_wait();
         pdl_trigger();
         histogram_block<DM_THREADS>(reinterpret_cast<int*>(dm_gamma), T, E, gate, count, offset, status, zero, zero_count);
@@ -447,22 +461,19 @@ dispatch_scatter_reg_kernel(int T, int D, int E, const float* __restrict__ X, co
     row.stats(D);
     if (early) pdl_wait();
     pdl_trigger();
-    const auto key = [&](int o) {
-        const int g = gate[o];
-        return (g >= 0 && g < E ? g : E) * DM_MAX_TOKENS + o;
-    };
+    const auto key_of = [&](int o, int g) { return (g >= 0 && g < E ? g : E) * DM_MAX_TOKENS + o; };
+    const auto key = [&](int o) { return key_of(o, gate[o]); };
     const int own = key(min(t, T - 1)), e = own / DM_MAX_TOKENS;
     float4* const s_gamma = dm_gamma + warp * (NV * 32);
     row.fetch_gamma(s_gamma, expert_gamma.of(e < E ? e : 0), D);
     int keys[DM_TOKENS], before[DM_TOKENS] = {};
 #pragma unroll
     for (int j = 0; j < DM_TOKENS; ++j) keys[j] = key(min(t0 + j, T - 1));
-#pragma unroll 4
-    for (int o = tid; o < T; o += DM_THREADS) {
-        const int k = key(o);
+    for_gates<DM_THREADS>(gate, T, [&](int o, int g) {
+        const int k = key_of(o, g);
 #pragma unroll
         for (int j = 0; j < DM_TOKENS; ++j) before[j] += k < keys[j] ? 1 : 0;
-    }
+    });
 #pragma unroll
     for (int j = 0; j < DM_TOKENS; ++j) {
         const int n = __reduce_add_sync(0xffffffffu, before[j]);
@@ -919,10 +930,10 @@ int launch_dispatch_scatter(long long T, int D, int E, const float* X, const flo
             set_error("dispatch_scatter: unaligned rows");
             return INFMOE_ERR_UNSUPPORTED;
         }
-        const int nv = D <= 1024 ? 8 : 16;
+        const int nv = D <= 512 ? 4 : D <= 1024 ? 8 : 16;
         size_t smem = (size_t)DM_TOKENS * nv * 512;
         if (smem < hist) smem = hist;
-        auto kern = nv == 8 ? dispatch_scatter_reg_kernel<8> : dispatch_scatter_reg_kernel<16>;
+        auto kern = nv == 4 ? dispatch_scatter_reg_kernel<4> : nv == 8 ? dispatch_scatter_reg_kernel<8> : dispatch_scatter_reg_kernel<16>;
         if (smem > 48 * 1024)
             INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)((T + DM_TOKENS - 1) / DM_TOKENS + 1), DM_THREADS, smem, 1, stream,
