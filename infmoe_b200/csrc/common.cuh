@@ -71,11 +71,13 @@ inline cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsign
 // ---------------------------------------------------------------------------
 // Programmatic dependent launch.  The kernels of a pass are short next to the time between two dependent launches
 // (1-2 us on an idle GPU), so each is launched while its predecessor still runs (launch_chained): its blocks start as
-// soon as every block of the predecessor has started (pdl_trigger) and left room, do what needs no memory, and wait
+// soon as every block of the predecessor has called pdl_trigger and left room, do what needs no memory, and wait
 // in pdl_wait until the predecessor has completed and its writes are visible.  Every block of every kernel launched
 // this way calls pdl_wait before it touches global memory; the predecessor did the same, so all earlier kernels of the
-// stream are complete too.  (Without the launch attribute both are no-ops.)  One kernel reads memory before its wait, the
-// second expert GEMM; see there.
+// stream are complete too.  (Without the launch attribute both are no-ops.)  The kernels of a
+// pass up to the first GEMM call pdl_trigger only after their own wait: when a block of the next one starts, everything before
+// its predecessor is complete, and it may read that before its wait.  The scatters read the tokens so, the GEMMs gates or
+// offsets and weights, the routing what no kernel writes; see there.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -21,7 +21,8 @@
 // Layer of 300 tokens, 6 experts, 510 x 1022: 423 -> 103 us (it was 64 x 64 tiles of scalar loads, one buffer, TF32 head
 // and tail planes added on the fly), 88 with the dispatch and scatter in one kernel, 67 with the clusters: 96 to 192 CTAs of
 // one chain each had left two or three of four schedulers of an SM without a warp, now 384 to 768 are in flight, six to an
-// SM (at 80 registers; five, at 96, left 28 of 768 CTAs for a second wave: 66.8 -> 65.6).  The shorter chains also halve the error against 64 bits, 4.6e-7 -> 2.4e-7.
+// SM (at 80 registers; five, at 96, left 28 of 768 CTAs for a second wave: 66.8 -> 65.6).  Half the threads with twice the
+// rows each, 16 loads for 256 multiply-adds, took 2.6 us longer.  The shorter chains also halve the error against 64 bits, 4.6e-7 -> 2.4e-7.
 #include <cooperative_groups.h>
 
 #include "common.cuh"

@@ -154,7 +154,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // L2 policies of a load: weights that one tile alone reads give way first, so that streaming them does not push out what
-// the passes come back to (activations, chunk sums, centroids, and the kernels' code).
+// the passes come back to (activations, chunk sums, centroids, and the kernels' code).  Layer, us: one token 32 x 4096 x 10240
+// 118.7 -> 108.8, 777 tokens 12 x 1000 x 2724 113 -> 104, 2500 tokens 16 x 512 x 2048 131 -> 118.
 __device__ __forceinline__ uint64_t l2_evict_first() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -402,7 +403,8 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, const int* s_prefix, c
 // one tile from each end of a stretch.  The R tiles left after the last whole round are cut into chunk units and dealt
 // out evenly when that pays: an uncut tail lasts one tile (m chunks), a cut one R m / G chunks plus storing and
 // re-reading the chunk sums, which is worth about two chunks.  A CTA whose share spans two tiles stores, fences and counts
-// twice, about as long as a chunk and a half; where shares that end with their tile are no longer than that, they are taken.
+// twice, about as long as a chunk and a half; where shares that end with their tile are at most that much longer, they are
+// taken.  Layer, us: 2500 tokens 16 x 512 x 2048 104 -> 90, one token 32 x 4096 x 10240 109 -> 105.
 struct Item {
     int tile;
     int c0, c1;        // chunks [c0, c1) of the tile
@@ -548,7 +550,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     // scatter is still running: offset[] is complete when a kernel of its own has made it, and the gates are when the scatter
     // makes offset[] itself.
     // Layer, us, second GEMM: 32 tokens 64 x 256 24.5 -> 22.3, one token 4096 x 10240 138.5 -> 133.7, 777 x 12 x 1000 x 2724
-    // 124 -> 120.
+    // 124 -> 120; first GEMM and scatter: one token 132.5 -> 125, 777 tokens 117 -> 112, 2500 x 16 x 512 x 2048 140 -> 130.
     const bool early = EPI == EPI_RESIDUAL || args.early;
     if (!early) pdl_wait();
     if (EPI == EPI_RESIDUAL || !early) pdl_trigger();
@@ -936,7 +938,8 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const int end = f < ((F + 31) & ~31) ? min(t.n_tok - col0, width) - odd : 0;    // columns this lane stores
                 // Eight columns at a time, every step for all of them before the next: one chain of shared-memory read, shuffle,
                 // exponential, reciprocal, conversions, shuffle and store is some 300 cycles, and a store keeps the
-                // compiler from starting the next one above it.
+                // compiler from starting the next one above it.  128 columns: 9.3 -> 6.8 thousand cycles.  (Conversions and
+                // the second shuffle for two columns at a time changed nothing.)
 #pragma unroll
                 for (int i = 0; i < 2 * C::SLICES; ++i) {
                     if (8 * i >= width) continue;     // uniform across the warp
@@ -1008,7 +1011,9 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     } else if (warp == ITEM_WARP) {
         // ================= list of items =================
         // The schedule and the place of a tile (searches, divisions) take one to two thousand cycles, and every role took them
-        // at each tile, the issuer and the accumulate warps while nothing else went on in their part.
+        // at each tile, the issuer and the accumulate warps while nothing else went on in their part.  Layer, us, with the
+        // column warp: 4096 tokens 8 x 1024 x 4096 331 -> 321, 16384 tokens 64 x 1024 x 4096 1481 -> 1432, 32 tokens 4 x 64 x 256,
+        // where the list is only a detour, 18.1 -> 18.5.
         Schedule<CTAS> sched(s_prefix[args.E], KB, args);
         Place at;
         bool more = true, first = true;
@@ -1041,6 +1046,8 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
     } else if (warp == COLUMN_WARP) {
         // ================= columns of the items =================
+        // Fetched by the accumulate warps, slice by slice when the sums were complete, these were a chain of trips to memory:
+        // 4096 tokens 8 x 1024 x 4096 355 -> 340 us, 2500 tokens 16 x 512 x 2048 118 -> 110.
         if (EPI == EPI_RESIDUAL) pdl_wait();
         wait_then_trigger();
         for (Place at;; at.advance()) {

@@ -637,7 +637,8 @@ route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // Behind a pass that has streamed its weights through L2 the same call took 17 us: the rows (twice, for their statistics), the
 // LayerNorm weights and the centroids (eight loads at a time) were one trip to HBM after the other.  While the blocks all
 // fit on the chip (AHEAD) everything is requested on entry, by cp.async into shared memory: 10 us.  (The centroid in 32 registers
-// per lane, fetched by unrolled loads, took 22: the code has to come from HBM too.)
+// per lane, fetched by unrolled loads, took 22: the code has to come from HBM too.)  Rows longer than 4224 floats do not fit
+// beside eight centroids, and with more blocks than SMs two of them share one: these read as they go.
 constexpr int RS_TOKENS = 4;
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
