@@ -77,7 +77,9 @@ inline cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsign
 // stream are complete too.  (Without the launch attribute both are no-ops.)  The kernels of a
 // pass up to the first GEMM call pdl_trigger only after their own wait: when a block of the next one starts, everything before
 // its predecessor is complete, and it may read that before its wait.  The scatters read the tokens so, the GEMMs gates or
-// offsets and weights, the routing what no kernel writes; see there.
+// offsets and weights, the routing what no kernel writes; see there.  Nothing that a predecessor may still be writing is read
+// through the read-only path: `const T* __restrict__` parameters and __ldg promise that nobody writes during the kernel, and a
+// load under that promise may be moved above the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -53,7 +53,7 @@ constexpr int DISPATCH_MAX_CLUSTER = 8;   // portable cluster size
 constexpr int DISPATCH_TABLES = 5 + DISPATCH_WARPS;
 
 __global__ void __launch_bounds__(DISPATCH_THREADS)
-dispatch_kernel(const int* __restrict__ gate, long long T, int E, const int* __restrict__ region_count,
+dispatch_kernel(const int* gate, long long T, int E, const int* region_count,
                 int region_size, int* __restrict__ pos, int* __restrict__ count, int* __restrict__ offset,
                 int* __restrict__ status, int* __restrict__ zero, int zero_count) {
     cg::cluster_group cluster = cg::this_cluster();

@@ -151,7 +151,7 @@ __device__ __forceinline__ void warp_four_row_stats(const float* const (&r)[4], 
 
 template <bool VEC>
 __global__ void __launch_bounds__(RT_THREADS, 1)
-route_kernel(const float* __restrict__ X, const float* __restrict__ C, const float* __restrict__ gamma,
+route_kernel(const float* X, const float* C, const float* gamma,
              long long T, int D, int E, int* __restrict__ gate, float* __restrict__ score,
              int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char rt_smem[];
@@ -412,7 +412,7 @@ __device__ __forceinline__ int rt_box_idx(int step, int l, int row) {
 
 __global__ void __launch_bounds__(RT_THREADS, 1)
 route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_c,
-                 const float* __restrict__ X, const float* __restrict__ gamma, long long T, int D, int E,
+                 const float* X, const float* gamma, long long T, int D, int E,
                  int* __restrict__ gate, float* __restrict__ score, int* __restrict__ status) {
     extern __shared__ unsigned char rt_smem_raw[];
     unsigned char* const rt_smem = rt_smem_raw + ((1024u - (rt_smem_u32(rt_smem_raw) & 1023u)) & 1023u);
@@ -651,7 +651,7 @@ __device__ __forceinline__ bool rs_better(float s, int e, float best, int best_e
 
 template <bool VEC, bool AHEAD>
 __global__ void __launch_bounds__(RS_THREADS)
-route_small_kernel(const float* __restrict__ X, const float* __restrict__ C, const float* __restrict__ gamma,
+route_small_kernel(const float* X, const float* C, const float* gamma,
                    long long T, int D, int E, int* __restrict__ gate, float* __restrict__ score,
                    int* __restrict__ status, int constant) {
     cg::cluster_group cluster = cg::this_cluster();
@@ -821,7 +821,7 @@ constexpr int RR_STAGE_EXPERTS = 8;
 
 template <int TOKENS, int NV>
 __global__ void __launch_bounds__(RR_THREADS, 1)
-route_rows_kernel(const float* __restrict__ X, const float* __restrict__ C, const float* __restrict__ gamma,
+route_rows_kernel(const float* X, const float* C, const float* gamma,
                   long long T, int D, int E, int* __restrict__ gate, float* __restrict__ score,
                   int* __restrict__ status, int constant) {
     constexpr int EB = 32 / TOKENS;                            // experts per reduction

@@ -37,8 +37,8 @@ __device__ __forceinline__ void copy_row(const float* __restrict__ src, float* _
 
 // routed[j,:] = X[pos[j],:]; rcoeff[j] = coeff[pos[j]]
 __global__ void __launch_bounds__(ROW_WARPS * 32)
-scatter_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ coeff,
-               const int* __restrict__ pos, float* __restrict__ routed, float* __restrict__ rcoeff) {
+scatter_kernel(long long T, int D, int vec, const float* X, const float* coeff,
+               const int* pos, float* __restrict__ routed, float* __restrict__ rcoeff) {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -73,9 +73,9 @@ __device__ __forceinline__ void warp_ln_rows(const float* __restrict__ src, cons
 }
 
 __global__ void __launch_bounds__(ROW_WARPS * 32)
-scatter_ln_rows_kernel(long long T, int D, int vec, const float* __restrict__ X, const float* __restrict__ score,
-                       const int* __restrict__ pos, const int* __restrict__ gate, const float* __restrict__ gamma_all,
-                       const int* __restrict__ valid_rows, float* __restrict__ rscore, float* __restrict__ h) {
+scatter_ln_rows_kernel(long long T, int D, int vec, const float* X, const float* score,
+                       const int* pos, const int* gate, const float* gamma_all,
+                       const int* valid_rows, float* __restrict__ rscore, float* __restrict__ h) {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -129,9 +129,9 @@ struct ExpertGamma {
     __device__ __forceinline__ const float* of(int e) const { return base + stride * (size_t)e; }
 };
 __global__ void __launch_bounds__(ROW_WARPS * 32)
-scatter_ln_pack_kernel(long long j0, long long T, int D, int vec, const float* __restrict__ X,
-                       const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
-                       const ExpertGamma gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
+scatter_ln_pack_kernel(long long j0, long long T, int D, int vec, const float* X,
+                       const float* score, const int* pos, const int* gate,
+                       const ExpertGamma gamma, const int* valid_rows, float* __restrict__ rscore,
                        uint16_t* __restrict__ h, float2* __restrict__ row_info) {
     pdl_wait();
     pdl_trigger();
@@ -233,9 +233,9 @@ struct RowInRegisters {
 
 template <int NV>
 __global__ void __launch_bounds__(128)
-scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* __restrict__ X,
-                           const float* __restrict__ score, const int* __restrict__ pos, const int* __restrict__ gate,
-                           const ExpertGamma expert_gamma, const int* __restrict__ valid_rows, float* __restrict__ rscore,
+scatter_ln_pack_reg_kernel(long long j0, long long T, int D, const float* X,
+                           const float* score, const int* pos, const int* gate,
+                           const ExpertGamma expert_gamma, const int* valid_rows, float* __restrict__ rscore,
                            uint16_t* __restrict__ h, float2* __restrict__ row_info) {
     pdl_wait();
     pdl_trigger();
@@ -314,8 +314,8 @@ __device__ __forceinline__ void histogram_block(int* hist, int T, int E, const i
 constexpr int DS_THREADS = 128;
 template <bool PACK>
 __global__ void __launch_bounds__(DS_THREADS)
-dispatch_scatter_kernel(int T, int D, int E, int vec, const float* __restrict__ X, const float* __restrict__ score,
-                        const int* __restrict__ gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
+dispatch_scatter_kernel(int T, int D, int E, int vec, const float* X, const float* score,
+                        const int* gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
                         int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
                         int* __restrict__ zero, int zero_count, float* __restrict__ rscore, void* __restrict__ h,
                         float2* __restrict__ row_info, int early) {
@@ -440,8 +440,8 @@ constexpr int DM_TOKENS = DM_THREADS / 32;
 constexpr int DM_MAX_TOKENS = 4096;
 template <int NV>
 __global__ void __launch_bounds__(DM_THREADS, NV <= 4 ? 4 : NV <= 8 ? 3 : 2)
-dispatch_scatter_reg_kernel(int T, int D, int E, const float* __restrict__ X, const float* __restrict__ score,
-                            const int* __restrict__ gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
+dispatch_scatter_reg_kernel(int T, int D, int E, const float* X, const float* score,
+                            const int* gate, const ExpertGamma expert_gamma, int* __restrict__ pos,
                             int* __restrict__ count, int* __restrict__ offset, int* __restrict__ status,
                             int* __restrict__ zero, int zero_count, float* __restrict__ rscore, uint16_t* __restrict__ h,
                             float2* __restrict__ row_info, int early) {
@@ -494,8 +494,8 @@ dispatch_scatter_reg_kernel(int T, int D, int E, const float* __restrict__ X, co
 
 // out[pos[j],:] = in[j,:] for the rows below *valid_rows (all rows when valid_rows is NULL)
 __global__ void __launch_bounds__(ROW_WARPS * 32)
-gather_kernel(long long T, int D, int vec, const float* __restrict__ in, const int* __restrict__ pos,
-              const int* __restrict__ valid_rows, float* __restrict__ out) {
+gather_kernel(long long T, int D, int vec, const float* in, const int* pos,
+              const int* valid_rows, float* __restrict__ out) {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -507,9 +507,9 @@ gather_kernel(long long T, int D, int vec, const float* __restrict__ in, const i
 // alpha = 1 / (1 + exp(-coeff[j])); out[pos[j],:] = alpha * post[j,:] + (1 - alpha) * routed[j,:]
 // (sigmoid: plugin/cuda/common.cuh:24-27)
 __global__ void __launch_bounds__(ROW_WARPS * 32)
-mix_gather_kernel(long long T, int D, int vec, const int* __restrict__ pos, const float* __restrict__ routed,
-                  const float* __restrict__ post, const float* __restrict__ coeff,
-                  const int* __restrict__ valid_rows, float* __restrict__ out) {
+mix_gather_kernel(long long T, int D, int vec, const int* pos, const float* routed,
+                  const float* post, const float* coeff,
+                  const int* valid_rows, float* __restrict__ out) {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31;

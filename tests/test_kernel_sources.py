@@ -8,8 +8,8 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "infmoe_b200", "csrc")
 
 
-def _kernels():
-    """(file, name, body) of every __global__ function, comments removed."""
+def _signatures():
+    """(file, name, parameter list, body) of every __global__ function, comments removed."""
     for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
         with open(path) as f:
             text = re.sub(r"//[^\n]*", "", f.read())
@@ -23,7 +23,11 @@ def _kernels():
                 i += 1
                 if depth == 0:
                     break
-            yield os.path.basename(path), m.group(1), text[start:i]
+            yield os.path.basename(path), m.group(1), text[m.end():start], text[start:i]
+
+
+def _kernels():
+    return [(file, name, body) for file, name, _, body in _signatures()]
 
 
 def test_kernels_are_found():
@@ -49,3 +53,14 @@ def test_sums_of_a_cut_tile_are_read_behind_a_warp_barrier():
     handed_on = body.rindex("__shfl_sync(0xffffffffu, done", counted, read)
     assert "__threadfence();" in body[counted:handed_on]
     assert "__syncwarp();" in body[handed_on:read]
+
+
+@pytest.mark.parametrize("file,name,params,body", [k for k in _signatures() if "pdl_wait" in k[3]],
+                         ids=lambda v: v if len(v) < 40 else "")
+def test_kernels_that_start_early_promise_nothing_about_what_others_still_write(file, name, params, body):
+    """A kernel that starts before its predecessor has ended may not read what that one writes through the read-only path:
+    `const T* __restrict__` parameters and __ldg promise that nobody writes during the kernel, and a load under that promise
+    may be moved above the wait."""
+    assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params), f"{file}: {name}"
+    for load in re.findall(r"__ldg\((?:[^()]|\([^()]*\))*\)", body):
+        assert re.search(r"\b(scales|bound)\b", load), f"{file}: {name}: {load}"      # of the weights, written before any pass
