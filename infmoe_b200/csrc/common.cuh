@@ -73,11 +73,14 @@ inline cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsign
 // (1-2 us on an idle GPU), so each is launched while its predecessor still runs (launch_chained): its blocks start as
 // soon as every block of the predecessor has called pdl_trigger and left room, do what needs no memory, and wait
 // in pdl_wait until the predecessor has completed and its writes are visible.  Every block of every kernel launched
-// this way calls pdl_wait before it touches global memory; the predecessor did the same, so all earlier kernels of the
-// stream are complete too.  (Without the launch attribute both are no-ops.)  The kernels of a
-// pass up to the first GEMM call pdl_trigger only after their own wait: when a block of the next one starts, everything before
-// its predecessor is complete, and it may read that before its wait.  The scatters read the tokens so, the GEMMs gates or
-// offsets and weights, the routing what no kernel writes; see there.  Nothing that a predecessor may still be writing is read
+// this way calls pdl_wait, and writes no global memory before it; the predecessor did the same, so all earlier kernels of the
+// stream are complete then too.  (Without the launch attribute both are no-ops.)
+// What may be read before the wait: what no kernel on the stream writes (the routing reads centroids and LayerNorm weights so),
+// and, behind a predecessor that calls pdl_trigger only after its own wait, what was complete when that one's wait ended.
+// Routing, dispatch and scatter kernels all trigger so: the scatters read the tokens, the first GEMM gates or offsets and
+// weights; it does too, for the second one.  The others (second GEMM, combine, weight layout) trigger first, and a kernel behind
+// them reads nothing of the second kind.
+// Nothing that a predecessor may still be writing is read
 // through the read-only path: `const T* __restrict__` parameters and __ldg promise that nobody writes during the kernel, and a
 // load under that promise may be moved above the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

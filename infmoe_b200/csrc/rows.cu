@@ -39,8 +39,8 @@ __device__ __forceinline__ void copy_row(const float* __restrict__ src, float* _
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 scatter_kernel(long long T, int D, int vec, const float* X, const float* coeff,
                const int* pos, float* __restrict__ routed, float* __restrict__ rcoeff) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T) return;
@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(ROW_WARPS * 32)
 scatter_ln_rows_kernel(long long T, int D, int vec, const float* X, const float* score,
                        const int* pos, const int* gate, const float* gamma_all,
                        const int* valid_rows, float* __restrict__ rscore, float* __restrict__ h) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const long long j = (long long)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
     if (j >= T || (valid_rows && j >= *valid_rows)) return;

@@ -64,3 +64,10 @@ def test_kernels_that_start_early_promise_nothing_about_what_others_still_write(
     assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params), f"{file}: {name}"
     for load in re.findall(r"__ldg\((?:[^()]|\([^()]*\))*\)", body):
         assert re.search(r"\b(scales|bound)\b", load), f"{file}: {name}: {load}"      # of the weights, written before any pass
+
+
+@pytest.mark.parametrize("file,name,body", [k for k in _kernels() if re.match(r"route_|dispatch_|scatter_", k[1]) and "pdl_wait" in k[2]],
+                         ids=lambda v: v if len(v) < 40 else "")
+def test_kernels_before_the_gemms_let_their_successor_start_after_their_own_wait(file, name, body):
+    """Their successors read, before their own wait, what was complete when this kernel's wait ended."""
+    assert body.index("pdl_wait()") < body.index("pdl_trigger()"), f"{file}: {name}"
