@@ -557,7 +557,8 @@ def test_cuda_core_experts_with_k_shared_by_a_cluster(oracle, D, F):
     assert oracle.rel_l2(out - x, want - x) <= 2e-6     # FP32 chains of up to 450 adds
 
 
-# Up to 1024 tokens one kernel computes the dispatch metadata and scatters; beyond, or with d_model > 6016, two do.
+# Up to 1024 tokens one kernel computes the dispatch metadata and scatters, unless d_model > 6016; up to 4096 another one does for
+# aligned rows of up to 2048 floats on the tensor-core path (more of its lines below); else two kernels do.
 @pytest.mark.parametrize("T,D,E,variant", [(1, 64, 4, "default"), (33, 66, 3, "base_layer"), (1023, 36, 70, "cpm_2"),
                                            (1024, 40, 5, "base_layer"), (1025, 40, 5, "base_layer"),
                                            (7, 6016, 2, "default"), (7, 6020, 2, "default"), (129, 130, 33, "default")])
@@ -721,3 +722,130 @@ def test_token_tiles_of_every_width(oracle, D, F):
     layer.terminate()
     np.testing.assert_array_equal(same, out)
     assert oracle.rel_l2(out[:64] - x[:64], oracle.expert_ffn_f64(x[:64], *expert) - x[:64]) <= TOL
+
+
+# Odd widths take the CUDA-core path, where two kernels dispatch and scatter from 1025 tokens on.
+def test_dispatch_of_a_few_thousand_tokens_of_odd_width_alike(oracle):
+    test_few_and_many_tokens_dispatch_alike(oracle, 1025, 42, 5, "cpm_2")
+    test_few_and_many_tokens_dispatch_alike(oracle, 1025, 41, 5, "base_layer")
+
+
+# Tokens that start one float past an aligned address: no wide loads, and from 1025 on two kernels; the same additions either way.
+@pytest.mark.parametrize("T", [33, 1024, 1025, 4097])
+@pytest.mark.parametrize("variant", ["cpm_2", "base_layer"])
+def test_unaligned_tokens_have_the_bits_of_aligned_ones(T, variant):
+    import torch
+    from infmoe_b200 import MoELayer
+    E, D, F = 5, 40, 44
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ln = np.linspace(0.9, 1.1, D, dtype=np.float32) if variant == "cpm_2" else None
+    layer = MoELayer.create(E, D, F, 2, torch.randn(E, D, generator=g, device="cuda").cpu().numpy(), None, "T5_FF", variant, ln)
+    for e in range(E):
+        layer.set_expert(e, torch.ones(D, device="cuda"), torch.randn(F, D, generator=g, device="cuda") / 6,
+                         torch.randn(F, D, generator=g, device="cuda") / 6, torch.randn(D, F, generator=g, device="cuda") / 6)
+    x = torch.randn(T, D, generator=g, device="cuda")
+    shifted = torch.empty(T * D + 1, device="cuda")[1:].view(T, D)
+    shifted.copy_(x)
+    assert x.data_ptr() % 16 == 0 and shifted.data_ptr() % 16 == 4
+    want, got = layer.forward(x), layer.forward(shifted)
+    layer.sync_status()
+    assert torch.equal(got, want)
+    layer.terminate()
+
+
+# Passes behind and in front of other kernels, one form of a pass each: separate dispatch and scatter for many tokens and for long
+# rows (pairs of CTAs), the CUDA-core path, LayerNorm weights and centroids that are read early, the mix.  Every step routes
+# differently, so that counts, positions or gates that an earlier step left in the workspace would show.
+@pytest.mark.parametrize("T,D,E,F,variant", [(4200, 256, 4, 512, "default"), (1500, 2052, 4, 132, "default"),
+                                             (300, 254, 4, 510, "cpm_2"), (1100, 130, 4, 66, "base_layer"), (5, 4096, 20, 64, "cpm_2"),
+                                             (600, 512, 6, 256, "cpm_2"), (2500, 256, 4, 512, "base_layer"), (16384, 64, 8, 64, "cpm_2")])
+def test_steps_that_route_differently_between_other_kernels(T, D, E, F, variant):
+    import torch
+    from infmoe_b200 import MoELayer
+    g = torch.Generator(device="cuda").manual_seed(T + D)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    centroids = normal(E, D)
+    layer = MoELayer.create(E, D, F, 2, centroids.cpu().numpy(), None, "T5_FF", variant,
+                            np.linspace(0.9, 1.1, D, dtype=np.float32) if variant == "cpm_2" else None)
+    for e in range(E):
+        layer.set_expert(e, 1 + normal(D) / 100, normal(F, D) / D ** 0.5, normal(F, D) / D ** 0.5, normal(D, F) / F ** 0.5)
+    # step i draws most of its tokens to expert i
+    src = torch.stack([normal(T, D) + (torch.rand(T, 1, generator=g, device="cuda") < 0.2 + 0.2 * i) * centroids[i % E] for i in range(4)])
+    want = []
+    for i in range(4):
+        want.append(layer.forward(src[i].contiguous()).clone())
+        layer.sync_status()
+    ref = torch.zeros(T, D, device="cuda")
+    for w in want:
+        ref.add_(w)
+    torch.cuda.synchronize()
+    x, out, acc = (torch.zeros(T, D, device="cuda") for _ in range(3))
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+
+    def steps():
+        acc.zero_()
+        for i in range(4):
+            x.copy_(src[i] * 1.0)
+            layer.forward(x, out)
+            acc.add_(out)
+            out.fill_(-1.0)
+            x.fill_(5.0)
+
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        steps()
+        steps()
+    side.synchronize()
+    assert torch.equal(acc, ref)
+    with torch.cuda.graph(graph, stream=side):
+        steps()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(acc, ref)
+    layer.sync_status()
+    layer.terminate()
+
+
+# The GEMMs fetch weights before their wait.  Experts are replaced on the device between passes of another stream that are issued
+# without a wait of the host: each pass has the results of a layer that only ever had its weights.
+@pytest.mark.parametrize("T", [3, 700, 4200])
+def test_experts_replaced_between_passes_of_another_stream(T):
+    import torch
+    from infmoe_b200 import MoELayer
+    E, D, F = 3, 256, 512
+    g = torch.Generator(device="cuda").manual_seed(T)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    centroids = normal(E, D).cpu().numpy()
+    sets = [[(1 + normal(D) / 100, normal(F, D) / 16, normal(F, D) / 16, normal(D, F) / 22) for _ in range(E)] for _ in range(4)]
+    x = normal(T, D)
+
+    def make(experts):
+        layer = MoELayer.create(E, D, F, 2, centroids, None, "T5_FF", "default", None)
+        for e in range(E):
+            layer.set_expert(e, *experts[e])
+        return layer
+
+    want = []
+    for experts in sets:
+        layer = make(experts)
+        want.append(layer.forward(x))
+        layer.sync_status()
+        layer.terminate()
+    layer = make(sets[0])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    outs = [torch.empty_like(x) for _ in sets]
+    for i in range(len(sets)):
+        with torch.cuda.stream(side):
+            layer.forward(x, outs[i])
+        torch.cuda.current_stream().wait_stream(side)      # the replacement runs on the default stream
+        if i + 1 < len(sets):
+            for e in range(E):
+                layer.set_expert(e, *sets[i + 1][e])
+    torch.cuda.synchronize()
+    layer.sync_status()
+    layer.terminate()
+    for got, w in zip(outs, want):
+        assert torch.equal(got, w)
