@@ -30,6 +30,7 @@
 #include <cooperative_groups.h>
 #include <cuda.h>
 
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 
@@ -636,9 +637,9 @@ route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // One token, d_model 4096, 32 experts: 47 -> 9.6 us; 64 tokens 52 -> 12.5; d_model 1024, 8 experts: 13 -> 3.5.
 // Behind a pass that has streamed its weights through L2 the same call took 17 us: the rows (twice, for their statistics), the
 // LayerNorm weights and the centroids (eight loads at a time) were one trip to HBM after the other.  While the blocks all
-// fit on the chip (AHEAD) everything is requested on entry, by cp.async into shared memory: 10 us.  (The centroid in 32 registers
+// run at once (AHEAD; rs_ahead_blocks) everything is requested on entry, by cp.async into shared memory: 10 us.  (The centroid in 32 registers
 // per lane, fetched by unrolled loads, took 22: the code has to come from HBM too.)  Rows longer than 4224 floats do not fit
-// beside eight centroids, and with more blocks than SMs two of them share one: these read as they go.
+// beside eight centroids; these, and calls of more blocks than run at once, read as they go.
 constexpr int RS_TOKENS = 4;
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
@@ -1087,6 +1088,40 @@ bool use_small_route(long long T, int D, int E, bool rows, bool vec, bool ln) {
     if (E <= 8) return !(vec && !ln && (E > 6 || one_block) && whole_wave);
     return T * e < 24576;
 }
+// Blocks of AHEAD that run at once.  Where its shared memory leaves one block per SM, a cluster has to fit into a GPC with all its
+// blocks, and 148 SMs hold 148 blocks alone or in pairs, but 132 in clusters of four and 120 in clusters of eight (asked of the
+// device, once each: it depends on the chip).  One block more, and a second wave costs more than reading as they go.  Routing stage
+// behind a pass, us, ahead | as they go: 32 experts, 4096 floats, 132 tokens (132 blocks) 14.8 | 16.6, 136 tokens 22.9 | 18.0;
+// 64 experts, 56 tokens (112 blocks) 14.7 | 16.7, 64 tokens 22.9 | 18.2; 64 experts, 2304 floats, 56 tokens 12.7 | 13.7, 64 tokens
+// 18.7 | 14.5.  Passes behind another kernel, d_ff 64: 32 x 4096, 136 tokens 61.0 | 55.0, 64 x 3072, 64 tokens 56.6 | 50.6, 200 x 4096, 64
+// tokens 116 | 93; only passes one right behind the other, where the second wave's constants arrive before the wait, would rather
+// have two waves: 57.7 | 57.3, 53.5 | 56.1, 112.6 | 103.4.
+int rs_ahead_blocks(size_t smem, int cluster, int* blocks) {
+    constexpr int DEVICES = 64;
+    static std::atomic<int> known[DEVICES][4];      // of clusters of 1, 2, 4, 8 blocks; 0: not asked yet
+    if (smem <= 112 * 1024) cluster = 1;            // two blocks to an SM: all clusters fit
+    int dev = 0;
+    INFMOE_CUDA_TRY(cudaGetDevice(&dev));
+    std::atomic<int>& entry = known[dev % DEVICES][cluster == 1 ? 0 : cluster == 2 ? 1 : cluster == 4 ? 2 : 3];
+    if (!(*blocks = entry.load(std::memory_order_relaxed))) {
+        auto kern = route_small_kernel<true, true>;
+        INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_AHEAD_SMEM));
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cluster);
+        cfg.blockDim = dim3(RS_THREADS);
+        cfg.dynamicSmemBytes = RS_AHEAD_SMEM;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        INFMOE_CUDA_TRY(cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg));
+        entry.store(*blocks = clusters * cluster, std::memory_order_relaxed);
+    }
+    return INFMOE_OK;
+}
 template <bool VEC>
 int launch_route_small(const float* X, const float* C, const float* gamma, long long T, int D, int E, int* gate,
                        float* score, int* status, bool constant, cudaStream_t stream) {
@@ -1094,7 +1129,9 @@ int launch_route_small(const float* X, const float* C, const float* gamma, long 
     size_t smem = rs_smem(D);
     const long long blocks = (T + RS_TOKENS - 1) / RS_TOKENS * cluster;
     const size_t all = smem / RS_TOKENS * (RS_TOKENS + 1 + RS_WARPS);     // rows, LayerNorm weights, a centroid per warp
-    const bool ahead = VEC && blocks <= 148 && all <= RS_AHEAD_SMEM;
+    int at_once = 0;
+    if (VEC && all <= RS_AHEAD_SMEM) INFMOE_TRY(rs_ahead_blocks(all, cluster, &at_once));
+    const bool ahead = blocks <= at_once;
     auto kern = ahead ? route_small_kernel<VEC, VEC> : route_small_kernel<VEC, false>;
     if (ahead) smem = all;
     if (smem > 40 * 1024)

@@ -80,11 +80,18 @@ def test_route_lines_between_the_kernels(g, oracle, T, D, E, ln):
 
 
 # The few-token kernel requests its rows, LayerNorm weights and first centroids together while these fit into shared memory
-# (rows of up to 4224 floats) and its blocks onto the chip at once (148): both sides of either line.
+# (rows of up to 4224 floats) and its blocks run at once (148, fewer in larger clusters): both sides of either line.
 @pytest.mark.parametrize("T,D,E,ln", [(1, 4224, 9, True), (3, 4228, 9, True), (72, 4096, 32, True), (73, 4096, 32, True),
                                       (72, 2052, 70, False), (296, 2052, 16, True), (297, 2052, 16, True), (592, 64, 4, True),
                                       (593, 64, 4, False), (4, 4221, 5, True)])
 def test_route_few_tokens_requested_at_once(g, oracle, T, D, E, ln):
+    test_route_bit_exact(g, oracle, T, D, E, ln)
+
+
+# One block per SM: 132 blocks run at once in clusters of four (17 to 32 experts), 120 in clusters of eight, on the chips seen so far.
+@pytest.mark.parametrize("T,D,E,ln", [(t, 4096, 32, True) for t in (128, 132, 133, 136, 148)] +
+                         [(t, 3072, 64, False) for t in (56, 60, 61, 64, 74)] + [(t, 2304, 17, True) for t in (129, 137)])
+def test_route_few_tokens_in_large_clusters(g, oracle, T, D, E, ln):
     test_route_bit_exact(g, oracle, T, D, E, ln)
 
 
