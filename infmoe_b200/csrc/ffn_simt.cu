@@ -11,9 +11,10 @@
 // 32 values (launch_retile), wi_0 and wi_1 sharing one matrix with interleaved rows (row 2f = wi_0[f], row
 // 2f+1 = wi_1[f]).  So whatever the widths are, every row of a k block is 128 aligned bytes.
 //
-// Bound by FP32 FMA issue for many rows per expert, by the number of CTAs for few.  A cluster of up to four CTAs computes 16
-// RI token rows x 32 outputs, each CTA a part of the k blocks, and adds the parts up through distributed shared memory; a
-// thread has RI x 4 (x 2 when both matrices are multiplied) outputs.  K blocks of 32 are fetched by 16-byte cp.async into two
+// Bound by shared-memory reads for many rows per expert, by the number of CTAs for few.  With few, a cluster of up to four CTAs
+// computes 16 RI token rows x 32 outputs, each CTA a part of the k blocks, and adds the parts up through distributed shared
+// memory; with many, one CTA takes the parts one after the other, with the same additions (launch_ffn_simt).  A thread has RI x 4
+// (x 2 when both matrices are multiplied) outputs.  K blocks of 32 are fetched by 16-byte cp.async into two
 // buffers.  Both operands stay row-major in shared memory at a pitch of 36 floats, and a thread reads
 // four k of a row at a time: 4 + 8 128-bit loads for 128 multiply-adds, without bank conflicts (the eight weight rows a
 // warp reads at once start 4 banks apart; token rows are broadcasts).  Every output is up to four chains of FMAs in
@@ -24,6 +25,8 @@
 // SM (at 80 registers; five, at 96, left 28 of 768 CTAs for a second wave: 66.8 -> 65.6).  Half the threads with twice the
 // rows each, 16 loads for 256 multiply-adds, took 2.6 us longer.  The shorter chains also halve the error against 64 bits, 4.6e-7 -> 2.4e-7.
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -38,6 +41,7 @@ constexpr int SIMT_THREADS = 128;
 constexpr int TN = 32;       // outputs per CTA
 constexpr int TK = 32;       // one k block of the weight tiles
 constexpr int PITCH = TK + 4;
+constexpr int SIMT_SMS = 148;
 
 // Finds the (expert, first row, valid rows) of row tile `tile` when every expert's rows are tiled separately by `tm`: one
 // warp, 32 experts at a time.  Returns false when `tile` is past the end.
@@ -90,18 +94,21 @@ struct SimtOutput {
 
 // DUAL = true : out[j][n] = gelu(A W0^T) * (A W1^T), padded rows of N outputs   (N = d_ff, K = d_model)
 // DUAL = false: out[.][n] = resid[.][n] + A W0^T, dense rows                    (N = d_model, K = d_ff)
-// Grid: clusters of S CTAs, one per (row tile, output tile), row tile major; CTA r of a cluster takes the r-th S-th of the
-// k blocks.
-template <bool DUAL, int RI>
-__global__ void __launch_bounds__(SIMT_THREADS, 6)
-ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, int K, const float* __restrict__ act,
+// The k blocks are cut into `parts` shares whose sums are added in ascending k.  A tile (row tile, output tile; row tile major)
+// belongs to a cluster of `parts` CTAs with a share each, or (WHOLE) to one CTA that takes the shares one after the other.
+template <bool DUAL, int RI, bool WHOLE>
+__global__ void __launch_bounds__(SIMT_THREADS, WHOLE && RI > 1 ? (DUAL ? 5 : 7) : 6)
+ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, int K, int parts, const float* __restrict__ act,
                 const float* __restrict__ w, const int* __restrict__ slot_of_expert, const SimtOutput o) {
     cg::cluster_group cluster = cg::this_cluster();
-    const int S = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
+    const int S = WHOLE ? 1 : (int)cluster.num_blocks(), part = WHOLE ? 0 : (int)cluster.block_rank();
     const unsigned n_tiles = (unsigned)(N + TN - 1) / TN, tile = blockIdx.x / (unsigned)S;
     constexpr int TM = 16 * RI, WROWS = DUAL ? 2 * TN : TN, NB = DUAL ? 2 : 1;
     constexpr int BUF = (TM + WROWS) * PITCH;                 // floats of one buffer: token rows, then weight rows
     __shared__ __align__(16) float smem[2 * BUF];
+    __shared__ int s_row[DUAL ? 1 : TM];                      // output rows of the tile, their addresses and mix coefficients
+    __shared__ float* s_dst[DUAL ? 1 : TM];
+    __shared__ float s_alpha[DUAL ? 1 : TM];
     __shared__ int s_info[4];
     if (threadIdx.x < 32) {
         int e = 0, r0 = 0, rows = 0;
@@ -143,7 +150,17 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
     float acc[NB][RI][4] = {};
     const int kb0 = KB * part / S, kb_end = KB * (part + 1) / S;
     fetch(kb0, kb0 & 1);
-    for (int kb = kb0; kb < kb_end; ++kb) {
+    // Where the outputs go; with four rows and more per warp while the first blocks are on their way: done row by row at the end, it
+    // was a chain of trips to memory.
+    const auto look_up_rows = [&]() {
+        if (DUAL || (int)threadIdx.x >= rows) return;
+        const int j = row0 + (int)threadIdx.x, row = o.out_pos ? o.out_pos[j] : j;
+        s_row[threadIdx.x] = row;
+        s_dst[threadIdx.x] = o.out_row_ptr ? reinterpret_cast<float*>(o.out_row_ptr[row]) : o.out + (size_t)row * N;
+        if (o.mix_score) s_alpha[threadIdx.x] = mix_alpha(o.mix_score[j]);
+    };
+    if (RI > 1) look_up_rows();
+    const auto multiply_block = [&](int kb) {
         const int buf = kb & 1;
         if (kb + 1 < kb_end) {
             fetch(kb + 1, buf ^ 1);
@@ -173,10 +190,38 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
                 }
         }
         __syncthreads();    // the next round's fetch refills this buffer
+    };
+    if constexpr (!WHOLE) {
+        for (int kb = kb0; kb < kb_end; ++kb) multiply_block(kb);
+    } else {
+        float total[NB][RI][4] = {};
+        for (int kb = 0, share = 0; share < parts; ++share) {
+            for (const int share_end = KB * (share + 1) / parts; kb < share_end; ++kb) multiply_block(kb);
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int i = 0; i < RI; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        total[b][i][j] += acc[b][i][j];
+                        acc[b][i][j] = share + 1 < parts ? 0.f : total[b][i][j];
+                    }
+        }
+    }
+    if constexpr (WHOLE && DUAL) {
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+            if (ty + 16 * i < rows)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)     // outputs past N are products of zero weights: the zeros the next GEMM's padding needs
+                    o.out[(size_t)(row0 + ty + 16 * i) * padded_row(N) + n0 + tx + 8 * j] = gelu_dot(acc[0][i][j], acc[NB - 1][i][j]);
+        return;
     }
     // Sums of the cluster's CTAs, added in ascending k; the CTAs share the outputs out.  A warp takes 32 consecutive outputs of a
-    // row, so that what it stores is one run (the rows may lie in host memory).
+    // row, so that what it stores is one run (the rows may lie in host memory), and several rows at a time: the stores may alias
+    // the loads as far as the compiler knows, and one row after the other each would cost a trip to memory.
     constexpr int RED = TN + 8;                 // floats per row: the four rows a warp stores to end in different banks
+    constexpr int AHEAD = WHOLE ? 4 : RI;
     static_assert(NB * TM * RED <= 2 * BUF, "the partial sums reuse the buffers");
     float* const red = smem;                    // [NB][TM][RED]
 #pragma unroll
@@ -185,31 +230,41 @@ ffn_simt_kernel(const int* __restrict__ offset, int e_begin, int e_end, int N, i
         for (int i = 0; i < RI; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) red[(b * TM + ty + 16 * i) * RED + tx + 8 * j] = acc[b][i][j];
-    cluster.sync();
-    const int lane = threadIdx.x & 31, n = n0 + lane;
-    for (int r = TM * part / S + (int)(threadIdx.x >> 5); r < min(rows, TM * (part + 1) / S); r += SIMT_THREADS / 32) {
-        float sum[NB] = {};
-        for (int q = 0; q < S; ++q) {
-            const float* from = cluster.map_shared_rank(red, q);
+    if (RI == 1) look_up_rows();
+    if (WHOLE) __syncthreads();
+    else cluster.sync();
+    constexpr int WARPS = SIMT_THREADS / 32;
+    const int lane = threadIdx.x & 31, n = n0 + lane, r_end = min(rows, TM * (part + 1) / S);
+    for (int r0 = TM * part / S + (int)(threadIdx.x >> 5); r0 < r_end; r0 += WARPS * AHEAD) {
+        float sum[AHEAD][NB] = {}, x[AHEAD];
+        if (!DUAL)
 #pragma unroll
-            for (int b = 0; b < NB; ++b) sum[b] += from[(b * TM + r) * RED + lane];
-        }
-        const int j = row0 + r;
-        if (DUAL) {     // outputs past N are products of zero weights: the zeros the next GEMM's padding needs
-            o.out[(size_t)j * padded_row(N) + n] = gelu_dot(sum[0], sum[NB - 1]);
-        } else if (n < N) {
-            const int row = o.out_pos ? o.out_pos[j] : j;
-            float* const dst = o.out_row_ptr ? reinterpret_cast<float*>(o.out_row_ptr[row]) : o.out + (size_t)row * N;
-            const float x = o.resid[(size_t)row * N + n];
-            float y = x + sum[0];
-            if (o.mix_score) {
-                const float alpha = mix_alpha(o.mix_score[j]);
-                y = mix_value(alpha, 1.0f - alpha, y, x);
+            for (int i = 0; i < AHEAD; ++i) {
+                const int r = r0 + WARPS * i;
+                x[i] = r < r_end && n < N ? o.resid[(size_t)s_row[r] * N + n] : 0.f;
             }
-            dst[n] = y;
+        for (int q = 0; q < S; ++q) {
+            const float* from = WHOLE ? red : cluster.map_shared_rank(red, q);
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i)
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+                    sum[i][b] += from[(b * TM + r0 + WARPS * i) * RED + lane];      // past `rows` too: never stored
+        }
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const int r = r0 + WARPS * i;
+            if (r >= r_end) continue;
+            if (DUAL) {     // outputs past N are products of zero weights: the zeros the next GEMM's padding needs
+                o.out[(size_t)(row0 + r) * padded_row(N) + n] = gelu_dot(sum[i][0], sum[i][NB - 1]);
+            } else if (n < N) {
+                float y = x[i] + sum[i][0];
+                if (o.mix_score) y = mix_value(s_alpha[r], 1.0f - s_alpha[r], y, x[i]);
+                s_dst[r][n] = y;
+            }
         }
     }
-    cluster.sync();      // nobody leaves while its sums are being read
+    if (!WHOLE) cluster.sync();      // nobody leaves while its sums are being read
 }
 
 }  // namespace
@@ -228,24 +283,38 @@ int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int
     const unsigned row_tiles = (unsigned)((T + tm - 1) / tm + experts);
     // Not chained (launch_chained): blocks put on the SMs while those of the kernel before are still there crowd on the
     // idle ones, and there are only a few per SM.  The pass of 300 tokens took 195 us so, 126 with a late trigger.
-    const auto launch = [&](auto kern, int N, int K, const float* act, const float* w, const SimtOutput& o) {
-        // CTAs per tile: by K alone, so that a row's additions do not depend on the other rows of the call
-        const unsigned S = K > 7 * TK ? 4 : K > 3 * TK ? 2 : 1;
+    const auto launch = [&](auto dual, int N, int K, const float* act, const float* w, const SimtOutput& o) {
+        constexpr bool DUAL = decltype(dual)::value;
+        // shares of K: by K alone, so that a row's additions do not depend on the other rows of the call
+        const unsigned parts = K > 7 * TK ? 4 : K > 3 * TK ? 2 : 1, tiles = (unsigned)((N + TN - 1) / TN) * row_tiles;
+        // One CTA per tile where there is nothing to share, and where the tiles alone keep the SMs busy: a cluster pays for its start,
+        // its sums and barriers with every share.  Tiles: half of one per expert may be missing from its last.  The line in tiles per
+        // SM; us of the kernel, cluster | one CTA per tile, tiles (experts x d_model x d_ff, tokens):
+        //   first GEMM      6 x 510 x 1022: 576: 77 | 80, 832: 110 | 104, 2240: 267 | 233, 8288: 994 | 846; 4 x 2050 x 4098: 645: 251 | 313
+        //   second GEMM     half the work per tile: 1072 (4096 tokens) 144 | 159, 64 x 510 x 1022 1504: 189 | 179, 6 x 510 x 1022 4144: 529 | 494
+        //   16-row tiles    either GEMM: 4 x 2050 x 4098 774: 243 | 254, 64 x 510 x 1022 1152: 104 | 97, 1536: 121 | 115
+        //   64-row tiles, shares of three k blocks and less    4 x 130 x 258: 117: 11.8 | 12.4, 234: 18.1 | 14.7, 594: 35 | 30
+        // Passes, before the clusters, with clusters always, now: 6 x 510 x 1022, 4096 tokens 403, 446, 401, 16384 1379, 1631, 1408;
+        // 4 x 130 x 258, 4096 69.5, 80.4, 69.2; 4 x 66 x 130, 300 23.8, 28.0, 22.4; 4 x 2050 x 4098, 1000 1414, 1493, 1376.
+        const long long busy = (long long)((N + TN - 1) / TN) * (T / tm + (experts < T ? experts : T) / 2);
+        const bool short_shares = !few && (K + TK - 1) / TK <= 3 * (int)parts;
+        const bool whole = parts == 1 || busy >= SIMT_SMS * (short_shares ? 1 : few ? 6 : DUAL ? 5 : 10);
+        const auto kern = few ? (whole ? ffn_simt_kernel<DUAL, 1, true> : ffn_simt_kernel<DUAL, 1, false>)
+                              : (whole ? ffn_simt_kernel<DUAL, 4, true> : ffn_simt_kernel<DUAL, 4, false>);
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)((N + TN - 1) / TN) * row_tiles * S);
+        cfg.gridDim = dim3(whole ? tiles : tiles * parts);
         cfg.blockDim = dim3(SIMT_THREADS);
         cfg.stream = stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = S;
+        attr[0].val.clusterDim.x = parts;
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kern, offset, e_begin, e_end, N, K, act, w, slot_of_expert, o);
+        cfg.numAttrs = whole ? 0 : 1;
+        return cudaLaunchKernelEx(&cfg, kern, offset, e_begin, e_end, N, K, (int)parts, act, w, slot_of_expert, o);
     };
-    INFMOE_CUDA_TRY(launch(few ? ffn_simt_kernel<true, 1> : ffn_simt_kernel<true, 4>, F, D, h, w01, SimtOutput{g, nullptr, nullptr, nullptr, nullptr}));
-    INFMOE_CUDA_TRY(launch(few ? ffn_simt_kernel<false, 1> : ffn_simt_kernel<false, 4>, D, F, (const float*)g, wo,
-                           SimtOutput{out, resid, out_pos, mix_score, out_row_ptr}));
+    INFMOE_CUDA_TRY(launch(std::true_type(), F, D, h, w01, SimtOutput{g, nullptr, nullptr, nullptr, nullptr}));
+    INFMOE_CUDA_TRY(launch(std::false_type(), D, F, (const float*)g, wo, SimtOutput{out, resid, out_pos, mix_score, out_row_ptr}));
     note_launch(2);
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

@@ -849,3 +849,40 @@ def test_experts_replaced_between_passes_of_another_stream(T):
     layer.terminate()
     for got, w in zip(outs, want):
         assert torch.equal(got, w)
+
+
+# Many rows: one CTA per tile, which takes the parts of the k blocks one after the other, instead of a cluster that shares them out.
+# Row counts on both sides of the lines (parts of up to three k blocks, longer ones, a single one; either GEMM), the last ones with
+# 16-row tiles; the bits are those of the same rows in a call of 16.
+@pytest.mark.parametrize("D,F,E,T", [(66, 34, 1, 700), (130, 258, 1, 1087), (130, 258, 1, 1088), (161, 450, 1, 15807), (161, 450, 1, 15808),
+                                     (450, 161, 1, 7935), (450, 161, 1, 7936), (1030, 33, 1, 3200), (510, 1022, 6, 2500),
+                                     (130, 320, 64, 1024), (322, 130, 64, 1024), (510, 70, 64, 1000)])
+def test_cuda_core_experts_of_one_cta_per_tile(oracle, D, F, E, T):
+    import torch
+    from infmoe_b200 import MoELayer
+    rng = np.random.default_rng(D * F + T)
+    layer = MoELayer.create(E, D, F, 2, np.ones((E, D), np.float32), None, "T5_FF", "default", None)
+    expert = [(1 + 0.01 * rng.standard_normal(D)).astype(np.float32)] + \
+             [(rng.standard_normal((F, D)) / np.sqrt(D)).astype(np.float32) for _ in range(2)] + \
+             [(rng.standard_normal((D, F)) / np.sqrt(F)).astype(np.float32)]
+    for e in range(E):
+        layer.set_expert(e, *(torch.from_numpy(a).cuda() for a in expert))
+    x = torch.from_numpy(rng.standard_normal((T, D)).astype(np.float32)).cuda()
+    gate = torch.from_numpy(rng.integers(0, E, T).astype(np.int32)).cuda()
+    score = torch.from_numpy(rng.standard_normal(T).astype(np.float32)).cuda()
+    out = layer.expert_forward(x, gate)
+    # rows to addresses, in another order and mixed with their scores
+    mixed, perm = torch.empty_like(x), torch.from_numpy(rng.permutation(T)).cuda()
+    if F >= D:       # what the call asks for
+        layer.expert_forward_scatter(x, gate, mixed.data_ptr() + 4 * D * perm, score)
+    few = [layer.expert_forward(x[i:i + 16].contiguous(), gate[i:i + 16].contiguous()) for i in (0, (T - 16) // 2, T - 16)]
+    layer.sync_status()
+    layer.terminate()
+    for i, rows in zip((0, (T - 16) // 2, T - 16), few):
+        assert torch.equal(rows, out[i:i + 16])
+    alpha = torch.sigmoid(score.double())[:, None]
+    want = alpha * out.double() + (1 - alpha) * x.double()
+    assert F < D or float((mixed[perm] - want).norm() / want.norm()) <= 5e-7     # eight roundings at most, the sigmoid included
+    head = x[:64].cpu().numpy()
+    want = oracle.expert_ffn_f64(head, *expert)
+    assert oracle.rel_l2(out[:64].cpu().numpy() - head, want - head) <= 2e-6     # FP32 chains of up to 1030 adds
