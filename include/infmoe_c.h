@@ -176,9 +176,10 @@ INFMOE_API int infmoe_layer_last_routing(const infmoe_layer* layer, const int32_
  * infmoe_layer_stage_ms waits for those calls and returns the average
  * milliseconds of: routing, dispatch, scatter, expert GEMM 1 (wi_0/wi_1 + gelu),
  * expert GEMM 2 (wo + residual), combine -- ms[6] -- then restarts the ring.
- * With streamed experts the two GEMM entries are reported together in ms[3].  With up to 1024 tokens the scatter
- * kernel computes the dispatch metadata on the way: the time of both is then in the scatter entry, and the dispatch
- * entry holds no kernel. */
+ * With streamed experts the two GEMM entries are reported together in ms[3].  With up to 1024 tokens (up to
+ * 4096 in 16-byte aligned rows of up to 2048 floats on the tensor-core path) the scatter kernel computes the dispatch
+ * metadata on the way: the time of both is then in the scatter entry, and the dispatch entry holds no kernel.  On the
+ * CUDA-core path (widths that are no multiple of four) the two GEMM entries are 0. */
 INFMOE_API int infmoe_layer_set_profiling(infmoe_layer* layer, int enable);
 INFMOE_API int infmoe_layer_stage_ms(infmoe_layer* layer, float* ms, int32_t* calls);
 

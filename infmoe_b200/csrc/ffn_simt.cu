@@ -23,7 +23,8 @@
 // and tail planes added on the fly), 88 with the dispatch and scatter in one kernel, 67 with the clusters: 96 to 192 CTAs of
 // one chain each had left two or three of four schedulers of an SM without a warp, now 384 to 768 are in flight, six to an
 // SM (at 80 registers; five, at 96, left 28 of 768 CTAs for a second wave: 66.8 -> 65.6).  Half the threads with twice the
-// rows each, 16 loads for 256 multiply-adds, took 2.6 us longer.  The shorter chains also halve the error against 64 bits, 4.6e-7 -> 2.4e-7.
+// rows each, 16 loads for 256 multiply-adds, took 2.6 us longer.  The shorter chains also halve the error against 64 bits,
+// 4.6e-7 -> 2.4e-7.
 #include <cooperative_groups.h>
 
 #include <type_traits>
@@ -83,7 +84,8 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid)
 
 // Where the outputs go: g (DUAL), or row j to row out_pos[j] (or j) of `out`, or to the address out_row_ptr[out_pos[j]]; the
 // residual is the same row of `resid`; mix_score != NULL applies the base_layer output mix.  With the combine step in here no
-// routed copy of x and no result in expert order are written and read back: 300 tokens, 6 experts, 510 x 1022 one kernel of 3.6 us less.
+// routed copy of x and no result in expert order are written and read back: 300 tokens, 6 experts, 510 x 1022 one kernel of
+// 3.6 us less.
 struct SimtOutput {
     float* out;
     const float* resid;
@@ -314,7 +316,8 @@ int launch_ffn_simt(long long T, int D, int F, int e_begin, int e_end, const int
         return cudaLaunchKernelEx(&cfg, kern, offset, e_begin, e_end, N, K, (int)parts, act, w, slot_of_expert, o);
     };
     INFMOE_CUDA_TRY(launch(std::true_type(), F, D, h, w01, SimtOutput{g, nullptr, nullptr, nullptr, nullptr}));
-    INFMOE_CUDA_TRY(launch(std::false_type(), D, F, (const float*)g, wo, SimtOutput{out, resid, out_pos, mix_score, out_row_ptr}));
+    INFMOE_CUDA_TRY(launch(std::false_type(), D, F, (const float*)g, wo,
+                           SimtOutput{out, resid, out_pos, mix_score, out_row_ptr}));
     note_launch(2);
     INFMOE_CUDA_TRY(cudaGetLastError());
     return INFMOE_OK;

@@ -69,6 +69,8 @@
 // ascending k and runs the epilogue.  Nobody waits, and the additions are those of an uncut tile, so the bits are too.
 // One token through one expert of 4096 x 10240 (32 tiles of 320 k blocks on 148 SMs): second GEMM 158 -> 58 us.
 //
+// Layer times beside a step are those before and after that step, in the code of its time: they do not add up to today's.
+//
 // Every mbarrier wait is bounded: on expiry the CTA raises STATUS_WAIT_TIMEOUT, lets
 // copies in flight land, frees its TMEM and returns.
 #include <cuda.h>
@@ -243,8 +245,8 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
 __device__ __forceinline__ void tma_load_2d_pair_hint(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
                                                       uint64_t policy) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], "
-        "[%2], %5;"
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], "
+        "[%1, {%3, %4}], [%2], %5;"
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
         : "memory");
 }
@@ -402,7 +404,8 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, const int* s_prefix, c
 // walk the (sorted) list forwards in even rounds and backwards in odd ones, so that over two rounds every CTA gets
 // one tile from each end of a stretch.  The R tiles left after the last whole round are cut into chunk units and dealt
 // out evenly when that pays: an uncut tail lasts one tile (m chunks), a cut one R m / G chunks plus storing and
-// re-reading the chunk sums, which is worth about two chunks.  A CTA whose share spans two tiles stores, fences and counts
+// re-reading the chunk sums, which is worth about two chunks (measured on narrow tiles, the same for wide ones by assumption), and
+// where the chunk sums fit into the scratch (ffn_umma_part_bytes).  A CTA whose share spans two tiles stores, fences and counts
 // twice, about as long as a chunk and a half; where shares that end with their tile are at most that much longer, they are
 // taken.  Layer, us: 2500 tokens 16 x 512 x 2048 104 -> 90, one token 32 x 4096 x 10240 109 -> 105.
 struct Item {
@@ -1013,7 +1016,7 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // The schedule and the place of a tile (searches, divisions) take one to two thousand cycles, and every role took them
         // at each tile, the issuer and the accumulate warps while nothing else went on in their part.  Layer, us, with the
         // column warp: 4096 tokens 8 x 1024 x 4096 331 -> 321, 16384 tokens 64 x 1024 x 4096 1481 -> 1432, 32 tokens 4 x 64 x 256,
-        // where the list is only a detour, 18.1 -> 18.5.
+        // where the list is only a detour, 18.1 -> 18.8.
         Schedule<CTAS> sched(s_prefix[args.E], KB, args);
         Place at;
         bool more = true, first = true;
@@ -1069,7 +1072,8 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     } else {
                         const int r = ok && args.out_pos ? __ldcg(args.out_pos + t.row0 + c) : t.row0 + c;
                         s_col[at.slot][c] = make_float2(exp2_int(-g_exp), __int_as_float(r));
-                        if (args.mix_score && ok) s_mix[EPI == EPI_RESIDUAL ? at.slot : 0][c] = mix_alpha(__ldcg(args.mix_score + t.row0 + c));
+                        if (args.mix_score && ok)
+                            s_mix[EPI == EPI_RESIDUAL ? at.slot : 0][c] = mix_alpha(__ldcg(args.mix_score + t.row0 + c));
                     }
                 }
                 reinterpret_cast<float4*>(s_winv[at.slot])[lane] = inv;
@@ -1288,8 +1292,9 @@ int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_be
     //                           579 / 585, 583 / 591, 32 x 4096 x 10240 20 and 36: 2389 / 2366, 2440 / 2466; the most it costs is
     //                           what 20 tokens cost at 64 x 2048 x 2048, 600 / 632.  With one 128-row weight block, of which
     //                           the second CTA has none: 4 x 128 x 4096, 1024 tokens 86 / 83, 8 x 128 x 2048, 4096 108 / 113
-    //   shorter K               one CTA: the epilogue, not the MMAs, is in front; first GEMM, us: K = 1024, 16 experts x 4096, 1000 tokens 104 / 112, K = 680, 6
-    //                           experts, 4640 tokens 65 / 80
+    //   shorter K               one CTA: the epilogue, not the MMAs, is in front, and from 144 columns on there are only two
+    //                           accumulators to compute the next tile's chunks into meanwhile; first GEMM, us: K = 1024, 16
+    //                           experts x 4096, 1000 tokens 104 / 112, K = 680, 6 experts, 4640 tokens 65 / 80
     const bool small = T <= 64 || T <= 16ll * (e_end - e_begin);
     const auto pick = [&](auto epi, const GemmArgs& a, const void* tokens) -> int {
         constexpr int EPI = decltype(epi)::value;
@@ -1304,7 +1309,10 @@ int launch_ffn_umma(const FfnUmma& f, long long T, int D, int F, int E, int e_be
 }
 
 // Room for the chunk sums of cut tiles: what the cut tail of either GEMM can need (fewer than FFN_CTAS tiles of up to
-// max(D, F) / 256 chunks), up to 64 MB; beyond that the tail stays uncut.
+// max(D, F) / 256 chunks), up to 64 MB; beyond that the tail stays uncut.  That is no rare case: from 192 tokens on a block
+// is 192 columns wide whatever the tiles are, 682 of them fit, one for each chunk, cut tile and CTA of a pair, and the second GEMM
+// of most batches wants more: 4096 tokens, 8 x 1024 x 4096, 704 (its second round of tiles has 22 of 74 pairs at work),
+// 777 tokens, 12 x 1000 x 2724, 1056.
 size_t ffn_umma_part_bytes(long long T, int D, int F) {
     const int K = D > F ? D : F;
     const size_t chunks = (size_t)((K + BK - 1) / BK + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;

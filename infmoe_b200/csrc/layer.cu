@@ -250,12 +250,13 @@ WsLayout ws_layout(const infmoe_layer* L, long long T, bool streamed) {
     w.score = take(4 * t);
     w.rscore = take(4 * t);
     // The GEMMs read their residual from the input through pos[] and write the layer output from their epilogue; routed rows
-    // and expert-ordered results are kept by the Identity and registered sublayers (and have room on the CUDA-core path).
+    // and expert-ordered results are kept by the Identity and registered sublayers.  The CUDA-core path has room for them, and
+    // in `g` for rows of d_model, that it does not use: its workspace keeps the size it always had.
     const bool row_planes = L->identity || L->custom || !uses_umma(L);
     w.routed = take(row_planes ? 4 * t * D : 0);
     w.post = take(row_planes ? 4 * t * D : 0);
-    // activations: FP16 pairs on the tensor-core path, FP32 on the CUDA-core path (where `g` also serves as a [T][D]
-    // buffer when the result goes to per-row addresses)
+    // activations: FP16 pairs on the tensor-core path, FP32 on the CUDA-core path; with the sublayers above `g` serves as a
+    // [T][D] buffer when the result goes to per-row addresses
     w.h = take(pack_bytes((long long)t, L->D));
     w.g = take(row_planes && D > F ? pack_bytes((long long)t, L->D) : pack_bytes((long long)t, L->F));
     w.row_info = take(row_planes ? 0 : 8 * t);

@@ -637,8 +637,8 @@ route_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // One token, d_model 4096, 32 experts: 47 -> 9.6 us; 64 tokens 52 -> 12.5; d_model 1024, 8 experts: 13 -> 3.5.
 // Behind a pass that has streamed its weights through L2 the same call took 17 us: the rows (twice, for their statistics), the
 // LayerNorm weights and the centroids (eight loads at a time) were one trip to HBM after the other.  While the blocks all
-// run at once (AHEAD; rs_ahead_blocks) everything is requested on entry, by cp.async into shared memory: 10 us.  (The centroid in 32 registers
-// per lane, fetched by unrolled loads, took 22: the code has to come from HBM too.)  Rows longer than 4224 floats do not fit
+// run at once (AHEAD; rs_ahead_blocks) everything is requested on entry, by cp.async into shared memory: 10 us.  (The centroid
+// in 32 registers per lane, fetched by unrolled loads, took 22: the code has to come from HBM too.)  Rows longer than 4224 floats do not fit
 // beside eight centroids; these, and calls of more blocks than run at once, read as they go.
 constexpr int RS_TOKENS = 4;
 constexpr int RS_THREADS = 256;

@@ -122,7 +122,8 @@ __device__ __forceinline__ void warp_ln_pack(const float* __restrict__ src, cons
     if (lane == 0) *info = token_row_info(s, squares);
 }
 
-// The scatter for the tensor-core GEMM, of rows j0 .. j0 + T - 1.  The LayerNorm weights are gamma' (see SplitExpert), which lies with the experts' planes.
+// The scatter for the tensor-core GEMM, of rows j0 .. j0 + T - 1.  The LayerNorm weights are gamma' (see SplitExpert), which
+// lies with the experts' planes.
 struct ExpertGamma {
     const float* base;              // first expert
     size_t stride;                  // floats from one expert to the next
@@ -434,7 +435,10 @@ dispatch_scatter_kernel(int T, int D, int E, int vec, const float* X, const floa
 // tokens are the most it takes: 8 MB and about 1.5 us of comparisons, against a kernel of one cluster between routing and
 // scatter.  Bound by latency: the gates' trips to L2, then the LayerNorm weights', in one to two rounds of blocks (three or four
 // to an SM by registers).  Dispatch and scatter, us, each timed by itself: 4096 tokens of 512 floats 12 + 10 -> 14.7, 1024 floats 11
-// + 12 -> 16.8, 2500 tokens of 512 floats 11 + 10 -> 10.9.
+// + 12 -> 16.8, 2500 tokens of 512 floats 11 + 10 -> 10.9, 2048 tokens of 1028 floats 12.6 + 10.5 -> 12.3 (64 experts), 4096 of 2048
+// 11.1 + 20.4 -> 22.9.  The line at 4096 is where the measurements end, not where the two forms meet: the comparisons grow with
+// T squared, and at the line this one is still ahead.  Whole passes, 5 experts, d_ff 64, at 4096 | 4097 tokens: 256 floats 33.1 |
+// 36.5, 1024 57.2 | 58.2, 2048 98.6 | 101.8.
 constexpr int DM_THREADS = 256;
 constexpr int DM_TOKENS = DM_THREADS / 32;
 constexpr int DM_MAX_TOKENS = 4096;
@@ -933,7 +937,8 @@ int launch_dispatch_scatter(long long T, int D, int E, const float* X, const flo
         const int nv = D <= 512 ? 4 : D <= 1024 ? 8 : 16;
         size_t smem = (size_t)DM_TOKENS * nv * 512;
         if (smem < hist) smem = hist;
-        auto kern = nv == 4 ? dispatch_scatter_reg_kernel<4> : nv == 8 ? dispatch_scatter_reg_kernel<8> : dispatch_scatter_reg_kernel<16>;
+        auto kern = nv == 4 ? dispatch_scatter_reg_kernel<4>
+                            : nv == 8 ? dispatch_scatter_reg_kernel<8> : dispatch_scatter_reg_kernel<16>;
         if (smem > 48 * 1024)
             INFMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         INFMOE_CUDA_TRY(launch_chained(kern, (unsigned)((T + DM_TOKENS - 1) / DM_TOKENS + 1), DM_THREADS, smem, 1, stream,

@@ -342,7 +342,8 @@ class MoELayer:
     def stage_ms(self):
         """Average device milliseconds per stage over the calls since the last read -> (dict, calls).
 
-        Up to 1024 tokens "scatter" holds the dispatch too (one kernel does both)."""
+        Up to 1024 tokens (4096 in aligned rows of up to 2048 floats on the tensor-core path) "scatter" holds the dispatch
+        too (one kernel does both)."""
         ms = (ctypes.c_float * 6)()
         n = ctypes.c_int32()
         capi.check(capi.lib().infmoe_layer_stage_ms(self._h, ms, ctypes.byref(n)))
