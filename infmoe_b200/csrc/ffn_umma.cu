@@ -1065,15 +1065,15 @@ ffn_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const float bound = (float)__ldg(args.bound + (size_t)t.slot * args.bound_stride);
                 for (int c = lane; c < t.n_pad; c += 32) {
                     const bool ok = c < t.n_tok;
-                    const float2 info = ok ? __ldcg(args.row_info + t.row0 + c) : make_float2(1.f, 0.f);
+                    const float2 info = ok ? args.row_info[t.row0 + c] : make_float2(1.f, 0.f);
                     const int g_exp = g_exponent(info.y, bound);
                     if (EPI == EPI_GELU_PAIR) {
                         s_col[at.slot][c] = make_float2(info.x, exp2_int(g_exp));
                     } else {
-                        const int r = ok && args.out_pos ? __ldcg(args.out_pos + t.row0 + c) : t.row0 + c;
+                        const int r = ok && args.out_pos ? args.out_pos[t.row0 + c] : t.row0 + c;
                         s_col[at.slot][c] = make_float2(exp2_int(-g_exp), __int_as_float(r));
                         if (args.mix_score && ok)
-                            s_mix[EPI == EPI_RESIDUAL ? at.slot : 0][c] = mix_alpha(__ldcg(args.mix_score + t.row0 + c));
+                            s_mix[EPI == EPI_RESIDUAL ? at.slot : 0][c] = mix_alpha(args.mix_score[t.row0 + c]);
                     }
                 }
                 reinterpret_cast<float4*>(s_winv[at.slot])[lane] = inv;
